@@ -49,13 +49,13 @@ def listed():
         # a long prompt's portion of 512 tokens beside 32 decoding requests, at the 14B layer sizes
         _case("mixed 512+32", "mixed", "qwen3", 5120, 4, 32, context=4096, rows=512),
         # the 32-bit path, which checks the other one: a prompt, then tokens one by one
-        _case("prompt 300, 32 bits", "prompt", "qwen3", 4096, 2, 1, rows=300, tail=4, dtype="float32"),
+        _case("prompt 300 fp32", "prompt", "qwen3", 4096, 2, 1, rows=300, tail=4, dtype="float32"),
         # the other designs at the benchmark's first size: a whole prompt ...
         _case("movivik 2048", "prompt", "movivik", 2048, 8, 1, rows=2048),
         _case("guvolix 1536 of 2", "prompt", "guvolix", 2048, 8, 2, rows=1536),
         _case("bozevik 2048", "prompt", "bozevik", 2048, 8, 1, rows=2048),
         # ... and eight short requests answered with two dozen tokens each: mostly decode steps over states of fixed size
-        _case("fusazen 777 of 8, 24 on", "prompt", "fusazen", 2048, 8, 8, rows=777, tail=24),
+        _case("fusazen 777 of 8", "prompt", "fusazen", 2048, 8, 8, rows=777, tail=24),
     ]
 
 
