@@ -824,7 +824,7 @@ EPILOGUE_RELU2 = 2       # as a product's `accumulate`: neither stored as it is 
 
 
 def gemm_plain(a, w, out, bias=None, accumulate=False) -> None:
-    """out (+)= a @ w.T (+ bias) on the CUDA cores with float32 accumulation in ascending k."""
+    """out (+)= a @ w.T (+ bias) on the CUDA cores with float32 accumulation; the order of an element's sum is fixed by K alone."""
     assert a.dtype == w.dtype and a.stride(-1) == 1 and w.stride(-1) == 1 and out.stride(-1) == 1
     _call("jllm_gemm_plain", a.data_ptr(), _DT[a.dtype], a.stride(0), w.data_ptr(), w.stride(0), _p(bias),
           _DT[bias.dtype] if bias is not None else F32, out.data_ptr(), _DT[out.dtype], out.stride(0),

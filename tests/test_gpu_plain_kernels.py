@@ -1,0 +1,86 @@
+"""The kernels of the 32-bit path at the edges of their tiles, against float64, and bit for bit between their forms.
+
+A product's tile follows the number of rows (4, 16, 32, 64 rows), the way its operands are loaded their alignment; a row's
+attention may be shared by a cluster of blocks. None of that may move a bit of a row's result."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from jllm_serve_b200.csrc import ops as o
+    o.require_device()
+    return o
+
+
+def rnd(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+@pytest.mark.parametrize("N,K", [(1, 1), (63, 12), (65, 36), (127, 515), (129, 1028), (300, 4096), (72, 12292)])
+def test_product_of_every_tile_and_loader(ops, N, K):
+    """Rows 1 to 150 run through all four tiles; the same operands in rows of another stride through the other loader."""
+    a, w, bias = rnd(150, K), rnd(N, K, seed=1), rnd(N, seed=2)
+    want = a.double() @ w.double().T + bias.double()
+    # two chains of K / 8 rounded products and sums per group, five more sums: |error| <= (K / 8 + 7) 2^-24 sum |a| |w|
+    bound = (K / 8 + 7) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs().double())
+    full = torch.empty(150, N, device=DEV)
+    ops.gemm_plain(a, w, full, bias)
+    assert bool(((full.double() - want).abs() <= bound).all())
+    for M in (1, 3, 4, 5, 16, 17, 32, 33, 64, 65, 96, 97, 128, 129):
+        out = torch.full((M + 1, N + 3), 7.0, device=DEV)
+        ops.gemm_plain(a[150 - M:], w, out[:M, :N], bias)
+        assert torch.equal(out[:M, :N], full[150 - M:]), M
+        assert float((out[M] - 7).abs().max()) == 0 and float((out[:, N:] - 7).abs().max()) == 0
+    odd_a, odd_w = torch.zeros(150, K + 1, device=DEV), torch.zeros(N, K + 3, device=DEV)
+    odd_a[:, :K], odd_w[:, :K] = a, w
+    for M in (2, 16, 30, 150):
+        out = torch.empty(M, N, device=DEV)
+        ops.gemm_plain(odd_a[:M, :K], odd_w[:, :K], out, bias)
+        assert torch.equal(out, full[:M]), M
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,dk,dv,window,keep", [(4, 4, 16, 16, 0, 0), (8, 2, 128, 128, 0, 0), (6, 1, 50, 140, 0, 0), (5, 1, 260, 300, 0, 0),
+                                                   (6, 3, 72, 64, 70, 9), (4, 1, 64, 64, -96, 0)])
+def test_attention_of_shared_rows(ops, dtype, H, G, dk, dv, window, keep):
+    """Lengths around a chunk of 64 keys and around the eight that a cluster takes at a time; one row alone (a cluster to a
+    row) has the bits it has among many (a block to a row)."""
+    page, width, scale = 8, max(dk, dv), 1.0 / math.sqrt(dk)
+    lens = [1, 63, 64, 65, 511, 512, 513, 700]
+    blocks = -(-max(lens) // page)
+    pool = len(lens) * blocks
+    order = torch.randperm(pool, generator=torch.Generator().manual_seed(5)).int()
+    tables = order.view(len(lens), blocks).to(DEV)
+    k, v = rnd(pool, G, page, width, seed=1).to(dtype), rnd(pool, G, page, width, seed=2).to(dtype)
+    sink = rnd(H, seed=3) if keep else None
+    rows = [(s, p) for s, n in enumerate(lens) for p in sorted({n - 1, max(0, n - 7)})] * 24
+    q = rnd(len(rows), H * dk, seed=4).to(dtype)
+    seg = torch.tensor([s for s, _ in rows], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([p for _, p in rows], dtype=torch.int32, device=DEV)
+
+    def run(lo, hi):
+        out = torch.full((hi - lo, H * dv), float("nan"), dtype=dtype, device=DEV)
+        ops.attention_plain(q[lo:hi], H * dk, k, v, out, seg[lo:hi], pos[lo:hi], tables, hi - lo, H, G, dk, page, window, scale, dv,
+                            keep, sink)
+        return out
+
+    full = run(0, len(rows))
+    for i, (s, p) in enumerate(rows[:len(rows) // 24]):
+        assert torch.equal(run(i, i + 1)[0], full[i]), (s, p)
+        at = torch.arange(p + 1, device=DEV)
+        first = max(0, p + 1 - window) if window > 0 else p - p % -window if window < 0 else 0
+        at = at[(at >= first) | (at < keep)]
+        keys, values = (t[tables[s][at // page].long(), :, at % page].double() for t in (k[..., :dk], v[..., :dv]))
+        x = torch.einsum("hd,jhd->hj", q[i].double().view(H, dk), keys.repeat_interleave(H // G, dim=1)) * scale
+        if sink is not None:
+            x = torch.cat([x, sink.double()[:, None]], dim=1)
+        want = torch.einsum("hj,jhd->hd", torch.softmax(x, dim=1)[:, :len(at)], values.repeat_interleave(H // G, dim=1))
+        # scores within about dk 2^-24 |q||k| scale, exponentials within a few 2^-24 of themselves, sums of 64 products
+        tol = 2e-5 if dtype == torch.float32 else 2.0 ** -8
+        assert float((full[i].double().view(H, dv) - want).abs().max()) <= tol * float(values.abs().max()), (s, p)
