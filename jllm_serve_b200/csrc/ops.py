@@ -125,6 +125,7 @@ class _Signatures:
     jllm_bounds_error_attention_prefill = [P]
     jllm_bounds_error_attention_prefill_tc = [P]
     jllm_bounds_error_attention_prefill_pair = [P]
+    jllm_bounds_error_attention_prefill_latent = [P]
     jllm_bounds_error_rowwise = [P]
     jllm_set_pdl = [I]
     jllm_launch_plan = [ctypes.c_longlong, I]
@@ -151,6 +152,7 @@ class _Signatures:
     jllm_attention_prefill = [P, I, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, P]
     jllm_attention_prefill_tc = [P, I, P, P, ctypes.c_longlong, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, P]
     jllm_attention_prefill_tc_error = []
+    jllm_attention_prefill_latent = [P, I, P, ctypes.c_longlong, P, I, P, P, P, P, I, I, I, I, I, I, I, I, I, F, F, P]
     jllm_attention_prefill_pair = [P, I, P, P, ctypes.c_longlong, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P]
     jllm_attention_decode_separate_combine = [I]
     jllm_attention_decode_fresh = [P, I, P, P, I, I, F, P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P]
@@ -1096,7 +1098,7 @@ def gemm_stream(a, packed: PackedWeight, out, bias=None, accumulate=False, swigl
 
 
 BOUNDS_FILES = ("attention_plain", "attention_decode", "attention_prefill", "attention_prefill_tc",
-                "attention_prefill_pair", "rowwise", "linear_attention", "latent_attention", "residual_paths",
+                "attention_prefill_pair", "attention_prefill_latent", "rowwise", "linear_attention", "latent_attention", "residual_paths",
                 "gated_recurrence", "attention_maps", "delta_recurrence")
 BOUNDS_WHAT = {1: "a block-table index", 2: "a page id", 3: "a cache slot", 4: "a token id", 5: "a row"}
 
@@ -1344,14 +1346,15 @@ def _combine_launches(how, n, rows, kv_heads, head_dim) -> int:
 
 
 def attention(q, k_cache, v_cache, out, batch, group, heads, kv_heads, head_dim, page_size, window, scale,
-              scratch=None, value_dim: int = 0, keep_first: int = 0, sink=None, softcap: float = 0.0) -> None:
+              scratch=None, value_dim: int = 0, keep_first: int = 0, sink=None, softcap: float = 0.0, read_cols: int = 0) -> None:
     """Causal attention of every row of the batch over its own request's cached keys and values. `window`: 0 every
     earlier key, w > 0 the last w keys, -c < 0 the keys of the row's own chunk of c positions (position p lies in chunk
     p // c). `value_dim`: a value head's width where it is not `head_dim`; the tile kernels take heads
     of one width only, so such a mixer runs on the plain kernel. `keep_first` (with a window): the request's first keys stay
     visible to every row. `sink` [heads]: a number per query head whose exponential joins the softmax's denominator. `softcap`
     > 0: every score s = scale (q . k) becomes softcap * tanh(s / softcap), in every kernel. With kept keys or a sink, single rows run on the general decode kernel and prompt portions on the tcgen05 kernel of one query tile (heads of
-    128) or the mma.sync kernel (64, 256)."""
+    128) or the mma.sync kernel (64, 256). `read_cols`: of a head's result the caller reads only so many columns from the first on
+    (0: all); a kernel may leave the others unwritten."""
     one_width = value_dim in (0, head_dim) and k_cache.shape[-1] == head_dim
     extras = bool(keep_first) or sink is not None
     if one_width and batch.decode_only and attention_decode_fits(q.dtype, heads, kv_heads, head_dim):
@@ -1367,7 +1370,7 @@ def attention(q, k_cache, v_cache, out, batch, group, heads, kv_heads, head_dim,
         if mr > 0:
             attention_prefill(q[:mr], k_cache, v_cache, out[:mr], batch.seg_start[:ms], batch.seg_len[:ms],
                               batch.seg_kv_len[:ms], batch.block_tables[group], mr, heads, kv_heads, head_dim, page_size,
-                              window, scale, keep_first=keep_first, sink=sink, softcap=softcap)
+                              window, scale, keep_first=keep_first, sink=sink, softcap=softcap, read_cols=read_cols)
         if mr < batch.rows:
             n = batch.rows - mr
             _attention_decode_rows(q[mr:], k_cache, v_cache, out[mr:], batch.row_seg[mr:], batch.positions[mr:],
@@ -1398,10 +1401,20 @@ def attention_prefill_tc_fits(q, out, k_cache, head_dim, page_size) -> bool:
 
 def attention_prefill(q, k_cache, v_cache, out, seg_start, seg_len, seg_kv_len, block_tables, rows, heads, kv_heads,
                       head_dim, page_size, window, scale, kernel: str = "auto", keep_first: int = 0, sink=None,
-                      softcap: float = 0.0) -> None:
+                      softcap: float = 0.0, read_cols: int = 0) -> None:
     """Flash attention of prompt portions: segments of consecutive rows, each over its own request's pages.
-    Head size 128 runs on tcgen05 (both products, accumulators in tensor memory; kernel "pair" or "tc"), other
-    sizes on mma.sync ("mma")."""
+    Head size 128 runs on tcgen05 (both products, accumulators in tensor memory; kernel "pair" or "tc"), and so does size
+    256 where keys and values are the same rows ("latent"); other sizes on mma.sync ("mma")."""
+    if kernel == "auto" and PREFILL_TC and not keep_first and sink is None and attention_prefill_latent_fits(
+            q, out, k_cache, v_cache, head_dim, page_size):
+        # one load of a row serves both products, and tcgen05 runs them: a causal prompt of 2,048 rows x 16 heads 270 us on mma.sync
+        # and 62 here, 128 rows 17.0 and 13.5, portions of 8 to 61 rows 13.2 to 14.2 and 12.9 to 13.5 (both then wait, not work)
+        kernel = "latent"
+    if kernel == "latent":
+        return _call("jllm_attention_prefill_latent", q.data_ptr(), q.stride(0), k_cache.data_ptr(), k_cache.shape[0], out.data_ptr(),
+                     out.stride(0), seg_start.data_ptr(), seg_len.data_ptr(), seg_kv_len.data_ptr(), block_tables.data_ptr(),
+                     block_tables.stride(0), seg_start.numel(), rows, heads, kv_heads, head_dim, read_cols or head_dim, page_size,
+                     int(window), float(scale), float(softcap), _stream())
     if kernel == "auto" and PREFILL_TC and attention_prefill_tc_fits(q, out, k_cache, head_dim, page_size):
         # two query tiles per block where the portions are long enough to fill them (the tiles take turns on the
         # tensor cores); one tile per block, with two S buffers, for short portions
@@ -1417,6 +1430,12 @@ def attention_prefill(q, k_cache, v_cache, out, seg_start, seg_len, seg_kv_len, 
                          heads, kv_heads, head_dim, page_size, int(window), float(scale), int(keep_first), _p(sink), sd, float(softcap),
                          _stream())
         return _call("jllm_attention_prefill_extras", q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
+def attention_prefill_latent_fits(q, out, k_cache, v_cache, head_dim, page_size) -> bool:
+    return (head_dim == 256 and q.dtype == torch.bfloat16 and k_cache.data_ptr() == v_cache.data_ptr()
+            and 1 <= page_size <= 128 and page_size & (page_size - 1) == 0 and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
+            and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and k_cache.data_ptr() % 16 == 0 and k_cache.is_contiguous())
+
+
                      out.data_ptr(), out.stride(0), seg_start.data_ptr(), seg_len.data_ptr(), seg_kv_len.data_ptr(),
                      block_tables.data_ptr(), block_tables.stride(0), seg_start.numel(), rows, heads, kv_heads, head_dim,
                      page_size, int(window), float(scale), int(keep_first), _p(sink), sd, float(softcap), _stream())

@@ -130,7 +130,7 @@ class LatentAttention(Mixer):
         for h0 in range(0, H, per):
             n = min(per, H - h0)
             ops.attention(q[:, h0 * W:(h0 + n) * W], cache.keys, cache.values, att[:, h0 * W:(h0 + n) * W], batch,
-                          cache.group, n, 1, W, self.rt.page_size, s.window, s.scale, scratch)
+                          cache.group, n, 1, W, self.rt.page_size, s.window, s.scale, scratch, read_cols=R)
         y = self.rt.buffer("latent_values", H * dv)[:rows]
         gate = proj[:, self.offsets["g"]:self.offsets["g"] + self.gate_width] if s.gated else None
         ops.gemm_heads(att, self.latent_to_v, y, gate, self.residual_scale, a_head=W)
@@ -172,7 +172,7 @@ class LatentAttention(Mixer):
         for h0 in range(0, H, per):
             n = min(per, H - h0)
             ops.attention(ql[:, h0 * W:(h0 + n) * W], cache.keys, cache.values, att[:, h0 * W:(h0 + n) * W], batch,
-                          cache.group, n, 1, W, self.rt.page_size, s.window, s.scale, scratch)
+                          cache.group, n, 1, W, self.rt.page_size, s.window, s.scale, scratch, read_cols=R)
         y = self.rt.buffer("latent_values", H * dv)[:rows]
         gate = proj_gate = None
         if s.gated:

@@ -42,7 +42,7 @@ def main() -> int:
     # ---- attention over the cache: every kernel, a clean run after the spoilt one ---------------------------------
     for name, hd, dtype in (("plain", 48, torch.float32), ("decode", 48, torch.bfloat16), ("decode", 128, torch.bfloat16),
                             ("flat", 128, torch.bfloat16), ("mma", 64, torch.bfloat16), ("tc", 128, torch.bfloat16),
-                            ("pair", 128, torch.bfloat16)):
+                            ("pair", 128, torch.bfloat16), ("latent", 256, torch.bfloat16)):
         scale = 1.0 / math.sqrt(hd)
         lens = [40, 300, 200, 70]
         q_lens = [1, 1, 1, 1] if name in ("decode", "flat") else [3, 260, 150, 2]
@@ -51,6 +51,10 @@ def main() -> int:
         pool = kc.shape[0]
         ops.set_pool_pages(pool)
         rows = q.shape[0]
+        if name == "latent":                                     # the same rows are keys and values
+            vc = kc
+            ops.attention_plain(q, q.stride(0), kc, kc, out, rseg, rpos, tables, rows, H, Hkv, hd, page, 0, scale)
+            want = out.float().cpu()
         starts = [sum(q_lens[:i]) for i in range(len(lens))]
         scratch = torch.empty(1 << 20, device=DEV)
 
@@ -69,7 +73,8 @@ def main() -> int:
 
         run(spoil(tables, pool))
         file = {"plain": "attention_plain", "decode": "attention_decode", "flat": "attention_decode",
-                "mma": "attention_prefill", "tc": "attention_prefill_tc", "pair": "attention_prefill_pair"}[name]
+                "mma": "attention_prefill", "tc": "attention_prefill_tc", "pair": "attention_prefill_pair",
+                "latent": "attention_prefill_latent"}[name]
         caught(file, "a page id")
         # a table whose row is shorter than the keys need: the index past its end is caught, not read
         short = tables[:, :3].contiguous()
@@ -80,7 +85,7 @@ def main() -> int:
         tol = dict(rtol=1e-4, atol=2e-5) if dtype == torch.float32 else dict(rtol=2e-2, atol=2e-2)
         assert torch.allclose(out.float().cpu(), want, **tol), (name, hd)
         ops.check_kernel_errors()
-        print(f"ok: {name} head size {hd}")
+        print(f"ok: {name} head size {hd}" if name != "latent" else f"and {name}, head size {hd}")
 
     # ---- the decode attention that makes its own rows' keys and values: a spoilt page of the newest position is neither
     # read nor written; afterwards the same bits as the row-wise kernel followed by the attention ----------------------

@@ -793,3 +793,24 @@ def test_sample_rows_have_their_own_parameters(ops):
     top4 = torch.topk(logits[2], 4).indices.tolist()
     assert out[0].item() == int(logits[0].argmax()) and out[1].item() == int(logits[1].argmax())
     assert out[2].item() == top4[3]
+
+
+@pytest.mark.parametrize("H,Hkv,page,window,cols", [(2, 1, 16, 0, 192), (5, 1, 1, 0, 256), (4, 2, 128, 0, 64), (3, 1, 8, 300, 200),
+                                                    (2, 2, 16, 128, 256), (2, 1, 32, -96, 130), (3, 1, 2, 1, 192)])
+def test_attention_prefill_over_rows_that_are_key_and_value(ops, H, Hkv, page, window, cols):
+    """The tcgen05 kernel for cached rows of 256 values that serve as key and value: portions that start and end anywhere in a
+    128-key tile, fewer result columns than a row has, against the same rows as keys and values."""
+    hd, scale, lens = 256, 1.0 / 16, [1, 17, 128, 129, 700, 1500, 256, 383]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    for far in MODES:
+        q, kc, _, out, rseg, rpos, tables, _, q_lens = attention_case(ops, torch.bfloat16, H, Hkv, hd, page, lens, max(window, 0), scale,
+                                                                       far, [1, 5, 128, 2, 513, 300, 129, 255])
+        out.fill_(float("nan"))
+        starts = [sum(q_lens[:i]) for i in range(len(lens))]
+        ops.attention_prefill(q, kc, kc, out, i32(starts), i32(q_lens), i32(lens), tables, q.shape[0], H, Hkv, hd, page, window, scale,
+                              read_cols=cols)
+        assert ops.attention_prefill_tc_error() == 0
+        want = torch.empty_like(out)
+        ops.attention_plain(q, q.stride(0), kc, kc, want, rseg, rpos, tables, q.shape[0], H, Hkv, hd, page, window, scale)
+        got = out.view(-1, H, hd)[:, :, :cols].reshape(q.shape[0], -1)
+        rows_close(got, want.float().cpu().view(-1, H, hd)[:, :, :cols].reshape(q.shape[0], -1), f"latent {far}")
