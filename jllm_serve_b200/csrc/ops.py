@@ -36,7 +36,7 @@ def library():
             if name.startswith("jllm_"):
                 fn = getattr(lib, name)
                 fn.argtypes = getattr(_Signatures, name)
-                fn.restype = c_int
+                fn.restype = ctypes.c_longlong if name == "jllm_chunk_workspace" else c_int
         _lib = lib
     return _lib
 
@@ -162,7 +162,11 @@ class _Signatures:
     jllm_dynamic_tanh = [P, P, P, I, F, P, I, P, I, I, P]
     jllm_add_scaled = [P, P, F, ctypes.c_longlong, P]
     jllm_gla_recurrent = [P, I, I, I, I, I, P, I, P, I, P, P, P, P, I, I, I, I, F, F, P, I, P]
-    jllm_gla_chunked = [P, I, I, I, I, I, P, I, P, P, P, P, I, P, P, P, P, I, I, I, I, I, F, F, P, I, P]
+    jllm_gla_chunked = [P, I, I, I, I, I, P, I, P, P, P, P, I, P, P, P, P, I, I, I, I, I, F, F, P, I, P, ctypes.c_longlong, P]
+    jllm_gla_chunks_fit = [P, I, I, I, I, I, I, I]
+    jllm_chunk_workspace = [I, I, I, I, I, I]
+    jllm_chunk_passes = [I, I, I, I, I, I]
+    jllm_bounds_error_chunk_scan = [P]
     jllm_gated_head_norm = [P, P, I, I, P, I, P, I, I, I, F, F, I, I, P]
     jllm_lightning_block_width = [I]
     jllm_head_prepare = [P, I, I, I, I, I, P, P, I, I, I, F, P, P, I, I, P, P, P, P, I, I, I, I, I, I, I, I, P]
@@ -190,7 +194,7 @@ class _Signatures:
     jllm_memory_gates = [P, I, I, I, P, P, I, F, P, I, P, P, P, P, P, P, I, I, P]
     jllm_causal_conv = [P, I, I, I, P, P, I, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P]
     jllm_scalar_gated_recurrent = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, P, I, P, P, I, P, P, P, P, I, I, I, I, F, P]
-    jllm_scalar_gated_chunked = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, F, P]
+    jllm_scalar_gated_chunked = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I, F, P, ctypes.c_longlong, P]
     jllm_memory_values = [P, I, I, I, P, I, I, I, I, P]
     jllm_memory_divide = [P, P, P, I, I, I, I, P]
     jllm_sigmoid_gate = [P, I, P, I, I, I, I, F, P]
@@ -286,17 +290,31 @@ def gla_chunked(proj, q_off, k_off, v_off, decay_logits, state, seg_start, seg_l
     assert proj.stride(1) == 1 and all(t.is_contiguous() for t in (decay_logits, state, out, qb, ke, scores))
     assert qb.shape == ke.shape == decay_logits.shape and scores.shape == (decay_logits.shape[0], heads * GLA_CHUNK)
     global launch_count
-    launch_count += 2
+    rows, segments, workspace = decay_logits.shape[0], seg_start.numel(), None
+    if head_decay is not None and rows and segments and library().jllm_gla_chunks_fit(
+            proj.data_ptr(), _DT[proj.dtype], proj.stride(0), q_off, k_off, v_off, key_dim, value_dim):
+        workspace, passes = _chunk_workspace(rows, segments, heads, heads, key_dim, value_dim, proj.device)
+        launch_count += 3 * passes - 1 + (1 if activation else 0)
+    else:
+        launch_count += 2
     _call("jllm_gla_chunked", proj.data_ptr(), _DT[proj.dtype], proj.stride(0), q_off, k_off, v_off, decay_logits.data_ptr(),
           decay_logits.shape[0], qb.data_ptr(), ke.data_ptr(), scores.data_ptr(), state.data_ptr(), state.shape[0],
           seg_start.data_ptr(), seg_len.data_ptr(), state_slots.data_ptr(), out.data_ptr(), seg_start.numel(), int(max_len),
           heads, key_dim, value_dim, float(query_scale), float(temperature), _head_decay(head_decay, heads), int(activation),
-          _stream())
+          _p(workspace), workspace.numel() if workspace is not None else 0, _stream())
+
+
+def _chunk_workspace(rows, segments, heads, groups, key_dim, value_dim, device):
+    """(workspace, passes) for the tensor-core chunks of a step: the states in front of all chunks, at most 256 MB of them at a
+    time (or one group's). It belongs to this call: the allocator's memory of the current stream, given back behind the launches."""
+    floats = library().jllm_chunk_workspace(int(rows), int(segments), int(heads), int(groups), int(key_dim), int(value_dim))
+    passes = library().jllm_chunk_passes(int(rows), int(segments), int(heads), int(groups), int(key_dim), int(value_dim))
+    return torch.empty(floats, dtype=torch.float32, device=device), passes
 
 
 def lightning_block_width(width: int = 0) -> None:
-    """A test's switch: the value columns a block of the tensor-core chunk kernel of the fixed-decay linear attention owns
-    (32 or 64); 0 (the default): 32 where blocks of 64 would leave SMs without one."""
+    """A test's switch: the value columns of an item of the tensor-core chunk kernels (32 or 64); 0 (the default): chosen from
+    the shape."""
     code = library().jllm_lightning_block_width(int(width))
     if code:
         raise KernelError(library().jllm_last_error().decode(errors="replace"))
@@ -594,7 +612,7 @@ GATED_CHUNKS = int(os.environ.get("JLLM_B200_GATED_CHUNKS", "1"))      # 0: prom
 
 def scalar_gated_chunked(q, q_off, q_groups, k, k_off, k_groups, v, v_off, log_decay, in_scale, state, batch, out, heads,
                          key_dim, value_dim, query_scale: float = 1.0, skip=None) -> bool:
-    """`scalar_gated_recurrent` (without a normalizer) for steps that hold prompt portions, in chunks of 64 tokens on the
+    """`scalar_gated_recurrent` (without a normalizer) for steps that hold prompt portions, all chunks of 64 tokens at once on the
     tensor cores: q, k, v enter as bfloat16 operands (float32 sources are rounded on their way in), the decays and scales are
     applied in float32 and every float32 factor becomes two bfloat16 operands. Key heads of 64 or 128 channels and 16-byte
     aligned pieces; says False, having launched nothing, where the shape is not taken."""
@@ -603,17 +621,19 @@ def scalar_gated_chunked(q, q_off, q_groups, k, k_off, k_groups, v, v_off, log_d
     assert q.dtype == k.dtype == v.dtype and q.stride(1) == k.stride(1) == v.stride(1) == 1
     assert state.dtype == out.dtype == torch.float32 and state.is_contiguous() and out.is_contiguous()
     fn = library().jllm_scalar_gated_chunked
+    rows, segments = out.shape[0], batch.seg_start.numel()
+    workspace, passes = _chunk_workspace(rows, segments, heads, q_groups if q_groups == k_groups else heads, key_dim, value_dim, out.device)
     code = fn(q.data_ptr(), q.stride(0), int(q_off), int(q_groups), k.data_ptr(), k.stride(0), int(k_off), int(k_groups),
               v.data_ptr(), v.stride(0), int(v_off), _DT[q.dtype], log_decay.data_ptr(), in_scale.data_ptr(), _p(skip),
               _DT[skip.dtype] if skip is not None else F32, state.data_ptr(), state.shape[0], batch.seg_start.data_ptr(),
-              batch.seg_len.data_ptr(), batch.state_slots.data_ptr(), out.data_ptr(), batch.seg_start.numel(), int(heads),
-              int(key_dim), int(value_dim), float(query_scale), _stream())
+              batch.seg_len.data_ptr(), batch.state_slots.data_ptr(), out.data_ptr(), rows, segments, int(heads),
+              int(key_dim), int(value_dim), float(query_scale), workspace.data_ptr(), workspace.numel(), _stream())
     if code == 3:        # the library's word for "this shape is not taken"
         return False
     if code != 0:
         raise KernelError(f"jllm_scalar_gated_chunked failed ({code}): {library().jllm_last_error().decode(errors='replace')}")
     global launch_count
-    launch_count += 1
+    launch_count += 3 * passes
     return True
 
 
@@ -1098,7 +1118,8 @@ def gemm_stream(a, packed: PackedWeight, out, bias=None, accumulate=False, swigl
 
 
 BOUNDS_FILES = ("attention_plain", "attention_decode", "attention_prefill", "attention_prefill_tc",
-                "attention_prefill_pair", "attention_prefill_latent", "rowwise", "linear_attention", "latent_attention", "residual_paths",
+                "attention_prefill_pair", "attention_prefill_latent", "rowwise", "linear_attention", "chunk_scan", "latent_attention",
+                "residual_paths",
                 "gated_recurrence", "attention_maps", "delta_recurrence")
 BOUNDS_WHAT = {1: "a block-table index", 2: "a page id", 3: "a cache slot", 4: "a token id", 5: "a row"}
 
@@ -1399,6 +1420,12 @@ def attention_prefill_tc_fits(q, out, k_cache, head_dim, page_size) -> bool:
             and k_cache.is_contiguous())
 
 
+def attention_prefill_latent_fits(q, out, k_cache, v_cache, head_dim, page_size) -> bool:
+    return (head_dim == 256 and q.dtype == torch.bfloat16 and k_cache.data_ptr() == v_cache.data_ptr()
+            and 1 <= page_size <= 128 and page_size & (page_size - 1) == 0 and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
+            and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and k_cache.data_ptr() % 16 == 0 and k_cache.is_contiguous())
+
+
 def attention_prefill(q, k_cache, v_cache, out, seg_start, seg_len, seg_kv_len, block_tables, rows, heads, kv_heads,
                       head_dim, page_size, window, scale, kernel: str = "auto", keep_first: int = 0, sink=None,
                       softcap: float = 0.0, read_cols: int = 0) -> None:
@@ -1430,12 +1457,6 @@ def attention_prefill(q, k_cache, v_cache, out, seg_start, seg_len, seg_kv_len, 
                          heads, kv_heads, head_dim, page_size, int(window), float(scale), int(keep_first), _p(sink), sd, float(softcap),
                          _stream())
         return _call("jllm_attention_prefill_extras", q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
-def attention_prefill_latent_fits(q, out, k_cache, v_cache, head_dim, page_size) -> bool:
-    return (head_dim == 256 and q.dtype == torch.bfloat16 and k_cache.data_ptr() == v_cache.data_ptr()
-            and 1 <= page_size <= 128 and page_size & (page_size - 1) == 0 and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
-            and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and k_cache.data_ptr() % 16 == 0 and k_cache.is_contiguous())
-
-
                      out.data_ptr(), out.stride(0), seg_start.data_ptr(), seg_len.data_ptr(), seg_kv_len.data_ptr(),
                      block_tables.data_ptr(), block_tables.stride(0), seg_start.numel(), rows, heads, kv_heads, head_dim,
                      page_size, int(window), float(scale), int(keep_first), _p(sink), sd, float(softcap), _stream())

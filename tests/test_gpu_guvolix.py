@@ -429,6 +429,68 @@ def test_the_recurrence_in_chunks_on_the_tensor_cores(H, G, dk, dv, block_width,
     assert float(state[0].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("H, G, dk, dv, lens", [(8, 8, 128, 264, [129, 1, 64, 1]), (6, 2, 64, 72, [65, 63, 128] + [1] * 7), (12, 1, 128, 8, [200])])
+def test_chunks_of_many_segments_and_cut_slabs(H, G, dk, dv, lens):
+    """All chunks at once over segments of one row to several chunks, values that end inside a slab of columns, more heads of a
+    group than a block takes, states that are not zero; and the same bits when the heads come in two calls (the workspace's passes)."""
+    o = ops()
+    g = torch.Generator().manual_seed(H * dk + dv)
+    rows = sum(lens)
+    q, k = torch.randn(rows, G, dk, generator=g).bfloat16().float(), (torch.randn(rows, G, dk, generator=g) / math.sqrt(dk)).bfloat16().float()
+    v = torch.randn(rows, H, dv, generator=g).bfloat16().float()
+    la, b = -torch.rand(rows, H, generator=g) * 0.3, torch.rand(rows, H, generator=g)
+    start = torch.randn(len(lens) + 1, H, dk, dv, generator=g)
+    batch = FakeBatch(lens, list(range(len(lens), 0, -1)))
+    buf = torch.cat([q.reshape(rows, -1), k.reshape(rows, -1), v.reshape(rows, -1)], dim=1).to(DEV)
+    state, out = start.to(DEV), torch.full((rows, H * dv), float("nan"), device=DEV)
+    assert o.scalar_gated_chunked(buf, 0, G, buf, G * dk, G, buf, 2 * G * dk, la.to(DEV), b.to(DEV), state, batch, out, H, dk, dv, 0.5)
+    at = 0
+    for s, n in enumerate(lens):
+        S = start[len(lens) - s].double()
+        part = slice(at, at + n)
+        want = plain_recurrence(q[part].double().repeat_interleave(H // G, 1), k[part].double().repeat_interleave(H // G, 1),
+                                v[part].double(), la[part].double(), b[part].double(), S, q_scale=0.5)
+        # (every float32 factor enters the products with 16 bits of mantissa)
+        close(out[part].cpu(), want.reshape(n, -1), torch.float32, f"segment {s}", loose=5)
+        close(state[len(lens) - s].cpu(), S, torch.float32, f"state {s}", loose=5)
+        at += n
+    assert torch.equal(state[0].cpu(), start[0])
+    if G == H:
+        o.lightning_block_width(64)
+        try:
+            whole, halves = [start.to(DEV), torch.empty_like(out)], []
+            o.scalar_gated_chunked(buf, 0, G, buf, G * dk, G, buf, 2 * G * dk, la.to(DEV), b.to(DEV), whole[0], batch, whole[1], H, dk, dv, 0.5)
+            for h in (0, H // 2):
+                n, one = H // 2, [start[:, h:h + H // 2].contiguous().to(DEV), torch.empty(rows, H // 2 * dv, device=DEV)]
+                o.scalar_gated_chunked(buf, h * dk, n, buf, (G + h) * dk, n, buf, 2 * G * dk + h * dv, la[:, h:h + n].contiguous().to(DEV),
+                                       b[:, h:h + n].contiguous().to(DEV), one[0], batch, one[1], n, dk, dv, 0.5)
+                halves.append(one)
+        finally:
+            o.lightning_block_width(0)
+        assert torch.equal(whole[0], torch.cat([x[0] for x in halves], 1)) and torch.equal(whole[1], torch.cat([x[1] for x in halves], 1))
+
+
+def test_chunks_whose_states_fill_the_workspace_more_than_once():
+    """256 heads with states of 128 x 128 over 1,100 rows: two passes over the heads give the bits of two calls of half the heads."""
+    o = ops()
+    H, dk, dv, rows = 256, 128, 128, 1100
+    g = torch.Generator(device=DEV).manual_seed(5)
+    buf = torch.randn(rows, H * (2 * dk + dv), generator=g, device=DEV).bfloat16() * 0.1
+    la, b = -torch.rand(rows, H, generator=g, device=DEV), torch.rand(rows, H, generator=g, device=DEV)
+    batch = FakeBatch([rows], [0])
+    assert o.library().jllm_chunk_passes(rows, 1, H, H, dk, dv) == 2 and o.library().jllm_chunk_passes(rows, 1, H // 2, H // 2, dk, dv) == 1
+    results = []
+    for n in (H, H // 2):
+        state, out = torch.zeros(1, H, dk, dv, device=DEV), torch.empty(rows, H, dv, device=DEV)
+        for h in range(0, H, n):
+            one, st = torch.empty(rows, n * dv, device=DEV), torch.zeros(1, n, dk, dv, device=DEV)
+            o.scalar_gated_chunked(buf, h * dk, n, buf, (H + h) * dk, n, buf, 2 * H * dk + h * dv, la[:, h:h + n].contiguous(),
+                                   b[:, h:h + n].contiguous(), st, batch, one, n, dk, dv, 1.0)
+            state[:, h:h + n], out[:, h:h + n] = st, one.view(rows, n, dv)
+        results.append((state, out))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("groups, width", [(2, 24), (1, 40), (3, 700), (5, 7)])
 def test_gate_in_front_of_a_norm_in_parts_and_a_gain_per_column(dtype, groups, width):
