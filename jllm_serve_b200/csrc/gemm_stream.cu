@@ -20,6 +20,9 @@
 // Roles: warp 0 (one lane) producer, warp 1 (one lane) MMA issuer, warps 2-5 epilogue (bias / float32 residual add /
 // SwiGLU over interleaved gate and up rows / store). Every wait is bounded and raises the error word of
 // gemm_tcgen05 (codes 11-13).
+#include <mutex>
+#include <unordered_map>
+
 #include "tcgen05_common.cuh"
 
 namespace {
@@ -39,6 +42,42 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
+}
+
+// What J tokens from m0 on of weight row n are added to (all the old values are requested before the first store: a load behind a
+// store through the same pointer would wait for it).
+template <typename Tout, int J>
+__device__ __forceinline__ void residual(float (&old)[J], const Tout* out, int ldo, int accumulate, int m0, int M, int n, int N) {
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+        old[j] = accumulate == EPI_ADD && n < N && m0 + j < M ? to_float(out[(size_t)(m0 + j) * ldo + n]) : 0.f;
+}
+// The values of those tokens: bias / residual / SwiGLU and the store. The lanes of a warp hold neighbouring weight rows.
+template <typename Tout, int J>
+__device__ __forceinline__ void finish(const float (&v)[J], const float (&old)[J], Tout* out, int ldo, int accumulate, const VecRef& bias,
+                                       int has_bias, const GluArgs& swiglu, int m0, int M, int n, int N) {
+    if (swiglu) {
+        // rows come in blocks of 16: 8 gate rows, then the 8 up rows of the same hidden units
+        const int unit = (n >> 4) * 8 + (n & 7);
+        float other[J], units[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) other[j] = __shfl_xor_sync(0xffffffffu, v[j], 8);
+        if ((threadIdx.x & 8) == 0 && n + 8 < N) {
+            glu_units<J>(swiglu.word_of(unit), [&](int j) { return v[j]; }, [&](int j) { return other[j]; }, 1.f, units);
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                if (m0 + j >= M) continue;
+                if (swiglu.weights != nullptr) units[j] = __fmul_rn(units[j], swiglu.weight(m0 + j, unit));
+                out[(size_t)(m0 + j) * ldo + unit] = from_float<Tout>(units[j]);
+            }
+        }
+    } else if (n < N) {
+        const float b = has_bias ? bias[n] : 0.f;
+        Tout* dst = out + (size_t)m0 * ldo + n;
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (m0 + j < M) dst[(size_t)j * ldo] = from_float<Tout>(epilogue_act(v[j] + b, accumulate) + old[j]);
+    }
 }
 
 template <typename Tout>
@@ -175,35 +214,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
             const int row_in_tile = quad * 32 + lane;
             const int n = tile * WM + row_in_tile;                 // this thread's weight row = output column
             const uint32_t taddr = tmem_base + buf * acc_cols + ((uint32_t)(quad * 32) << 16);
-            // value of (token m, weight row n): bias / residual / SwiGLU and the store
             auto finalize16 = [&](const float (&v)[16], int m0) {
-                if (swiglu) {
-                    // rows come in blocks of 16: 8 gate rows, then the 8 up rows of the same hidden units
-                    const int unit = (n >> 4) * 8 + (n & 7);
-                    float other[16], units[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) other[j] = __shfl_xor_sync(0xffffffffu, v[j], 8);
-                    if ((lane & 8) == 0 && n + 8 < N) {
-                        glu_units<16>(swiglu.word_of(unit), [&](int j) { return v[j]; }, [&](int j) { return other[j]; }, 1.f, units);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            if (m0 + j >= M) continue;
-                            if (swiglu.weights != nullptr) units[j] = __fmul_rn(units[j], swiglu.weight(m0 + j, unit));
-                            out[(size_t)(m0 + j) * ldo + unit] = from_float<Tout>(units[j]);
-                        }
-                    }
-                } else if (n < N) {
-                    const float b = has_bias ? bias[n] : 0.f;
-                    Tout* dst = out + (size_t)m0 * ldo + n;
-                    float old[16];
-                    // all the old values are requested before the first store (a load behind a store through the
-                    // same pointer would wait for it: 16 round trips instead of one)
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) old[j] = (accumulate == EPI_ADD && m0 + j < M) ? to_float(dst[(size_t)j * ldo]) : 0.f;
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (m0 + j < M) dst[(size_t)j * ldo] = from_float<Tout>(epilogue_act(v[j] + b, accumulate) + old[j]);
-                }
+                float old[16];
+                residual(old, out, ldo, accumulate, m0, M, n, N);
+                finish(v, old, out, ldo, accumulate, bias, has_bias, swiglu, m0, M, n, N);
             };
             if (kb0 == 0 && kb1 == k_blocks) {                      // the whole tile is this block's
 #pragma unroll 1
@@ -317,6 +331,253 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
     }
 }
 
+
+// ---- a cluster of blocks to a tile --------------------------------------------------------------------------------------
+// What the equal runs above pay for is the meeting: a tile's parts go to a workspace and back, a fence and a counter between
+// (5 to 7 us of a product whose bytes take 5 to 15). Where the tiles come out even, a cluster of `gridDim.x / tiles` blocks has
+// one tile instead, each block a part of its k blocks, and the parts never leave the SMs: every block finishes a share of the
+// tokens, the others write their parts of it straight into its shared memory (st.shared::cluster), and after the cluster's
+// barrier it adds them up in k order. Launched back to back, equal runs and clusters: 64 rows against O (4,096 x 4,096) 14.0 and
+// 11.5 us, against down (4,096 x 12,288) 24.5 and 21.7, 24 rows against them 13.8 and 10.5, 23.4 and 20.3; 64 rows against 2,048 x
+// 8,192 16.5 and 12.7. What bounds it is what an SM takes in, 60 GB/s of weights and activations (0.33 us per k block with 32 tokens,
+// 0.40 with 64) on the SMs that have a block, and about 5 us from launch to first bytes and for the meeting.
+// `overlay`: the parts lie over the ring (many tokens leave no room beside it); the cluster then meets once more, when every block
+// is done with its ring, before anything is written.
+constexpr int CLUSTER_MAX = 8;
+constexpr double MEETING_K_BLOCKS = 16;         // k blocks an SM streams in the time of a meeting in the workspace (5 to 6 us)
+
+__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+template <typename Tout>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat16* __restrict__ w_packed, VecRef bias,
+                    int has_bias, Tout* __restrict__ out, int ldo, int accumulate, int M, int N, int k_blocks, GluArgs swiglu,
+                    int ntok, int stages, uint32_t tmem_cols, int blocks, int share, int overlay, int* __restrict__ error_word) {
+    // `share`: tokens (a multiple of 8) that a block of the cluster finishes: block p those from p * share on
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t stage_bytes = W_TILE_BYTES + (uint32_t)ntok * 128u, ring = (uint32_t)stages * stage_bytes;
+    const uint32_t part_bytes = (uint32_t)share * WM * 4;          // one block's part of a share, [share / 4][128 rows][4 tokens]
+    const uint32_t parts_at = overlay ? 0u : ring;
+    const uint32_t bars_at = overlay ? max(ring, (blocks - 1) * part_bytes) : ring + (blocks - 1) * part_bytes;
+    const uint32_t bars = base + bars_at;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (stages + s); };
+    const uint32_t acc_bar = bars + 16u * stages;
+    uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(aligned + bars_at + 8 * (2 * stages + 1));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = (int)blockIdx.x / blocks, rank = (int)blockIdx.x % blocks;      // (clusters lie along x: this is the rank)
+    const int kb_lo = k_blocks * rank / blocks, kb_hi = k_blocks * (rank + 1) / blocks, n_kb = kb_hi - kb_lo;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        mbar_init(acc_bar, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)),
+                     "r"(tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem_base = *tmem_base_slot;
+    // The first meeting says that every block runs (without overlay: from here on its shared memory may be written), or
+    // that every block is done with its ring (overlay: the epilogue warps arrive then).
+    if (!overlay || warp < 2) cluster_arrive();
+
+    if (warp == 0) {
+        // ---------------- producer: weights by bulk copy, activations by TMA ----------------
+        if (lane == 0) {
+            bool ok = true;
+            const __nv_bfloat16* w = w_packed + ((size_t)tile * k_blocks + kb_lo) * (WM * BK);
+            const int early = min(stages, n_kb);
+            // the first weights are requested before the kernel in front of this one has finished
+            for (int i = 0; i < early; ++i) {
+                mbar_expect_tx(full_bar(i), stage_bytes);
+                bulk_copy(base + (uint32_t)i * stage_bytes, w + (size_t)i * (WM * BK), W_TILE_BYTES, full_bar(i));
+            }
+            pdl_wait();
+            pdl_trigger();
+            for (int i = 0; i < early; ++i)
+                tma_load_2d(base + (uint32_t)i * stage_bytes + W_TILE_BYTES, &map_a, (kb_lo + i) * BK, 0, full_bar(i));
+            int s = 0;
+            uint32_t parity = 0;                                   // the ring's second lap waits for the first lap's release
+            for (int i = stages; i < n_kb; ++i) {
+                if (!mbar_wait(empty_bar(s), parity, abort_flag)) { ok = false; break; }
+                const uint32_t dst = base + (uint32_t)s * stage_bytes;
+                mbar_expect_tx(full_bar(s), stage_bytes);
+                bulk_copy(dst, w + (size_t)i * (WM * BK), W_TILE_BYTES, full_bar(s));
+                tma_load_2d(dst + W_TILE_BYTES, &map_a, (kb_lo + i) * BK, 0, full_bar(s));
+                if (++s == stages) { s = 0; parity ^= 1u; }
+            }
+            if (!ok) { *abort_flag = 1; atomicExch(error_word, 14); }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        if (lane == 0) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ntok >> 3) << 17) | ((uint32_t)(WM >> 4) << 24);
+            bool ok = true;
+            int s = 0;
+            uint32_t parity = 0;
+            for (int i = 0; i < n_kb; ++i) {
+                if (!mbar_wait(full_bar(s), parity, abort_flag)) { ok = false; break; }
+                tcgen05_fence_after();
+                const uint32_t w_addr = base + (uint32_t)s * stage_bytes, b_addr = w_addr + W_TILE_BYTES;
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k)
+                    tcgen05_mma_bf16(tmem_base, smem_desc_sw128(w_addr + k * 32), smem_desc_sw128(b_addr + k * 32), idesc,
+                                     (i > 0 || k > 0) ? 1u : 0u);
+                tcgen05_commit(empty_bar(s));
+                if (++s == stages) { s = 0; parity ^= 1u; }
+            }
+            if (ok) tcgen05_commit(acc_bar);
+            else { *abort_flag = 1; atomicExch(error_word, 15); }
+        }
+        __syncwarp();
+    } else {
+        pdl_wait();          // the residual stream it may add into was written by the kernels before
+        pdl_trigger();
+    }
+    if (warp < 2) {
+        cluster_wait();
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        // ---------------- epilogue: warps 2..5, TMEM lanes 32 * (warp % 4) = weight rows of the tile ----------------
+        const int quad = warp & 3, row = quad * 32 + lane, n = tile * WM + row, mine = rank * share;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+        float old[8];
+        residual(old, out, ldo, accumulate, mine, min(M, ntok), n, N);      // asked for while the weights still come
+        bool ok = mbar_wait(acc_bar, 0, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        tcgen05_fence_after();
+        if (overlay) cluster_arrive();
+        cluster_wait();
+        if (ok)
+            for (int d = 1; d < blocks; ++d) {          // (every block begins with its neighbour: nobody is written by all at once)
+                const int p = (rank + d) % blocks, t0 = p * share;
+                // of block p's blocks - 1 parts this block's is number `rank`, or rank - 1 if p is below it
+                const uint32_t at = base + parts_at + (uint32_t)(rank - (rank > p ? 1 : 0)) * part_bytes + (uint32_t)row * 16;
+                uint32_t dst;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(at), "r"(p));
+                for (int t = t0; t < min(t0 + share, ntok); t += 8) {
+                    uint32_t v[8];
+                    tmem_ld_32x32b_x8(taddr + t, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(dst + (uint32_t)((t - t0) / 4 + q) * (WM * 16)), "r"(v[4 * q]), "r"(v[4 * q + 1]),
+                                     "r"(v[4 * q + 2]), "r"(v[4 * q + 3])
+                                     : "memory");
+                }
+            }
+        cluster_arrive();
+        cluster_wait();
+        if (ok) {
+            const uint8_t* parts = aligned + parts_at + (size_t)row * 16;
+            for (int t = mine; t < min(mine + share, ntok); t += 8) {
+                uint32_t own[8];
+                tmem_ld_32x32b_x8(taddr + t, own);
+                tmem_ld_wait();
+                float v[8] = {};
+                for (int p = 0; p < blocks; ++p) {      // in k order
+                    if (p == rank) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] += __uint_as_float(own[j]);
+                    } else {
+                        const uint8_t* src = parts + (size_t)(p - (p > rank ? 1 : 0)) * part_bytes + (size_t)((t - mine) / 4) * (WM * 16);
+                        const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + WM * 16);
+                        v[0] += x.x, v[1] += x.y, v[2] += x.z, v[3] += x.w, v[4] += y.x, v[5] += y.y, v[6] += y.z, v[7] += y.w;
+                    }
+                }
+                if (t > mine) residual(old, out, ldo, accumulate, t, M, n, N);
+                finish(v, old, out, ldo, accumulate, bias, has_bias, swiglu, t, M, n, N);
+            }
+        } else if (lane == 0) { *abort_flag = 1; atomicExch(error_word, 16); }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 2) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    }
+}
+
+// How a cluster product of `ntok` tokens lies in shared memory
+struct ClusterCut {
+    int blocks, share, overlay, stages;
+    size_t smem;
+};
+ClusterCut cluster_cut(int blocks, int ntok) {
+    ClusterCut c{blocks, ((ntok + 7) / 8 + blocks - 1) / blocks * 8, 0, 0, 0};
+    const size_t stage = W_TILE_BYTES + (size_t)ntok * 128, parts = (size_t)(blocks - 1) * c.share * WM * 4, room = 224 * 1024;
+    c.stages = (int)((room - parts) / stage);
+    if (c.stages < 6) c.overlay = 1, c.stages = (int)(room / stage);
+    if (c.stages > 12) c.stages = 12;
+    const size_t ring = c.stages * stage;
+    c.smem = (c.overlay ? (ring > parts ? ring : parts) : ring + parts) + 1024 + 8 * (2 * c.stages + 1) + 16;
+    return c;
+}
+
+template <typename Tout>
+cudaLaunchConfig_t cluster_config(const ClusterCut& c, int tiles, cudaLaunchAttribute* attr, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles * c.blocks);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = c.smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = c.blocks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// clusters of that many blocks the device runs at a time with that much shared memory (asked once per size)
+template <typename Tout>
+int resident_clusters(int blocks, size_t smem) {
+    static std::mutex mu;
+    static std::unordered_map<long long, int> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const long long key = ((long long)dev * 16 + blocks) * (1 << 20) + (long long)smem;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    int n = 0;
+    ClusterCut c{blocks, 0, 0, 0, smem};
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = cluster_config<Tout>(c, 1, attr, nullptr);
+    if (cudaFuncSetAttribute(gemm_cluster_kernel<Tout>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_cluster_kernel<Tout>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    known[key] = n;
+    return n;
+}
+
 }  // namespace
 
 // The error word is gemm_tcgen05's (one word for the tcgen05 products).
@@ -361,13 +622,45 @@ JLLM_EXPORT int jllm_gemm_stream(const void* a, int lda, const void* w_packed, i
     if (rc != JLLM_OK) return rc;
     int* error_word = jllm_gemm_error_word();
     if (!error_word) return jllm_fail(JLLM_CUDA_ERROR, "gemm_stream: no error word");
+    const VecRef b{bias, bias_dtype};
+    // A cluster to a tile where the clusters of all tiles are resident at once and a block's k blocks take no longer than an equal run
+    // and the meeting it saves; of the sizes that fit, the one with the fewest k blocks a block (a larger cluster meets for longer).
+    if (max_blocks <= 0) {
+        ClusterCut c{};
+        double best = (double)tiles * k_blocks / sms + MEETING_K_BLOCKS;
+        for (int n = 1; n <= CLUSTER_MAX && n <= k_blocks; ++n) {
+            const ClusterCut one = cluster_cut(n, ntok);
+            const double cost = (k_blocks + n - 1) / n + 0.5 * n;
+            if (one.stages < 2 || cost >= best) continue;
+            if (tiles <= (out_dtype == JLLM_F32 ? resident_clusters<float>(n, one.smem) : resident_clusters<__nv_bfloat16>(n, one.smem)))
+                best = cost, c = one;
+        }
+        if (c.blocks > 0) {
+#define JLLM_CLUSTER_GO(T)                                                                                          \
+    do {                                                                                                            \
+        auto kern = gemm_cluster_kernel<T>;                                                                         \
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);                       \
+        cudaLaunchAttribute attr[2];                                                                                \
+        cudaLaunchConfig_t cfg = cluster_config<T>(c, tiles, attr, stream);                                         \
+        if (jllm_launch_overlaps(c.smem, LAUNCH_DEPENDENT)) {                                                       \
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;                                        \
+            attr[1].val.programmaticStreamSerializationAllowed = 1;                                                 \
+            cfg.numAttrs = 2;                                                                                       \
+        }                                                                                                           \
+        cudaLaunchKernelEx(&cfg, kern, map_a, (const __nv_bfloat16*)w_packed, b, (int)(bias != nullptr), (T*)out, ldo, accumulate, \
+                           M, N, k_blocks, swiglu, ntok, c.stages, acc_cols, c.blocks, c.share, c.overlay, error_word); \
+    } while (0)
+            if (out_dtype == JLLM_F32) JLLM_CLUSTER_GO(float); else JLLM_CLUSTER_GO(__nv_bfloat16);
+#undef JLLM_CLUSTER_GO
+            return jllm_check_launch("gemm_cluster");
+        }
+    }
     const long long total = (long long)tiles * k_blocks;
     int grid = total < sms ? (int)total : sms;
     if (grid > 160) grid = 160;
     if (max_blocks > 0 && grid > max_blocks) grid = max_blocks;
     int* counters = reinterpret_cast<int*>(workspace);
     float* partials = workspace + 2 * MAX_TILES;      // two counters per tile (counted in, done), then the parked parts
-    const VecRef b{bias, bias_dtype};
 #define JLLM_STREAM_GO(T)                                                                                           \
     do {                                                                                                            \
         auto kern = gemm_stream_kernel<T>;                                                                          \

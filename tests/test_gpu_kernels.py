@@ -141,6 +141,22 @@ def test_gemm_stream(ops, M, N, K):
     assert float(out16[:, N:].abs().max()) == 0 and ops.gemm_tcgen05_error() == 0
 
 
+@pytest.mark.parametrize("M", [3, 24, 61, 130, 250])
+@pytest.mark.parametrize("N,K", [(300, 8192), (2048, 8192), (1111, 320), (2500, 2056)])
+def test_gemm_stream_by_clusters(ops, M, N, K):
+    """A cluster of two to eight blocks to a tile, their shares of the tokens uneven or empty, few k blocks, parts beside the ring and
+    over it: against float64, and the same bits twice."""
+    a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
+    packed, base, bias = ops.pack_weight(w), rnd(M, N, seed=3), rnd(N, dtype=torch.float32, seed=2)
+    want = gemm_want(a, w, bias, base)
+    acc, again = base.clone(), base.clone()
+    ops.gemm_stream(a, packed, acc, bias, accumulate=True)
+    ops.gemm_stream(a, packed, again, bias, accumulate=True)
+    assert ops.gemm_tcgen05_error() == 0
+    assert torch.allclose(acc.cpu(), want, rtol=1e-4, atol=1e-4 * math.sqrt(K) * 0.05)
+    assert torch.equal(acc, again)
+
+
 @pytest.mark.parametrize("M", [1, 8, 20, 64, 128, 250])
 @pytest.mark.parametrize("hidden,K", [(8, 8), (200, 72), (12288, 4096), (1000, 136)])
 def test_gemm_stream_with_swiglu_epilogue(ops, M, hidden, K):
