@@ -302,6 +302,7 @@ int g_separate_combine = 0;
 JLLM_EXPORT void jllm_attention_decode_separate_combine(int on) { g_separate_combine = on; }
 
 #include "attention_decode_staged.cuh"
+#include "attention_decode_ring.cuh"
 
 // Floats of scratch the split path needs: (head_dim + 2) per (row, head, split).
 JLLM_EXPORT long long jllm_attention_decode_scratch_floats(int rows, int heads, int head_dim, int splits) {
@@ -348,7 +349,14 @@ int decode_split(const void* q, int q_stride, const void* k_cache, const void* v
     staged::launch<HD>(q, q_stride, k_cache, v_cache, out, out_stride, row_seg, row_pos, block_tables, table_stride, \
                        rows, heads, kv_heads, page_size, window, scale_log2, splits, part_o, part_ml, counters, fresh, stream, \
                        keep_first, sk, cap)
-        if (head_dim == 64) JLLM_STAGED(64); else if (head_dim == 128) JLLM_STAGED(128); else JLLM_STAGED(256);
+        if (ring::fits(heads, kv_heads, head_dim, page_size, window, keep_first)) {
+            const ring::Args a{(const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, row_seg, row_pos, block_tables,
+                               table_stride, rows, heads, kv_heads, page_size, 0, 0, window, scale_log2, splits, part_o, part_ml,
+                               counters, fresh, sk, has_sink, cap, nullptr};
+            const int rc = head_dim == 64 ? ring::launch<64, false>(a, k_cache, v_cache, grid, stream)
+                                          : ring::launch<128, false>(a, k_cache, v_cache, grid, stream);
+            if (rc != JLLM_OK) return rc;
+        } else if (head_dim == 64) JLLM_STAGED(64); else if (head_dim == 128) JLLM_STAGED(128); else JLLM_STAGED(256);
 #undef JLLM_STAGED
         int rc2 = jllm_check_launch("attention_decode_staged");
         if (rc2 != JLLM_OK || splits == 1 || counters != nullptr) return rc2;
@@ -436,7 +444,17 @@ int decode_flat(const void* q, int q_stride, const void* k_cache, const void* v_
     staged::launch_flat<HD>(q, q_stride, k_cache, v_cache, out, out_stride, row_seg, row_pos, block_tables, table_stride, \
                             rows, heads, kv_heads, page_size, window, scale_log2, blocks, part_o, part_ml, counters, fresh, stream, \
                             score_cap(softcap, scale))
-    if (head_dim == 64) JLLM_FLAT(64); else if (head_dim == 128) JLLM_FLAT(128); else JLLM_FLAT(256);
+    if (ring::fits(heads, kv_heads, head_dim, page_size, window, 0)) {
+        const ring::Args a{(const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, row_seg, row_pos, block_tables,
+                           table_stride, rows, heads, kv_heads, page_size, 0, 0, window, scale_log2, 1, part_o, part_ml, counters,
+                           fresh, VecRef{nullptr, JLLM_F32}, 0, score_cap(softcap, scale), nullptr};
+        const int rc = head_dim == 64 ? ring::launch<64, true>(a, k_cache, v_cache, dim3(blocks), stream)
+                                      : ring::launch<128, true>(a, k_cache, v_cache, dim3(blocks), stream);
+        if (rc != JLLM_OK) return rc;
+        if (counters == nullptr)
+            jllm_launch(staged::attention_combine_flat_kernel, dim3(rows, heads), dim3(128), 0, stream, true, (const float*)part_o,
+                        (const float*)part_ml, (__nv_bfloat16*)out, out_stride, row_pos, rows, heads, kv_heads, head_dim, window, blocks);
+    } else if (head_dim == 64) JLLM_FLAT(64); else if (head_dim == 128) JLLM_FLAT(128); else JLLM_FLAT(256);
 #undef JLLM_FLAT
     return jllm_check_launch("attention_decode_flat");
 }

@@ -555,6 +555,30 @@ def test_attention_prefill_tcgen05_tiles(ops, H, Hkv, page, window, kernel):
                             [128, 2, 513, 300, 129, 255], kernel)
 
 
+@pytest.mark.parametrize("H,Hkv,hd,page,window", [(8, 1, 128, 32, 0), (5, 1, 64, 64, 0), (3, 3, 128, 128, 0), (10, 2, 64, 16, 0),
+                                                   (7, 1, 128, 16, -96), (4, 2, 64, 32, -64), (9, 1, 128, 16, 0), (4, 2, 128, 16, -40)])
+def test_attention_decode_tiles_and_pages(ops, H, Hkv, hd, page, window):
+    """Key counts around the 64-key tiles and the ring's three stages, boxes of a page, of two and of half a page, chunks of whole
+    pages, one to eight query heads to a kv head (nine, and chunks that cut a page, go to the other kernels), one block per pair,
+    several, and the tiles of all pairs dealt out: against the plain kernel, whose own test has the float64 attention."""
+    lens, scale = [1, 15, 16, 63, 64, 65, 128, 191, 192, 193, 257, 700], 1.0 / math.sqrt(hd)
+    for far in MODES:
+        q, kc, vc, _, rseg, rpos, tables, _, q_lens = attention_case(ops, torch.bfloat16, H, Hkv, hd, page, lens, 0, scale, far, [1] * len(lens))
+        R = len(lens)
+        want = torch.empty_like(q)
+        ops.attention_plain(q, q.stride(0), kc, vc, want, rseg, rpos, tables, R, H, Hkv, hd, page, window, scale)
+        for how, n in (("split", 1), ("split", 3), ("split", 12), ("flat", 1), ("flat", 5), ("flat", 12)):
+            out = torch.full_like(q, float("nan"))
+            if how == "split":
+                scratch = torch.full((ops.attention_decode_scratch_floats(R, H, hd, n) + 1,), float("nan"), device=DEV)
+                ops.attention_decode(q, kc, vc, out, rseg, rpos, tables, R, H, Hkv, hd, page, window, scale, n, scratch)
+            else:
+                scratch = torch.full((ops.attention_decode_flat_scratch_floats(R, H, Hkv, hd, n),), float("nan"), device=DEV)
+                ops.attention_decode_flat(q, kc, vc, out, rseg, rpos, tables, R, H, Hkv, hd, page, window, scale, n, scratch)
+            rows_close(out, want, f"{how} {n} {far}")
+        assert ops.attention_prefill_tc_error() == 0
+
+
 @pytest.mark.parametrize("splits", [1, 3, 8])
 @pytest.mark.parametrize("H,Hkv,hd,page,window", [(6, 2, 48, 16, 0), (4, 4, 16, 4, 0), (32, 8, 128, 16, 0),
                                                    (6, 3, 80, 8, 21), (16, 1, 256, 16, 0), (2, 1, 32, 1, 7),
