@@ -316,6 +316,153 @@ gemm_heads_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_b
     }
 }
 
+// The same product for many rows (prompts): 128 x 64 tiles, 64 values of k at a time through a ring of three stages filled by
+// cp.async, fragments by ldmatrix, results through shared memory in 16-byte stores; the rotated part in pieces of eight values. The
+// products are short (K of 128 to 256), so what bounds them is the way in and out (29 MB for 2,048 rows x 16 heads of 128 -> 192
+// values and 64 rotated ones: 4.5 us at the memory's rate). 64 x 64 tiles with plain loads of 32 values of k, a barrier in front and
+// behind, and a block that turned the rotated part value by value took 41 us, 192 -> 128 values 22; these take 14 and 11 (launched
+// back to back), and eight layers of a prompt 0.26 ms less of 3.2. Needs VEC's alignment; the sums run over k in the same order.
+namespace many {
+
+constexpr int ROWS = 128, COLS = 64, KS = 64, STAGES = 3, THREADS = 256;
+constexpr int A_BYTES = ROWS * KS * 2, STAGE_BYTES = A_BYTES + COLS * KS * 2, OUT_LD = COLS + 8;
+constexpr size_t SMEM = STAGES * STAGE_BYTES;
+static_assert(SMEM >= ROWS * OUT_LD * 2, "the results are staged where the ring was");
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// byte offset of 16-byte chunk c of row r of a tile of 64-value rows
+__device__ __forceinline__ uint32_t off(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
+
+// The rotated part of 128 rows of a head, eight values at a time (rope_dim and rotary_dim multiples of 8, 16-byte aligned pieces).
+__device__ __forceinline__ void rope_rows(const __nv_bfloat16* __restrict__ ah, int lda, __nv_bfloat16* __restrict__ oh, int ldo, int m0, int M,
+                                          int K, int N, const HeadRope& rp) {
+    const int half = rp.rotary_dim / 2, pieces = rp.rope_dim / 8;
+    for (int e = threadIdx.x; e < ROWS * pieces; e += THREADS) {
+        const int m = m0 + e / pieces, i = e % pieces;
+        if (m >= M) break;
+        uint4 v = *reinterpret_cast<const uint4*>(ah + (size_t)m * lda + K + 8 * i);
+        if (4 * i < half) {
+            const size_t at = (size_t)rp.positions[m] * half + 4 * i;
+            const float4 c = *reinterpret_cast<const float4*>(rp.cos_t + at), sn = *reinterpret_cast<const float4*>(rp.sin_t + at);
+            const float cs[4] = {c.x, c.y, c.z, c.w}, ss[4] = {sn.x, sn.y, sn.z, sn.w};
+            uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+                float p, q;
+                turn_pair(x.x, x.y, cs[j], ss[j], p, q);
+                __nv_bfloat162 b = __floats2bfloat162_rn(p, q);
+                w[j] = *reinterpret_cast<uint32_t*>(&b);
+            }
+            v = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        *reinterpret_cast<uint4*>(oh + (size_t)m * ldo + N + 8 * i) = v;
+    }
+}
+
+__global__ void __launch_bounds__(THREADS, 3)
+gemm_heads_many_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w,
+                       __nv_bfloat16* __restrict__ out, int ldo, const __nv_bfloat16* __restrict__ gate, int ld_gate, int gate_full,
+                       float alpha, int M, int N, int K, int a_head, int o_head, int wide_out, int wide_rope, HeadRope rp) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, h = blockIdx.z;
+    const int m0 = blockIdx.y * ROWS, n0 = blockIdx.x * COLS;
+    const __nv_bfloat16* ah = a + (size_t)h * a_head;
+    const __nv_bfloat16* wh = w + (size_t)h * N * K;
+    __nv_bfloat16* oh = out + (size_t)h * o_head;
+    pdl_wait();
+    pdl_trigger();
+    if (rp.rope_dim > 0 && blockIdx.x == gridDim.x - 1) {
+        if (wide_rope) return rope_rows(ah, lda, oh, ldo, m0, M, K, N, rp);
+        for (int m = m0; m < min(M, m0 + ROWS); m += 64) rope_tile(ah, lda, oh, ldo, m, M, K, N, rp);
+        return;
+    }
+    const int steps = (K + KS - 1) / KS;
+    auto load = [&](int s) {
+        if (s < steps) {
+            const uint32_t dst = base + (s % STAGES) * STAGE_BYTES;
+            const int c = tid & 7, k = s * KS + c * 8;               // (K is a multiple of 8: a chunk is inside or outside as a whole)
+#pragma unroll
+            for (int j = 0; j < ROWS / 32; ++j) {
+                const int r = (tid >> 3) + 32 * j;
+                const bool in = m0 + r < M && k < K;
+                cp16(dst + off(r, c), in ? ah + (size_t)(m0 + r) * lda + k : ah, in ? 16 : 0);
+            }
+#pragma unroll
+            for (int j = 0; j < COLS / 32; ++j) {
+                const int r = (tid >> 3) + 32 * j;
+                const bool in = n0 + r < N && k < K;
+                cp16(dst + A_BYTES + off(r, c), in ? wh + (size_t)(n0 + r) * K + k : wh, in ? 16 : 0);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load(0);
+    load(1);
+    float acc[8][4] = {};
+    for (int s = 0; s < steps; ++s) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();            // step s has landed, and everyone is done with step s - 1, whose stage is filled again
+        load(s + 2);
+        const uint32_t sa = base + (s % STAGES) * STAGE_BYTES, sw = sa + A_BYTES;
+#pragma unroll
+        for (int kk = 0; kk < KS / 16; ++kk) {
+            uint32_t x[4];
+            ldsm4(x, sa + off(warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, kk * 2 + (lane >> 4)));
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                uint32_t b[4];
+                ldsm4(b, sw + off(j * 8 + (lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
+                mma_bf16_16816(acc[j], x[0], x[1], x[2], x[3], b[0], b[1]);
+                mma_bf16_16816(acc[j + 1], x[0], x[1], x[2], x[3], b[2], b[3]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();                // the ring is free
+    __nv_bfloat16* stage = reinterpret_cast<__nv_bfloat16*>(smem) + (size_t)warp * 16 * OUT_LD;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int m = m0 + warp * 16 + g + 8 * half;
+        float f = alpha;
+        if (gate != nullptr && !gate_full && m < M) f = __fmul_rn(alpha, 1.f / (1.f + expf(-__bfloat162float(gate[(size_t)m * ld_gate + h]))));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int n = n0 + 8 * j + 2 * t;
+            float f0 = f, f1 = f;
+            if (gate_full && m < M) {
+                const __nv_bfloat16* gm = gate + (size_t)m * ld_gate + (size_t)h * N + n;
+                if (n < N) f0 = __fmul_rn(f, 1.f / (1.f + expf(-__bfloat162float(gm[0]))));
+                if (n + 1 < N) f1 = __fmul_rn(f, 1.f / (1.f + expf(-__bfloat162float(gm[1]))));
+            }
+            *reinterpret_cast<__nv_bfloat162*>(stage + (g + 8 * half) * OUT_LD + 8 * j + 2 * t) =
+                __floats2bfloat162_rn(__fmul_rn(acc[j][2 * half], f0), __fmul_rn(acc[j][2 * half + 1], f1));
+        }
+    }
+    __syncwarp();
+    if (wide_out) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = (lane >> 3) + 4 * i, c = (lane & 7) * 8, m = m0 + warp * 16 + r;
+            if (m < M && n0 + c < N) *reinterpret_cast<uint4*>(oh + (size_t)m * ldo + n0 + c) = *reinterpret_cast<const uint4*>(stage + r * OUT_LD + c);
+        }
+    } else {
+        for (int e = lane; e < 16 * COLS; e += 32) {
+            const int r = e / COLS, c = e % COLS, m = m0 + warp * 16 + r;
+            if (m < M && n0 + c < N) oh[(size_t)m * ldo + n0 + c] = stage[r * OUT_LD + c];
+        }
+    }
+}
+
+}  // namespace many
+
 }  // namespace
 
 JLLM_BOUNDS_READER(latent_attention)
@@ -363,7 +510,15 @@ JLLM_EXPORT int jllm_gemm_heads(const void* a, int dtype, int lda, const void* w
         return jllm_check_launch("gemm_heads");
     }
     const bool vec = K % 8 == 0 && lda % 8 == 0 && a_head % 8 == 0 && ((uintptr_t)a % 16) == 0 && ((uintptr_t)w % 16) == 0;
-    if (vec)
+    if (vec && M > 64) {        // (up to 64 rows the small tiles give more blocks)
+        const int wide_out = ldo % 8 == 0 && o_head % 8 == 0 && N % 8 == 0 && ((uintptr_t)out % 16) == 0;
+        const int wide_rope = wide_out && rope_dim % 8 == 0 && rotary_dim % 8 == 0 && ((uintptr_t)cos_t % 16) == 0 && ((uintptr_t)sin_t % 16) == 0;
+        cudaFuncSetAttribute(many::gemm_heads_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)many::SMEM);
+        jllm_launch(many::gemm_heads_many_kernel, dim3(grid.x, (M + many::ROWS - 1) / many::ROWS, heads), dim3(many::THREADS), many::SMEM,
+                    stream, LAUNCH_DEPENDENT, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, ldo,
+                    (const __nv_bfloat16*)gate, ld_gate, (int)(gate != nullptr && gate_full), alpha, M, N, K, a_head, o_head, wide_out,
+                    wide_rope, rp);
+    } else if (vec)
         jllm_launch(gemm_heads_mma_kernel<true>, grid, dim3(128), 0, stream, LAUNCH_DEPENDENT, (const __nv_bfloat16*)a, lda,
                     (const __nv_bfloat16*)w, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)gate, ld_gate, gate != nullptr && gate_full, alpha, M, N, K, a_head, o_head, rp);
     else

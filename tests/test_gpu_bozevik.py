@@ -198,6 +198,37 @@ def test_products_per_head_that_carry_the_rotated_part_along(dtype, heads, K, N,
     close(out, want.reshape(rows, -1), dtype, "latent-space queries")
 
 
+@pytest.mark.parametrize("rows", [65, 128, 300])
+@pytest.mark.parametrize("heads, K, N, rope_dim, rotary, gate", [(2, 128, 192, 64, 64, ""), (3, 72, 40, 16, 8, ""), (2, 200, 70, 0, 0, "head"),
+                                                                 (2, 64, 130, 0, 0, "value"), (2, 8, 64, 6, 4, "")])
+def test_products_per_head_of_many_rows(heads, K, N, rope_dim, rotary, gate, rows):
+    """The tiles of 128 rows: rows, columns and k that end inside a tile, rotated parts of whole and of cut pieces, gates, rows of more
+    values than the heads have (they stay as they were)."""
+    from jllm_serve_b200.config import RopeTableSpec
+    from jllm_serve_b200.parts import RotaryTable
+    o_ = ops()
+    g = torch.Generator().manual_seed(heads * K + rows)
+    a_head, wide = -(-(K + rope_dim) // 8) * 8, heads * (N + rope_dim) + 8
+    q = torch.randn(rows, heads * a_head, generator=g).bfloat16()
+    w = (torch.randn(heads, N, K, generator=g) / math.sqrt(K)).bfloat16()
+    positions = torch.tensor([(11 * r) % 900 for r in range(rows)], dtype=torch.int32)
+    gates = torch.randn(rows, heads * N if gate == "value" else heads, generator=g).bfloat16() if gate else None
+    rope = None
+    if rope_dim:
+        table = RotaryTable(RopeTableSpec(rotary_dim=rotary, theta=1000.0, pairing="interleaved"), 1024, torch.device(DEV))
+        rope = (rope_dim, table.cos, table.sin, rotary, positions.to(DEV))
+    out = torch.full((rows, wide), 7.0, dtype=torch.bfloat16, device=DEV)
+    o_.gemm_heads(q.to(DEV), w.to(DEV), out[:, :wide - 8], gates.to(DEV) if gate else None, 0.5, a_head=a_head, out_head=N + rope_dim, rope=rope)
+    qh = q.double().view(rows, heads, a_head)
+    want = 0.5 * torch.einsum("rhk,hnk->rhn", qh[:, :, :K], w.double())
+    if gate:
+        want = want * torch.sigmoid(gates.double().view(rows, heads, -1))
+    if rope_dim:
+        want = torch.cat([want, P.rotate_pairs(qh[:, :, K:K + rope_dim], positions.tolist(), rotary, 1000.0)], dim=2)
+    close(out[:, :wide - 8], want.reshape(rows, -1), torch.bfloat16, "products of many rows")
+    assert (out[:, wide - 8:] == 7).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("experts, ff, shared_ff", [(1, 40, 0), (4, 24, 16), (3, 10, 0), (16, 96, 128), (5, 7, 3)])
 def test_clamped_gated_unit_with_a_weight_on_the_input(dtype, experts, ff, shared_ff):
