@@ -491,6 +491,28 @@ def test_chunks_whose_states_fill_the_workspace_more_than_once():
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
 
 
+@pytest.mark.parametrize("gate_dtype, dtype", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("heads, width", [(8, 128), (4, 256), (3, 512), (2, 1024), (1, 2048), (1, 4096), (1, 8192), (1, 1536)])
+def test_gated_norms_of_many_rows(heads, width, gate_dtype, dtype):
+    """The norm that keeps a thread's values in registers (rows of 128 to 8,192 values; 1,536 go to the general kernels), the gate in
+    front and behind, a gain per column and per head, a gate that is part of wider rows, against float64."""
+    o_ = ops()
+    g = torch.Generator().manual_seed(width)
+    rows = -(-1030 // heads)
+    o, gate = torch.randn(rows, heads * width, generator=g) * 2, torch.randn(rows, heads * width + 8, generator=g).to(gate_dtype)
+    for first, per_column, kind in ((True, True, "silu"), (False, False, "sigmoid"), (False, True, "silu")):
+        gain = 1 + 0.1 * torch.randn(heads * width if per_column else width, generator=g)
+        out = torch.full((rows, heads * width), float("nan"), dtype=dtype, device=DEV)
+        o_.gated_head_norm(o.to(DEV), gate.to(DEV)[:, 8:], gain.to(DEV), 1e-5, 0.5, out, heads, width, kind, gate_first=first,
+                           gain_per_column=per_column)
+        z = gate[:, 8:].double().view(rows, heads, width)
+        act = torch.sigmoid(z) * (z if kind == "silu" else 1.0)
+        v = o.double().view(rows, heads, width) * (act if first else 1.0)
+        want = v / (v.square().mean(-1, keepdim=True) + 1e-5).sqrt() * gain.double().view(heads if per_column else 1, width)
+        want = (want * (1.0 if first else act) * 0.5).reshape(rows, -1)
+        close(out, want, dtype, f"{heads} x {width} first={first}")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("groups, width", [(2, 24), (1, 40), (3, 700), (5, 7)])
 def test_gate_in_front_of_a_norm_in_parts_and_a_gain_per_column(dtype, groups, width):
