@@ -329,8 +329,6 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(const __grid_constant
     __nv_bfloat16* Vs = Ks + C * LDK;                                       // [C][LDV]
     float* cl = reinterpret_cast<float*>(Vs + C * LDV);
     float* bs = cl + C;
-    pdl_wait();
-    pdl_trigger();
     int seg, t0;
     if (!find_chunk(a, blockIdx.x, seg, t0)) return;
     if (!jllm_in_bounds(a.state_slots[seg], a.num_slots, BOUNDS_SLOT)) return;
@@ -342,16 +340,21 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(const __grid_constant
     const int h0 = a.group0 * a.per_group, hg = h0 + group * a.per_group;
     Values<TS, SLAB> v;
     Gates<FIXED> gates;
-    auto fetch = [&](int i) {
+    auto fetch_state = [&](int i) {
         const Item it = item_of(a, group, i);
         const float4* src = a.ws + (((size_t)blockIdx.x * a.pass_heads + it.head) * a.slabs + it.slab) * STATE;
         uint4* dst = S0 + ((i - i0) & 1) * STATE;
 #pragma unroll
         for (int e = 0; e < STATE / 256; ++e) cp_async_16(dst + e * 256 + tid, src + e * 256 + tid);
+    };
+    auto fetch_values = [&](int i) {
+        const Item it = item_of(a, group, i);
         v.fetch(a, row0, nt, h0 + it.head, it.slab * SLAB);
         gates.fetch(a, row0, nt, h0 + it.head);
     };
-    fetch(i0);
+    // q, k, v and the gates were there before chunk_states began, whose end chunk_scan's blocks have waited for before they let this
+    // kernel in: only the states are waited for, and the rest overlaps chunk_scan.
+    fetch_values(i0);
     load_rows<TS, DK>(Qs, static_cast<const TS*>(a.q) + (size_t)row0 * a.ld_q + a.q_off + (size_t)(hg / a.q_share) * DK, a.ld_q, nt);
     load_rows<TS, DK>(Ks, static_cast<const TS*>(a.k) + (size_t)row0 * a.ld_k + a.k_off + (size_t)(hg / a.k_share) * DK, a.ld_k, nt);
     __syncthreads();
@@ -370,6 +373,9 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(const __grid_constant
                 mma_bf16(qk[j + 1], q, b[2], b[3]);
             }
     }
+    pdl_wait();
+    pdl_trigger();
+    fetch_state(i0);
     const size_t row_o = (size_t)a.heads * a.dv;
     const int tok0 = mt * 16 + g;
     for (int i = i0; i < i_end; ++i) {
@@ -380,7 +386,10 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(const __grid_constant
 #pragma unroll
         for (int u = 0; u < v.N; ++u) *reinterpret_cast<uint4*>(Vs + v.row(u) * LDV + v.col(u)) = v.piece[u];
         gates.put(cl, bs);
-        if (i + 1 < i_end) fetch(i + 1);
+        if (i + 1 < i_end) {
+            fetch_state(i + 1);
+            fetch_values(i + 1);
+        }
         // ---- q^T S0 ----
         const uint4* s0 = S0 + ((i - i0) & 1) * STATE + side * NT * 32 + lane;
         float acc[NT][4] = {};
