@@ -92,9 +92,10 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
 #pragma unroll
         for (int c = 0; c < NC; ++c) acc[h][c] = 0.f;
     }
+    // (Nothing is skipped: a chunk without a finite score has weights of 0, or of NaN where a score was NaN, and either goes on
+    // into the sums. Its maximum is -inf, from which no difference is taken.)
     auto merge = [&](int h, float t, float s, const float (&v)[NC]) {
-        if (t == -INFINITY) return;                     // a chunk of absent keys (the checked build skips bad pages)
-        const float m = fmaxf(top[h], t), old = expf(top[h] - m), add = expf(t - m);
+        const float m = fmaxf(top[h], t), from = m == -INFINITY ? 0.f : m, old = expf(top[h] - from), add = expf(t - from);
         top[h] = m;
         sum[h] = __fmaf_rn(s, add, __fmul_rn(sum[h], old));
 #pragma unroll
@@ -156,9 +157,10 @@ attention_plain_kernel(const T* __restrict__ q, int q_stride, const T* __restric
         for (int h = warp; h < HG; h += WARPS) {
             float t = -INFINITY, s = 0.f;
             for (int j = lane; j < n; j += 32) t = fmaxf(t, es[j * HG + h]);
-            t = warp_max(t);
+            t = warp_max(t);                            // (-inf: no score is above it, but some may be NaN)
+            const float from = t == -INFINITY ? 0.f : t;
             for (int j = lane; j < n; j += 32) {
-                const float e = t == -INFINITY ? 0.f : expf(es[j * HG + h] - t);
+                const float e = expf(es[j * HG + h] - from);
                 es[j * HG + h] = e;
                 s += e;
             }

@@ -84,3 +84,40 @@ def test_attention_of_shared_rows(ops, dtype, H, G, dk, dv, window, keep):
         # scores within about dk 2^-24 |q||k| scale, exponentials within a few 2^-24 of themselves, sums of 64 products
         tol = 2e-5 if dtype == torch.float32 else 2.0 ** -8
         assert float((full[i].double().view(H, dv) - want).abs().max()) <= tol * float(values.abs().max()), (s, p)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("copies", [1, 160])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_attention_keeps_what_is_not_a_number(ops, dtype, copies, with_sink):
+    """A row of 65 keys, so that key 64 is a chunk of its own, in a cluster's form (one row) and in a block's (160 rows): a key that is
+    NaN makes the row's heads NaN, a query head that is NaN itself alone (beside a sink too), and a key whose score is -inf only
+    drops out: the result is, bit for bit, that of a score far below the others."""
+    H, G, d, page, n = 4, 2, 64, 16, 65
+    k, v = rnd(5, G, page, d, seed=1).to(dtype), rnd(5, G, page, d, seed=2).to(dtype)
+    q = rnd(1, H * d, seed=3).abs().to(dtype)
+    table = torch.arange(5, dtype=torch.int32, device=DEV).view(1, 5)
+    seg, pos = torch.zeros(copies, dtype=torch.int32, device=DEV), torch.full((copies,), n - 1, dtype=torch.int32, device=DEV)
+    sink = rnd(H, seed=4) if with_sink else None
+
+    def run(q, k):
+        out = torch.full((copies, H * d), 7.0, dtype=dtype, device=DEV)
+        ops.attention_plain(q.expand(copies, -1).contiguous(), H * d, k, v, out, seg, pos, table, copies, H, G, d, page, 0, 0.125, sink=sink)
+        assert bool((out == out[:1]).all() or (out.isnan() == out[:1].isnan()).all())
+        return out[0].view(H, d)
+
+    whole = run(q, k)
+    assert bool(whole.isfinite().all())
+    bad = k.clone()
+    bad[4, 0, 0] = float("nan")                    # key 64 of the first kv head
+    got = run(q, bad)
+    assert bool(got[:2].isnan().all()) and torch.equal(got[2:], whole[2:])
+    bad[4, 0, 0], bad[4, 0, 0, 5] = k[4, 0, 0], float("-inf")
+    low = k.clone()
+    low[4, 0, 0] = -1e4
+    got, want = run(q, bad), run(q, low)
+    assert bool(want.isfinite().all()) and torch.equal(got, want)
+    bad_q = q.clone()
+    bad_q[0, d + 3] = float("nan")                 # the second head
+    got = run(bad_q, k)
+    assert bool(got[1].isnan().all()) and torch.equal(got[[0, 2, 3]], whole[[0, 2, 3]])
