@@ -582,6 +582,17 @@ int jllm_fixed_decay_chunks(const __nv_bfloat16* proj, int ld, int q_off, int k_
     return run_chunks<__nv_bfloat16, true>(a, rows, dk, workspace, workspace_floats, stream);
 }
 
+// Whether jllm_scalar_gated_chunked takes a shape: key heads of 64 or 128 channels, 16-byte aligned rows and pieces.
+JLLM_EXPORT int jllm_scalar_gated_chunks_fit(const void* q, int ld_q, int q_off, int q_groups, const void* k, int ld_k, int k_off,
+                                             int k_groups, const void* v, int ld_v, int v_off, int dtype, int heads, int dk, int dv) {
+    const int per = dtype == JLLM_F32 ? 4 : 8;          // values of a 16-byte piece
+    const bool aligned = ld_q % per == 0 && ld_k % per == 0 && ld_v % per == 0 && q_off % per == 0 && k_off % per == 0 &&
+                         v_off % per == 0 && dv % 8 == 0 && ((uintptr_t)q % 16) == 0 && ((uintptr_t)k % 16) == 0 &&
+                         ((uintptr_t)v % 16) == 0;
+    return (dk == 64 || dk == 128) && aligned && q_groups > 0 && k_groups > 0 && heads % q_groups == 0 && heads % k_groups == 0 &&
+           heads <= 65535;
+}
+
 // The recurrence with a decay and an input scale per token and head (`jllm_scalar_gated_recurrent`, which this stands in for
 // where a step holds prompt portions): key heads of 64 or 128 channels, no normalizer. q, k, v: views of type `dtype` (float32 or
 // bfloat16) with 16-byte aligned rows and pieces. Returns JLLM_UNSUPPORTED without launching where the shape is not taken (the caller
@@ -592,11 +603,8 @@ JLLM_EXPORT int jllm_scalar_gated_chunked(const void* q, int ld_q, int q_off, in
                                           const int* seg_start, const int* seg_len, const int* state_slots, float* o,
                                           int rows, int segments, int heads, int dk, int dv, float q_scale, float* workspace,
                                           long long workspace_floats, cudaStream_t stream) {
-    const int per = dtype == JLLM_F32 ? 4 : 8;          // values of a 16-byte piece
-    const bool aligned = ld_q % per == 0 && ld_k % per == 0 && ld_v % per == 0 && q_off % per == 0 && k_off % per == 0 &&
-                         v_off % per == 0 && dv % 8 == 0 && ((uintptr_t)q % 16) == 0 && ((uintptr_t)k % 16) == 0 &&
-                         ((uintptr_t)v % 16) == 0;
-    if (!(dk == 64 || dk == 128) || !aligned || heads % q_groups || heads % k_groups || heads > 65535) return JLLM_UNSUPPORTED;
+    if (!jllm_scalar_gated_chunks_fit(q, ld_q, q_off, q_groups, k, ld_k, k_off, k_groups, v, ld_v, v_off, dtype, heads, dk, dv))
+        return JLLM_UNSUPPORTED;
     if (segments == 0 || rows == 0) return JLLM_OK;
     ChunkArgs a{};
     a.q = q, a.k = k, a.v = v;

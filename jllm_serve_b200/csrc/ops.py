@@ -195,6 +195,7 @@ class _Signatures:
     jllm_causal_conv = [P, I, I, I, P, P, I, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P]
     jllm_scalar_gated_recurrent = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, P, I, P, P, I, P, P, P, P, I, I, I, I, F, P]
     jllm_scalar_gated_chunked = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I, F, P, ctypes.c_longlong, P]
+    jllm_scalar_gated_chunks_fit = [P, I, I, I, P, I, I, I, P, I, I, I, I, I, I]
     jllm_memory_values = [P, I, I, I, P, I, I, I, I, P]
     jllm_memory_divide = [P, P, P, I, I, I, I, P]
     jllm_sigmoid_gate = [P, I, P, I, I, I, I, F, P]
@@ -620,16 +621,17 @@ def scalar_gated_chunked(q, q_off, q_groups, k, k_off, k_groups, v, v_off, log_d
         return False
     assert q.dtype == k.dtype == v.dtype and q.stride(1) == k.stride(1) == v.stride(1) == 1
     assert state.dtype == out.dtype == torch.float32 and state.is_contiguous() and out.is_contiguous()
+    operands = (q.data_ptr(), q.stride(0), int(q_off), int(q_groups), k.data_ptr(), k.stride(0), int(k_off), int(k_groups),
+                v.data_ptr(), v.stride(0), int(v_off), _DT[q.dtype])
+    if not library().jllm_scalar_gated_chunks_fit(*operands, int(heads), int(key_dim), int(value_dim)):
+        return False
     fn = library().jllm_scalar_gated_chunked
     rows, segments = out.shape[0], batch.seg_start.numel()
     workspace, passes = _chunk_workspace(rows, segments, heads, q_groups if q_groups == k_groups else heads, key_dim, value_dim, out.device)
-    code = fn(q.data_ptr(), q.stride(0), int(q_off), int(q_groups), k.data_ptr(), k.stride(0), int(k_off), int(k_groups),
-              v.data_ptr(), v.stride(0), int(v_off), _DT[q.dtype], log_decay.data_ptr(), in_scale.data_ptr(), _p(skip),
+    code = fn(*operands, log_decay.data_ptr(), in_scale.data_ptr(), _p(skip),
               _DT[skip.dtype] if skip is not None else F32, state.data_ptr(), state.shape[0], batch.seg_start.data_ptr(),
               batch.seg_len.data_ptr(), batch.state_slots.data_ptr(), out.data_ptr(), rows, segments, int(heads),
               int(key_dim), int(value_dim), float(query_scale), workspace.data_ptr(), workspace.numel(), _stream())
-    if code == 3:        # the library's word for "this shape is not taken"
-        return False
     if code != 0:
         raise KernelError(f"jllm_scalar_gated_chunked failed ({code}): {library().jllm_last_error().decode(errors='replace')}")
     global launch_count

@@ -491,6 +491,20 @@ def test_chunks_whose_states_fill_the_workspace_more_than_once():
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
 
 
+def test_a_shape_the_chunks_do_not_take_costs_no_workspace():
+    """Values of 12 columns, and keys that begin off a 16-byte boundary: the call says no before any memory is asked for."""
+    o = ops()
+    H, dk, rows = 64, 128, 2048
+    buf = torch.zeros(rows, H * (2 * dk + 16), device=DEV)
+    gates, batch = torch.zeros(rows, H, device=DEV), FakeBatch([rows], [0])
+    for dv, k_off in ((12, H * dk), (8, H * dk + 2)):
+        state, out = torch.zeros(1, H, dk, dv, device=DEV), torch.empty(rows, H * dv, device=DEV)
+        torch.cuda.reset_peak_memory_stats()
+        before, launches = torch.cuda.memory_allocated(), o.launch_count
+        assert not o.scalar_gated_chunked(buf, 0, H, buf, k_off, H, buf, 2 * H * dk, gates, gates, state, batch, out, H, dk, dv)
+        assert torch.cuda.max_memory_allocated() == before and o.launch_count == launches
+
+
 @pytest.mark.parametrize("gate_dtype, dtype", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
 @pytest.mark.parametrize("heads, width", [(8, 128), (4, 256), (3, 512), (2, 1024), (1, 2048), (1, 4096), (1, 8192), (1, 1536)])
 def test_gated_norms_of_many_rows(heads, width, gate_dtype, dtype):
