@@ -9,6 +9,7 @@
 //     chunk_states   every chunk's own sum_s k_s (w_s v_s)^T                      (a block per chunk and some heads)
 //     chunk_scan     the states in front of every chunk, element by element       (a thread per four state values)
 //     chunk_out      every chunk's o from its q, k, v and the state in front      (a block per chunk and some heads)
+// Short segments have no chunks to run beside one another: a fourth kernel, chunk_walk, takes theirs one after the other.
 // An item is a head and a slab of 32 or 64 of its value columns. Heads whose q and k are the same (a group) share the chunk's q, k
 // and their product q k^T, which a warp keeps in registers. q, k and v are projections and enter as bfloat16 operands (float32 sources are rounded on their way
 // into shared memory); the float32 factors meet float32 values (the scores behind their product, the values in front of theirs,
@@ -25,6 +26,8 @@
 // themselves); 8 heads of 128 x 264: 112 and 60; 2,048 tokens, 16 heads of 128 x 128, one decay per head: 148 and 53.
 // It is mma.sync, not tcgen05: the products are 64 tokens high, the scores and the states are float32 values that become
 // operands by an elementwise step, and registers are where that step happens.
+#include <climits>
+
 #include "common.cuh"
 
 namespace {
@@ -98,30 +101,58 @@ struct ChunkArgs {
     float4* ws;                         // the chunks' states: [chunk][head of the pass][slab][DK / 16][SLAB / 8][32]
     float* ends;                        // [chunk][head of the pass]: exp(cl_n)
     int chunks;                         // room for so many chunks
+    int walked;                         // segments of so many chunks and fewer are left to chunk_walk (0: none)
     int group0, pass_heads;             // this pass covers the heads from group0 * per_group on
     int slabs, items;                   // slabs of a head; items a block takes
 };
 
+// the chunks of a segment; those that the three launches take care of
+__device__ __forceinline__ int all_chunks(const ChunkArgs& a, int seg) { return (a.seg_len[seg] + C - 1) / C; }
+__device__ __forceinline__ int scanned_chunks(const ChunkArgs& a, int seg) {
+    const int n = all_chunks(a, seg);
+    return n <= a.walked ? 0 : n;
+}
 // which chunk of which segment a block has; false past the last
 __device__ __forceinline__ bool find_chunk(const ChunkArgs& a, int chunk, int& seg, int& t0) {
     for (seg = 0; seg < a.segments; ++seg) {
-        const int n = (a.seg_len[seg] + C - 1) / C;
+        const int n = scanned_chunks(a, seg);
         if (chunk < n) { t0 = chunk * C; return true; }
         chunk -= n;
     }
     return false;
 }
 
-// 64 rows of DK values into shared memory, zeros from row nt on
+// `rows` (64) rows of DK values into shared memory, zeros from row nt on
 template <typename TS, int DK>
-__device__ __forceinline__ void load_rows(__nv_bfloat16* dst, const TS* src, int ld, int nt) {
+__device__ __forceinline__ void load_rows(__nv_bfloat16* dst, const TS* src, int ld, int nt, int rows = C) {
 #pragma unroll 4
-    for (int e = threadIdx.x; e < C * (DK / 8); e += 256) {
+    for (int e = threadIdx.x; e < rows * (DK / 8); e += 256) {
         const int row = e / (DK / 8), piece = e % (DK / 8);
         *reinterpret_cast<uint4*>(dst + row * (DK + 8) + piece * 8) =
             row < nt ? load8(src + (size_t)row * ld + piece * 8) : make_uint4(0, 0, 0, 0);
     }
 }
+
+// The same by way of registers: fetched while the rows before are still read
+template <typename TS, int DK>
+struct Rows {
+    static constexpr int N = C * (DK / 8) / 256;
+    uint4 piece[N];
+    __device__ __forceinline__ void fetch(const TS* src, int ld, int nt) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int e = threadIdx.x + u * 256, row = e / (DK / 8);
+            piece[u] = row < nt ? load8(src + (size_t)row * ld + e % (DK / 8) * 8) : make_uint4(0, 0, 0, 0);
+        }
+    }
+    __device__ __forceinline__ void put(__nv_bfloat16* dst) const {
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int e = threadIdx.x + u * 256;
+            *reinterpret_cast<uint4*>(dst + e / (DK / 8) * (DK + 8) + e % (DK / 8) * 8) = piece[u];
+        }
+    }
+};
 
 // An item's gates: cl [C] and bs [C] (not FIXED; zeros of bs past the chunk's end), or pw [C + 1] = d^0 .. d^C (FIXED, in the same
 // place). They are fetched an item ahead (`fetch`: the first warp, a lane two neighbouring tokens) and put in place by that warp.
@@ -183,6 +214,148 @@ __device__ __forceinline__ Item item_of(const ChunkArgs& a, int group, int i) {
 
 constexpr int GATES = 2 * C + 8;        // floats of an item's gates
 
+// An item's values times their weights towards the chunk's end, as two operands [C][LDV]
+template <typename TS, int SLAB, bool FIXED>
+__device__ __forceinline__ void weigh(const Values<TS, SLAB>& v, __nv_bfloat16* Vh, __nv_bfloat16* Vl, const float* cl, const float* bs,
+                                      int nt) {
+    constexpr int LDV = SLAB + 8;
+#pragma unroll
+    for (int u = 0; u < v.N; ++u) {
+        const int row = v.row(u);
+        const float w = row >= nt ? 0.f : FIXED ? cl[nt - 1 - row] : __fmul_rn(bs[row], expf(cl[nt - 1] - cl[row]));
+        const uint32_t in[4] = {v.piece[u].x, v.piece[u].y, v.piece[u].z, v.piece[u].w};
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&in[x]));
+            split2(f.x * w, f.y * w, hi[x], lo[x]);
+        }
+        *reinterpret_cast<uint4*>(Vh + row * LDV + v.col(u)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(Vl + row * LDV + v.col(u)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+// ... and U^T [value columns x key channels] = (w v)^T k over the chunk's first `rows` tokens: 16 value columns from mt * 16 on, NT
+// tiles of channels from tile part * NT on
+template <int DK, int SLAB, int NT>
+__device__ __forceinline__ void own_state(float (&acc)[NT][4], const __nv_bfloat16* Vh, const __nv_bfloat16* Vl, const __nv_bfloat16* Ks,
+                                          int mt, int part, int lane, int rows = C) {
+    constexpr int LDK = DK + 8, LDV = SLAB + 8;
+#pragma unroll
+    for (int k0 = 0; k0 < C; k0 += 16)
+        if (k0 < rows) {
+            uint32_t ah[4], al[4];
+            load_a_trans(ah, Vh, LDV, mt * 16, k0, lane);
+            load_a_trans(al, Vl, LDV, mt * 16, k0, lane);
+#pragma unroll
+            for (int j = 0; j < NT; j += 2) {
+                uint32_t b[4];
+                load_b2_trans(b, Ks, LDK, (part * NT + j) * 8, k0, lane);
+                mma_bf16(acc[j], ah, b[0], b[1]);
+                mma_bf16(acc[j + 1], ah, b[2], b[3]);
+                mma_bf16(acc[j], al, b[0], b[1]);
+                mma_bf16(acc[j + 1], al, b[2], b[3]);
+            }
+        }
+}
+
+// q k^T of 16 tokens (from mt * 16 on) and the keys up to the last of them
+template <int DK>
+__device__ __forceinline__ void own_scores(float (&qk)[8][4], const __nv_bfloat16* Qs, const __nv_bfloat16* Ks, int mt, int lane) {
+    constexpr int LDK = DK + 8;
+#pragma unroll 1
+    for (int k0 = 0; k0 < DK; k0 += 16) {
+        uint32_t q[4];
+        load_a(q, Qs, LDK, mt * 16, k0, lane);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2)
+            if (j <= 2 * mt) {
+                uint32_t b[4];
+                load_b2(b, Ks, LDK, j * 8, k0, lane);
+                mma_bf16(qk[j], q, b[0], b[1]);
+                mma_bf16(qk[j + 1], q, b[2], b[3]);
+            }
+    }
+}
+// acc = q^T S0 of those tokens and the first `live` of NT tiles of value columns; `s0`: the lane's operands of the first
+template <int DK, int NT>
+__device__ __forceinline__ void from_state(float (&acc)[NT][4], const __nv_bfloat16* Qs, const uint4* s0, int live, int mt, int lane) {
+    constexpr int LDK = DK + 8;
+#pragma unroll 2
+    for (int kt = 0; kt < DK / 16; ++kt) {
+        uint32_t q[4];
+        load_a(q, Qs, LDK, mt * 16, kt * 16, lane);
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+            if (j < live) {
+                const uint4 x = s0[(kt * 2 * NT + j) * 32];
+                mma_bf16(acc[j], q, x.x, x.y);
+                mma_bf16(acc[j], q, x.z, x.w);
+            }
+    }
+}
+// o = exp(cl_t) s acc + P v [+ D v]; `c0`: the first of the warp's value columns, `at`: its place in the slab, dst0: o of row 0
+template <int SLAB, bool FIXED, int NT>
+__device__ __forceinline__ void finish(const ChunkArgs& a, float (&acc)[NT][4], const float (&qk)[8][4], const __nv_bfloat16* Vs,
+                                       const float* cl, const float* bs, int h, int c0, int at, int live, int row0, int nt, int mt, int lane) {
+    constexpr int LDV = SLAB + 8;
+    const int g = lane >> 2, t = lane & 3, tok0 = mt * 16 + g;
+    const size_t row_o = (size_t)a.heads * a.dv;
+    const float f0 = __fmul_rn(FIXED ? cl[tok0 + 1] : expf(cl[tok0]), a.q_scale);
+    const float f1 = __fmul_rn(FIXED ? cl[tok0 + 9] : expf(cl[tok0 + 8]), a.q_scale);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        acc[j][0] = __fmul_rn(acc[j][0], f0), acc[j][1] = __fmul_rn(acc[j][1], f0);
+        acc[j][2] = __fmul_rn(acc[j][2], f1), acc[j][3] = __fmul_rn(acc[j][3], f1);
+    }
+    // the accumulators of q k^T, weighted, are the A operand as they lie
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+        if (kk <= mt) {
+            uint32_t ph[4], pl[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {                     // rows g, g + 8; keys 2t and 2t + 8 of the sixteen
+                const int j = 2 * kk + (x >> 1), tok = tok0 + (x & 1) * 8, key = j * 8 + 2 * t;
+                float w0, w1;
+                if constexpr (FIXED) {
+                    w0 = cl[max(tok - key, 0)], w1 = cl[max(tok - key - 1, 0)];
+                } else {
+                    const float ct = cl[tok];
+                    w0 = __fmul_rn(expf(ct - cl[key]), bs[key]), w1 = __fmul_rn(expf(ct - cl[key + 1]), bs[key + 1]);
+                }
+                const float p0 = key <= tok ? __fmul_rn(__fmul_rn(qk[j][2 * (x & 1)], a.q_scale), w0) : 0.f;
+                const float p1 = key + 1 <= tok ? __fmul_rn(__fmul_rn(qk[j][2 * (x & 1) + 1], a.q_scale), w1) : 0.f;
+                split2(p0, p1, ph[x], pl[x]);
+            }
+#pragma unroll
+            for (int j = 0; j < NT; j += 2) {
+                uint32_t b[4];
+                load_b2_trans(b, Vs, LDV, at + j * 8, kk * 16, lane);
+                mma_bf16(acc[j], ph, b[0], b[1]);
+                mma_bf16(acc[j + 1], ph, b[2], b[3]);
+                mma_bf16(acc[j], pl, b[0], b[1]);
+                mma_bf16(acc[j + 1], pl, b[2], b[3]);
+            }
+        }
+    const float d_skip = a.has_skip ? a.skip[h] : 0.f;
+#pragma unroll
+    for (int below = 0; below < 2; ++below) {
+        const int tok = tok0 + below * 8;
+        if (tok < nt) {
+            float* dst = a.o + (size_t)(row0 + tok) * row_o + (size_t)h * a.dv + c0 + 2 * t;
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+                if (j < live) {
+                    float2 r = make_float2(acc[j][2 * below], acc[j][2 * below + 1]);
+                    if (a.has_skip) {
+                        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Vs + tok * LDV + at + j * 8 + 2 * t));
+                        r.x = fmaf(d_skip, x.x, r.x), r.y = fmaf(d_skip, x.y, r.y);
+                    }
+                    *reinterpret_cast<float2*>(dst + j * 8) = r;
+                }
+        }
+    }
+}
+
 // ---- every chunk's own part of the state: U^T [value columns x key channels] = (w v)^T k ----
 template <typename TS, int DK, int SLAB, bool FIXED>
 __global__ void __launch_bounds__(256, 2) chunk_states_kernel(const __grid_constant__ ChunkArgs a) {
@@ -221,41 +394,14 @@ __global__ void __launch_bounds__(256, 2) chunk_states_kernel(const __grid_const
         const int c0 = it.slab * SLAB;
         gates.put(cl, bs);
         __syncthreads();
-#pragma unroll
-        for (int u = 0; u < v.N; ++u) {
-            const int row = v.row(u);
-            const float w = row >= nt ? 0.f : FIXED ? cl[nt - 1 - row] : __fmul_rn(bs[row], expf(cl[nt - 1] - cl[row]));
-            const uint32_t in[4] = {v.piece[u].x, v.piece[u].y, v.piece[u].z, v.piece[u].w};
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&in[x]));
-                split2(f.x * w, f.y * w, hi[x], lo[x]);
-            }
-            *reinterpret_cast<uint4*>(Vh + row * LDV + v.col(u)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(Vl + row * LDV + v.col(u)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        }
+        weigh<TS, SLAB, FIXED>(v, Vh, Vl, cl, bs, nt);
         const size_t place = (size_t)blockIdx.x * a.pass_heads + it.head;
         if (it.slab == 0 && threadIdx.x == 0) a.ends[place] = FIXED ? cl[nt] : expf(cl[nt - 1]);
         if (i + 1 < i_end) fetch(i + 1);
         __syncthreads();
         if (c0 + mt * 16 < a.dv) {
             float acc[NT][4] = {};
-#pragma unroll
-            for (int k0 = 0; k0 < C; k0 += 16) {
-                uint32_t ah[4], al[4];
-                load_a_trans(ah, Vh, LDV, mt * 16, k0, lane);
-                load_a_trans(al, Vl, LDV, mt * 16, k0, lane);
-#pragma unroll
-                for (int j = 0; j < NT; j += 2) {
-                    uint32_t b[4];
-                    load_b2_trans(b, Ks, LDK, (part * NT + j) * 8, k0, lane);
-                    mma_bf16(acc[j], ah, b[0], b[1]);
-                    mma_bf16(acc[j + 1], ah, b[2], b[3]);
-                    mma_bf16(acc[j], al, b[0], b[1]);
-                    mma_bf16(acc[j + 1], al, b[2], b[3]);
-                }
-            }
+            own_state<DK, SLAB, NT>(acc, Vh, Vl, Ks, mt, part, lane);
             float4* dst = a.ws + ((place * a.slabs + it.slab) * (DK / 16) + part * (NT / 2)) * (SLAB / 8) * 32 + mt * 64 + lane;
 #pragma unroll
             for (int j = 0; j < NT; j += 2) {
@@ -274,7 +420,7 @@ __global__ void __launch_bounds__(256) chunk_scan_kernel(const __grid_constant__
     pdl_wait();
     pdl_trigger();
     const int seg = blockIdx.y, per_head = a.slabs * (DK / 16) * (SLAB / 8) * 32;
-    const int n = (a.seg_len[seg] + C - 1) / C, slot = a.state_slots[seg];
+    const int n = scanned_chunks(a, seg), slot = a.state_slots[seg];
     if (n == 0 || !jllm_in_bounds(slot, a.num_slots, BOUNDS_SLOT)) return;
     const long long e = (long long)blockIdx.x * 256 + threadIdx.x;
     if (e >= (long long)a.pass_heads * per_head) return;
@@ -283,7 +429,7 @@ __global__ void __launch_bounds__(256) chunk_scan_kernel(const __grid_constant__
     const int col = slab * SLAB + nt * 8 + (lane >> 2), ch = kt * 16 + 2 * (lane & 3);
     if (slab * SLAB + nt * 8 >= a.dv) return;
     int first = 0;
-    for (int s = 0; s < seg; ++s) first += (a.seg_len[s] + C - 1) / C;
+    for (int s = 0; s < seg; ++s) first += scanned_chunks(a, s);
     float* S = a.state + (((size_t)slot * a.heads + a.group0 * a.per_group + head) * DK + ch) * a.dv + col;
     float s[4] = {S[0], S[a.dv], S[8 * (size_t)a.dv], S[9 * (size_t)a.dv]};
     float4* u = a.ws + (size_t)first * a.pass_heads * per_head + e;
@@ -336,7 +482,7 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(const __grid_constant
     const int group = blockIdx.y / blocks_per_group, i0 = blockIdx.y % blocks_per_group * a.items;
     const int i_end = min(i0 + a.items, a.per_group * a.slabs);
     const int row0 = a.seg_start[seg] + t0, nt = min(C, a.seg_len[seg] - t0);
-    const int tid = threadIdx.x, side = tid >> 7, mt = (tid >> 5) & 3, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, side = tid >> 7, mt = (tid >> 5) & 3, lane = tid & 31;
     const int h0 = a.group0 * a.per_group, hg = h0 + group * a.per_group;
     Values<TS, SLAB> v;
     Gates<FIXED> gates;
@@ -358,26 +504,11 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(const __grid_constant
     load_rows<TS, DK>(Qs, static_cast<const TS*>(a.q) + (size_t)row0 * a.ld_q + a.q_off + (size_t)(hg / a.q_share) * DK, a.ld_q, nt);
     load_rows<TS, DK>(Ks, static_cast<const TS*>(a.k) + (size_t)row0 * a.ld_k + a.k_off + (size_t)(hg / a.k_share) * DK, a.ld_k, nt);
     __syncthreads();
-    // q k^T of the warp's 16 tokens and the keys up to its last one
     float qk[8][4] = {};
-#pragma unroll 1
-    for (int k0 = 0; k0 < DK; k0 += 16) {
-        uint32_t q[4];
-        load_a(q, Qs, LDK, mt * 16, k0, lane);
-#pragma unroll
-        for (int j = 0; j < 8; j += 2)
-            if (j <= 2 * mt) {
-                uint32_t b[4];
-                load_b2(b, Ks, LDK, j * 8, k0, lane);
-                mma_bf16(qk[j], q, b[0], b[1]);
-                mma_bf16(qk[j + 1], q, b[2], b[3]);
-            }
-    }
+    own_scores<DK>(qk, Qs, Ks, mt, lane);
     pdl_wait();
     pdl_trigger();
     fetch_state(i0);
-    const size_t row_o = (size_t)a.heads * a.dv;
-    const int tok0 = mt * 16 + g;
     for (int i = i0; i < i_end; ++i) {
         const Item it = item_of(a, group, i);
         const int h = h0 + it.head, c0 = it.slab * SLAB + side * NT * 8, live = min(NT, (a.dv - c0 + 7) / 8);     // (live <= 0: no column)
@@ -390,79 +521,107 @@ __global__ void __launch_bounds__(256, 2) chunk_out_kernel(const __grid_constant
             fetch_state(i + 1);
             fetch_values(i + 1);
         }
-        // ---- q^T S0 ----
-        const uint4* s0 = S0 + ((i - i0) & 1) * STATE + side * NT * 32 + lane;
         float acc[NT][4] = {};
-#pragma unroll 2
-        for (int kt = 0; kt < DK / 16; ++kt) {
-            uint32_t q[4];
-            load_a(q, Qs, LDK, mt * 16, kt * 16, lane);
-#pragma unroll
-            for (int j = 0; j < NT; ++j)
-                if (j < live) {
-                    const uint4 x = s0[(kt * 2 * NT + j) * 32];
-                    mma_bf16(acc[j], q, x.x, x.y);
-                    mma_bf16(acc[j], q, x.z, x.w);
-                }
-        }
+        from_state<DK, NT>(acc, Qs, S0 + ((i - i0) & 1) * STATE + side * NT * 32 + lane, live, mt, lane);
         __syncthreads();       // values and gates are in place
-        // ---- ... times exp(cl_t) s ----
-        const float f0 = __fmul_rn(FIXED ? cl[tok0 + 1] : expf(cl[tok0]), a.q_scale);
-        const float f1 = __fmul_rn(FIXED ? cl[tok0 + 9] : expf(cl[tok0 + 8]), a.q_scale);
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            acc[j][0] = __fmul_rn(acc[j][0], f0), acc[j][1] = __fmul_rn(acc[j][1], f0);
-            acc[j][2] = __fmul_rn(acc[j][2], f1), acc[j][3] = __fmul_rn(acc[j][3], f1);
-        }
-        // ---- ... + P v: the accumulators of q k^T, weighted, are the A operand as they lie ----
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-            if (kk <= mt) {
-                uint32_t ph[4], pl[4];
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {                     // rows g, g + 8; keys 2t and 2t + 8 of the sixteen
-                    const int j = 2 * kk + (x >> 1), tok = tok0 + (x & 1) * 8, key = j * 8 + 2 * t;
-                    float w0, w1;
-                    if constexpr (FIXED) {
-                        w0 = cl[max(tok - key, 0)], w1 = cl[max(tok - key - 1, 0)];
-                    } else {
-                        const float ct = cl[tok];
-                        w0 = __fmul_rn(expf(ct - cl[key]), bs[key]), w1 = __fmul_rn(expf(ct - cl[key + 1]), bs[key + 1]);
-                    }
-                    const float p0 = key <= tok ? __fmul_rn(__fmul_rn(qk[j][2 * (x & 1)], a.q_scale), w0) : 0.f;
-                    const float p1 = key + 1 <= tok ? __fmul_rn(__fmul_rn(qk[j][2 * (x & 1) + 1], a.q_scale), w1) : 0.f;
-                    split2(p0, p1, ph[x], pl[x]);
-                }
-#pragma unroll
-                for (int j = 0; j < NT; j += 2) {
-                    uint32_t b[4];
-                    load_b2_trans(b, Vs, LDV, (side * NT + j) * 8, kk * 16, lane);
-                    mma_bf16(acc[j], ph, b[0], b[1]);
-                    mma_bf16(acc[j + 1], ph, b[2], b[3]);
-                    mma_bf16(acc[j], pl, b[0], b[1]);
-                    mma_bf16(acc[j + 1], pl, b[2], b[3]);
-                }
-            }
-        const float d_skip = a.has_skip ? a.skip[h] : 0.f;
-#pragma unroll
-        for (int below = 0; below < 2; ++below) {
-            const int tok = tok0 + below * 8;
-            if (tok < nt) {
-                float* dst = a.o + (size_t)(row0 + tok) * row_o + (size_t)h * a.dv + c0 + 2 * t;
-#pragma unroll
-                for (int j = 0; j < NT; ++j)
-                    if (j < live) {
-                        float2 r = make_float2(acc[j][2 * below], acc[j][2 * below + 1]);
-                        if (a.has_skip) {
-                            const float2 x = __bfloat1622float2(
-                                *reinterpret_cast<const __nv_bfloat162*>(Vs + tok * LDV + (side * NT + j) * 8 + 2 * t));
-                            r.x = fmaf(d_skip, x.x, r.x), r.y = fmaf(d_skip, x.y, r.y);
-                        }
-                        *reinterpret_cast<float2*>(dst + j * 8) = r;
-                    }
-            }
-        }
+        finish<SLAB, FIXED, NT>(a, acc, qk, Vs, cl, bs, h, c0, side * NT * 8, live, row0, nt, mt, lane);
     }
+}
+
+// ---- short segments: a block walks the chunks of one (segment, head, slab), the state in its registers ----
+// A segment of a chunk or two has no chunks to run beside one another, and the way of its states through the workspace and two more
+// launches are what it would wait for. The pieces and their order are those of the three kernels: the results have the same bits.
+template <typename TS, int DK, int SLAB, bool FIXED>
+__global__ void __launch_bounds__(256, 2) chunk_walk_kernel(const __grid_constant__ ChunkArgs a) {
+    constexpr int LDK = DK + 8, LDV = SLAB + 8, STATE = DK * SLAB / 4;
+    constexpr int MT = SLAB / 16, PARTS = 8 / MT, NS = DK / 8 / PARTS, NT = SLAB / 16;
+    extern __shared__ __align__(16) unsigned char chunk_smem[];
+    uint4* S0 = reinterpret_cast<uint4*>(chunk_smem);
+    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(S0 + STATE);
+    __nv_bfloat16 *Ks = Qs + C * LDK, *Vs = Ks + C * LDK, *Vh = Vs + C * LDV, *Vl = Vh + C * LDV;
+    float *cl = reinterpret_cast<float*>(Vl + C * LDV), *bs = cl + C;
+    const int seg = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * SLAB, chunks = all_chunks(a, seg), slot = a.state_slots[seg];
+    pdl_wait();
+    pdl_trigger();
+    if (chunks == 0 || chunks > a.walked) return;
+    if (!jllm_in_bounds(slot, a.num_slots, BOUNDS_SLOT)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int first = a.seg_start[seg], n = a.seg_len[seg];
+    const int smt = warp % MT, part = warp / MT;                // the state: 16 value columns, NS tiles of channels
+    const int side = warp >> 2, mt = warp & 3;                  // the results: half of the columns, 16 tokens
+    const int col0 = c0 + side * NT * 8, live = min(NT, (a.dv - col0 + 7) / 8);
+    Values<TS, SLAB> v;
+    Gates<FIXED> gates;
+    v.fetch(a, first, min(C, n), h, c0);
+    gates.fetch(a, first, min(C, n), h);
+    // (channels of 64: the next chunk's q and k wait in registers; of 128 they do not fit, and other blocks hide the way)
+    constexpr bool AHEAD = DK == 64;
+    auto q_from = [&](int row) { return static_cast<const TS*>(a.q) + (size_t)row * a.ld_q + a.q_off + (size_t)(h / a.q_share) * DK; };
+    auto k_from = [&](int row) { return static_cast<const TS*>(a.k) + (size_t)row * a.ld_k + a.k_off + (size_t)(h / a.k_share) * DK; };
+    Rows<TS, DK> qr, kr;
+    if constexpr (AHEAD) {
+        qr.fetch(q_from(first), a.ld_q, min(C, n));
+        kr.fetch(k_from(first), a.ld_k, min(C, n));
+    }
+    float* S = a.state + (((size_t)slot * a.heads + h) * DK + part * (NS * 8) + 2 * t) * a.dv + c0 + smt * 16 + g;
+    float s[NS][4];
+#pragma unroll
+    for (int j = 0; j < NS; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            s[j][e] = c0 + smt * 16 + (e >> 1) * 8 < a.dv ? S[(size_t)(j * 8 + (e & 1)) * a.dv + (e >> 1) * 8] : 0.f;
+    for (int t0 = 0; t0 < n; t0 += C) {
+        const int row0 = first + t0, nt = min(C, n - t0), rows = (nt + 15) / 16 * 16;
+        if (t0 > 0) __syncthreads();       // nobody reads the chunk before any more
+        if constexpr (AHEAD) {
+            qr.put(Qs);
+            kr.put(Ks);
+        } else {
+            load_rows<TS, DK>(Qs, q_from(row0), a.ld_q, nt, rows);
+            load_rows<TS, DK>(Ks, k_from(row0), a.ld_k, nt, rows);
+        }
+        gates.put(cl, bs);
+#pragma unroll
+        for (int u = 0; u < v.N; ++u) *reinterpret_cast<uint4*>(Vs + v.row(u) * LDV + v.col(u)) = v.piece[u];
+#pragma unroll
+        for (int j = 0; j < NS; j += 2)
+#pragma unroll
+            for (int below = 0; below < 2; ++below) {
+                uint4 p;
+                split2(s[j][2 * below], s[j][2 * below + 1], p.x, p.z);
+                split2(s[j + 1][2 * below], s[j + 1][2 * below + 1], p.y, p.w);
+                S0[((part * (NS / 2) + j / 2) * (SLAB / 8) + smt * 2 + below) * 32 + lane] = p;
+            }
+        __syncthreads();
+        weigh<TS, SLAB, FIXED>(v, Vh, Vl, cl, bs, nt);
+        if (t0 + C < n) {
+            v.fetch(a, row0 + C, min(C, n - t0 - C), h, c0);
+            gates.fetch(a, row0 + C, min(C, n - t0 - C), h);
+            if constexpr (AHEAD) {
+                qr.fetch(q_from(row0 + C), a.ld_q, min(C, n - t0 - C));
+                kr.fetch(k_from(row0 + C), a.ld_k, min(C, n - t0 - C));
+            }
+        }
+        if (mt * 16 < nt) {
+            float qk[8][4] = {}, acc[NT][4] = {};
+            own_scores<DK>(qk, Qs, Ks, mt, lane);
+            from_state<DK, NT>(acc, Qs, S0 + side * NT * 32 + lane, live, mt, lane);
+            finish<SLAB, FIXED, NT>(a, acc, qk, Vs, cl, bs, h, col0, side * NT * 8, live, row0, nt, mt, lane);
+        }
+        __syncthreads();                   // the weighted values are in place
+        float own[NS][4] = {};
+        own_state<DK, SLAB, NS>(own, Vh, Vl, Ks, smt, part, lane, rows);
+        const float d = FIXED ? cl[nt] : expf(cl[nt - 1]);
+#pragma unroll
+        for (int j = 0; j < NS; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[j][e] = __fadd_rn(__fmul_rn(s[j][e], d), own[j][e]);
+    }
+#pragma unroll
+    for (int j = 0; j < NS; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (c0 + smt * 16 + (e >> 1) * 8 < a.dv) S[(size_t)(j * 8 + (e & 1)) * a.dv + (e >> 1) * 8] = s[j][e];
 }
 
 // A test's switch: the value columns of an item (32 or 64; 0: chosen from the shape).
@@ -474,15 +633,43 @@ int g_slab = 0;
 // product) costs about 0.7 of an item; the number of rounds times their length is least. Where all heads' states do not fit the
 // workspace, a pass takes as many groups as do.
 struct Cut {
+    int walked, walk_slab;       // segments of so many chunks and fewer are walked, in slabs of so many columns
     int slab, slabs, chunks, items, pass_groups;
-    long long floats;
+    long long floats;            // 0: every segment is walked
+    int launches;
 };
 constexpr long long WORKSPACE_FLOATS = 64ll << 20;      // 256 MB: 2,048 tokens of 64 heads with states of 128 x 64 take a quarter
 
-Cut cut_of(int rows, int segments, int heads, int groups, int dk, int dv) {
+// All segments are walked where that takes no longer than the three launches: a walked chunk takes as long as its block's chain (3.5 to
+// 5 us), once more for every block beyond the first on an SM; the three launches take about two such chunks and 0.0095 for a chunk of
+// one head and 64 value columns. Launched back to back, 64 heads with states of 128 x 64: one segment of 64 tokens 7 us walked and 16 in
+// three launches, of 256 tokens 23 and 28, of 512 43 and 35; eight of 512 160 and 206. 16 fixed-decay heads of 128 x 128: one of 64
+// tokens 6 and 12, of 192 14 and 13, of 512 35 and 20; eight of 512 71 and 101. Where the longer segments take the three launches, those
+// of up to two chunks are walked all the same: their states would go the long way (32 single tokens beside a portion of 512, 64
+// heads of 128 x 64: 179 us in three launches, 115 with the single ones walked).
+constexpr int WALKED = 2, WALKED_MOST = 12;      // (no more chunks than measured)
+bool walks_all(int rows, int segments, int longest, int heads, int dv, int sms) {
+    const long long pairs = (long long)segments * heads, wide = pairs * ((dv + 63) / 64);
+    const bool narrow = wide < sms;
+    const double rounds = (double)(((narrow ? pairs * ((dv + 31) / 32) : wide) + sms - 1) / sms) * (narrow ? 0.9 : 1.);
+    const double chunks = (double)((rows + 32ll * segments) / C);          // (a segment's last chunk is half full)
+    return longest <= WALKED_MOST * C && (longest + C - 1) / C * (rounds > 1. ? rounds : 1.) < 2. + 0.0095 * chunks * heads * (dv / 64.);
+}
+
+// `longest`: the rows of the longest segment
+Cut cut_of(int rows, int segments, int longest, int heads, int groups, int dk, int dv) {
     const int sms = jllm_device_sm_count() > 0 ? jllm_device_sm_count() : 148;
-    Cut c;
-    c.chunks = rows / C + segments;
+    Cut c{};
+    longest = longest > rows ? rows : longest;
+    const bool scans = longest > WALKED * C && !walks_all(rows, segments, longest, heads, dv, sms);
+    if (!scans || segments > 1) {
+        c.walked = scans ? WALKED : INT_MAX;
+        c.walk_slab = g_slab ? g_slab : (dv <= 32 || (long long)segments * heads * ((dv + 63) / 64) < sms ? 32 : 64);
+        c.launches = 1;
+    }
+    if (!scans) return c;
+    const int longs = rows / (c.walked * C + 1);                 // no more segments than that are longer
+    c.chunks = rows / C + (longs < segments ? longs : segments);
     const int per_group = heads / groups;
     c.slab = g_slab ? g_slab : (dv <= 32 || (long long)c.chunks * heads * ((dv + 63) / 64) < 4ll * sms ? 32 : 64);
     c.slabs = (dv + c.slab - 1) / c.slab;
@@ -497,7 +684,18 @@ Cut cut_of(int rows, int segments, int heads, int groups, int dk, int dv) {
     c.pass_groups = (int)(WORKSPACE_FLOATS / group_floats);
     c.pass_groups = c.pass_groups < 1 ? 1 : c.pass_groups > groups ? groups : c.pass_groups;
     c.floats = group_floats * c.pass_groups;
+    c.launches += 3 * ((groups + c.pass_groups - 1) / c.pass_groups);
     return c;
+}
+
+template <typename TS, int DK, int SLAB, bool FIXED>
+int run_walk(const ChunkArgs& a, cudaStream_t stream) {
+    constexpr size_t smem = (size_t)DK * SLAB * 4 + 2 * (size_t)C * (DK + 8) * 2 + 3 * (size_t)C * (SLAB + 8) * 2 + GATES * sizeof(float);
+    if (cudaFuncSetAttribute(chunk_walk_kernel<TS, DK, SLAB, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return jllm_fail(JLLM_CUDA_ERROR, "chunk_walk: %zu bytes of shared memory refused", smem);
+    jllm_launch(chunk_walk_kernel<TS, DK, SLAB, FIXED>, dim3(a.segments, a.heads, (a.dv + SLAB - 1) / SLAB), dim3(256), smem, stream,
+                LAUNCH_DEPENDENT, a);
+    return jllm_check_launch("chunk_walk");
 }
 
 template <typename TS, int DK, int SLAB, bool FIXED>
@@ -530,13 +728,19 @@ int run_passes(ChunkArgs a, const Cut& c, float* workspace, cudaStream_t stream)
 }
 
 template <typename TS, bool FIXED>
-int run_chunks(ChunkArgs a, int rows, int dk, float* workspace, long long workspace_floats, cudaStream_t stream) {
-    const Cut c = cut_of(rows, a.segments, a.heads, a.groups, dk, a.dv);
-    JLLM_REQUIRE(workspace != nullptr && workspace_floats >= c.floats && ((uintptr_t)workspace % 16) == 0,
+int run_chunks(ChunkArgs a, int rows, int longest, int dk, float* workspace, long long workspace_floats, cudaStream_t stream) {
+    const Cut c = cut_of(rows, a.segments, longest, a.heads, a.groups, dk, a.dv);
+    JLLM_REQUIRE(c.floats == 0 || (workspace != nullptr && workspace_floats >= c.floats && ((uintptr_t)workspace % 16) == 0),
                  "chunk_scan: a workspace of %lld floats where %lld are needed (16-byte aligned)", workspace_floats, c.floats);
-    JLLM_REQUIRE((long long)a.groups * ((a.per_group * c.slabs + c.items - 1) / c.items) <= 65535 && a.segments <= 65535,
+    JLLM_REQUIRE(c.floats == 0 || ((long long)a.groups * ((a.per_group * c.slabs + c.items - 1) / c.items) <= 65535 && a.segments <= 65535),
                  "chunk_scan: %d heads in %d segments are too many blocks", a.heads, a.segments);
-    a.chunks = c.chunks, a.slabs = c.slabs, a.items = c.items;
+    a.chunks = c.chunks, a.walked = c.walked, a.slabs = c.slabs, a.items = c.items;
+    if (c.walked) {
+        const bool wide = c.walk_slab == 64;
+        const int code = dk == 64 ? (wide ? run_walk<TS, 64, 64, FIXED>(a, stream) : run_walk<TS, 64, 32, FIXED>(a, stream))
+                                  : (wide ? run_walk<TS, 128, 64, FIXED>(a, stream) : run_walk<TS, 128, 32, FIXED>(a, stream));
+        if (code || c.floats == 0) return code;
+    }
     if (dk == 64) return c.slab == 64 ? run_passes<TS, 64, 64, FIXED>(a, c, workspace, stream) : run_passes<TS, 64, 32, FIXED>(a, c, workspace, stream);
     return c.slab == 64 ? run_passes<TS, 128, 64, FIXED>(a, c, workspace, stream) : run_passes<TS, 128, 32, FIXED>(a, c, workspace, stream);
 }
@@ -551,24 +755,28 @@ JLLM_EXPORT int jllm_lightning_block_width(int width) {
     return JLLM_OK;
 }
 
-// floats that the chunks of a step's states need (heads in `groups` that share q and k)
-JLLM_EXPORT long long jllm_chunk_workspace(int rows, int segments, int heads, int groups, int dk, int dv) {
+// What a step's chunks take: the launches; `floats`: the workspace (0: none). Heads in `groups` that share q and k, the longest segment
+// of `longest` rows.
+JLLM_EXPORT int jllm_chunk_plan(int rows, int segments, int longest, int heads, int groups, int dk, int dv, long long* floats) {
+    *floats = 0;
     if (rows <= 0 || segments <= 0 || heads <= 0 || groups <= 0 || heads % groups || dk <= 0 || dv <= 0) return 0;
-    return cut_of(rows, segments, heads, groups, dk, dv).floats;
+    const Cut c = cut_of(rows, segments, longest, heads, groups, dk, dv);
+    *floats = c.floats;
+    return c.launches;
 }
 
-// ... and the passes over the heads it makes in them
+// ... and the passes over the heads that segments of any length make in it
 JLLM_EXPORT int jllm_chunk_passes(int rows, int segments, int heads, int groups, int dk, int dv) {
     if (rows <= 0 || segments <= 0 || heads <= 0 || groups <= 0 || heads % groups || dk <= 0 || dv <= 0) return 0;
-    const int at_once = cut_of(rows, segments, heads, groups, dk, dv).pass_groups;
-    return (groups + at_once - 1) / at_once;
+    const int at_once = cut_of(rows, segments, rows, heads, groups, dk, dv).pass_groups;
+    return at_once ? (groups + at_once - 1) / at_once : 0;
 }
 
 // one fixed decay per head, q, k, v pieces of one bfloat16 matrix (called by jllm_gla_chunked)
 int jllm_fixed_decay_chunks(const __nv_bfloat16* proj, int ld, int q_off, int k_off, int v_off, const float* head_decay, float* state,
                             int num_slots, const int* seg_start, const int* seg_len, const int* state_slots, float* o, int rows,
-                            int segments, int heads, int dk, int dv, float q_scale, float* workspace, long long workspace_floats,
-                            cudaStream_t stream) {
+                            int segments, int longest, int heads, int dk, int dv, float q_scale, float* workspace,
+                            long long workspace_floats, cudaStream_t stream) {
     ChunkArgs a{};
     a.q = a.k = a.v = proj;
     a.ld_q = a.ld_k = a.ld_v = ld;
@@ -579,7 +787,7 @@ int jllm_fixed_decay_chunks(const __nv_bfloat16* proj, int ld, int q_off, int k_
     a.state = state, a.num_slots = num_slots;
     a.seg_start = seg_start, a.seg_len = seg_len, a.state_slots = state_slots;
     a.o = o, a.segments = segments, a.heads = heads, a.dv = dv, a.q_scale = q_scale;
-    return run_chunks<__nv_bfloat16, true>(a, rows, dk, workspace, workspace_floats, stream);
+    return run_chunks<__nv_bfloat16, true>(a, rows, longest, dk, workspace, workspace_floats, stream);
 }
 
 // Whether jllm_scalar_gated_chunked takes a shape: key heads of 64 or 128 channels, 16-byte aligned rows and pieces.
@@ -594,15 +802,16 @@ JLLM_EXPORT int jllm_scalar_gated_chunks_fit(const void* q, int ld_q, int q_off,
 }
 
 // The recurrence with a decay and an input scale per token and head (`jllm_scalar_gated_recurrent`, which this stands in for
-// where a step holds prompt portions): key heads of 64 or 128 channels, no normalizer. q, k, v: views of type `dtype` (float32 or
-// bfloat16) with 16-byte aligned rows and pieces. Returns JLLM_UNSUPPORTED without launching where the shape is not taken (the caller
-// then runs token by token). `workspace`: jllm_chunk_workspace(rows, segments, heads, q_groups if it equals k_groups else heads, dk, dv).
+// where a step holds prompt portions), without a normalizer. q, k, v: views of type `dtype` (float32 or bfloat16). Returns
+// JLLM_UNSUPPORTED without launching where jllm_scalar_gated_chunks_fit says no (the caller then runs token by token). `longest`: the
+// rows of the longest segment; `workspace`: what jllm_chunk_plan says for the heads in q_groups groups if that equals k_groups, else
+// a group per head.
 JLLM_EXPORT int jllm_scalar_gated_chunked(const void* q, int ld_q, int q_off, int q_groups, const void* k, int ld_k, int k_off,
                                           int k_groups, const void* v, int ld_v, int v_off, int dtype, const float* la,
                                           const float* b, const void* skip, int skip_dtype, float* state, int num_slots,
                                           const int* seg_start, const int* seg_len, const int* state_slots, float* o,
-                                          int rows, int segments, int heads, int dk, int dv, float q_scale, float* workspace,
-                                          long long workspace_floats, cudaStream_t stream) {
+                                          int rows, int segments, int longest, int heads, int dk, int dv, float q_scale,
+                                          float* workspace, long long workspace_floats, cudaStream_t stream) {
     if (!jllm_scalar_gated_chunks_fit(q, ld_q, q_off, q_groups, k, ld_k, k_off, k_groups, v, ld_v, v_off, dtype, heads, dk, dv))
         return JLLM_UNSUPPORTED;
     if (segments == 0 || rows == 0) return JLLM_OK;
@@ -618,6 +827,6 @@ JLLM_EXPORT int jllm_scalar_gated_chunked(const void* q, int ld_q, int q_off, in
     a.state = state, a.num_slots = num_slots;
     a.seg_start = seg_start, a.seg_len = seg_len, a.state_slots = state_slots;
     a.o = o, a.segments = segments, a.heads = heads, a.dv = dv, a.q_scale = q_scale;
-    return dtype == JLLM_F32 ? run_chunks<float, false>(a, rows, dk, workspace, workspace_floats, stream)
-                             : run_chunks<__nv_bfloat16, false>(a, rows, dk, workspace, workspace_floats, stream);
+    return dtype == JLLM_F32 ? run_chunks<float, false>(a, rows, longest, dk, workspace, workspace_floats, stream)
+                             : run_chunks<__nv_bfloat16, false>(a, rows, longest, dk, workspace, workspace_floats, stream);
 }

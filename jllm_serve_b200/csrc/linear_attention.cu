@@ -738,8 +738,8 @@ JLLM_BOUNDS_READER(linear_attention)
 // chunk_scan.cu
 int jllm_fixed_decay_chunks(const __nv_bfloat16* proj, int ld, int q_off, int k_off, int v_off, const float* head_decay, float* state,
                             int num_slots, const int* seg_start, const int* seg_len, const int* state_slots, float* o, int rows,
-                            int segments, int heads, int dk, int dv, float q_scale, float* workspace, long long workspace_floats,
-                            cudaStream_t stream);
+                            int segments, int longest, int heads, int dk, int dv, float q_scale, float* workspace,
+                            long long workspace_floats, cudaStream_t stream);
 
 // proj [rows, ld]: q at column q_off (heads x dk), k at k_off, v at v_off (heads x dv); z [rows, heads x dk] float32:
 // the decay logits, which this call turns into the decays in place; state [num_slots, heads, dk, dv] float32; o [rows,
@@ -810,8 +810,8 @@ JLLM_EXPORT int jllm_gla_chunked(const void* proj, int dtype, int ld, int q_off,
             if (code) return code;
         }
         return jllm_fixed_decay_chunks((const __nv_bfloat16*)proj, ld, q_off, k_off, v_off, head_decay, state, num_slots, seg_start,
-                                       seg_len, state_slots, o, rows, segments, heads, dk, dv, q_scale, workspace, workspace_floats,
-                                       stream);
+                                       seg_len, state_slots, o, rows, segments, max_len, heads, dk, dv, q_scale, workspace,
+                                       workspace_floats, stream);
     }
     if (head_decay) {
         const int code = dtype == JLLM_F32

@@ -7,6 +7,7 @@ these functions: without the library or without a B200 they raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_char_p, c_double, c_float, c_int, c_void_p
 
@@ -36,7 +37,7 @@ def library():
             if name.startswith("jllm_"):
                 fn = getattr(lib, name)
                 fn.argtypes = getattr(_Signatures, name)
-                fn.restype = ctypes.c_longlong if name == "jllm_chunk_workspace" else c_int
+                fn.restype = c_int
         _lib = lib
     return _lib
 
@@ -164,7 +165,7 @@ class _Signatures:
     jllm_gla_recurrent = [P, I, I, I, I, I, P, I, P, I, P, P, P, P, I, I, I, I, F, F, P, I, P]
     jllm_gla_chunked = [P, I, I, I, I, I, P, I, P, P, P, P, I, P, P, P, P, I, I, I, I, I, F, F, P, I, P, ctypes.c_longlong, P]
     jllm_gla_chunks_fit = [P, I, I, I, I, I, I, I]
-    jllm_chunk_workspace = [I, I, I, I, I, I]
+    jllm_chunk_plan = [I, I, I, I, I, I, I, P]
     jllm_chunk_passes = [I, I, I, I, I, I]
     jllm_bounds_error_chunk_scan = [P]
     jllm_gated_head_norm = [P, P, I, I, P, I, P, I, I, I, F, F, I, I, P]
@@ -194,7 +195,7 @@ class _Signatures:
     jllm_memory_gates = [P, I, I, I, P, P, I, F, P, I, P, P, P, P, P, P, I, I, P]
     jllm_causal_conv = [P, I, I, I, P, P, I, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P]
     jllm_scalar_gated_recurrent = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, P, I, P, P, I, P, P, P, P, I, I, I, I, F, P]
-    jllm_scalar_gated_chunked = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I, F, P, ctypes.c_longlong, P]
+    jllm_scalar_gated_chunked = [P, I, I, I, P, I, I, I, P, I, I, I, P, P, P, I, P, I, P, P, P, P, I, I, I, I, I, I, F, P, ctypes.c_longlong, P]
     jllm_scalar_gated_chunks_fit = [P, I, I, I, P, I, I, I, P, I, I, I, I, I, I]
     jllm_memory_values = [P, I, I, I, P, I, I, I, I, P]
     jllm_memory_divide = [P, P, P, I, I, I, I, P]
@@ -294,8 +295,8 @@ def gla_chunked(proj, q_off, k_off, v_off, decay_logits, state, seg_start, seg_l
     rows, segments, workspace = decay_logits.shape[0], seg_start.numel(), None
     if head_decay is not None and rows and segments and library().jllm_gla_chunks_fit(
             proj.data_ptr(), _DT[proj.dtype], proj.stride(0), q_off, k_off, v_off, key_dim, value_dim):
-        workspace, passes = _chunk_workspace(rows, segments, heads, heads, key_dim, value_dim, proj.device)
-        launch_count += 3 * passes - 1 + (1 if activation else 0)
+        workspace, launches = _chunk_workspace(rows, segments, max_len, heads, heads, key_dim, value_dim, proj.device)
+        launch_count += launches - 1 + (1 if activation else 0)
     else:
         launch_count += 2
     _call("jllm_gla_chunked", proj.data_ptr(), _DT[proj.dtype], proj.stride(0), q_off, k_off, v_off, decay_logits.data_ptr(),
@@ -305,12 +306,19 @@ def gla_chunked(proj, q_off, k_off, v_off, decay_logits, state, seg_start, seg_l
           _p(workspace), workspace.numel() if workspace is not None else 0, _stream())
 
 
-def _chunk_workspace(rows, segments, heads, groups, key_dim, value_dim, device):
-    """(workspace, passes) for the tensor-core chunks of a step: the states in front of all chunks, at most 256 MB of them at a
-    time (or one group's). It belongs to this call: the allocator's memory of the current stream, given back behind the launches."""
-    floats = library().jllm_chunk_workspace(int(rows), int(segments), int(heads), int(groups), int(key_dim), int(value_dim))
-    passes = library().jllm_chunk_passes(int(rows), int(segments), int(heads), int(groups), int(key_dim), int(value_dim))
-    return torch.empty(floats, dtype=torch.float32, device=device), passes
+@functools.lru_cache(maxsize=256)
+def _chunk_plan(rows, segments, longest, heads, groups, key_dim, value_dim):
+    floats = ctypes.c_longlong()
+    launches = library().jllm_chunk_plan(rows, segments, longest, heads, groups, key_dim, value_dim, ctypes.byref(floats))
+    return floats.value, launches
+
+
+def _chunk_workspace(rows, segments, longest, heads, groups, key_dim, value_dim, device):
+    """(workspace or None, launches) for the tensor-core chunks of a step: the states in front of all chunks of its longer segments, at
+    most 256 MB of them at a time (or one group's). It belongs to this call: the allocator's memory of the current stream, given back
+    behind the launches."""
+    floats, launches = _chunk_plan(int(rows), int(segments), int(longest), int(heads), int(groups), int(key_dim), int(value_dim))
+    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, launches
 
 
 def lightning_block_width(width: int = 0) -> None:
@@ -319,6 +327,7 @@ def lightning_block_width(width: int = 0) -> None:
     code = library().jllm_lightning_block_width(int(width))
     if code:
         raise KernelError(library().jllm_last_error().decode(errors="replace"))
+    _chunk_plan.cache_clear()
 
 
 def gated_head_norm(o, gate, gain, eps, scale, out, heads, value_dim, gate_kind: str = "silu", gate_first: bool = False,
@@ -627,15 +636,18 @@ def scalar_gated_chunked(q, q_off, q_groups, k, k_off, k_groups, v, v_off, log_d
         return False
     fn = library().jllm_scalar_gated_chunked
     rows, segments = out.shape[0], batch.seg_start.numel()
-    workspace, passes = _chunk_workspace(rows, segments, heads, q_groups if q_groups == k_groups else heads, key_dim, value_dim, out.device)
+    longest = getattr(batch, "max_q_len", rows)
+    workspace, launches = _chunk_workspace(rows, segments, longest, heads, q_groups if q_groups == k_groups else heads, key_dim,
+                                           value_dim, out.device)
     code = fn(*operands, log_decay.data_ptr(), in_scale.data_ptr(), _p(skip),
               _DT[skip.dtype] if skip is not None else F32, state.data_ptr(), state.shape[0], batch.seg_start.data_ptr(),
-              batch.seg_len.data_ptr(), batch.state_slots.data_ptr(), out.data_ptr(), rows, segments, int(heads),
-              int(key_dim), int(value_dim), float(query_scale), workspace.data_ptr(), workspace.numel(), _stream())
+              batch.seg_len.data_ptr(), batch.state_slots.data_ptr(), out.data_ptr(), rows, segments, int(longest),
+              int(heads), int(key_dim), int(value_dim), float(query_scale), _p(workspace),
+              workspace.numel() if workspace is not None else 0, _stream())
     if code != 0:
         raise KernelError(f"jllm_scalar_gated_chunked failed ({code}): {library().jllm_last_error().decode(errors='replace')}")
     global launch_count
-    launch_count += 3 * passes
+    launch_count += launches
     return True
 
 

@@ -491,6 +491,62 @@ def test_chunks_whose_states_fill_the_workspace_more_than_once():
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
 
 
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("H, G, dk, dv", [(4, 2, 128, 72), (6, 6, 64, 64), (3, 1, 128, 24), (40, 40, 64, 136)])
+def test_short_segments_are_walked_with_the_bits_of_the_chunks_side_by_side(H, G, dk, dv, fixed):
+    """Segments of one or two chunks are walked by one launch, longer ones take three. Five segments, of 1 to 300 tokens: all in one
+    step, each alone, and each cut behind every second chunk into steps that are walked only; outputs and states have the same
+    bits, and those of the first way are the float64 recurrence's."""
+    o = ops()
+    g = torch.Generator().manual_seed(dk + dv)
+    lens, per_head = [300, 1, 128, 64, 129], G if not fixed else H
+    rows = sum(lens)
+    k_of = per_head * dk
+    q, k = torch.randn(rows, k_of, generator=g).bfloat16(), (torch.randn(rows, k_of, generator=g) / math.sqrt(dk)).bfloat16()
+    v = torch.randn(rows, H * dv, generator=g).bfloat16()
+    buf = torch.cat([q, k, v], dim=1).to(DEV)
+    decay = 0.9 + 0.09 * torch.rand(H, generator=g)
+    la, b = (decay.double().log().float().expand(rows, H), torch.ones(rows, H)) if fixed else \
+        (-torch.rand(rows, H, generator=g) * 0.3, torch.rand(rows, H, generator=g))
+    start = torch.randn(len(lens), H, dk, dv, generator=g)
+
+    def step(state, out, parts):          # parts: (segment, first token, tokens)
+        at = torch.cat([torch.arange(sum(lens[:s]) + a, sum(lens[:s]) + a + n) for s, a, n in parts]).to(DEV)
+        batch = FakeBatch([n for _, _, n in parts], [s for s, _, _ in parts])
+        batch.max_q_len = max(n for _, _, n in parts)
+        part, n = buf[at].contiguous(), len(at)
+        y = torch.full((n, H * dv), float("nan"), device=DEV)
+        if fixed:
+            f32 = lambda *s: torch.empty(*s, device=DEV)
+            o.gla_chunked(part, 0, k_of, 2 * k_of, f32(n, H * dk), state, batch.seg_start, batch.seg_len, batch.state_slots, y, H, dk, dv,
+                          0.5, 1.0, batch.max_q_len, f32(n, H * dk), f32(n, H * dk), f32(n, H * o.GLA_CHUNK), head_decay=decay.to(DEV))
+        else:
+            assert o.scalar_gated_chunked(part, 0, G, part, k_of, G, part, 2 * k_of, la.to(DEV)[at].contiguous(), b.to(DEV)[at].contiguous(),
+                                          state, batch, y, H, dk, dv, 0.5)
+        out[at] = y
+
+    ways = []
+    for way in range(3):
+        state, out = start.to(DEV), torch.full((rows, H * dv), float("nan"), device=DEV)
+        if way == 0:
+            step(state, out, [(s, 0, n) for s, n in enumerate(lens)])
+        for s, n in enumerate(lens):
+            for a in range(0, n, 128) if way == 2 else [0] * way:
+                step(state, out, [(s, a, min(128, n - a) if way == 2 else n)])
+        ways.append((state, out))
+    for state, out in ways[1:]:
+        assert torch.equal(state, ways[0][0]) and torch.equal(out, ways[0][1])
+    at = 0
+    for s, n in enumerate(lens):
+        part, S, share = slice(at, at + n), start[s].double(), H // per_head
+        want = plain_recurrence(q[part].double().view(n, per_head, dk).repeat_interleave(share, 1),
+                                k[part].double().view(n, per_head, dk).repeat_interleave(share, 1), v[part].double().view(n, H, dv),
+                                la[part].double(), b[part].double(), S, q_scale=0.5)
+        close(ways[0][1][part].cpu(), want.reshape(n, -1), torch.float32, f"segment {s}", loose=5)
+        close(ways[0][0][s].cpu(), S, torch.float32, f"state {s}", loose=5)
+        at += n
+
+
 def test_a_shape_the_chunks_do_not_take_costs_no_workspace():
     """Values of 12 columns, and keys that begin off a 16-byte boundary: the call says no before any memory is asked for."""
     o = ops()
