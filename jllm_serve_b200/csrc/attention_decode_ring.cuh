@@ -436,7 +436,8 @@ int launch(Args a, const void* k_cache, const void* v_cache, dim3 grid, cudaStre
     if (rc == JLLM_OK) rc = tc::tensor_map_for(v_cache, 0x7fffffffll, HD, HD, box, &map_v);
     if (rc != JLLM_OK) return rc;
     auto kern = attention_decode_ring_kernel<HD, FLAT>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES);
+    if (jllm_allow_smem((const void*)kern, L::BYTES) != cudaSuccess)
+        return jllm_fail(JLLM_CUDA_ERROR, "attention_decode: %zu bytes of shared memory refused", L::BYTES);
     jllm_launch(kern, grid, dim3(THREADS), L::BYTES, stream, LAUNCH_DEPENDENT, map_k, map_v, a);
     return JLLM_OK;
 }

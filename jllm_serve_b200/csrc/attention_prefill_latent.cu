@@ -400,7 +400,8 @@ JLLM_EXPORT int jllm_attention_prefill_latent(const void* q, int q_stride, const
     int page_shift = 0;
     while ((1 << page_shift) < page_size) ++page_shift;
     auto kern = softcap > 0.f ? attention_prefill_latent_kernel<true> : attention_prefill_latent_kernel<false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    if (jllm_allow_smem((const void*)kern, SMEM_BYTES) != cudaSuccess)
+        return jllm_fail(JLLM_CUDA_ERROR, "attention_prefill_latent: %zu bytes of shared memory refused", SMEM_BYTES);
     const dim3 grid(heads, (rows + BQ - 1) / BQ + num_segs);
     jllm_launch(kern, grid, dim3(THREADS), SMEM_BYTES, stream, true, map_q, map_k, (const __nv_bfloat16*)cache,
                 (__nv_bfloat16*)out, out_stride, seg_start, seg_len, seg_kv_len, block_tables, table_stride, num_segs, heads,

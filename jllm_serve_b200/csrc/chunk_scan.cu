@@ -691,7 +691,7 @@ Cut cut_of(int rows, int segments, int longest, int heads, int groups, int dk, i
 template <typename TS, int DK, int SLAB, bool FIXED>
 int run_walk(const ChunkArgs& a, cudaStream_t stream) {
     constexpr size_t smem = (size_t)DK * SLAB * 4 + 2 * (size_t)C * (DK + 8) * 2 + 3 * (size_t)C * (SLAB + 8) * 2 + GATES * sizeof(float);
-    if (cudaFuncSetAttribute(chunk_walk_kernel<TS, DK, SLAB, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (jllm_allow_smem((const void*)chunk_walk_kernel<TS, DK, SLAB, FIXED>, smem) != cudaSuccess)
         return jllm_fail(JLLM_CUDA_ERROR, "chunk_walk: %zu bytes of shared memory refused", smem);
     jllm_launch(chunk_walk_kernel<TS, DK, SLAB, FIXED>, dim3(a.segments, a.heads, (a.dv + SLAB - 1) / SLAB), dim3(256), smem, stream,
                 LAUNCH_DEPENDENT, a);
@@ -702,8 +702,8 @@ template <typename TS, int DK, int SLAB, bool FIXED>
 int run_passes(ChunkArgs a, const Cut& c, float* workspace, cudaStream_t stream) {
     const size_t tail = GATES * sizeof(float), values = (size_t)C * (SLAB + 8) * 2, rows = (size_t)C * (DK + 8) * 2;
     const size_t smem_s = rows + 2 * values + tail, smem_o = 2 * (size_t)DK * SLAB * 4 + 2 * rows + values + tail;
-    if (cudaFuncSetAttribute(chunk_states_kernel<TS, DK, SLAB, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s) != cudaSuccess ||
-        cudaFuncSetAttribute(chunk_out_kernel<TS, DK, SLAB, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o) != cudaSuccess)
+    if (jllm_allow_smem((const void*)chunk_states_kernel<TS, DK, SLAB, FIXED>, smem_s) != cudaSuccess ||
+        jllm_allow_smem((const void*)chunk_out_kernel<TS, DK, SLAB, FIXED>, smem_o) != cudaSuccess)
         return jllm_fail(JLLM_CUDA_ERROR, "chunk_scan: %zu bytes of shared memory refused", smem_s > smem_o ? smem_s : smem_o);
     const int per_head = c.slabs * (DK / 16) * (SLAB / 8) * 32;
     for (int g0 = 0; g0 < a.groups; g0 += c.pass_groups) {

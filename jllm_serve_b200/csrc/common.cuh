@@ -123,6 +123,9 @@ bool jllm_pdl_enabled();
 enum : int { LAUNCH_PLAIN = 0, LAUNCH_DEPENDENT = 1, LAUNCH_DEPENDENT_WANTS_L1 = 2 };
 bool jllm_launch_overlaps(size_t dynamic_smem, int how);     // decides, and keeps the record the decision needs
 
+// Lets a kernel have `bytes` of dynamic shared memory: asked of the driver once per kernel and device, not per launch.
+cudaError_t jllm_allow_smem(const void* kernel, size_t bytes);
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t jllm_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                int how, Args... args) {

@@ -513,7 +513,8 @@ JLLM_EXPORT int jllm_gemm_heads(const void* a, int dtype, int lda, const void* w
     if (vec && M > 64) {        // (up to 64 rows the small tiles give more blocks)
         const int wide_out = ldo % 8 == 0 && o_head % 8 == 0 && N % 8 == 0 && ((uintptr_t)out % 16) == 0;
         const int wide_rope = wide_out && rope_dim % 8 == 0 && rotary_dim % 8 == 0 && ((uintptr_t)cos_t % 16) == 0 && ((uintptr_t)sin_t % 16) == 0;
-        cudaFuncSetAttribute(many::gemm_heads_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)many::SMEM);
+        if (jllm_allow_smem((const void*)many::gemm_heads_many_kernel, many::SMEM) != cudaSuccess)
+            return jllm_fail(JLLM_CUDA_ERROR, "gemm_heads: %zu bytes of shared memory refused", many::SMEM);
         jllm_launch(many::gemm_heads_many_kernel, dim3(grid.x, (M + many::ROWS - 1) / many::ROWS, heads), dim3(many::THREADS), many::SMEM,
                     stream, LAUNCH_DEPENDENT, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, ldo,
                     (const __nv_bfloat16*)gate, ld_gate, (int)(gate != nullptr && gate_full), alpha, M, N, K, a_head, o_head, wide_out,

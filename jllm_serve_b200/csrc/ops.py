@@ -293,8 +293,8 @@ def gla_chunked(proj, q_off, k_off, v_off, decay_logits, state, seg_start, seg_l
     assert qb.shape == ke.shape == decay_logits.shape and scores.shape == (decay_logits.shape[0], heads * GLA_CHUNK)
     global launch_count
     rows, segments, workspace = decay_logits.shape[0], seg_start.numel(), None
-    if head_decay is not None and rows and segments and library().jllm_gla_chunks_fit(
-            proj.data_ptr(), _DT[proj.dtype], proj.stride(0), q_off, k_off, v_off, key_dim, value_dim):
+    if head_decay is not None and rows and segments and _gla_chunks_fit(
+            proj.data_ptr() % 16, _DT[proj.dtype], proj.stride(0), q_off, k_off, v_off, key_dim, value_dim):
         workspace, launches = _chunk_workspace(rows, segments, max_len, heads, heads, key_dim, value_dim, proj.device)
         launch_count += launches - 1 + (1 if activation else 0)
     else:
@@ -304,6 +304,16 @@ def gla_chunked(proj, q_off, k_off, v_off, decay_logits, state, seg_start, seg_l
           seg_start.data_ptr(), seg_len.data_ptr(), state_slots.data_ptr(), out.data_ptr(), seg_start.numel(), int(max_len),
           heads, key_dim, value_dim, float(query_scale), float(temperature), _head_decay(head_decay, heads), int(activation),
           _p(workspace), workspace.numel() if workspace is not None else 0, _stream())
+
+
+@functools.lru_cache(maxsize=256)
+def _gla_chunks_fit(*shape):             # (the first: the address's place in 16 bytes)
+    return bool(library().jllm_gla_chunks_fit(*shape))
+
+
+@functools.lru_cache(maxsize=256)
+def _scalar_gated_chunks_fit(*shape):    # (addresses: their place in 16 bytes)
+    return bool(library().jllm_scalar_gated_chunks_fit(*shape))
 
 
 @functools.lru_cache(maxsize=256)
@@ -317,7 +327,7 @@ def _chunk_workspace(rows, segments, longest, heads, groups, key_dim, value_dim,
     """(workspace or None, launches) for the tensor-core chunks of a step: the states in front of all chunks of its longer segments, at
     most 256 MB of them at a time (or one group's). It belongs to this call: the allocator's memory of the current stream, given back
     behind the launches."""
-    floats, launches = _chunk_plan(int(rows), int(segments), int(longest), int(heads), int(groups), int(key_dim), int(value_dim))
+    floats, launches = _chunk_plan(rows, segments, int(longest), heads, groups, key_dim, value_dim)
     return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, launches
 
 
@@ -630,20 +640,22 @@ def scalar_gated_chunked(q, q_off, q_groups, k, k_off, k_groups, v, v_off, log_d
         return False
     assert q.dtype == k.dtype == v.dtype and q.stride(1) == k.stride(1) == v.stride(1) == 1
     assert state.dtype == out.dtype == torch.float32 and state.is_contiguous() and out.is_contiguous()
-    operands = (q.data_ptr(), q.stride(0), int(q_off), int(q_groups), k.data_ptr(), k.stride(0), int(k_off), int(k_groups),
-                v.data_ptr(), v.stride(0), int(v_off), _DT[q.dtype])
-    if not library().jllm_scalar_gated_chunks_fit(*operands, int(heads), int(key_dim), int(value_dim)):
+    q_off, q_groups, k_off, k_groups, v_off, heads, key_dim, value_dim = map(
+        int, (q_off, q_groups, k_off, k_groups, v_off, heads, key_dim, value_dim))
+    qp, kp, vp, dt = q.data_ptr(), k.data_ptr(), v.data_ptr(), _DT[q.dtype]
+    lq, lk, lv = q.stride(0), k.stride(0), v.stride(0)
+    if not _scalar_gated_chunks_fit(qp % 16, lq, q_off, q_groups, kp % 16, lk, k_off, k_groups, vp % 16, lv, v_off, dt, heads, key_dim,
+                                    value_dim):
         return False
-    fn = library().jllm_scalar_gated_chunked
     rows, segments = out.shape[0], batch.seg_start.numel()
     longest = getattr(batch, "max_q_len", rows)
     workspace, launches = _chunk_workspace(rows, segments, longest, heads, q_groups if q_groups == k_groups else heads, key_dim,
                                            value_dim, out.device)
-    code = fn(*operands, log_decay.data_ptr(), in_scale.data_ptr(), _p(skip),
-              _DT[skip.dtype] if skip is not None else F32, state.data_ptr(), state.shape[0], batch.seg_start.data_ptr(),
-              batch.seg_len.data_ptr(), batch.state_slots.data_ptr(), out.data_ptr(), rows, segments, int(longest),
-              int(heads), int(key_dim), int(value_dim), float(query_scale), _p(workspace),
-              workspace.numel() if workspace is not None else 0, _stream())
+    code = library().jllm_scalar_gated_chunked(
+        qp, lq, q_off, q_groups, kp, lk, k_off, k_groups, vp, lv, v_off, dt, log_decay.data_ptr(), in_scale.data_ptr(), _p(skip),
+        _DT[skip.dtype] if skip is not None else F32, state.data_ptr(), state.shape[0], batch.seg_start.data_ptr(),
+        batch.seg_len.data_ptr(), batch.state_slots.data_ptr(), out.data_ptr(), rows, segments, int(longest), heads, key_dim, value_dim,
+        float(query_scale), _p(workspace), workspace.numel() if workspace is not None else 0, _stream())
     if code != 0:
         raise KernelError(f"jllm_scalar_gated_chunked failed ({code}): {library().jllm_last_error().decode(errors='replace')}")
     global launch_count
@@ -1435,9 +1447,11 @@ def attention_prefill_tc_fits(q, out, k_cache, head_dim, page_size) -> bool:
 
 
 def attention_prefill_latent_fits(q, out, k_cache, v_cache, head_dim, page_size) -> bool:
-    return (head_dim == 256 and q.dtype == torch.bfloat16 and k_cache.data_ptr() == v_cache.data_ptr()
-            and 1 <= page_size <= 128 and page_size & (page_size - 1) == 0 and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
-            and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and k_cache.data_ptr() % 16 == 0 and k_cache.is_contiguous())
+    if head_dim != 256 or q.dtype != torch.bfloat16:
+        return False
+    keys = k_cache.data_ptr()
+    return (keys == v_cache.data_ptr() and 1 <= page_size <= 128 and page_size & (page_size - 1) == 0 and q.stride(0) % 8 == 0
+            and out.stride(0) % 8 == 0 and (q.data_ptr() | out.data_ptr() | keys) % 16 == 0 and k_cache.is_contiguous())
 
 
 def attention_prefill(q, k_cache, v_cache, out, seg_start, seg_len, seg_kv_len, block_tables, rows, heads, kv_heads,

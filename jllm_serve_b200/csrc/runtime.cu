@@ -3,6 +3,8 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <unordered_map>
 
 namespace {
 thread_local char g_error[1024] = "";
@@ -83,6 +85,22 @@ int jllm_device_sm_count() {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) counts[dev] = n;
     }
     return counts[dev];
+}
+
+// (A call to the driver takes about as long as the launch's own preparation; a kernel that was let have more keeps it.)
+cudaError_t jllm_allow_smem(const void* kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::unordered_map<const void*, size_t> allowed[64];
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& known = allowed[dev][kernel];
+    if (bytes <= known) return cudaSuccess;
+    const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (set == cudaSuccess) known = bytes;
+    return set;
 }
 
 // Pages of the cache pool that the launches which follow read and write (0 = not known). Only the build with bounds

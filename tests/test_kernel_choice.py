@@ -83,3 +83,20 @@ def test_a_decode_steps_bucket_is_clamped_where_it_stops_mattering():
     assert all(l <= max(1, b) and l in ops.KV_BUCKET_LEVELS for b, l in enumerate(levels))
     assert all(4 * b <= 5 * l + 4 for b, l in enumerate(levels[:33]))                # never more than a quarter below
     assert len(set(levels)) == 16
+
+
+def test_what_the_recurrence_chunks_take_is_asked_once_per_shape(monkeypatch):
+    """Launches and workspace of a step's chunks: one launch and nothing where the segments are short, three for a long one, four where
+    both are there; passes over the heads where a pass's states fill 256 MB. A second layer of the step asks nothing."""
+    ops._chunk_plan.cache_clear()
+    plan = lambda *shape: ops._chunk_plan(*shape)
+    assert plan(64, 1, 64, 64, 8, 128, 64) == (0, 1) and plan(33, 33, 1, 64, 8, 128, 64) == (0, 1)
+    floats, launches = plan(2048, 1, 2048, 64, 8, 128, 64)
+    assert launches == 3 and floats == 33 * 64 * (128 * 64 + 1)
+    assert plan(2080, 33, 2048, 64, 8, 128, 64)[1] == 4                   # 32 single rows beside a portion
+    assert plan(1100, 1, 1100, 256, 256, 128, 128)[1] == 6 and plan(1100, 1, 1100, 256, 256, 128, 128)[0] <= 64 << 20
+    floats, launches = plan(2048, 8, 256, 64, 8, 128, 64)                 # eight of 256: their blocks fill the SMs
+    assert (floats, launches) == (0, 1)
+    monkeypatch.setattr(ops, "library", lambda: (_ for _ in ()).throw(AssertionError("the library was asked again")))
+    assert plan(64, 1, 64, 64, 8, 128, 64) == (0, 1)
+    ops._chunk_plan.cache_clear()
