@@ -19,7 +19,7 @@
 //     launch): weights do not depend on it.
 // Roles: warp 0 (one lane) producer, warp 1 (one lane) MMA issuer, warps 2-5 epilogue (bias / float32 residual add /
 // SwiGLU over interleaved gate and up rows / store). Every wait is bounded and raises the error word of
-// gemm_tcgen05 (codes 11-13).
+// gemm_tcgen05 (codes 11-13; the clusters' kernel 14-16).
 #include <mutex>
 #include <unordered_map>
 
@@ -214,10 +214,35 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
             const int row_in_tile = quad * 32 + lane;
             const int n = tile * WM + row_in_tile;                 // this thread's weight row = output column
             const uint32_t taddr = tmem_base + buf * acc_cols + ((uint32_t)(quad * 32) << 16);
+            // value of (token m, weight row n): bias / residual / SwiGLU and the store
             auto finalize16 = [&](const float (&v)[16], int m0) {
-                float old[16];
-                residual(old, out, ldo, accumulate, m0, M, n, N);
-                finish(v, old, out, ldo, accumulate, bias, has_bias, swiglu, m0, M, n, N);
+                if (swiglu) {
+                    // rows come in blocks of 16: 8 gate rows, then the 8 up rows of the same hidden units
+                    const int unit = (n >> 4) * 8 + (n & 7);
+                    float other[16], units[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) other[j] = __shfl_xor_sync(0xffffffffu, v[j], 8);
+                    if ((lane & 8) == 0 && n + 8 < N) {
+                        glu_units<16>(swiglu.word_of(unit), [&](int j) { return v[j]; }, [&](int j) { return other[j]; }, 1.f, units);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            if (m0 + j >= M) continue;
+                            if (swiglu.weights != nullptr) units[j] = __fmul_rn(units[j], swiglu.weight(m0 + j, unit));
+                            out[(size_t)(m0 + j) * ldo + unit] = from_float<Tout>(units[j]);
+                        }
+                    }
+                } else if (n < N) {
+                    const float b = has_bias ? bias[n] : 0.f;
+                    Tout* dst = out + (size_t)m0 * ldo + n;
+                    float old[16];
+                    // all the old values are requested before the first store (a load behind a store through the
+                    // same pointer would wait for it: 16 round trips instead of one)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) old[j] = (accumulate == EPI_ADD && m0 + j < M) ? to_float(dst[(size_t)j * ldo]) : 0.f;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (m0 + j < M) dst[(size_t)j * ldo] = from_float<Tout>(epilogue_act(v[j] + b, accumulate) + old[j]);
+                }
             };
             if (kb0 == 0 && kb1 == k_blocks) {                      // the whole tile is this block's
 #pragma unroll 1
@@ -344,7 +369,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
 // `overlay`: the parts lie over the ring (many tokens leave no room beside it); the cluster then meets once more, when every block
 // is done with its ring, before anything is written.
 constexpr int CLUSTER_MAX = 8;
-constexpr double MEETING_K_BLOCKS = 16;         // k blocks an SM streams in the time of a meeting in the workspace (5 to 6 us)
 
 __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -554,28 +578,59 @@ cudaLaunchConfig_t cluster_config(const ClusterCut& c, int tiles, cudaLaunchAttr
     return cfg;
 }
 
-// clusters of that many blocks the device runs at a time with that much shared memory (asked once per size)
+// clusters of that many blocks the device runs at a time with that much shared memory
 template <typename Tout>
-int resident_clusters(int blocks, size_t smem) {
+int resident_clusters(const ClusterCut& c) {
+    int n = 0;
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = cluster_config<Tout>(c, 1, attr, nullptr);
+    if (jllm_allow_smem((const void*)gemm_cluster_kernel<Tout>, c.smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_cluster_kernel<Tout>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+// The cluster of `n` blocks to a tile for a product, or one of no blocks where it does not fit: fewer k blocks than blocks, no room for
+// two stages, or more tiles than clusters are resident at once
+ClusterCut cluster_of(int n, int ntok, int tiles, int k_blocks, int out_dtype) {
+    if (n < 1 || n > CLUSTER_MAX || n > k_blocks) return ClusterCut{};
+    const ClusterCut one = cluster_cut(n, ntok);
+    if (one.stages < 2) return ClusterCut{};
+    const int resident = out_dtype == JLLM_F32 ? resident_clusters<float>(one) : resident_clusters<__nv_bfloat16>(one);
+    return tiles <= resident ? one : ClusterCut{};
+}
+
+// A cluster to a tile where the clusters of all tiles are resident at once and it costs less than equal runs; of the sizes that fit, the
+// cheapest. Costs are in k blocks that an SM streams (0.3 to 0.4 us): a block's own, and what the meetings take. In the workspace that
+// is 10 to 16, more where a tile falls to more blocks; in a cluster half a k block for every block of it and a third more where the
+// cluster meets twice (`overlay`); tokens, which either has to add up, cost a cluster of one nothing. Equal runs and clusters, launched
+// back to back: 2,048 x 8,192 (six to a cluster), 64 rows 15.0 and 12.6 us; 7,168 x 5,120 (two), 128 rows 27.1 and 25.3; 12,288 x 2,048
+// (one), 32 rows 15.4 and 15.9, 128 rows 28.2 and 26.7; 6,144 x 4,096 (two, 96 of the SMs), 32 rows 14.7 and 14.6, 128 rows 20.0 and
+// 21.3; 2,048 x 12,288 (six), 64 rows 16.4 and 15.8, 128 rows, with overlay, 17.8 and 19.0.
+// (The driver is asked once per shape and device: the choice is kept.)
+ClusterCut choose_cluster(int ntok, int tiles, int k_blocks, int out_dtype, int sms) {
     static std::mutex mu;
-    static std::unordered_map<long long, int> known;
+    static std::unordered_map<unsigned long long, ClusterCut> known;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    const long long key = ((long long)dev * 16 + blocks) * (1 << 20) + (long long)smem;
+    if (cudaGetDevice(&dev) != cudaSuccess) return ClusterCut{};
+    const unsigned long long key =
+        ((((unsigned long long)k_blocks << 24 | (unsigned)tiles) << 5 | (unsigned)(ntok / 16)) << 2 | (unsigned)out_dtype) << 6 | (unsigned)dev;
     std::lock_guard<std::mutex> lock(mu);
     const auto it = known.find(key);
     if (it != known.end()) return it->second;
-    int n = 0;
-    ClusterCut c{blocks, 0, 0, 0, smem};
-    cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = cluster_config<Tout>(c, 1, attr, nullptr);
-    if (cudaFuncSetAttribute(gemm_cluster_kernel<Tout>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, gemm_cluster_kernel<Tout>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
+    ClusterCut c{};
+    const double tokens = ntok / 40., meeting = 8.5 + 1.1 * sms / tiles;
+    double best = (double)tiles * k_blocks / sms + (meeting < 16. ? meeting : 16.) + tokens;
+    for (int n = 1; n <= CLUSTER_MAX && n <= k_blocks; ++n) {
+        const double cost = (k_blocks + n - 1) / n + 0.5 * n + (n > 1 ? tokens : 0.) + (cluster_cut(n, ntok).overlay ? n / 3. : 0.);
+        if (cost >= best) continue;
+        const ClusterCut one = cluster_of(n, ntok, tiles, k_blocks, out_dtype);
+        if (one.blocks > 0) best = cost, c = one;
     }
-    known[key] = n;
-    return n;
+    if (known.size() >= 4096) known.clear();
+    return known[key] = c;
 }
 
 }  // namespace
@@ -585,13 +640,21 @@ int* jllm_gemm_error_word();
 
 JLLM_EXPORT long long jllm_gemm_stream_workspace_floats() { return 2LL * MAX_TILES + 2LL * 160 * MAX_TOKENS * WM; }
 
+// The blocks of the clusters that a product of M rows against an [N, K] weight runs in (0: equal runs)
+JLLM_EXPORT int jllm_gemm_stream_cluster(int M, int N, int K, int out_dtype) {
+    if (M < 1 || M > MAX_TOKENS || N < 1 || K < 1) return 0;
+    const int sms = jllm_device_sm_count() > 0 ? jllm_device_sm_count() : 1;
+    return choose_cluster((M + 15) / 16 * 16, (N + WM - 1) / WM, (K + BK - 1) / BK, out_dtype, sms).blocks;
+}
+
 // a [M, K] bfloat16 (row stride lda), w_packed: ops.pack_weight of the [N, K] weight (k padded to k_blocks * 64, rows
 // to a multiple of 128, zeros), out [M, N] (or [M, N / 2] with swiglu) float32 or bfloat16. `workspace`: zeroed floats
-// (counters, then parked parts), at least jllm_gemm_stream_workspace_floats().
+// (counters, then parked parts), at least jllm_gemm_stream_workspace_floats(). `cluster` (tests): the blocks of a cluster, 0 as the
+// shape has it, -1 equal runs.
 JLLM_EXPORT int jllm_gemm_stream(const void* a, int lda, const void* w_packed, int k_blocks, const void* bias,
                                  int bias_dtype, void* out, int out_dtype, int ldo, int accumulate, int M, int N, int K,
                                  int swiglu_word, const void* glu_more, float* workspace, long long workspace_floats, int max_blocks,
-                                 cudaStream_t stream) {
+                                 int cluster, cudaStream_t stream) {
     const GluArgs swiglu = glu_args(swiglu_word, glu_more);
     JLLM_REQUIRE(swiglu.in_eights(), "gemm_stream: units of %d in front of %d do not come in eights", swiglu.ff, swiglu.split);
     JLLM_REQUIRE(M >= 1 && M <= MAX_TOKENS && N >= 1 && K >= 8 && K % 8 == 0 && lda % 8 == 0 && ((uintptr_t)a % 16) == 0 &&
@@ -623,23 +686,17 @@ JLLM_EXPORT int jllm_gemm_stream(const void* a, int lda, const void* w_packed, i
     int* error_word = jllm_gemm_error_word();
     if (!error_word) return jllm_fail(JLLM_CUDA_ERROR, "gemm_stream: no error word");
     const VecRef b{bias, bias_dtype};
-    // A cluster to a tile where the clusters of all tiles are resident at once and a block's k blocks take no longer than an equal run
-    // and the meeting it saves; of the sizes that fit, the one with the fewest k blocks a block (a larger cluster meets for longer).
-    if (max_blocks <= 0) {
-        ClusterCut c{};
-        double best = (double)tiles * k_blocks / sms + MEETING_K_BLOCKS;
-        for (int n = 1; n <= CLUSTER_MAX && n <= k_blocks; ++n) {
-            const ClusterCut one = cluster_cut(n, ntok);
-            const double cost = (k_blocks + n - 1) / n + 0.5 * n;
-            if (one.stages < 2 || cost >= best) continue;
-            if (tiles <= (out_dtype == JLLM_F32 ? resident_clusters<float>(n, one.smem) : resident_clusters<__nv_bfloat16>(n, one.smem)))
-                best = cost, c = one;
-        }
+    if (max_blocks <= 0 && cluster >= 0) {
+        const ClusterCut c = cluster > 0 ? cluster_of(cluster, ntok, tiles, k_blocks, out_dtype)
+                                         : choose_cluster(ntok, tiles, k_blocks, out_dtype, sms);
+        JLLM_REQUIRE(cluster == 0 || c.blocks == cluster, "gemm_stream: clusters of %d blocks do not take %d tiles of %d k blocks, %d rows",
+                     cluster, tiles, k_blocks, M);
         if (c.blocks > 0) {
 #define JLLM_CLUSTER_GO(T)                                                                                          \
     do {                                                                                                            \
         auto kern = gemm_cluster_kernel<T>;                                                                         \
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);                       \
+        if (jllm_allow_smem((const void*)kern, c.smem) != cudaSuccess)                                              \
+            return jllm_fail(JLLM_CUDA_ERROR, "gemm_stream: %zu bytes of shared memory refused", c.smem);           \
         cudaLaunchAttribute attr[2];                                                                                \
         cudaLaunchConfig_t cfg = cluster_config<T>(c, tiles, attr, stream);                                         \
         if (jllm_launch_overlaps(c.smem, LAUNCH_DEPENDENT)) {                                                       \

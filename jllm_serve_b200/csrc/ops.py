@@ -141,7 +141,8 @@ class _Signatures:
     jllm_gemm_pair = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, P]
     jllm_gemm_pair_resident = []
     jllm_gemm_plain_stores = [I]
-    jllm_gemm_stream = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, P]
+    jllm_gemm_stream = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, I, P]
+    jllm_gemm_stream_cluster = [I, I, I, I]
     jllm_gemm_tcgen05_error = []
     jllm_gemm_tcgen05_starve_next = []
     jllm_attention_plain = [P, I, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P, I, F, P]
@@ -1130,17 +1131,24 @@ def gemm_stream_fits(a, packed: PackedWeight) -> bool:
             and a.data_ptr() % 16 == 0)
 
 
-def gemm_stream(a, packed: PackedWeight, out, bias=None, accumulate=False, swiglu=False, max_blocks: int = 0) -> None:
+def gemm_stream_cluster(rows: int, out_features: int, in_features: int, out_dtype) -> int:
+    """The blocks to a cluster in which `gemm_stream` runs such a product (0: equal runs of all tiles' k blocks)."""
+    return int(library().jllm_gemm_stream_cluster(int(rows), int(out_features), int(in_features), _DT[out_dtype]))
+
+
+def gemm_stream(a, packed: PackedWeight, out, bias=None, accumulate=False, swiglu=False, max_blocks: int = 0, cluster: int = 0) -> None:
     """out (+)= a @ W^T (+ bias) for at most 256 rows: the packed weight streamed once through tcgen05.mma with the
     weight rows as the M side (see gemm_stream.cu). With `swiglu` the rows of W are blocks of 8 gate rows followed by
     their 8 up rows and out[m, j] = silu(gate_j) * up_j. A tile's parts (its k blocks may fall to several blocks) are
-    added in k order: two runs give the same bits."""
+    added in k order: two runs give the same bits. `cluster` (tests): the blocks of a cluster, 0 as `gemm_stream_cluster` says, -1 equal
+    runs."""
     packed = _packed(packed)
     assert a.dtype == torch.bfloat16 and out.stride(-1) == 1 and a.shape[1] == packed.cols
     ws = gemm_workspace((a.device, "stream"), SWAP_WORKSPACE_FLOATS)     # its own: it keeps counters of its own there
     _call("jllm_gemm_stream", a.data_ptr(), a.stride(0), packed.data.data_ptr(), packed.k_blocks, _p(bias),
           _DT[bias.dtype] if bias is not None else F32, out.data_ptr(), _DT[out.dtype], out.stride(0), int(accumulate),
-          a.shape[0], packed.rows, packed.cols, glu_kind(swiglu), glu_more(swiglu), ws.data_ptr(), ws.numel(), int(max_blocks), _stream())
+          a.shape[0], packed.rows, packed.cols, glu_kind(swiglu), glu_more(swiglu), ws.data_ptr(), ws.numel(), int(max_blocks), int(cluster),
+          _stream())
 
 
 BOUNDS_FILES = ("attention_plain", "attention_decode", "attention_prefill", "attention_prefill_tc",

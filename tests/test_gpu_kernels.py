@@ -144,8 +144,8 @@ def test_gemm_stream(ops, M, N, K):
 @pytest.mark.parametrize("M", [3, 24, 61, 130, 250])
 @pytest.mark.parametrize("N,K", [(300, 8192), (2048, 8192), (1111, 320), (2500, 2056)])
 def test_gemm_stream_by_clusters(ops, M, N, K):
-    """A cluster of two to eight blocks to a tile, their shares of the tokens uneven or empty, few k blocks, parts beside the ring and
-    over it: against float64, and the same bits twice."""
+    """Products as the shape has them, clusters of one to eight blocks and (300 x 8,192) equal runs, few and uneven k blocks: against
+    float64, and the same bits twice."""
     a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
     packed, base, bias = ops.pack_weight(w), rnd(M, N, seed=3), rnd(N, dtype=torch.float32, seed=2)
     want = gemm_want(a, w, bias, base)
@@ -155,6 +155,37 @@ def test_gemm_stream_by_clusters(ops, M, N, K):
     assert ops.gemm_tcgen05_error() == 0
     assert torch.allclose(acc.cpu(), want, rtol=1e-4, atol=1e-4 * math.sqrt(K) * 0.05)
     assert torch.equal(acc, again)
+
+
+@pytest.mark.parametrize("M", [3, 24, 61, 130, 250])
+@pytest.mark.parametrize("blocks", [-1, 1, 2, 3, 4, 5, 6, 7, 8])
+def test_gemm_stream_in_clusters_of_every_size(ops, M, blocks):
+    """Clusters of one to eight blocks to a tile (and equal runs) asked for by size: residual add, bfloat16 results and the gated
+    epilogue against float64, the same bits twice."""
+    N, K = 304, 1032
+    a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
+    packed, base, bias = ops.pack_weight(w), rnd(M, N, seed=3), rnd(N, dtype=torch.float32, seed=2)
+    acc, again, out16 = base.clone(), base.clone(), torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_stream(a, packed, acc, bias, accumulate=True, cluster=blocks)
+    ops.gemm_stream(a, packed, again, bias, accumulate=True, cluster=blocks)
+    ops.gemm_stream(a, packed, out16, cluster=blocks)
+    units = torch.empty(M, N // 2, device=DEV)
+    ops.gemm_stream(a, packed, units, swiglu=True, cluster=blocks)
+    assert ops.gemm_tcgen05_error() == 0
+    tol = 1e-4 * math.sqrt(K) * 0.05
+    assert torch.allclose(acc.cpu(), gemm_want(a, w, bias, base), rtol=1e-4, atol=tol) and torch.equal(acc, again)
+    assert torch.allclose(out16.float().cpu(), gemm_want(a, w), rtol=2 ** -7, atol=2e-3)
+    z = gemm_want(a, w).view(M, N // 16, 2, 8)
+    want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2)
+    assert torch.allclose(units.cpu(), want, rtol=1e-3, atol=1e-3)
+
+
+def test_gemm_stream_refuses_a_cluster_that_does_not_fit(ops):
+    a, w = rnd(20, 64, dtype=torch.bfloat16), ops.pack_weight(rnd(256, 64, dtype=torch.bfloat16, seed=1))
+    out = torch.empty(20, 256, device=DEV)
+    for blocks in (2, 9):                        # one k block; more blocks than a cluster has
+        with pytest.raises(ops.KernelError, match="clusters of"):
+            ops.gemm_stream(a, w, out, cluster=blocks)
 
 
 @pytest.mark.parametrize("M", [1, 8, 20, 64, 128, 250])
