@@ -21,7 +21,8 @@
 // bounds it: from 32 rows on the multiply-adds, below that the weights' bytes. 300 rows of the 8B layer products: 43 TFLOP/s
 // (5 before: 4 x 4 elements a thread, scalar loads, no loads ahead); one row: 5.3 TB/s of weights (a prompt of 300 rows and
 // four rows behind it, two layers and the head: 44.3 ms of products before, 9.8 now). Operands whose rows are no multiples of 16
-// bytes, and bfloat16 ones, are loaded value by value into the same ring.
+// bytes are loaded value by value into the same ring. So are bfloat16 ones, or four at a time where rows and pieces allow; theirs wait
+// in registers while the step in hand is worked on.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -32,6 +33,29 @@ constexpr int BK = 32, GROUPS = 4, THREADS = 128;
 
 __device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// four bfloat16 values as they lie in memory
+struct Four {
+    uint2 v;
+    __device__ __forceinline__ float4 floats() const {
+        return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                           __uint_as_float(v.y & 0xffff0000u));
+    }
+};
+// the values k .. k + 3 of a row in front of `end`, zeros behind it; `whole`: the four lie inside or outside together, aligned
+__device__ __forceinline__ Four fetch4(const __nv_bfloat16* p, int k, int end, int whole) {
+    Four x = {make_uint2(0u, 0u)};
+    if (whole) {
+        if (k < end) x.v = *reinterpret_cast<const uint2*>(p + k);
+    } else {
+        const uint16_t* u = reinterpret_cast<const uint16_t*>(p);
+        if (k + 0 < end) x.v.x = u[k];
+        if (k + 1 < end) x.v.x |= (uint32_t)u[k + 1] << 16;
+        if (k + 2 < end) x.v.y = u[k + 2];
+        if (k + 3 < end) x.v.y |= (uint32_t)u[k + 3] << 16;
+    }
+    return x;
 }
 
 __device__ __forceinline__ void copy16(uint32_t smem, const void* p, bool inside) {
@@ -46,8 +70,11 @@ __host__ __device__ __forceinline__ int group_size(int K) { return ((K + GROUPS 
 template <int TI, int TJ, int WM, int WN, int STAGES, typename Tin, typename Tout, bool WIDE>
 __global__ void __cluster_dims__(GROUPS, 1, 1) __launch_bounds__(THREADS)
 gemm_plain_kernel(const Tin* __restrict__ a, int lda, const Tin* __restrict__ w, int ldw, VecRef bias, int has_bias,
-                  Tout* __restrict__ out, int ldo, int accumulate, int M, int N, int K, int row_tiles) {
+                  Tout* __restrict__ out, int ldo, int accumulate, int M, int N, int K, int row_tiles, int whole) {
     constexpr int BM = 4 * TI * WM, BN = 8 * TJ * WN, ROWS = BM + BN, STAGE = ROWS * BK;
+    constexpr int PIECES = (ROWS * 8 + THREADS - 1) / THREADS;
+    constexpr bool HELD = sizeof(Tin) == 2;
+    constexpr int AHEAD = HELD ? 1 : STAGES - 1;         // steps between a load and the step in hand
     static_assert(32 * WM * WN == THREADS, "four warps");
     extern __shared__ __align__(128) float smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -56,12 +83,13 @@ gemm_plain_kernel(const Tin* __restrict__ a, int lda, const Tin* __restrict__ w,
     const int per = group_size(K), k_lo = min(K, group * per), k_hi = min(K, k_lo + per);
     const int steps = (k_hi - k_lo + BK - 1) / BK;
 
-    // stage `s` takes the k values from k_lo + step * BK on: rows [0, BM) are a's, the rest w's
+    // stage `s` takes the k values from k_lo + step * BK on: rows [0, BM) are a's, the rest w's (HELD: they are fetched here and `put` there)
+    Four held[HELD ? PIECES : 1];
     auto load = [&](int step, int s) {
         const int kb = k_lo + step * BK;
         float* to = smem + s * STAGE;
 #pragma unroll
-        for (int i = 0; i < (ROWS * 8 + THREADS - 1) / THREADS; ++i) {
+        for (int i = 0; i < PIECES; ++i) {
             const int u = tid + i * THREADS, r = u >> 3, c = u & 7;
             if (ROWS * 8 % THREADS != 0 && u >= ROWS * 8) break;
             const int k = kb + c * 4, row = r < BM ? m0 + r : n0 + r - BM;
@@ -71,6 +99,8 @@ gemm_plain_kernel(const Tin* __restrict__ a, int lda, const Tin* __restrict__ w,
             if constexpr (WIDE) {
                 const bool inside = there && k < k_hi;
                 copy16((uint32_t)__cvta_generic_to_shared(dst), inside ? p + k : p, inside);
+            } else if constexpr (HELD) {
+                held[i] = fetch4(p, k, there ? k_hi : 0, whole);
             } else {
                 float4 v;
                 v.x = there && k + 0 < k_hi ? to_float(p[k + 0]) : 0.f;
@@ -78,6 +108,16 @@ gemm_plain_kernel(const Tin* __restrict__ a, int lda, const Tin* __restrict__ w,
                 v.z = there && k + 2 < k_hi ? to_float(p[k + 2]) : 0.f;
                 v.w = there && k + 3 < k_hi ? to_float(p[k + 3]) : 0.f;
                 *reinterpret_cast<float4*>(dst) = v;
+            }
+        }
+    };
+    auto put = [&](int s) {
+        if constexpr (HELD) {
+#pragma unroll
+            for (int i = 0; i < PIECES; ++i) {
+                const int u = tid + i * THREADS, r = u >> 3, c = u & 7;
+                if (ROWS * 8 % THREADS != 0 && u >= ROWS * 8) break;
+                *reinterpret_cast<float4*>(smem + s * STAGE + r * BK + ((c ^ (r & 7)) << 2)) = held[i].floats();
             }
         }
     };
@@ -98,15 +138,18 @@ gemm_plain_kernel(const Tin* __restrict__ a, int lda, const Tin* __restrict__ w,
         for (int j = 0; j < TJ; ++j) acc[i][j] = 0;
 
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < steps) load(s, s);
+    for (int s = 0; s < AHEAD; ++s) {
+        if (s < steps) {
+            load(s, s);
+            put(s);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     const int ar = (warp / WN) * 4 * TI + (lane >> 3), wr = BM + (warp % WN) * 8 * TJ + (lane & 7);
     for (int step = 0; step < steps; ++step) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
         __syncthreads();
-        if (step + STAGES - 1 < steps) load(step + STAGES - 1, (step + STAGES - 1) % STAGES);
+        if (step + AHEAD < steps) load(step + AHEAD, (step + AHEAD) % STAGES);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* s = smem + (step % STAGES) * STAGE;
 #pragma unroll
@@ -124,6 +167,7 @@ gemm_plain_kernel(const Tin* __restrict__ a, int lda, const Tin* __restrict__ w,
                 for (int j = 0; j < TJ; ++j) fma2(acc[i][j], av.y, wv[j].y);
             }
         }
+        if (HELD && step + AHEAD < steps) put((step + AHEAD) % STAGES);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -166,34 +210,33 @@ int launch_tile(const void* a, int lda, const void* w, int ldw, VecRef bias, int
     constexpr int BM = 4 * TI * WM, BN = 8 * TJ * WN;
     constexpr size_t smem = (size_t)STAGES * (BM + BN) * BK * sizeof(float);
     auto kernel = gemm_plain_kernel<TI, TJ, WM, WN, STAGES, Tin, Tout, WIDE>;
-    static bool asked[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return jllm_fail(JLLM_CUDA_ERROR, "gemm: no current device");
-    if (!asked[dev]) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return jllm_check_launch("gemm_plain");
-        asked[dev] = true;
-    }
+    if (jllm_allow_smem((const void*)kernel, smem) != cudaSuccess) return jllm_check_launch("gemm_plain");
     const long long row_tiles = (M + BM - 1) / BM, tiles = row_tiles * ((N + BN - 1) / BN);
     JLLM_REQUIRE(tiles <= 0x7fffffffll / GROUPS, "gemm: M=%d N=%d are too many tiles", M, N);
+    const size_t piece = 4 * sizeof(Tin);
+    const int whole = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)a % piece == 0 && (uintptr_t)w % piece == 0;
     if (jllm_launch(kernel, dim3((unsigned)(tiles * GROUPS)), dim3(THREADS), smem, stream, LAUNCH_DEPENDENT, (const Tin*)a, lda,
-                    (const Tin*)w, ldw, bias, has_bias, (Tout*)out, ldo, accumulate, M, N, K, (int)row_tiles) != cudaSuccess)
+                    (const Tin*)w, ldw, bias, has_bias, (Tout*)out, ldo, accumulate, M, N, K, (int)row_tiles, whole) != cudaSuccess)
         return jllm_check_launch("gemm_plain");
     return jllm_check_launch("gemm_plain");
 }
 
 // The tile for M rows. A tile of 64 rows reads least from shared memory per multiply-add; the smaller ones are for products
 // that would leave most of it empty: up to 4 and 16 rows the weights' stream is the bound (more, smaller tiles keep more
-// bytes on their way), up to 32 rows, and where 32-row tiles leave a fifth fewer rows empty, the multiply-adds.
+// bytes on their way), up to 32 rows, and where 32-row tiles leave a fifth fewer rows empty, the multiply-adds. Where even the blocks
+// of 16-row tiles are on the SMs at once, a larger tile only makes the few blocks longer (64 rows, 48 x 32: 7.9 us in one tile, 3.9
+// in four); of a short k two such blocks share an SM and wait together (300 rows, 300 x 64, bfloat16: 10.3 us in 64-row tiles).
 template <typename Tin, typename Tout, bool WIDE>
 int launch(const void* a, int lda, const void* w, int ldw, VecRef bias, int has_bias, void* out, int ldo, int accumulate, int M,
            int N, int K, cudaStream_t stream) {
     if (M <= 4) return launch_tile<1, 2, 1, 4, 6, Tin, Tout, WIDE>(a, lda, w, ldw, bias, has_bias, out, ldo, accumulate, M, N, K, stream);
-    if (M <= 16) return launch_tile<4, 4, 1, 4, 4, Tin, Tout, WIDE>(a, lda, w, ldw, bias, has_bias, out, ldo, accumulate, M, N, K, stream);
+    const int sms = jllm_device_sm_count();
+    if (M <= 16 || (M + 15ll) / 16 * ((N + 127ll) / 128) * GROUPS <= (K <= 128 ? 2 : 1) * sms)
+        return launch_tile<4, 4, 1, 4, 4, Tin, Tout, WIDE>(a, lda, w, ldw, bias, has_bias, out, ldo, accumulate, M, N, K, stream);
     const long long in32 = (M + 31) / 32 * 32ll, in64 = (M + 63) / 64 * 64ll;
-    if (in32 * 6 <= in64 * 5)
-        return launch_tile<8, 4, 1, 4, 3, Tin, Tout, WIDE>(a, lda, w, ldw, bias, has_bias, out, ldo, accumulate, M, N, K, stream);
-    return launch_tile<8, 8, 2, 2, 3, Tin, Tout, WIDE>(a, lda, w, ldw, bias, has_bias, out, ldo, accumulate, M, N, K, stream);
+    if (in32 * 6 > in64 * 5)
+        return launch_tile<8, 8, 2, 2, 3, Tin, Tout, WIDE>(a, lda, w, ldw, bias, has_bias, out, ldo, accumulate, M, N, K, stream);
+    return launch_tile<8, 4, 1, 4, 3, Tin, Tout, WIDE>(a, lda, w, ldw, bias, has_bias, out, ldo, accumulate, M, N, K, stream);
 }
 
 bool wide_rows(const void* p, int stride) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && stride % 4 == 0; }

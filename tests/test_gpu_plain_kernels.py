@@ -46,6 +46,50 @@ def test_product_of_every_tile_and_loader(ops, N, K):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K", [(100, 1), (100, 7), (129, 32), (3, 100), (100, 128), (130, 129)])
+def test_product_of_a_short_k(ops, dtype, N, K):
+    """Groups of few or no k; products whose 16-row tiles are on the SMs at once (70 rows) and larger ones (2,560). Bias, residual,
+    bfloat16 results, operands in rows of another stride: a row has the same bits in all of them."""
+    M, few = 16 * 160, 70
+    a, w, bias = rnd(M, K).to(dtype), rnd(N, K, seed=1).to(dtype), rnd(N, seed=2)
+    base = rnd(M, N, seed=3)
+    full, part = base.clone(), torch.full((few + 1, N + 3), 7.0, device=DEV)
+    part[:few, :N] = base[:few]
+    ops.gemm_plain(a, w, full, bias, accumulate=True)
+    ops.gemm_plain(a[:few], w, part[:few, :N], bias, accumulate=True)
+    assert torch.equal(part[:few, :N], full[:few]) and bool((part[few] == 7).all()) and bool((part[:, N:] == 7).all())
+    want = a.double() @ w.double().T + bias.double() + base.double()
+    bound = (K / 8 + 8) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T + bias.abs().double() + base.abs().double())
+    assert bool(((full.double() - want).abs() <= bound).all())
+    odd_a, odd_w = torch.zeros(M, K + 1, device=DEV, dtype=dtype), torch.zeros(N, K + 3, device=DEV, dtype=dtype)
+    odd_a[:, :K], odd_w[:, :K] = a, w
+    for rows in (1, few, M):
+        out = base[:rows].clone()
+        ops.gemm_plain(odd_a[:rows, :K], odd_w[:, :K], out, bias, accumulate=True)
+        assert torch.equal(out, full[:rows]), rows
+    if dtype == torch.bfloat16:
+        out, many = torch.empty(few, N, device=DEV, dtype=dtype), torch.empty(M, N, device=DEV, dtype=dtype)
+        ops.gemm_plain(a[:few], w, out)
+        ops.gemm_plain(a, w, many)
+        assert torch.equal(out, many[:few])
+
+
+@pytest.mark.parametrize("N,K", [(65, 515), (129, 1028), (300, 333)])
+def test_product_of_bfloat16_operands(ops, N, K):
+    """The loader by way of registers, four values at a time and value by value, in all tiles: the bits of the float32 loader."""
+    a, w = rnd(150, K).bfloat16(), rnd(N, K, seed=1).bfloat16()
+    odd_a, odd_w = torch.zeros(150, K + 1, device=DEV, dtype=torch.bfloat16), torch.zeros(N, K + 3, device=DEV, dtype=torch.bfloat16)
+    odd_a[:, :K], odd_w[:, :K] = a, w
+    want = torch.empty(150, N, device=DEV)
+    ops.gemm_plain(a.float(), w.float(), want)
+    for M in (1, 4, 5, 16, 17, 33, 64, 97, 150):
+        out, odd = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+        ops.gemm_plain(a[:M], w, out)
+        ops.gemm_plain(odd_a[:M, :K], odd_w[:, :K], odd)
+        assert torch.equal(out, want[:M]) and torch.equal(odd, want[:M]), M
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,G,dk,dv,window,keep", [(4, 4, 16, 16, 0, 0), (8, 2, 128, 128, 0, 0), (6, 1, 50, 140, 0, 0), (5, 1, 260, 300, 0, 0),
                                                    (6, 3, 72, 64, 70, 9), (4, 1, 64, 64, -96, 0)])
 def test_attention_of_shared_rows(ops, dtype, H, G, dk, dv, window, keep):
