@@ -349,7 +349,8 @@ int decode_split(const void* q, int q_stride, const void* k_cache, const void* v
     staged::launch<HD>(q, q_stride, k_cache, v_cache, out, out_stride, row_seg, row_pos, block_tables, table_stride, \
                        rows, heads, kv_heads, page_size, window, scale_log2, splits, part_o, part_ml, counters, fresh, stream, \
                        keep_first, sk, cap)
-        if (ring::fits(heads, kv_heads, head_dim, page_size, window, keep_first)) {
+        const bool by_ring = ring::fits(heads, kv_heads, head_dim, page_size, window, keep_first);
+        if (by_ring) {
             const ring::Args a{(const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, row_seg, row_pos, block_tables,
                                table_stride, rows, heads, kv_heads, page_size, 0, 0, window, scale_log2, splits, part_o, part_ml,
                                counters, fresh, sk, has_sink, cap, nullptr};
@@ -358,7 +359,7 @@ int decode_split(const void* q, int q_stride, const void* k_cache, const void* v
             if (rc != JLLM_OK) return rc;
         } else if (head_dim == 64) JLLM_STAGED(64); else if (head_dim == 128) JLLM_STAGED(128); else JLLM_STAGED(256);
 #undef JLLM_STAGED
-        int rc2 = jllm_check_launch("attention_decode_staged");
+        int rc2 = jllm_check_launch(by_ring ? "attention_decode_ring" : "attention_decode_staged");
         if (rc2 != JLLM_OK || splits == 1 || counters != nullptr) return rc2;
         jllm_launch(attention_combine_kernel, dim3(rows, heads), dim3(128), 0, stream, true, (const float*)part_o,
                     (const float*)part_ml, (__nv_bfloat16*)out, out_stride, heads, head_dim, splits, sk, has_sink);

@@ -1184,16 +1184,27 @@ def bounds_errors() -> dict:
     return out
 
 
+# Which kernel a code in an error word is from: the products share one word, the attention kernels another.
+WAIT_KERNELS = {"products": ((1, 3, "gemm_tcgen05"), (11, 13, "gemm_stream"), (14, 16, "gemm_stream (clusters)"), (21, 23, "gemm_pair")),
+                "attention": ((21, 23, "attention_prefill_tc"), (31, 33, "attention_prefill_pair"), (41, 43, "attention_prefill_latent"),
+                              (51, 52, "attention_decode_ring"))}
+
+
+def wait_kernel(word: str, code: int) -> str:
+    """The kernel that raised `code` in the error word of the `products` or the `attention`."""
+    return next((name for lo, hi, name in WAIT_KERNELS[word] if lo <= code <= hi), f"a kernel of the {word}")
+
+
 def check_kernel_errors() -> None:
     """Raises if a tcgen05 kernel gave up on one of its bounded waits since the last check (its results are then
     not to be trusted), or, in the build with bounds checks, if a kernel was handed a table index, page id, cache
     slot or token id outside its array (the access was skipped). Reads a few words from the device, so it
     synchronises."""
     lib = library()
-    raised = {name: code for name, code in (("gemm_tcgen05", lib.jllm_gemm_tcgen05_error()),
-                                            ("attention_prefill_tc", lib.jllm_attention_prefill_tc_error())) if code}
+    raised = [f"{wait_kernel(word, code)} (code {code})" for word, code in (("products", lib.jllm_gemm_tcgen05_error()),
+                                                                            ("attention", lib.jllm_attention_prefill_tc_error())) if code]
     if raised:
-        raise KernelError("a bounded wait ran out inside " + ", ".join(f"{k} (code {v})" for k, v in raised.items()))
+        raise KernelError("a bounded wait ran out inside " + ", ".join(raised))
     if checks_bounds():
         caught = bounds_errors()
         if caught:

@@ -100,3 +100,33 @@ def test_what_the_recurrence_chunks_take_is_asked_once_per_shape(monkeypatch):
     monkeypatch.setattr(ops, "library", lambda: (_ for _ in ()).throw(AssertionError("the library was asked again")))
     assert plan(64, 1, 64, 64, 8, 128, 64) == (0, 1)
     ops._chunk_plan.cache_clear()
+
+
+def test_a_wait_that_ran_out_is_reported_with_its_kernel(monkeypatch):
+    """Every code that a kernel's source raises in an error word is named as that kernel's, and the report says so."""
+    import re
+    from pathlib import Path
+
+    import pytest
+    folder, seen = Path(ops.__file__).parent, 0
+    for file in sorted(list(folder.glob("*.cu")) + list(folder.glob("*.cuh"))):
+        text = file.read_text()
+        codes = [int(c) for c in re.findall(r"atomicExch\((?:a\.)?error_word, (?:warp == 4 \? )?(\d+)", text) + re.findall(r"give_up\((\d+)\)", text)
+                 + re.findall(r"warp == 4 \? \d+ : (\d+)\)", text)]
+        for code in codes:
+            word = "products" if file.stem.startswith("gemm") else "attention"
+            assert ops.wait_kernel(word, code).split()[0] == file.stem, (file.name, code)
+        seen += len(codes)
+    assert seen >= 25
+
+    class Fake:
+        def __init__(self, products, attention):
+            self.jllm_gemm_tcgen05_error, self.jllm_attention_prefill_tc_error = lambda: products, lambda: attention
+            self.jllm_checks_bounds = lambda: 0
+    for products, attention, what in ((16, 0, r"inside gemm_stream \(clusters\) \(code 16\)$"), (0, 51, r"inside attention_decode_ring \(code 51\)$"),
+                                      (2, 43, r"gemm_tcgen05 \(code 2\), attention_prefill_latent \(code 43\)$")):
+        monkeypatch.setattr(ops, "library", lambda: Fake(products, attention))
+        with pytest.raises(ops.KernelError, match=what):
+            ops.check_kernel_errors()
+    monkeypatch.setattr(ops, "library", lambda: Fake(0, 0))
+    ops.check_kernel_errors()
