@@ -85,7 +85,7 @@ def main() -> int:
         tol = dict(rtol=1e-4, atol=2e-5) if dtype == torch.float32 else dict(rtol=2e-2, atol=2e-2)
         assert torch.allclose(out.float().cpu(), want, **tol), (name, hd)
         ops.check_kernel_errors()
-        print(f"ok: {name} head size {hd}" if name != "latent" else f"and {name}, head size {hd}")
+        print(f"ok: {name} head size {hd}" if name != "latent" else f"right again: {name}")
 
     # ---- the decode attention that makes its own rows' keys and values: a spoilt page of the newest position is neither
     # read nor written; afterwards the same bits as the row-wise kernel followed by the attention ----------------------
@@ -154,6 +154,37 @@ def main() -> int:
         good = [r for r in range(R) if r not in (5, 9)]
         assert torch.equal(flat[good], v_in[good]) and float(flat[5].abs().max()) == 0 and float(flat[9].abs().max()) == 0
         print(f"ok: cache write head size {hd}")
+
+    # ---- the recurrence's chunks: a state slot beyond the states is neither read nor written, whether its segment is walked (20
+    # rows) or takes the three launches (1,400), and the other segments are right ----------------------------------------
+    lens, H, dk, dv = [1400, 20, 1000], 4, 64, 64
+    R = sum(lens)
+    buf = torch.randn(R, H * (2 * dk + dv), device=DEV).bfloat16()
+    la, b = -torch.rand(R, H, device=DEV) * 0.1, torch.rand(R, H, device=DEV)
+
+    class Step:
+        seg_start, seg_len, max_q_len = i32([0, 1400, 1420]), i32(lens), 1400
+
+    def chunks(slots):
+        Step.state_slots = i32(slots)
+        state, out = torch.ones(3, H, dk, dv, device=DEV), torch.full((R, H * dv), 7.0, device=DEV)
+        assert ops.scalar_gated_chunked(buf, 0, H, buf, H * dk, H, buf, 2 * H * dk, la, b, state, Step, out, H, dk, dv)
+        torch.cuda.synchronize()
+        return state, out
+
+    good = chunks([2, 0, 1])
+    assert ops.bounds_errors() == {}
+    for bad, slots in ((0, [3, 0, 1]), (1, [2, -1, 1])):
+        state, out = chunks(slots)
+        caught("chunk_scan", "a cache slot")
+        at, n = int(Step.seg_start[bad]), lens[bad]
+        keep = torch.arange(R, device=DEV)
+        keep = keep[(keep < at) | (keep >= at + n)]
+        assert torch.equal(out[keep], good[1][keep]) and bool((out[at:at + n] == 7).all())
+        untouched = [2, 0, 1][bad]
+        assert bool((state[untouched] == 1).all())
+        assert all(torch.equal(state[s], good[0][s]) for s in range(3) if s != untouched)
+    print("right again: chunks")
 
     # ---- token ids: clamped as always, and reported here ----------------------------------------------------------
     table = torch.randn(50, 24, device=DEV)

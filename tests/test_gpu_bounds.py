@@ -32,6 +32,7 @@ def test_bad_tables_slots_and_tokens_are_skipped_and_reported():
                           capture_output=True, text=True, timeout=900)
     assert proc.returncode == 0, (proc.stdout[-3000:], proc.stderr[-3000:])
     assert proc.stdout.count("ok:") == 10, proc.stdout
+    assert [line for line in proc.stdout.splitlines() if line.startswith("right again:")] == ["right again: latent", "right again: chunks"]
 
 
 def test_replay_traces_run_clean_under_the_checked_library():

@@ -610,6 +610,30 @@ def test_attention_decode_tiles_and_pages(ops, H, Hkv, hd, page, window):
         assert ops.attention_prefill_tc_error() == 0
 
 
+@pytest.mark.parametrize("H,Hkv,hd,page,window", [(8, 1, 128, 16, 0), (6, 2, 64, 32, 0), (5, 1, 128, 16, -96), (4, 4, 64, 64, -64)])
+@pytest.mark.parametrize("splits", [1, 3, 8, 12])
+def test_attention_decode_with_a_sink(ops, H, Hkv, hd, page, window, splits):
+    """A number per query head in the softmax's denominator where the tiles come by TMA (all keys, chunks of whole pages): one block
+    per pair, parts that the last block adds up, parts that a kernel of their own adds up; sinks among the scores, far above and far
+    below all of them. Against float64."""
+    lens, scale = [1, 16, 64, 65, 130, 193, 700], 1.0 / math.sqrt(hd)
+    q, kc, vc, _, rseg, rpos, tables, _, _ = attention_case(ops, torch.bfloat16, H, Hkv, hd, page, lens, 0, scale, "far", [1] * len(lens))
+    R, sink = len(lens), torch.randn(H, generator=torch.Generator().manual_seed(H)).to(DEV)
+    sink[0], sink[-1] = 80.0, -80.0
+    scratch = torch.full((ops.attention_decode_scratch_floats(R, H, hd, splits) + 1,), float("nan"), device=DEV)
+    out = torch.full_like(q, float("nan"))
+    ops.attention_decode_extras(q, kc, vc, out, rseg, rpos, tables, R, H, Hkv, hd, page, window, scale, splits, scratch, 0, sink)
+    assert ops.attention_prefill_tc_error() == 0
+    want = torch.empty(R, H, hd, dtype=torch.float64)
+    for r, n in enumerate(lens):
+        at = torch.arange(n - 1 - (n - 1) % -window if window else 0, n, device=DEV)
+        keys, values = (t[tables[r][at // page].long(), :, at % page].double().repeat_interleave(H // Hkv, 1) for t in (kc, vc))
+        x = torch.cat([torch.einsum("hd,jhd->hj", q[r].double().view(H, hd), keys) * scale, sink.double()[:, None]], 1)
+        want[r] = torch.einsum("hj,jhd->hd", torch.softmax(x, 1)[:, :-1], values).cpu()
+    assert float(out.view(R, H, hd)[:, 0].float().abs().max()) < 1e-3                # all of the weight is the sink's
+    rows_close(out, want.reshape(R, H * hd).float(), f"sink {splits}")
+
+
 @pytest.mark.parametrize("splits", [1, 3, 8])
 @pytest.mark.parametrize("H,Hkv,hd,page,window", [(6, 2, 48, 16, 0), (4, 4, 16, 4, 0), (32, 8, 128, 16, 0),
                                                    (6, 3, 80, 8, 21), (16, 1, 256, 16, 0), (2, 1, 32, 1, 7),
