@@ -12,9 +12,12 @@
 // beside the products of its neighbours. Two softmax warpgroups share a tile's columns (64 each, the row's maximum exchanged
 // through shared memory): one warp a scheduler alone is bound by the latency of its own chain of 128 exponentials.
 // The MMAs of one thread complete in order, so S_(j+2) may overwrite P_j once O += P_j K_j has been issued.
-// What bounds it: per key tile the two products (2,048 clocks on the tensor cores, as many of shared-memory reads) beside
-// 1,024 clocks of exponentials. A causal prompt of 2,048 rows x 16 heads: 274 us on mma.sync (attention_prefill.cu, which
-// fetches every row twice and keeps 64-key tiles), 62 us here (54 where 192 of the 256 columns are read).
+// What bounds it is a block's chain, not a unit: a key tile's products are 2,048 clocks on the tensor cores and as many of
+// shared-memory reads, its exponentials 1,024, and a tile takes 2.7 us (5,200 clocks; 16 heads of 128 rows over 8,000 keys, 16
+// blocks, 179 us; over none 8.8): scores, their maxima, the exponentials and the next product wait for one another with one
+// block to an SM, and only neighbouring tiles overlap. A causal prompt of 2,048 rows x 16 heads: 274 us on mma.sync
+// (attention_prefill.cu, which fetches every row twice and keeps 64-key tiles), 62 us here, 54 where 192 of the 256 columns are
+// read: 2,176 key tiles over 148 SMs are 40 of them, the rest is the blocks' starts and ends and the uneven last ones.
 // Every mbarrier wait is bounded; the softmax threads agree at the exchange of the maxima whether to go on.
 //
 // Requirements: bfloat16, rows of 256 values, page_size a power of two <= 128, 16-byte aligned q rows.

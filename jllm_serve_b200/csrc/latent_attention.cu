@@ -510,7 +510,10 @@ JLLM_EXPORT int jllm_gemm_heads(const void* a, int dtype, int lda, const void* w
         return jllm_check_launch("gemm_heads");
     }
     const bool vec = K % 8 == 0 && lda % 8 == 0 && a_head % 8 == 0 && ((uintptr_t)a % 16) == 0 && ((uintptr_t)w % 16) == 0;
-    if (vec && M > 64) {        // (up to 64 rows the small tiles give more blocks)
+    // (Up to 64 rows a 128-row tile would be half empty. From 65 on it is the faster one however few the blocks, launched back to back:
+    // 65 rows x 16 heads of 128 -> 192 values and 64 rotated ones 9.5 us on 64 x 64 tiles and 3.4 here, 256 rows 10.4 and 3.7, four
+    // heads 9.3 and 3.4; 65 rows x 16 heads of 192 -> 128 6.4 and 4.0.)
+    if (vec && M > 64) {
         const int wide_out = ldo % 8 == 0 && o_head % 8 == 0 && N % 8 == 0 && ((uintptr_t)out % 16) == 0;
         const int wide_rope = wide_out && rope_dim % 8 == 0 && rotary_dim % 8 == 0 && ((uintptr_t)cos_t % 16) == 0 && ((uintptr_t)sin_t % 16) == 0;
         if (jllm_allow_smem((const void*)many::gemm_heads_many_kernel, many::SMEM) != cudaSuccess)

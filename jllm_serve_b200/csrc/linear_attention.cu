@@ -660,7 +660,9 @@ gated_norm_vec_kernel(const float* __restrict__ o, const TG* __restrict__ gate, 
 }
 
 // launches it where it takes the shape: 1,024 rows x heads and more (fewer leave SMs idle: the kernel below gives a block to each), whole
-// pieces of four values
+// pieces of four values. At 1,024 rows x heads, float32 gate, launched back to back, the general kernels and this one: 128 values 2.8 and
+// 2.0 us, 256 3.4 and 2.5, 512 4.2 and 3.5, 1,024 5.9 and 4.1, 2,048 9.3 and 5.2, 4,096 15.9 and 8.2, 8,192 37.6 and 20.4; at 4,096
+// 512 values 6.9 and 4.9, 2,048 30.2 and 14.6, 8,192 167 and 72.
 template <typename T, typename TG>
 bool launch_gated_norm_vec(const float* o, const TG* gate, int ld_gate, VecRef gain, T* y, long long total, int heads, int dv, float eps,
                            float scale, int gate_kind, cudaStream_t stream) {

@@ -985,9 +985,11 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
     wide = rows >= 16 and out_features >= WIDE_ROWS and tiles_fit
     if tiles_fit and not wide and 16 < rows <= 128 and (out_features * in_features * 2 >= SWAP_MIN_BYTES or rows > 40):
         return "swap"
-    # 129 to 256 rows (the tokens are still one tcgen05 N side): the parked parts grow with the rows, so it keeps only
-    # what the tiles kernel is worst at, matrices much longer than high (down: 12,288 k for 4,096 rows; 31 to 41 us
-    # against 58), and everything up to 160 rows (QKV 20 to 22 us against 23, O 19 to 20 against 22)
+    # 129 to 256 rows (the tokens are still one tcgen05 N side): what the tiles kernel is worst at, matrices much longer than
+    # high (down: 12,288 k for 4,096 rows; 160, 200, 256 rows 28.6, 32.9, 37.7 us against 59), and everything up to 160 rows
+    # (QKV 22.7 us against 24.6, O 16.3 against 22.8; at 200 rows QKV 26.2 against 24.8). The lines of O were drawn before a
+    # cluster took a tile of it: since then swap is ahead of the row kernel from 17 rows on (24 rows 10.3 us against 12.3, 40 rows
+    # 11.5 against 18.2) and of the tiles up to 256 (200 rows 19.1 against 22.7, 256 rows 21.3 against 22.8).
     if tiles_fit and not wide and 128 < rows <= SWAP_MAX_ROWS and (rows <= 160 or in_features >= 2 * out_features):
         return "swap"
     if rows <= min(SMALL_M_ROWS, 64) and rows_fit and not wide:
@@ -1290,7 +1292,10 @@ def decode_plan(rows, kv_heads, kv_bucket, heads, head_dim, scratch, places: int
     when there are more (row, kv head) pairs than places for blocks (`places`, by default two per SM of the device)
     and they would fill the last round of places
     badly (by less than 93 %), the key tiles of all pairs dealt out evenly over as many blocks as there are places
-    (with fewer pairs than places the even deal is the slower one). `kv_bucket` = the longest request's keys in
+    (with fewer pairs than places the even deal is the slower one). 32 heads of 128 over 8, launched back to back, 4,096 keys: 8 rows
+    25.0 us in the 4 splits this takes, 28.0 in 3, 31.7 dealt out; 16 rows 43.6 in 2, 50.3 dealt out; 32 rows 77.8 whole, 86.5 dealt
+    out; 64 rows of equal lengths 150 whole, 158 dealt out, which ragged rows turn round; one row 7.4 in 16, 7.9 in the 32 it
+    takes. `kv_bucket` = the longest request's keys in
     units of 256."""
     places = places or resident_blocks()
     splits = decode_splits(rows, kv_heads, kv_bucket, heads, head_dim, scratch, places)
