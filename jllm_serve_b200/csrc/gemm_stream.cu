@@ -369,6 +369,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
 // `overlay`: the parts lie over the ring (many tokens leave no room beside it); the cluster then meets once more, when every block
 // is done with its ring, before anything is written.
 constexpr int CLUSTER_MAX = 8;
+constexpr double MEETING_K_BLOCKS = 16;         // k blocks an SM streams in the time of a meeting in the workspace (5 to 6 us)
 
 __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -602,13 +603,13 @@ ClusterCut cluster_of(int n, int ntok, int tiles, int k_blocks, int out_dtype) {
     return tiles <= resident ? one : ClusterCut{};
 }
 
-// A cluster to a tile where the clusters of all tiles are resident at once and it costs less than equal runs; of the sizes that fit, the
-// cheapest. Costs are in k blocks that an SM streams (0.3 to 0.4 us): a block's own, and what the meetings take. In the workspace that
-// is 10 to 16, more where a tile falls to more blocks; in a cluster half a k block for every block of it and a third more where the
-// cluster meets twice (`overlay`); tokens, which either has to add up, cost a cluster of one nothing. Equal runs and clusters, launched
-// back to back: 2,048 x 8,192 (six to a cluster), 64 rows 15.0 and 12.6 us; 7,168 x 5,120 (two), 128 rows 27.1 and 25.3; 12,288 x 2,048
-// (one), 32 rows 15.4 and 15.9, 128 rows 28.2 and 26.7; 6,144 x 4,096 (two, 96 of the SMs), 32 rows 14.7 and 14.6, 128 rows 20.0 and
-// 21.3; 2,048 x 12,288 (six), 64 rows 16.4 and 15.8, 128 rows, with overlay, 17.8 and 19.0.
+// A cluster to a tile where the clusters of all tiles are resident at once and a block's k blocks take no longer than an equal run and
+// the meeting it saves; of the sizes that fit, the one with the fewest k blocks a block (a larger cluster meets for longer). The meeting
+// counts what it costs in a step, more than back to back, where the next product's start hides it: QKV (6,144 x 4,096, two blocks to a
+// cluster) at 64 rows takes 16.4 us in equal runs and 16.8 in clusters launched back to back, and a decode step of 64 requests,
+// eight layers, 1,621 us with it in equal runs and 1,587 in clusters (a prompt of 47 rows 1,092 and 1,067). Back to back, equal runs and
+// clusters: 2,048 x 8,192 (six), 64 rows 15.0 and 12.6 us; 7,168 x 5,120 (two), 128 rows 27.1 and 25.3; 12,288 x 2,048 (one), 32 rows
+// 15.4 and 15.9, 128 rows 28.2 and 26.7; 6,144 x 4,096, 128 rows 20.0 and 21.3; 2,048 x 12,288 (six), 64 rows 16.4 and 15.8, 128 17.8 and 19.0.
 // (The driver is asked once per shape and device: the choice is kept.)
 ClusterCut choose_cluster(int ntok, int tiles, int k_blocks, int out_dtype, int sms) {
     static std::mutex mu;
@@ -621,10 +622,9 @@ ClusterCut choose_cluster(int ntok, int tiles, int k_blocks, int out_dtype, int 
     const auto it = known.find(key);
     if (it != known.end()) return it->second;
     ClusterCut c{};
-    const double tokens = ntok / 40., meeting = 8.5 + 1.1 * sms / tiles;
-    double best = (double)tiles * k_blocks / sms + (meeting < 16. ? meeting : 16.) + tokens;
+    double best = (double)tiles * k_blocks / sms + MEETING_K_BLOCKS;
     for (int n = 1; n <= CLUSTER_MAX && n <= k_blocks; ++n) {
-        const double cost = (k_blocks + n - 1) / n + 0.5 * n + (n > 1 ? tokens : 0.) + (cluster_cut(n, ntok).overlay ? n / 3. : 0.);
+        const double cost = (k_blocks + n - 1) / n + 0.5 * n;
         if (cost >= best) continue;
         const ClusterCut one = cluster_of(n, ntok, tiles, k_blocks, out_dtype);
         if (one.blocks > 0) best = cost, c = one;
