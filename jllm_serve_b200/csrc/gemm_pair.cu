@@ -109,7 +109,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t fix_bar = bars + 8u * (2 * STAGES + 4) + 16u;   // parked parts arriving by bulk copy (behind the three words)
     uint8_t* staging = aligned + STAGES * STAGE_BYTES;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();             // 0: the pair's first block, which issues the MMAs
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int tiles_m = (M + PAIR_M - 1) / PAIR_M, tiles_n = (N + BN - 1) / BN, tiles = tiles_m * tiles_n;
@@ -187,7 +187,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
     if (warp == 0) {
         // ---------------- producer (both blocks) ----------------
-        if (lane == 0) {
+        {
+            const uint32_t first_full = in_block(full_bar(0), 0);
             int s = 0;
             uint32_t parity = 1, dst = base;
             bool ok = true;
@@ -199,45 +200,53 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 const uint32_t tx = 2 * A_BYTES + (tn + 1 < packed_tiles ? 2 : 1) * W_BYTES;     // both blocks' bytes
                 int wy = ((tn + (int)rank) * k_blocks + lo) * 128;         // row of the packed weight's k block
                 for (int kb = lo; kb < hi; ++kb, wy += 128) {
-                    if (!mbar_wait(empty_bar(s), parity, abort_flag)) { ok = false; break; }
-                    const uint32_t full0 = in_block(full_bar(s), 0);
-                    if (rank == 0) mbar_expect_tx(full_bar(s), tx);
-                    tma_load_2d_pair(dst, &map_a, kb * BK, m0, full0);
-                    if (mine) tma_load_2d_pair(dst + A_BYTES, &map_w, 0, wy, full0);
+                    if (!warp_wait(empty_bar(s), parity, abort_flag)) { ok = false; break; }
+                    const uint32_t full0 = first_full + 8u * s;
+                    if (elect_one()) {
+                        if (rank == 0) mbar_expect_tx(full_bar(s), tx);
+                        tma_load_2d_pair(dst, &map_a, kb * BK, m0, full0);
+                        if (mine) tma_load_2d_pair(dst + A_BYTES, &map_w, 0, wy, full0);
+                    }
+                    __syncwarp();
                     dst += STAGE_BYTES;
                     if (++s == STAGES) { s = 0; parity ^= 1u; dst = base; }
                 }
             }
-            if (!ok) give_up(21);
+            if (!ok && lane == 0) give_up(21);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (the first block) ----------------
-        if (lane == 0 && rank == 0) {
-            uint32_t local_tile = 0, parity = 0, a_addr = base;
+        if (rank == 0) {
+            const uint64_t desc_a0 = smem_desc_sw128(base), desc_b0 = smem_desc_sw128(base + A_BYTES);
+            uint64_t desc_a = desc_a0, desc_b = desc_b0;          // (a stage further is an addition to the address field)
+            uint32_t local_tile = 0, parity = 0;
             int s = 0;
             bool ok = true;
             Walk walk = first_unit();
             int tile, lo, hi;
             for (; ok && next_unit(walk, tile, lo, hi); ++local_tile) {
                 const uint32_t buf = local_tile & 1u;
-                if (!mbar_wait(acc_empty_bar(buf), ((local_tile >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+                if (!warp_wait(acc_empty_bar(buf), ((local_tile >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * BN;
                 for (int kb = lo; kb < hi; ++kb) {
-                    if (!mbar_wait(full_bar(s), parity, abort_flag)) { ok = false; break; }
+                    if (!warp_wait(full_bar(s), parity, abort_flag)) { ok = false; break; }
                     tcgen05_fence_after();
-                    const uint32_t b_addr = a_addr + A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        mma_pair(tmem_d, smem_desc_sw128(a_addr + k * 32), smem_desc_sw128(b_addr + k * 32), IDESC,
-                                 (kb > lo || k > 0) ? 1u : 0u);
-                    commit_pair(empty_bar(s));          // both blocks' stage is free when these MMAs have read it
-                    a_addr += STAGE_BYTES;
-                    if (++s == STAGES) { s = 0; parity ^= 1u; a_addr = base; }
+                        for (int k = 0; k < BK / 16; ++k)
+                            mma_pair(tmem_d, desc_a + 2 * k, desc_b + 2 * k, IDESC, (kb > lo || k > 0) ? 1u : 0u);
+                        commit_pair(empty_bar(s));          // both blocks' stage is free when these MMAs have read it
+                    }
+                    __syncwarp();
+                    desc_a += STAGE_BYTES >> 4;
+                    desc_b += STAGE_BYTES >> 4;
+                    if (++s == STAGES) { s = 0; parity ^= 1u; desc_a = desc_a0; desc_b = desc_b0; }
                 }
-                if (ok) commit_pair(acc_full_bar(buf));
+                if (ok && elect_one()) commit_pair(acc_full_bar(buf));
+                __syncwarp();
             }
-            if (!ok) give_up(22);
+            if (!ok && lane == 0) give_up(22);
         }
     } else {
         // ---------------- epilogue: warps 2..5 of both blocks, TMEM lanes 32 * (warp % 4) ----------------

@@ -99,7 +99,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
     volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int tiles = (N + WM - 1) / WM;
     // the work: (tile, k block) pairs in tile order, one equal run per block
     const long long total = (long long)tiles * k_blocks;
@@ -131,41 +131,47 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
 
     if (warp == 0) {
         // ---------------- producer: weights by bulk copy, activations by TMA ----------------
-        if (lane == 0) {
-            bool ok = true;
-            const long long n = run_hi - run_lo;
-            const int early = (int)min((long long)stages, n);
-            // the first weights are requested before the kernel in front of this one has finished
+        bool ok = true;
+        const int n = (int)(run_hi - run_lo), early = min(stages, n);
+        const __nv_bfloat16* src = w_packed + (size_t)run_lo * (WM * BK);
+        // the first weights are requested before the kernel in front of this one has finished
+        if (elect_one())
             for (int i = 0; i < early; ++i) {
-                const long long g = run_lo + i;
                 mbar_expect_tx(full_bar(i), stage_bytes);
-                bulk_copy(base + (uint32_t)i * stage_bytes, w_packed + (size_t)g * (WM * BK), W_TILE_BYTES, full_bar(i));
+                bulk_copy(base + (uint32_t)i * stage_bytes, src + (size_t)i * (WM * BK), W_TILE_BYTES, full_bar(i));
             }
-            pdl_wait();
-            pdl_trigger();
-            for (int i = 0; i < early; ++i) {
-                const int kb = (int)((run_lo + i) % k_blocks);
-                tma_load_2d(base + (uint32_t)i * stage_bytes + W_TILE_BYTES, &map_a, kb * BK, 0, full_bar(i));
-            }
-            int s = early == stages ? 0 : early;
-            uint32_t parity = early == stages ? 0u : 1u;      // the ring's second lap waits for the first lap's release
-            for (long long i = early; i < n; ++i) {
-                const long long g = run_lo + i;
-                const int kb = (int)(g % k_blocks);
-                if (!mbar_wait(empty_bar(s), parity, abort_flag)) { ok = false; break; }
+        __syncwarp();
+        pdl_wait();
+        pdl_trigger();
+        int kb = (int)(run_lo % k_blocks);
+        for (int i = 0; i < early; ++i) {
+            if (elect_one()) tma_load_2d(base + (uint32_t)i * stage_bytes + W_TILE_BYTES, &map_a, kb * BK, 0, full_bar(i));
+            __syncwarp();
+            if (++kb == k_blocks) kb = 0;
+        }
+        src += (size_t)early * (WM * BK);
+        int s = early == stages ? 0 : early;
+        uint32_t parity = early == stages ? 0u : 1u;      // the ring's second lap waits for the first lap's release
+        for (int i = early; i < n; ++i, src += WM * BK) {
+            if (!warp_wait(empty_bar(s), parity, abort_flag)) { ok = false; break; }
+            if (elect_one()) {
                 const uint32_t dst = base + (uint32_t)s * stage_bytes;
                 mbar_expect_tx(full_bar(s), stage_bytes);
-                bulk_copy(dst, w_packed + (size_t)g * (WM * BK), W_TILE_BYTES, full_bar(s));
+                bulk_copy(dst, src, W_TILE_BYTES, full_bar(s));
                 tma_load_2d(dst + W_TILE_BYTES, &map_a, kb * BK, 0, full_bar(s));
-                if (++s == stages) { s = 0; parity ^= 1u; }
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 11); }
+            __syncwarp();
+            if (++kb == k_blocks) kb = 0;
+            if (++s == stages) { s = 0; parity ^= 1u; }
         }
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 11); }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        {
             // kind::f16: float32 accumulate, A and B bfloat16, both K-major, N = tokens, M = 128 weight rows
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ntok >> 3) << 17) | ((uint32_t)(WM >> 4) << 24);
+            const uint64_t desc_w0 = smem_desc_sw128(base), desc_b0 = smem_desc_sw128(base + W_TILE_BYTES);
+            uint64_t desc_w = desc_w0, desc_b = desc_b0;          // (a stage further is an addition to the address field)
             bool ok = true;
             int s = 0;
             uint32_t parity = 0, segment = 0;
@@ -174,24 +180,28 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
                 const int kb0 = (int)(g % k_blocks);
                 const long long seg_end = min(run_hi, g + (k_blocks - kb0));      // the tile's k blocks that are this block's
                 const uint32_t buf = segment & 1u;
-                if (!mbar_wait(acc_empty_bar(buf), ((segment >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+                if (!warp_wait(acc_empty_bar(buf), ((segment >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * acc_cols;
                 for (bool first = true; g < seg_end; ++g, first = false) {
-                    if (!mbar_wait(full_bar(s), parity, abort_flag)) { ok = false; break; }
+                    if (!warp_wait(full_bar(s), parity, abort_flag)) { ok = false; break; }
                     tcgen05_fence_after();
-                    const uint32_t w_addr = base + (uint32_t)s * stage_bytes, b_addr = w_addr + W_TILE_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k)
-                        tcgen05_mma_bf16(tmem_d, smem_desc_sw128(w_addr + k * 32), smem_desc_sw128(b_addr + k * 32), idesc,
-                                         (!first || k > 0) ? 1u : 0u);
-                    tcgen05_commit(empty_bar(s));
-                    if (++s == stages) { s = 0; parity ^= 1u; }
+                        for (int k = 0; k < BK / 16; ++k)
+                            tcgen05_mma_bf16(tmem_d, desc_w + 2 * k, desc_b + 2 * k, idesc, (!first || k > 0) ? 1u : 0u);
+                        tcgen05_commit(empty_bar(s));
+                    }
+                    __syncwarp();
+                    desc_w += stage_bytes >> 4;
+                    desc_b += stage_bytes >> 4;
+                    if (++s == stages) { s = 0; parity ^= 1u; desc_w = desc_w0; desc_b = desc_b0; }
                 }
-                if (ok) tcgen05_commit(acc_full_bar(buf));
+                if (ok && elect_one()) tcgen05_commit(acc_full_bar(buf));
+                __syncwarp();
                 ++segment;
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 12); }
+            if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 12); }
         }
     } else {
         // ---------------- epilogue: warps 2..5, TMEM lanes 32 * (warp % 4) = weight rows of the tile ----------------
@@ -400,7 +410,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(aligned + bars_at + 8 * (2 * stages + 1));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int tile = (int)blockIdx.x / blocks, rank = (int)blockIdx.x % blocks;      // (clusters lie along x: this is the rank)
     const int kb_lo = k_blocks * rank / blocks, kb_hi = k_blocks * (rank + 1) / blocks, n_kb = kb_hi - kb_lo;
 
@@ -429,53 +439,61 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat
 
     if (warp == 0) {
         // ---------------- producer: weights by bulk copy, activations by TMA ----------------
-        if (lane == 0) {
-            bool ok = true;
-            const __nv_bfloat16* w = w_packed + ((size_t)tile * k_blocks + kb_lo) * (WM * BK);
-            const int early = min(stages, n_kb);
-            // the first weights are requested before the kernel in front of this one has finished
+        bool ok = true;
+        const __nv_bfloat16* w = w_packed + ((size_t)tile * k_blocks + kb_lo) * (WM * BK);
+        const int early = min(stages, n_kb);
+        // the first weights are requested before the kernel in front of this one has finished
+        if (elect_one())
             for (int i = 0; i < early; ++i) {
                 mbar_expect_tx(full_bar(i), stage_bytes);
                 bulk_copy(base + (uint32_t)i * stage_bytes, w + (size_t)i * (WM * BK), W_TILE_BYTES, full_bar(i));
             }
-            pdl_wait();
-            pdl_trigger();
+        __syncwarp();
+        pdl_wait();
+        pdl_trigger();
+        if (elect_one())
             for (int i = 0; i < early; ++i)
                 tma_load_2d(base + (uint32_t)i * stage_bytes + W_TILE_BYTES, &map_a, (kb_lo + i) * BK, 0, full_bar(i));
-            int s = 0;
-            uint32_t parity = 0;                                   // the ring's second lap waits for the first lap's release
-            for (int i = stages; i < n_kb; ++i) {
-                if (!mbar_wait(empty_bar(s), parity, abort_flag)) { ok = false; break; }
+        __syncwarp();
+        int s = 0;
+        uint32_t parity = 0;                                   // the ring's second lap waits for the first lap's release
+        for (int i = stages; i < n_kb; ++i) {
+            if (!warp_wait(empty_bar(s), parity, abort_flag)) { ok = false; break; }
+            if (elect_one()) {
                 const uint32_t dst = base + (uint32_t)s * stage_bytes;
                 mbar_expect_tx(full_bar(s), stage_bytes);
                 bulk_copy(dst, w + (size_t)i * (WM * BK), W_TILE_BYTES, full_bar(s));
                 tma_load_2d(dst + W_TILE_BYTES, &map_a, (kb_lo + i) * BK, 0, full_bar(s));
-                if (++s == stages) { s = 0; parity ^= 1u; }
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 14); }
+            __syncwarp();
+            if (++s == stages) { s = 0; parity ^= 1u; }
         }
-        __syncwarp();
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 14); }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ntok >> 3) << 17) | ((uint32_t)(WM >> 4) << 24);
-            bool ok = true;
-            int s = 0;
-            uint32_t parity = 0;
-            for (int i = 0; i < n_kb; ++i) {
-                if (!mbar_wait(full_bar(s), parity, abort_flag)) { ok = false; break; }
-                tcgen05_fence_after();
-                const uint32_t w_addr = base + (uint32_t)s * stage_bytes, b_addr = w_addr + W_TILE_BYTES;
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ntok >> 3) << 17) | ((uint32_t)(WM >> 4) << 24);
+        const uint64_t desc_w0 = smem_desc_sw128(base), desc_b0 = smem_desc_sw128(base + W_TILE_BYTES);
+        uint64_t desc_w = desc_w0, desc_b = desc_b0;          // (a stage further is an addition to the address field)
+        bool ok = true;
+        int s = 0;
+        uint32_t parity = 0;
+        for (int i = 0; i < n_kb; ++i) {
+            if (!warp_wait(full_bar(s), parity, abort_flag)) { ok = false; break; }
+            tcgen05_fence_after();
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
-                    tcgen05_mma_bf16(tmem_base, smem_desc_sw128(w_addr + k * 32), smem_desc_sw128(b_addr + k * 32), idesc,
-                                     (i > 0 || k > 0) ? 1u : 0u);
+                    tcgen05_mma_bf16(tmem_base, desc_w + 2 * k, desc_b + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
                 tcgen05_commit(empty_bar(s));
-                if (++s == stages) { s = 0; parity ^= 1u; }
             }
-            if (ok) tcgen05_commit(acc_bar);
-            else { *abort_flag = 1; atomicExch(error_word, 15); }
+            __syncwarp();
+            desc_w += stage_bytes >> 4;
+            desc_b += stage_bytes >> 4;
+            if (++s == stages) { s = 0; parity ^= 1u; desc_w = desc_w0; desc_b = desc_b0; }
         }
+        if (ok) {
+            if (elect_one()) tcgen05_commit(acc_bar);
+        } else if (lane == 0) { *abort_flag = 1; atomicExch(error_word, 15); }
         __syncwarp();
     } else {
         pdl_wait();          // the residual stream it may add into was written by the kernels before

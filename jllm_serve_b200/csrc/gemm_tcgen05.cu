@@ -76,7 +76,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 2);
     uint8_t* staging = aligned + STAGES * STAGE_BYTES;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN, tiles = tiles_m * tiles_n;
     const int k_blocks = (K + BK - 1) / BK;
     const int padded_rows = (N + 127) & ~127;       // rows of the packed weight
@@ -145,9 +145,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            // (stage and phase are counted, not divided out: with narrow tiles this one thread's instructions per
-            // k block are what the product waits for)
+        {
+            // (stage and phase are counted, not divided out: with narrow tiles this warp's instructions per k block are
+            // what the product waits for)
             int s = 0;
             uint32_t parity = 1, dst = base;
             bool ok = true;
@@ -159,7 +159,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 // (a piece ends where a packed tile of 128 rows ends; a BN-row tile meets at most two of them). Rows
                 // beyond the padded matrix do not exist: their part of a stage keeps what it held, and the columns they
                 // would give are never stored. Everything that does not change with the k block is worked out here:
-                // this one thread's instructions per k block are what a product of narrow tiles waits for.
+                // this warp's instructions per k block are what a product of narrow tiles waits for.
                 const int w_rows = min(BN, padded_rows - n0);
                 const int in_tile = n0 & 127;
                 const uint32_t bytes0 = (uint32_t)min(128 - in_tile, w_rows) * 128u;
@@ -169,48 +169,54 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const uint32_t tx = A_BYTES + bytes0 + bytes1;
                 uint32_t extra = starve ? 16u : 0u;         // the wait test: the first barrier expects too much
                 for (int kb = lo; kb < hi; ++kb, src += 8192) {
-                    if (!mbar_wait(empty_bar(s), parity, abort_flag, spin)) { ok = false; break; }
-                    mbar_expect_tx(full_bar(s), tx + extra);
+                    if (!warp_wait(empty_bar(s), parity, abort_flag, spin)) { ok = false; break; }
+                    if (elect_one()) {
+                        mbar_expect_tx(full_bar(s), tx + extra);
+                        tma_load_2d(dst, &map_a, kb * BK, m0, full_bar(s));
+                        bulk_copy(dst + A_BYTES, src, bytes0, full_bar(s));
+                        if (bytes1) bulk_copy(dst + A_BYTES + bytes0, src + next_tile, bytes1, full_bar(s));
+                    }
+                    __syncwarp();
                     extra = 0;
-                    tma_load_2d(dst, &map_a, kb * BK, m0, full_bar(s));
-                    bulk_copy(dst + A_BYTES, src, bytes0, full_bar(s));
-                    if (bytes1) bulk_copy(dst + A_BYTES + bytes0, src + next_tile, bytes1, full_bar(s));
                     dst += STAGE_BYTES;
                     if (++s == STAGES) { s = 0; parity ^= 1u; dst = base; }
                 }
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 1); }
+            if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 1); }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            uint32_t local_tile = 0, parity = 0, a_addr = base;
+        {
+            const uint64_t desc_a0 = smem_desc_sw128(base), desc_b0 = smem_desc_sw128(base + A_BYTES);
+            uint64_t desc_a = desc_a0, desc_b = desc_b0;          // (a stage further is an addition to the address field)
+            uint32_t local_tile = 0, parity = 0;
             int s = 0;
             bool ok = true;
             Walk walk = first_unit();
             int tile, lo, hi;
             for (; ok && next_unit(walk, tile, lo, hi); ++local_tile) {
                 const uint32_t buf = local_tile & 1u;
-                if (!mbar_wait(acc_empty_bar(buf), ((local_tile >> 1) & 1u) ^ 1u, abort_flag, spin)) { ok = false; break; }
+                if (!warp_wait(acc_empty_bar(buf), ((local_tile >> 1) & 1u) ^ 1u, abort_flag, spin)) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * BN;
                 for (int kb = lo; kb < hi; ++kb) {
-                    if (!mbar_wait(full_bar(s), parity, abort_flag, spin)) { ok = false; break; }
+                    if (!warp_wait(full_bar(s), parity, abort_flag, spin)) { ok = false; break; }
                     tcgen05_fence_after();
-                    const uint32_t b_addr = a_addr + A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
-                        // 16 bfloat16 = 32 bytes further along k inside the 128-byte swizzled rows
-                        tcgen05_mma_bf16(tmem_d, smem_desc_sw128(a_addr + k * 32), smem_desc_sw128(b_addr + k * 32), IDESC,
-                                         (kb > lo || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < BK / 16; ++k)      // 16 bfloat16 = 32 bytes further along k inside the 128-byte swizzled rows
+                            tcgen05_mma_bf16(tmem_d, desc_a + 2 * k, desc_b + 2 * k, IDESC, (kb > lo || k > 0) ? 1u : 0u);
+                        tcgen05_commit(empty_bar(s));   // arrives when the MMAs above have read the stage
                     }
-                    tcgen05_commit(empty_bar(s));   // arrives when the MMAs above have read the stage
-                    a_addr += STAGE_BYTES;
-                    if (++s == STAGES) { s = 0; parity ^= 1u; a_addr = base; }
+                    __syncwarp();
+                    desc_a += STAGE_BYTES >> 4;
+                    desc_b += STAGE_BYTES >> 4;
+                    if (++s == STAGES) { s = 0; parity ^= 1u; desc_a = desc_a0; desc_b = desc_b0; }
                 }
-                if (ok) tcgen05_commit(acc_full_bar(buf));
+                if (ok && elect_one()) tcgen05_commit(acc_full_bar(buf));
+                __syncwarp();
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 2); }
+            if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 2); }
         }
     } else {
         // ---------------- epilogue: warps 2..5, TMEM lanes 32 * (warp % 4) ----------------

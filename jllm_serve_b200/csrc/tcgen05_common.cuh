@@ -44,6 +44,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
     return false;
 }
+// ---- a warp that only issues (copies, MMAs) --------------------------------------------------------------------------
+// tcgen05.mma, tcgen05.commit and the bulk copies take their operands from the warp's uniform registers. Issued under `if (lane == 0)`
+// every operand is moved there one by one behind a branch that the compiler has to think divergent, and a loop of one wait, four MMAs and
+// a commit takes 330 ns whatever the tile (205 ns with nothing but the barriers): longer than the MMAs of every tile but the largest.
+// So the WHOLE warp walks the loop, its control flow follows from votes (which are uniform), and one elected lane issues: 115 ns for the
+// barriers alone, and from there on the MMAs are what is waited for (128 weight rows a block x 160 tokens: 318 -> 176 ns a k block of 64).
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// mbar_wait by a whole warp
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t limit = SPIN_LIMIT) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
