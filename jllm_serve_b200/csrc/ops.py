@@ -139,6 +139,7 @@ class _Signatures:
     jllm_gemm_small_m = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, P, P]
     jllm_gemm_tcgen05 = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, I, P]
     jllm_gemm_pair = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, P]
+    jllm_gemm_pair_swap = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, I, I, P, P]
     jllm_gemm_pair_resident = []
     jllm_gemm_plain_stores = [I]
     jllm_gemm_stream = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, I, P]
@@ -953,6 +954,8 @@ def gemm_bf16_fits(a, w, out) -> bool:
 #            256 for matrices much longer than high (down); not for very wide matrices (gate_up), which whole tiles of
 #            the tiles kernel fill the SMs with;
 #   "tiles"  gemm_tcgen05: tokens as the M side, 128 x BN tiles; above that, and from 16 rows for very wide matrices.
+# From 129 rows on `pair_swap_tokens` then says whether pairs of SMs with the weight rows as their M side (gemm_pair_swap) are faster
+# than the kernel named here.
 SWAP_MAX_ROWS = 256      # gemm_stream: the tokens are the N side of one tcgen05.mma
 TILE_ROWS = 128          # rows of a tcgen05 product tile (BM in gemm_tcgen05.cu): a step of 129 rows pays for 256
 SMALL_M_ROWS = int(os.environ.get("JLLM_B200_SMALL_M_ROWS", "64"))
@@ -1015,6 +1018,47 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
     return "tiles"
 
 
+@functools.lru_cache(maxsize=4096)
+def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str, sms: int = 148, pairs: int = 74) -> int:
+    """The tokens of a tile with which `gemm_pair_swap` takes a product of `rows` rows that would else go to `kernel`
+    (`gemm_kernel_for`), or 0 where it is not the faster one.
+
+    What a product takes is counted in clocks a k block of 64: a round of tiles takes T + 256 (shared memory: 128 weight rows
+    and half of the T tokens of every block are written and read once at 128 bytes a clock), one-SM tiles of 128 x w 2 w + 256,
+    pairs of 256 x 256 512; and because the SMs share one power limit, twice the multiply-adds of all tiles, spread over all
+    pairs, come on top. 8B layer shapes, us, before and with it: QKV of 300 rows 18.5 and 16.5, of 613 28.9 and 24.7, of 1,024
+    42.5 and 38.1; O of 512 17.7 and 15.9; gate_up of 144 47.7 and 38.6, of 400 73.0 and 63.3, of 613 101 and 88; down of 300
+    47.3 and 35.5, of 613 59.6 and 50.7. From there on 256 x 256 tiles with the tokens as the M side are as good (gate_up of 1,536 rows
+    195 and 213): it takes a twelfth less by this count to change. Below 129 rows there are too few tiles; of few k blocks a pair's start and
+    end are most of it (3,072 x 768, 613 rows 6.6 and 7.4); matrices much longer than high stay with `gemm_stream` up to 208 rows
+    (down of 200 rows 38.4 and 40, of 256 48.5 and 45.4). A matrix of few rows, which the streamed pairs took between 257 and 512
+    rows, was worst off there (768 x 2,048, 300 rows: 49.6 and 7.1)."""
+    if pairs <= 0 or rows <= TILE_ROWS or kernel not in ("swap", "tiles", "pair", "pair-streamed"):
+        return 0
+    if kernel == "swap" and rows <= 208 and in_features >= 2 * out_features:
+        return 0
+    if kernel in ("tiles", "pair") and in_features < 1024:
+        return 0
+    high = -(-out_features // 256)
+
+    def cost(tiles, places, per_round, multiply):
+        return -(-tiles // places) * per_round + 2.0 * tiles * multiply / places
+
+    best = tokens = 0
+    for cut in range(-(-rows // 256), -(-rows // 256) + 9):
+        t = -(-rows // (16 * cut)) * 16
+        c = cost(-(-rows // t) * high, pairs, 256 + t, 2 * t)
+        if t >= 48 and (not tokens or c < best):
+            best, tokens = c, t
+    if kernel == "pair":
+        other = cost(-(-rows // 256) * high, pairs, 512, 512)
+    elif kernel == "tiles":
+        other = min(cost(-(-rows // 128) * -(-out_features // w), sms, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
+    else:
+        return tokens
+    return tokens if best < 0.92 * other else 0
+
+
 def gemm_bf16(a, w, out, bias=None, accumulate=False, swiglu=False) -> None:
     """out (+)= a @ w.T (+ bias) on the tensor cores: bfloat16 operands, float32 accumulation; `w` a PackedWeight (a
     plain [out, in] matrix is packed on the spot). With `swiglu` the rows of w are blocks of 8 gate rows followed by
@@ -1023,6 +1067,10 @@ def gemm_bf16(a, w, out, bias=None, accumulate=False, swiglu=False) -> None:
     rows = a.shape[0]
     kernel = gemm_kernel_for(rows, w.rows, w.cols, _rows_fit(a, w), _tcgen05_fits(a, w), sm_count(),
                              resident_pairs() if rows > 128 else 0)
+    if rows > TILE_ROWS and kernel and _tcgen05_fits(a, w):
+        tokens = pair_swap_tokens(rows, w.rows, w.cols, kernel, sm_count(), resident_pairs())
+        if tokens:
+            return gemm_pair_swap(a, w, out, tokens, bias, accumulate, swiglu=swiglu)
     if kernel == "rows":
         return gemm_small_m(a, w, out, bias, accumulate, swiglu=swiglu)
     if kernel == "swap":
@@ -1065,6 +1113,16 @@ def gemm_pair(a, w, out, bias=None, accumulate=False, swiglu=False, max_pairs: i
           _DT[bias.dtype] if bias is not None else F32, out.data_ptr(), _DT[out.dtype], out.stride(0),
           int(accumulate), a.shape[0], w.rows, w.cols, int(max_pairs), glu_kind(swiglu), glu_more(swiglu), _p(ws),
           ws.numel() if ws is not None else 0, int(stream_mode), _stream())
+
+
+def gemm_pair_swap(a, w, out, tokens: int, bias=None, accumulate=False, swiglu=False, max_pairs: int = 0) -> None:
+    """As `gemm_pair`, with the weight rows as the M side: tiles of 256 weight rows by `tokens` tokens (a multiple of 16 up to 256)."""
+    w = _packed(w)
+    assert a.dtype == torch.bfloat16 and out.stride(-1) == 1 and a.shape[1] == w.cols
+    _call("jllm_gemm_pair_swap", a.data_ptr(), a.stride(0), w.data.data_ptr(), w.k_blocks, _p(bias),
+          _DT[bias.dtype] if bias is not None else F32, out.data_ptr(), _DT[out.dtype], out.stride(0),
+          int(accumulate), a.shape[0], w.rows, w.cols, int(tokens), int(max_pairs) or resident_pairs(), glu_kind(swiglu), glu_more(swiglu),
+          _stream())
 
 
 _resident_pairs = None
@@ -1187,7 +1245,7 @@ def bounds_errors() -> dict:
 
 
 # Which kernel a code in an error word is from: the products share one word, the attention kernels another.
-WAIT_KERNELS = {"products": ((1, 3, "gemm_tcgen05"), (11, 13, "gemm_stream"), (14, 16, "gemm_stream (clusters)"), (21, 23, "gemm_pair")),
+WAIT_KERNELS = {"products": ((1, 3, "gemm_tcgen05"), (11, 13, "gemm_stream"), (14, 16, "gemm_stream (clusters)"), (21, 23, "gemm_pair"), (34, 36, "gemm_pair_swap")),
                 "attention": ((21, 23, "attention_prefill_tc"), (31, 33, "attention_prefill_pair"), (41, 43, "attention_prefill_latent"),
                               (51, 52, "attention_decode_ring"))}
 

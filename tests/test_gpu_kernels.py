@@ -909,3 +909,31 @@ def test_attention_prefill_over_rows_that_are_key_and_value(ops, H, Hkv, page, w
         ops.attention_plain(q, q.stride(0), kc, kc, want, rseg, rpos, tables, q.shape[0], H, Hkv, hd, page, window, scale)
         got = out.view(-1, H, hd)[:, :, :cols].reshape(q.shape[0], -1)
         rows_close(got, want.float().cpu().view(-1, H, hd)[:, :, :cols].reshape(q.shape[0], -1), f"latent {far}")
+
+
+@pytest.mark.parametrize("M,N,K,tokens", [(1, 8, 8, 16), (130, 40, 72, 48), (257, 517, 200, 256), (300, 256, 4096, 112), (613, 1040, 1032, 208),
+                                          (500, 2500, 136, 80)])
+def test_gemm_pair_swap(ops, M, N, K, tokens):
+    """Weight rows as the M side of a pair's tile: edges of tokens, rows and k, tiles whose second block has no weight rows, many tiles on
+    few pairs (both accumulators in turn), bias, residual add, relu squared, bfloat16 results into a wider row, gate and up rows."""
+    a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
+    packed, bias, base = ops.pack_weight(w), rnd(N, dtype=torch.float32, seed=2), rnd(M, N, seed=3)
+    tol, plain = 1e-4 * math.sqrt(K) * 0.05, gemm_want(a, w, bias)
+    for pairs in (0, 2):
+        acc, again, sq = base.clone(), base.clone(), torch.full((M, N), float("nan"), device=DEV)
+        ops.gemm_pair_swap(a, packed, acc, tokens, bias, accumulate=True, max_pairs=pairs)
+        ops.gemm_pair_swap(a, packed, again, tokens, bias, accumulate=True, max_pairs=pairs)
+        ops.gemm_pair_swap(a, packed, sq, tokens, bias, accumulate=ops.EPILOGUE_RELU2, max_pairs=pairs)
+        out16 = torch.zeros(M, N + 6, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_pair_swap(a, packed, out16[:, :N], tokens, max_pairs=pairs)
+        assert ops.gemm_tcgen05_error() == 0
+        assert torch.allclose(acc.cpu(), plain + base.cpu(), rtol=1e-4, atol=tol) and torch.equal(acc, again)
+        assert torch.allclose(sq.cpu(), torch.relu(plain) ** 2, rtol=1e-3, atol=4 * tol)
+        assert torch.allclose(out16[:, :N].float().cpu(), gemm_want(a, w), rtol=2 ** -7, atol=2e-3) and float(out16[:, N:].abs().max()) == 0
+        if N % 16 == 0:
+            z = gemm_want(a, w).view(M, N // 16, 2, 8)
+            want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2)
+            for dtype, t in ((torch.float32, 1e-3), (torch.bfloat16, 2 ** -7)):
+                units = torch.full((M, N // 2), float("nan"), dtype=dtype, device=DEV)
+                ops.gemm_pair_swap(a, packed, units, tokens, swiglu=True, max_pairs=pairs)
+                assert torch.allclose(units.float().cpu(), want, rtol=t, atol=1e-3)

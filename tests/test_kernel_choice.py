@@ -130,3 +130,16 @@ def test_a_wait_that_ran_out_is_reported_with_its_kernel(monkeypatch):
             ops.check_kernel_errors()
     monkeypatch.setattr(ops, "library", lambda: Fake(0, 0))
     ops.check_kernel_errors()
+
+
+def test_tokens_of_a_tile_with_the_weight_rows_as_m_side():
+    """Where the product of a pair with the weight rows as its M side takes another kernel's place, and the tiles it then has cover the rows."""
+    def tokens(rows, n, k, **more):
+        return ops.pair_swap_tokens(rows, n, k, ops.gemm_kernel_for(rows, n, k), **more)
+    assert tokens(613, 24576, 4096) == 208 and tokens(613, 4096, 12288) == 160 and tokens(300, 4096, 12288) == 80
+    assert tokens(128, 6144, 4096) == 0 and tokens(2048, 24576, 4096) == 0 and tokens(200, 4096, 12288) == 0
+    assert tokens(613, 24576, 4096, pairs=0) == 0 and ops.pair_swap_tokens(613, 24576, 4096, "rows") == 0
+    for rows in list(range(129, 700, 13)) + [1000, 1536, 2048, 5000]:
+        for n, k in ((6144, 4096), (4096, 4096), (24576, 4096), (4096, 12288), (2048, 2048), (768, 2048), (64, 2048)):
+            t = tokens(rows, n, k)
+            assert t % 16 == 0 and 0 <= t <= 256 and (t == 0 or t >= 48)
