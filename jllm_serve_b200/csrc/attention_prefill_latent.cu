@@ -87,7 +87,7 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap map_q, const
         tile -= nt;
     }
     if (seg >= num_segs) return;                       // whole block: before any barrier or allocation
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int head = blockIdx.x, kvh = head / (heads / kv_heads);
     const int n_rows = seg_len[seg], q0 = tile * BQ;
     const int rows_here = min(BQ, n_rows - q0);
@@ -198,28 +198,31 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap map_q, const
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 41); }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            bool ok = mbar_wait(bar(Q_FULL), 0, abort_flag);
+        // (the whole warp walks the tiles, one elected lane issues: see tcgen05_common.cuh)
+        {
+            bool ok = warp_wait(bar(Q_FULL), 0, abort_flag);
             auto issue_s = [&](int j) {       // S[j & 1] = Q K_j^T, piece by piece
                 const uint32_t d = tmem_base + (j & 1) * 128;
 #pragma unroll 1
                 for (int c = 0; c < QUARTERS; ++c) {
                     const int n = j * QUARTERS + c, slot = n % SLOTS;
-                    if (!mbar_wait(bar(FULL + slot), (uint32_t)(n / SLOTS) & 1u, abort_flag)) return false;
+                    if (!warp_wait(bar(FULL + slot), (uint32_t)(n / SLOTS) & 1u, abort_flag)) return false;
                     tcgen05_fence_after();
+                    if (elect_one()) {
+                        const uint64_t q = smem_desc_sw128(s_q(c)), key = smem_desc_sw128(s_k(slot));
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        tcgen05_mma_bf16(d, smem_desc_sw128(s_q(c) + k * 32), smem_desc_sw128(s_k(slot) + k * 32), IDESC_128x128_KK,
-                                         (c > 0 || k > 0) ? 1u : 0u);
-                    if (c >= value_quarters) tcgen05_commit(bar(EMPTY + slot));
+                        for (int k = 0; k < 4; ++k) tcgen05_mma_bf16(d, q + 2 * k, key + 2 * k, IDESC_128x128_KK, (c > 0 || k > 0) ? 1u : 0u);
+                        if (c >= value_quarters) tcgen05_commit(bar(EMPTY + slot));
+                        if (c == QUARTERS - 1) tcgen05_commit(bar(S_FULL + (j & 1)));
+                    }
+                    __syncwarp();
                 }
-                tcgen05_commit(bar(S_FULL + (j & 1)));
                 return true;
             };
             if (ok) ok = issue_s(0);
             for (int j = 0; j < n_tiles && ok; ++j) {
                 if (j + 1 < n_tiles) ok = issue_s(j + 1);
-                if (!ok || !mbar_wait(bar(P_READY + (j & 1)), (uint32_t)(j >> 1) & 1u, abort_flag)) {
+                if (!ok || !warp_wait(bar(P_READY + (j & 1)), (uint32_t)(j >> 1) & 1u, abort_flag)) {
                     ok = false;
                     break;
                 }
@@ -227,16 +230,19 @@ attention_prefill_latent_kernel(const __grid_constant__ CUtensorMap map_q, const
 #pragma unroll 1
                 for (int c = 0; c < value_quarters; ++c) {
                     const int slot = (j * QUARTERS + c) % SLOTS;
-                    const uint32_t d = tmem_base + 256 + c * 64, a = tmem_base + (j & 1) * 128;
+                    if (elect_one()) {
+                        const uint32_t d = tmem_base + 256 + c * 64, a = tmem_base + (j & 1) * 128;
+                        const uint64_t value = smem_desc_mn_sw128(s_k(slot), PIECE_BYTES);
 #pragma unroll
-                    for (int k = 0; k < BKV / 16; ++k)
-                        mma_bf16_ts(d, a + k * 8, smem_desc_mn_sw128(s_k(slot) + k * 2048, PIECE_BYTES), IDESC_128x64_KMN,
-                                    (j > 0 || k > 0) ? 1u : 0u);
-                    tcgen05_commit(bar(EMPTY + slot));
+                        for (int k = 0; k < BKV / 16; ++k)
+                            mma_bf16_ts(d, a + k * 8, value + k * (2048 >> 4), IDESC_128x64_KMN, (j > 0 || k > 0) ? 1u : 0u);
+                        tcgen05_commit(bar(EMPTY + slot));
+                        if (c == value_quarters - 1) tcgen05_commit(bar(PV_DONE + (j & 1)));
+                    }
+                    __syncwarp();
                 }
-                tcgen05_commit(bar(PV_DONE + (j & 1)));
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 42); }
+            if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 42); }
         }
     } else {
         // ---------------- softmax: two threads to a query row (= TMEM lane), 64 of a tile's keys each ----------------

@@ -73,7 +73,7 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
         pair -= np;
     }
     if (seg >= num_segs) return;                       // whole block: before any barrier or allocation
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int head = blockIdx.x, kvh = head / (heads / kv_heads);
     const int n_rows = seg_len[seg], q0 = pair * 2 * BQ;
     const int rows_here = min(2 * BQ, n_rows - q0);                    // rows of both tiles
@@ -175,50 +175,62 @@ attention_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const _
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 31); }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            bool ok = mbar_wait(bar(Q_FULL), 0, abort_flag);
+        // (the whole warp walks the tiles, one elected lane issues: see tcgen05_common.cuh)
+        {
+            bool ok = warp_wait(bar(Q_FULL), 0, abort_flag);
             auto issue_s = [&](int x, int j) {      // S_x = Q_x K_j^T (the K tile has been waited for)
-                const uint32_t d = tmem_base + x * 128;
+                if (elect_one()) {
+                    const uint32_t d = tmem_base + x * 128;
+                    const uint64_t q = smem_desc_sw128(s_q(x)), key = smem_desc_sw128(s_k(j & 1));
 #pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
-                    const uint32_t o = (k >> 2) * HALF_BYTES + (k & 3) * 32;
-                    tcgen05_mma_bf16(d, smem_desc_sw128(s_q(x) + o), smem_desc_sw128(s_k(j & 1) + o), IDESC_128x128_KK, k > 0);
+                    for (int k = 0; k < HD / 16; ++k) {
+                        const uint32_t o = ((k >> 2) * HALF_BYTES + (k & 3) * 32) >> 4;
+                        tcgen05_mma_bf16(d, q + o, key + o, IDESC_128x128_KK, k > 0);
+                    }
+                    tcgen05_commit(bar(S_FULL + x));
                 }
-                tcgen05_commit(bar(S_FULL + x));
+                __syncwarp();
+            };
+            auto commit = [&](int which) {
+                if (elect_one()) tcgen05_commit(bar(which));
+                __syncwarp();
             };
             auto issue_pv = [&](int x, int j) {     // O_x += P_x V_j
-                const uint32_t d = tmem_base + 256 + x * 128, a = tmem_base + x * 128;
+                if (elect_one()) {
+                    const uint32_t d = tmem_base + 256 + x * 128, a = tmem_base + x * 128;
+                    const uint64_t value = smem_desc_mn_sw128(s_v(j & 1), HALF_BYTES);
 #pragma unroll
-                for (int k = 0; k < BKV / 16; ++k)
-                    tcgen05_mma_bf16_ts(d, a + k * 8, smem_desc_mn_sw128(s_v(j & 1) + k * 2048, HALF_BYTES), IDESC_128x128_KMN,
-                                        (j > 0 || k > 0) ? 1u : 0u);
-                tcgen05_commit(bar(PV_DONE + x));
+                    for (int k = 0; k < BKV / 16; ++k)
+                        tcgen05_mma_bf16_ts(d, a + k * 8, value + k * (2048 >> 4), IDESC_128x128_KMN, (j > 0 || k > 0) ? 1u : 0u);
+                    tcgen05_commit(bar(PV_DONE + x));
+                }
+                __syncwarp();
             };
-            if (ok) ok = mbar_wait(bar(K_FULL + 0), 0, abort_flag);
+            if (ok) ok = warp_wait(bar(K_FULL + 0), 0, abort_flag);
             if (ok) {
                 tcgen05_fence_after();
                 for (int x = 0; x < 2; ++x)
                     if (n_x[x] > 0) issue_s(x, 0);
-                tcgen05_commit(bar(K_EMPTY + 0));
+                commit(K_EMPTY + 0);
             }
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int b = j & 1;
-                if (!mbar_wait(bar(V_FULL + b), (j >> 1) & 1u, abort_flag)) { ok = false; break; }
+                if (!warp_wait(bar(V_FULL + b), (j >> 1) & 1u, abort_flag)) { ok = false; break; }
                 const bool more = j + 1 < n_tiles;
-                if (more && !mbar_wait(bar(K_FULL + (b ^ 1)), ((j + 1) >> 1) & 1u, abort_flag)) { ok = false; break; }
+                if (more && !warp_wait(bar(K_FULL + (b ^ 1)), ((j + 1) >> 1) & 1u, abort_flag)) { ok = false; break; }
                 for (int x = 0; x < 2 && ok; ++x) {
                     if (j < n_x[x]) {
-                        if (!mbar_wait(bar(P_READY + x), j & 1u, abort_flag)) { ok = false; break; }
+                        if (!warp_wait(bar(P_READY + x), j & 1u, abort_flag)) { ok = false; break; }
                         tcgen05_fence_after();
                         issue_pv(x, j);
                     }
                     if (j + 1 < n_x[x]) issue_s(x, j + 1);
                 }
                 if (!ok) break;
-                tcgen05_commit(bar(V_EMPTY + b));
-                if (more) tcgen05_commit(bar(K_EMPTY + (b ^ 1)));
+                commit(V_EMPTY + b);
+                if (more) commit(K_EMPTY + (b ^ 1));
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 32); }
+            if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 32); }
         }
     } else {
         // ---------------- softmax of tile x: thread = query row = TMEM lane ----------------

@@ -66,7 +66,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         tile -= nt;
     }
     if (seg >= num_segs) return;                       // whole block: before any barrier or allocation
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int head = blockIdx.x, kvh = head / (heads / kv_heads);
     const int n_rows = seg_len[seg], q0 = tile * BQ;
     const int rows_here = min(BQ, n_rows - q0);
@@ -167,21 +167,26 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 21); }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            bool ok = mbar_wait(bar(Q_FULL), 0, abort_flag);
+        // (the whole warp walks the tiles, one elected lane issues: see tcgen05_common.cuh)
+        {
+            bool ok = warp_wait(bar(Q_FULL), 0, abort_flag);
             auto issue_s = [&](int j) {       // S[j & 1] = Q K_j^T
                 const int b = j & 1;
-                if (!mbar_wait(bar(K_FULL + b), (j >> 1) & 1u, abort_flag)) return false;
-                if (j >= 2 && !mbar_wait(bar(S_EMPTY + b), ((j >> 1) - 1) & 1u, abort_flag)) return false;
+                if (!warp_wait(bar(K_FULL + b), (j >> 1) & 1u, abort_flag)) return false;
+                if (j >= 2 && !warp_wait(bar(S_EMPTY + b), ((j >> 1) - 1) & 1u, abort_flag)) return false;
                 tcgen05_fence_after();
-                const uint32_t d = tmem_base + b * 128;
+                if (elect_one()) {
+                    const uint32_t d = tmem_base + b * 128;
+                    const uint64_t q = smem_desc_sw128(s_q), key = smem_desc_sw128(s_k(b));
 #pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
-                    const uint32_t o = (k >> 2) * HALF_BYTES + (k & 3) * 32;
-                    tcgen05_mma_bf16(d, smem_desc_sw128(s_q + o), smem_desc_sw128(s_k(b) + o), IDESC_128x128_KK, k > 0);
+                    for (int k = 0; k < HD / 16; ++k) {
+                        const uint32_t o = ((k >> 2) * HALF_BYTES + (k & 3) * 32) >> 4;
+                        tcgen05_mma_bf16(d, q + o, key + o, IDESC_128x128_KK, k > 0);
+                    }
+                    tcgen05_commit(bar(S_FULL + b));
+                    tcgen05_commit(bar(K_EMPTY + b));
                 }
-                tcgen05_commit(bar(S_FULL + b));
-                tcgen05_commit(bar(K_EMPTY + b));
+                __syncwarp();
                 return true;
             };
             if (ok) ok = issue_s(0);
@@ -189,23 +194,24 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const int b = j & 1;
                 if (j + 1 < n_tiles) ok = issue_s(j + 1);
                 if (!ok) break;
-                if (!mbar_wait(bar(P_READY), j & 1u, abort_flag) || !mbar_wait(bar(V_FULL + b), (j >> 1) & 1u, abort_flag)) {
+                if (!warp_wait(bar(P_READY), j & 1u, abort_flag) || !warp_wait(bar(V_FULL + b), (j >> 1) & 1u, abort_flag)) {
                     ok = false;
                     break;
                 }
                 tcgen05_fence_after();
-                const uint32_t d = tmem_base + 256;
+                if (elect_one()) {
+                    const uint32_t d = tmem_base + 256;
+                    const uint64_t p = smem_desc_sw128(s_p), value = smem_desc_mn_sw128(s_v(b), HALF_BYTES);
 #pragma unroll
-                for (int k = 0; k < BKV / 16; ++k) {
-                    // A: 16 keys further along P's rows; B: 16 key rows further down V (two 8-row groups)
-                    const uint32_t pa = s_p + (k >> 2) * HALF_BYTES + (k & 3) * 32;
-                    tcgen05_mma_bf16(d, smem_desc_sw128(pa), smem_desc_mn_sw128(s_v(b) + k * 2048, HALF_BYTES), IDESC_128x128_KMN,
-                                     (j > 0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < BKV / 16; ++k)      // A: 16 keys further along P's rows; B: 16 key rows further down V (two 8-row groups)
+                        tcgen05_mma_bf16(d, p + (((k >> 2) * HALF_BYTES + (k & 3) * 32) >> 4), value + k * (2048 >> 4), IDESC_128x128_KMN,
+                                         (j > 0 || k > 0) ? 1u : 0u);
+                    tcgen05_commit(bar(PV_DONE));
+                    tcgen05_commit(bar(V_EMPTY + b));
                 }
-                tcgen05_commit(bar(PV_DONE));
-                tcgen05_commit(bar(V_EMPTY + b));
+                __syncwarp();
             }
-            if (!ok) { *abort_flag = 1; atomicExch(error_word, 22); }
+            if (!ok && lane == 0) { *abort_flag = 1; atomicExch(error_word, 22); }
         }
     } else {
         // ---------------- softmax: thread = query row = TMEM lane ----------------
