@@ -333,7 +333,30 @@ struct VecRef {
         return dtype == JLLM_F32 ? static_cast<const float*>(p)[i]
                                  : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
     }
+    // the four values from i on (i a multiple of 4), in one access where the vector's start allows it
+    __device__ __forceinline__ float4 four(int i) const {
+        if (dtype == JLLM_F32) {
+            if (((uintptr_t)p & 15u) == 0) return *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i);
+        } else if (((uintptr_t)p & 7u) == 0) {
+            const uint2 v = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p) + i);
+            return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                               __uint_as_float(v.y & 0xffff0000u));
+        }
+        return make_float4((*this)[i], (*this)[i + 1], (*this)[i + 2], (*this)[i + 3]);
+    }
 };
+
+// item = row * per + at, without a 64-bit division where 32 bits hold the item
+__device__ __forceinline__ void split_item(long long item, int per, int& row, int& at) {
+    if (item < 0x100000000ll) {
+        const unsigned q = (unsigned)item / (unsigned)per;
+        row = (int)q;
+        at = (int)((unsigned)item - q * (unsigned)per);
+    } else {
+        row = (int)(item / per);
+        at = (int)(item % per);
+    }
+}
 
 // ---- reductions with a fixed order: the result of a row never depends on what else is in the batch ----
 
@@ -353,16 +376,10 @@ __device__ __forceinline__ float warp_max(float v) {
 __device__ __forceinline__ float block_sum(float v, float* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
     v = warp_sum(v);
-    __syncthreads();
+    __syncthreads();               // (the warps' sums of a call in front of this one have been read)
     if (lane == 0) scratch[warp] = v;
     __syncthreads();
-    if (warp == 0) {
-        float t = lane < warps ? scratch[lane] : 0.f;
-        t = warp_sum(t);
-        if (lane == 0) scratch[32] = t;
-    }
-    __syncthreads();
-    return scratch[32];
+    return warp_sum(lane < warps ? scratch[lane] : 0.f);        // every warp adds them up, in the same order
 }
 
 __device__ __forceinline__ float block_max(float v, float* scratch) {

@@ -8,8 +8,16 @@
 
 // The scale of an RMSNorm, taken in double from a float mean, as the reference does.
 __device__ __forceinline__ float rms_scale(float sum_squares, int n, float eps) {
+    // 1 / sqrt(mean) in double by two of Newton's steps y <- y (1.5 - 0.5 mean y^2) from the single-precision estimate: each squares the
+    // relative error (2^-22, 2^-43, below 2^-52), where a division and a root in double were half of what a head's norm took (its warps
+    // all compute it). Values a step could leave the range of go the long way.
     const float mean = sum_squares / (float)n + eps;
-    return (float)(1.0 / sqrt((double)mean));
+    if (!(mean > 1e-30f && mean < 1e30f)) return (float)(1.0 / sqrt((double)mean));
+    const double half = 0.5 * (double)mean;
+    double y = (double)rsqrtf(mean);
+    y = y * fma(-half, y * y, 1.5);
+    y = y * fma(-half, y * y, 1.5);
+    return (float)y;
 }
 
 // a[i] = x[lane * V + i], b[i] = x[32 * V + lane * V + i]; cos_row / sin_row: the 32 * V angles of the row's position

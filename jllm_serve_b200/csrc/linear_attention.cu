@@ -613,8 +613,8 @@ gated_norm_vec_kernel(const float* __restrict__ o, const TG* __restrict__ gate, 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = warp % W;
     const long long at = (long long)blockIdx.x * (8 / W) + warp / W;           // (row, head)
     const bool live = at < total;
-    const long long r = live ? at / heads : 0;
-    const int h = live ? (int)(at - r * heads) : 0;
+    int r = 0, h = 0;
+    if (live) split_item(at, heads, r, h);
     const bool logistic = gate_kind & 1, gate_first = gate_kind & 2;
     const int g0 = (gate_kind & 4) ? h * DV : 0;
     const float* src = o + ((size_t)r * heads + h) * DV;
@@ -650,9 +650,11 @@ gated_norm_vec_kernel(const float* __restrict__ o, const TG* __restrict__ gate, 
     for (int c = 0; c < NV; ++c) {
         const int i = ((c * W + sub) * 32 + lane) * 4;
         float out[4];
+        const float4 g4 = gain.four(g0 + i);
+        const float gn[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const float n = __fmul_rn(__fmul_rn(v[c][e], inv), gain[g0 + i + e]);
+            const float n = __fmul_rn(__fmul_rn(v[c][e], inv), gn[e]);
             out[e] = __fmul_rn(gate_first ? n : __fmul_rn(n, gt[c][e]), scale);
         }
         store_four(dst + i, out);

@@ -111,6 +111,88 @@ norm_add_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef gain,
     }
 }
 
+// The row in registers (widths that are a multiple of 4, at most 1,024 V): one trip to memory for both statistics and the result, the
+// gains on their way before the kernel in front has ended. Sums are grouped by thread, four neighbouring values at a time.
+template <int V>
+struct HeldRow {
+    float4 v[V], g[V];
+    __device__ __forceinline__ void gains(const VecRef& gain, int n4) {
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            const int i = threadIdx.x + 256 * j;
+            g[j] = i < n4 ? gain.four(4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ void load(const float* src, int n4) {
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            const int i = threadIdx.x + 256 * j;
+            v[j] = i < n4 ? reinterpret_cast<const float4*>(src)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ void statistics(int dim, float eps, int center, float* scratch, float& mean, float& inv) const {
+        mean = 0.f;
+        if (center) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < V; ++j) s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+            mean = block_sum(s, scratch) / (float)dim;
+        }
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            if (4 * (threadIdx.x + 256 * j) >= dim) break;
+            const float a = v[j].x - mean, b = v[j].y - mean, c = v[j].z - mean, d = v[j].w - mean;
+            ss = fmaf(a, a, ss); ss = fmaf(b, b, ss); ss = fmaf(c, c, ss); ss = fmaf(d, d, ss);
+        }
+        inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)dim + eps);
+    }
+    // o + norm(v) * g, piece j
+    __device__ __forceinline__ float4 added(int j, const float4& o, float mean, float inv) const {
+        return make_float4(__fadd_rn(o.x, __fmul_rn(__fmul_rn(v[j].x - mean, inv), g[j].x)), __fadd_rn(o.y, __fmul_rn(__fmul_rn(v[j].y - mean, inv), g[j].y)),
+                           __fadd_rn(o.z, __fmul_rn(__fmul_rn(v[j].z - mean, inv), g[j].z)), __fadd_rn(o.w, __fmul_rn(__fmul_rn(v[j].w - mean, inv), g[j].w)));
+    }
+};
+template <typename T>
+__device__ __forceinline__ void store_piece(T* dst, int i, const float4& y) {
+    if constexpr (sizeof(T) == 4) {
+        reinterpret_cast<float4*>(dst)[i] = y;
+    } else {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+        reinterpret_cast<uint2*>(dst)[i] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    }
+}
+
+template <typename Tnext, int V>
+__global__ void __launch_bounds__(256)
+norm_add_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef gain, Tnext* __restrict__ next_out, int dim, float eps,
+                    int center) {
+    __shared__ float scratch[33];
+    const int n4 = dim >> 2;
+    HeldRow<V> row;
+    row.gains(gain, n4);
+    pdl_wait();
+    pdl_trigger();
+    row.load(a + (size_t)blockIdx.x * dim, n4);
+    float4* xr = reinterpret_cast<float4*>(x + (size_t)blockIdx.x * dim);
+    float4 o[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int i = threadIdx.x + 256 * j;
+        o[j] = i < n4 ? xr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float mean, inv;
+    row.statistics(dim, eps, center, scratch, mean, inv);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int i = threadIdx.x + 256 * j;
+        if (i >= n4) break;
+        const float4 y = row.added(j, o[j], mean, inv);
+        xr[i] = y;
+        if (next_out != nullptr) store_piece(next_out + (size_t)blockIdx.x * dim, i, y);
+    }
+}
+
 template <typename Tout>
 __global__ void __launch_bounds__(256)
 token_shift_kernel(const float* __restrict__ x, VecRef mu, float* __restrict__ state, const int* __restrict__ row_seg,
@@ -128,8 +210,9 @@ token_shift_kernel(const float* __restrict__ x, VecRef mu, float* __restrict__ s
     if (rows_vec4(cur, saved, dim) && (((uintptr_t)dst) & 7u) == 0) {
         for (int i = threadIdx.x * 4; i < dim; i += blockDim.x * 4) {
             const float4 c = *reinterpret_cast<const float4*>(cur + i), p = *reinterpret_cast<const float4*>(before + i);
-            const float y0 = __fadd_rn(c.x, __fmul_rn(p.x - c.x, mu[i])), y1 = __fadd_rn(c.y, __fmul_rn(p.y - c.y, mu[i + 1]));
-            const float y2 = __fadd_rn(c.z, __fmul_rn(p.z - c.z, mu[i + 2])), y3 = __fadd_rn(c.w, __fmul_rn(p.w - c.w, mu[i + 3]));
+            const float4 m = mu.four(i);
+            const float y0 = __fadd_rn(c.x, __fmul_rn(p.x - c.x, m.x)), y1 = __fadd_rn(c.y, __fmul_rn(p.y - c.y, m.y));
+            const float y2 = __fadd_rn(c.z, __fmul_rn(p.z - c.z, m.z)), y3 = __fadd_rn(c.w, __fmul_rn(p.w - c.w, m.w));
             if constexpr (sizeof(Tout) == 4) {
                 dst[i] = y0; dst[i + 1] = y1; dst[i + 2] = y2; dst[i + 3] = y3;
             } else {
@@ -268,6 +351,86 @@ norm_add_mix_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef g
         if (shift) {
             hr[i] = from_float<Tout>(__fadd_rn(acc, __fmul_rn(saved[i] - acc, mu[i])));
             saved[i] = acc;
+        }
+    }
+}
+
+// The same with the row in registers (see HeldRow), the planes below it four at a time: a thread has 4 V of their pieces on their way
+// where it waited for one after the other (2,048 rows of 2,048, the layers' results of two to nine planes: 37 us on average before).
+template <typename Tout, int V>
+__global__ void __launch_bounds__(256)
+norm_add_mix_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef gain, int dim, float eps, int center,
+                        const float* __restrict__ stack, size_t plane, VecRef weights, int n, float* __restrict__ mix_out, int shift,
+                        VecRef mu, float* __restrict__ state, int slots, const int* __restrict__ row_seg,
+                        const int* __restrict__ state_slots, Tout* __restrict__ h_out) {
+    constexpr int BATCH = V >= 4 ? 2 : 4;
+    __shared__ float scratch[33];
+    __shared__ float wj[MIX_MAX];
+    const int r = blockIdx.x, n4 = dim >> 2;
+    HeldRow<V> row;
+    row.gains(gain, n4);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) wj[j] = weights[j];
+    pdl_wait();
+    pdl_trigger();
+    row.load(a + (size_t)r * dim, n4);
+    float4* xr = reinterpret_cast<float4*>(x + (size_t)r * dim);
+    const float4* lower = reinterpret_cast<const float4*>(stack + (size_t)r * dim);
+    const size_t step = plane >> 2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 o[V], p[BATCH][V], acc[V];
+    auto fetch = [&](int j0) {
+#pragma unroll
+        for (int b = 0; b < BATCH; ++b)
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                const int i = threadIdx.x + 256 * j;
+                p[b][j] = j0 + b < n - 1 && i < n4 ? lower[(size_t)(j0 + b) * step + i] : zero;
+            }
+    };
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int i = threadIdx.x + 256 * j;
+        o[j] = i < n4 ? xr[i] : zero;
+        acc[j] = zero;
+    }
+    fetch(0);
+    float mean, inv;
+    row.statistics(dim, eps, center, scratch, mean, inv);      // (its barriers also publish wj)
+    for (int j0 = 0; j0 < n - 1; j0 += BATCH) {
+#pragma unroll
+        for (int b = 0; b < BATCH; ++b) {
+            if (j0 + b >= n - 1) break;
+            const float w = wj[j0 + b];
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                acc[j].x = fmaf(w, p[b][j].x, acc[j].x);
+                acc[j].y = fmaf(w, p[b][j].y, acc[j].y);
+                acc[j].z = fmaf(w, p[b][j].z, acc[j].z);
+                acc[j].w = fmaf(w, p[b][j].w, acc[j].w);
+            }
+        }
+        if (j0 + BATCH < n - 1) fetch(j0 + BATCH);
+    }
+    float* saved = nullptr;
+    if (shift) {
+        const int slot = state_slots[row_seg[r]];
+        if (!jllm_in_bounds(slot, slots, BOUNDS_SLOT)) return;
+        saved = state + (size_t)slot * dim;
+    }
+    const float w = wj[n - 1];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int i = threadIdx.x + 256 * j;
+        if (i >= n4) break;
+        const float4 y = row.added(j, o[j], mean, inv);
+        xr[i] = y;
+        const float4 m = make_float4(fmaf(w, y.x, acc[j].x), fmaf(w, y.y, acc[j].y), fmaf(w, y.z, acc[j].z), fmaf(w, y.w, acc[j].w));
+        reinterpret_cast<float4*>(mix_out + (size_t)r * dim)[i] = m;
+        if (shift) {
+            const float4 b = reinterpret_cast<const float4*>(saved)[i], u = mu.four(4 * i);
+            store_piece(h_out + (size_t)r * dim, i, make_float4(__fadd_rn(m.x, __fmul_rn(b.x - m.x, u.x)), __fadd_rn(m.y, __fmul_rn(b.y - m.y, u.y)),
+                                                               __fadd_rn(m.z, __fmul_rn(b.z - m.z, u.z)), __fadd_rn(m.w, __fmul_rn(b.w - m.w, u.w))));
+            reinterpret_cast<float4*>(saved)[i] = m;
         }
     }
 }
@@ -493,6 +656,18 @@ JLLM_EXPORT int jllm_norm_add(float* x, const float* a, const void* gain, int ga
     JLLM_REQUIRE(rows >= 0 && dim > 0, "norm_add: rows=%d dim=%d", rows, dim);
     if (rows == 0) return JLLM_OK;
     const VecRef g{gain, gain_dtype};
+    if (dim % 4 == 0 && dim <= 4096 && (((uintptr_t)x | (uintptr_t)a | (uintptr_t)next_out) & 15u) == 0) {
+#define JLLM_NORM_ADD(T, V)                                                                                                        \
+    jllm_launch(norm_add_vec_kernel<T, V>, dim3(rows), dim3(256), 0, stream, LAUNCH_DEPENDENT, x, a, g, (T*)next_out, dim, eps, center)
+#define JLLM_NORM_ADD_T(T)                                                                                                         \
+    do {                                                                                                                           \
+        if (dim <= 1024) JLLM_NORM_ADD(T, 1); else if (dim <= 2048) JLLM_NORM_ADD(T, 2); else JLLM_NORM_ADD(T, 4);                 \
+    } while (0)
+        if (next_dtype == JLLM_F32) JLLM_NORM_ADD_T(float); else JLLM_NORM_ADD_T(__nv_bfloat16);
+#undef JLLM_NORM_ADD_T
+#undef JLLM_NORM_ADD
+        return jllm_check_launch("norm_add");
+    }
     if (next_dtype == JLLM_F32)
         jllm_launch(norm_add_kernel<float>, dim3(rows), dim3(256), 0, stream, LAUNCH_DEPENDENT, x, a, g, (float*)next_out, dim, eps,
                     center);
@@ -553,6 +728,20 @@ JLLM_EXPORT int jllm_norm_add_mix(float* x, const float* a, const void* gain, in
     if (rows == 0) return JLLM_OK;
     const VecRef g{gain, gain_dtype}, w{weights, weights_dtype}, m{mu, mu_dtype};
     const int shift = mu != nullptr;
+    if (dim % 4 == 0 && dim <= 4096 && plane % 4 == 0 &&
+        (((uintptr_t)x | (uintptr_t)a | (uintptr_t)stack | (uintptr_t)mix_out | (uintptr_t)state | (uintptr_t)h_out) & 15u) == 0) {
+#define JLLM_MIX(T, V)                                                                                                             \
+    jllm_launch(norm_add_mix_vec_kernel<T, V>, dim3(rows), dim3(256), 0, stream, LAUNCH_DEPENDENT, x, a, g, dim, eps, center, stack, \
+                (size_t)plane, w, n, mix_out, shift, m, state, slots, row_seg, state_slots, (T*)h_out)
+#define JLLM_MIX_T(T)                                                                                                              \
+    do {                                                                                                                           \
+        if (dim <= 1024) JLLM_MIX(T, 1); else if (dim <= 2048) JLLM_MIX(T, 2); else JLLM_MIX(T, 4);                                \
+    } while (0)
+        if (out_dtype == JLLM_F32) JLLM_MIX_T(float); else JLLM_MIX_T(__nv_bfloat16);
+#undef JLLM_MIX_T
+#undef JLLM_MIX
+        return jllm_check_launch("norm_add_mix");
+    }
     if (out_dtype == JLLM_F32)
         jllm_launch(norm_add_mix_kernel<float>, dim3(rows), dim3(256), 0, stream, LAUNCH_DEPENDENT, x, a, g, dim, eps, center, stack,
                     (size_t)plane, w, n, mix_out, shift, m, state, slots, row_seg, state_slots, (float*)h_out);

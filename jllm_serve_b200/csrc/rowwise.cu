@@ -93,19 +93,26 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, VecRef gain, Tout* _
 
 // The same for widths that are a multiple of 4 and at most 8192: the row is read once, as float4, and kept in
 // registers between the sum of squares and the scaling.
-template <typename Tout>
+template <typename Tout, int V>
 __global__ void __launch_bounds__(256)
 rmsnorm_vec_kernel(const float* __restrict__ x, VecRef gain, Tout* __restrict__ out, const int* __restrict__ row_index,
                    int dim, float eps) {
     __shared__ float scratch[33];
+    const int r = blockIdx.x, n4 = dim >> 2;
+    // (the gains are nobody's output: they are on their way while the kernel in front ends)
+    float4 g[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+        const int i = threadIdx.x + 256 * j;
+        g[j] = i < n4 ? gain.four(4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     pdl_wait();
     pdl_trigger();
-    const int r = blockIdx.x, n4 = dim >> 2;
     const float4* src = reinterpret_cast<const float4*>(x + (size_t)(row_index ? row_index[r] : r) * dim);
-    float4 v[8];
+    float4 v[V];
     float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < V; ++j) {
         const int i = threadIdx.x + 256 * j;
         v[j] = i < n4 ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         ss = fmaf(v[j].x, v[j].x, ss);
@@ -117,11 +124,11 @@ rmsnorm_vec_kernel(const float* __restrict__ x, VecRef gain, Tout* __restrict__ 
     const float s = rms_scale(ss, dim, eps);
     Tout* dst = out + (size_t)r * dim;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < V; ++j) {
         const int i = threadIdx.x + 256 * j;
         if (i >= n4) break;
-        const float a = __fmul_rn(__fmul_rn(v[j].x, s), gain[4 * i + 0]), b = __fmul_rn(__fmul_rn(v[j].y, s), gain[4 * i + 1]);
-        const float c = __fmul_rn(__fmul_rn(v[j].z, s), gain[4 * i + 2]), d = __fmul_rn(__fmul_rn(v[j].w, s), gain[4 * i + 3]);
+        const float a = __fmul_rn(__fmul_rn(v[j].x, s), g[j].x), b = __fmul_rn(__fmul_rn(v[j].y, s), g[j].y);
+        const float c = __fmul_rn(__fmul_rn(v[j].z, s), g[j].z), d = __fmul_rn(__fmul_rn(v[j].w, s), g[j].w);
         if constexpr (sizeof(Tout) == 4) {
             reinterpret_cast<float4*>(dst)[i] = make_float4(a, b, c, d);
         } else {
@@ -140,12 +147,17 @@ JLLM_EXPORT int jllm_rmsnorm(const float* x, const void* gain, int gain_dtype, v
     if (rows == 0) return JLLM_OK;
     const VecRef g{gain, gain_dtype};
     if (dim % 4 == 0 && dim <= 8192 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0) {
-        if (out_dtype == JLLM_F32)
-            jllm_launch(rmsnorm_vec_kernel<float>, dim3(rows), dim3(256), 0, stream, true, x, g, (float*)out, row_index, dim,
-                        eps);
-        else
-            jllm_launch(rmsnorm_vec_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, true, x, g,
-                        (__nv_bfloat16*)out, row_index, dim, eps);
+#define JLLM_NORM(V)                                                                                                             \
+    do {                                                                                                                         \
+        if (out_dtype == JLLM_F32)                                                                                               \
+            jllm_launch(rmsnorm_vec_kernel<float, V>, dim3(rows), dim3(256), 0, stream, true, x, g, (float*)out, row_index, dim, eps); \
+        else                                                                                                                     \
+            jllm_launch(rmsnorm_vec_kernel<__nv_bfloat16, V>, dim3(rows), dim3(256), 0, stream, true, x, g, (__nv_bfloat16*)out, \
+                        row_index, dim, eps);                                                                                    \
+    } while (0)
+        const int v = (dim / 4 + 255) / 256;
+        if (v <= 1) JLLM_NORM(1); else if (v <= 2) JLLM_NORM(2); else if (v <= 4) JLLM_NORM(4); else JLLM_NORM(8);
+#undef JLLM_NORM
         return jllm_check_launch("rmsnorm");
     }
     const int threads = dim >= 2048 ? 512 : 256;
@@ -329,7 +341,9 @@ qk_norm_rope_store_warp_kernel(T* __restrict__ qkv, VecRef q_gain, VecRef k_gain
     pdl_trigger();
     const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (item >= items) return;
-    const int r = (int)(item / heads_total), h = (int)(item % heads_total), lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
+    int r, h;
+    split_item(item, heads_total, r, h);
     T* src = qkv + (size_t)r * row_stride + (size_t)h * HD;
     const bool is_q = h < heads, is_k = !is_q && h < heads + kv_heads;
     float a[V], b[V];
@@ -373,10 +387,19 @@ qk_norm_rope_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, VecRef q_gain, Ve
     const int lane = threadIdx.x & 31, sub = lane % LANES;
     const long long item = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * PER_WARP + lane / LANES;
     const bool live = item < items;
-    const int r = live ? (int)(item / heads_total) : 0, h = live ? (int)(item % heads_total) : 0;
+    int r = 0, h = 0;
+    if (live) split_item(item, heads_total, r, h);
     __nv_bfloat16* src = qkv + (size_t)r * row_stride + (size_t)h * HD;
     const bool is_q = h < heads, is_k = !is_q && h < heads + kv_heads;
     float a[8], b[8];
+    // (the angles' trip, position and row of the table, goes beside the values': a warp has nothing else to hide it behind)
+    const int slot = live && !is_q ? slots[r] : 0;
+    float4 c0, c1, s0, s1;
+    if (is_q || is_k) {
+        const size_t at = (size_t)positions[r] * HALF + sub * 8;
+        const float4 *c4 = reinterpret_cast<const float4*>(cos_t + at), *s4 = reinterpret_cast<const float4*>(sin_t + at);
+        c0 = c4[0], c1 = c4[1], s0 = s4[0], s1 = s4[1];
+    }
     {
         const uint4 ua = live ? *reinterpret_cast<const uint4*>(src + sub * 8) : make_uint4(0, 0, 0, 0);
         const uint4 ub = live ? *reinterpret_cast<const uint4*>(src + HALF + sub * 8) : make_uint4(0, 0, 0, 0);
@@ -401,14 +424,16 @@ qk_norm_rope_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, VecRef q_gain, Ve
             const float s = rms_scale(ss, HD, eps);
             const VecRef g = is_q ? q_gain : k_gain;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                a[i] = __fmul_rn(__fmul_rn(a[i], s), g[sub * 8 + i]);
-                b[i] = __fmul_rn(__fmul_rn(b[i], s), g[HALF + sub * 8 + i]);
+            for (int q = 0; q < 8; q += 4) {
+                const float4 ga4 = g.four(sub * 8 + q), gb4 = g.four(HALF + sub * 8 + q);
+                const float ga[4] = {ga4.x, ga4.y, ga4.z, ga4.w}, gb[4] = {gb4.x, gb4.y, gb4.z, gb4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    a[q + i] = __fmul_rn(__fmul_rn(a[q + i], s), ga[i]);
+                    b[q + i] = __fmul_rn(__fmul_rn(b[q + i], s), gb[i]);
+                }
             }
         }
-        const float4* c4 = reinterpret_cast<const float4*>(cos_t + (size_t)positions[r] * HALF + sub * 8);
-        const float4* s4 = reinterpret_cast<const float4*>(sin_t + (size_t)positions[r] * HALF + sub * 8);
-        const float4 c0 = c4[0], c1 = c4[1], s0 = s4[0], s1 = s4[1];
         const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
         const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
@@ -422,7 +447,6 @@ qk_norm_rope_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, VecRef q_gain, Ve
     __nv_bfloat16* dst = src;
     if (!is_q) {
         const int kvh = is_k ? h - heads : h - heads - kv_heads;
-        const int slot = slots[r];
         if (!jllm_in_bounds(slot, num_slots, BOUNDS_SLOT)) return;      // checked build: the write is dropped
         const size_t page = slot / page_size, off = slot % page_size;
         dst = (is_k ? k_cache : v_cache) + ((page * kv_heads + kvh) * page_size + off) * HD;
@@ -619,7 +643,8 @@ head_prepare_vec_kernel(__nv_bfloat16* __restrict__ qkv, int row_stride, int q_o
     const int lane = threadIdx.x & 31, sub = lane % LANES;
     const long long item = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * PER_WARP + lane / LANES;
     const bool live = item < items;
-    const int r = live ? (int)(item / heads_total) : 0, h = live ? (int)(item % heads_total) : 0;
+    int r = 0, h = 0;
+    if (live) split_item(item, heads_total, r, h);
     const bool is_q = h < heads, is_k = !is_q && h < heads + kv_heads;
     __nv_bfloat16* src = qkv + (size_t)r * row_stride +
                          (is_q ? q_off + (size_t)h * HD : is_k ? k_off + (size_t)(h - heads) * HD
@@ -649,7 +674,12 @@ head_prepare_vec_kernel(__nv_bfloat16* __restrict__ qkv, int row_stride, int q_o
         const VecRef g = is_q ? q_gain : k_gain;
         if (turns) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = __fmul_rn(__fmul_rn(x[i], s), g[sub * 8 + i]);
+            for (int q = 0; q < 8; q += 4) {
+                const float4 g4 = g.four(sub * 8 + q);
+                const float gv[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[q + i] = __fmul_rn(__fmul_rn(x[q + i], s), gv[i]);
+            }
         }
     }
     if (rotary_dim > 0) {
@@ -902,11 +932,12 @@ norm_sum_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef g
         const float pa[4] = {va[u].x, va[u].y, va[u].z, va[u].w}, pb[4] = {vb[u].x, vb[u].y, vb[u].z, vb[u].w};
         float4 old = accumulate ? *reinterpret_cast<const float4*>(x + row + 4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
         float res[4] = {old.x, old.y, old.z, old.w};
+        const float4 ga4 = gain_a.four(4 * gi), gb4 = b ? gain_b.four(4 * gi) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float ga[4] = {ga4.x, ga4.y, ga4.z, ga4.w}, gb[4] = {gb4.x, gb4.y, gb4.z, gb4.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int i = 4 * gi + k;
-            float v = __fmul_rn(__fmul_rn(pa[k], ra), gain_a[i]);
-            if (b) v = __fadd_rn(v, __fmul_rn(__fmul_rn(pb[k], rb), gain_b[i]));
+            float v = __fmul_rn(__fmul_rn(pa[k], ra), ga[k]);
+            if (b) v = __fadd_rn(v, __fmul_rn(__fmul_rn(pb[k], rb), gb[k]));
             v = __fmul_rn(v, scale);
             res[k] = accumulate ? __fadd_rn(res[k], v) : v;
         }
@@ -996,10 +1027,10 @@ __global__ void __launch_bounds__(256)
 norm_chain_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef gain_a, const float* __restrict__ b,
                       VecRef gain_b, float scale, VecRef gain_post, VecRef gain_next, Tnext* __restrict__ next, int dim, float eps) {
     __shared__ float scratch[33];
-    pdl_wait();
-    pdl_trigger();
     const size_t row = (size_t)blockIdx.x * dim;
     const int n4 = dim >> 2;
+    pdl_wait();
+    pdl_trigger();
     const float4* pa = reinterpret_cast<const float4*>(a + row);
     const float4* pb = b ? reinterpret_cast<const float4*>(b + row) : nullptr;
     float4* px = reinterpret_cast<float4*>(x + row);
@@ -1028,9 +1059,11 @@ norm_chain_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef
             if (i >= dim) break;
             float* pva = reinterpret_cast<float*>(&va[j]);
             const float* pvb = reinterpret_cast<const float*>(&vb[j]);
+            const float4 ga4 = gain_a.four(i), gb4 = gain_b.four(i);
+            const float ga[4] = {ga4.x, ga4.y, ga4.z, ga4.w}, gb[4] = {gb4.x, gb4.y, gb4.z, gb4.w};
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                pva[c] = __fmul_rn(__fadd_rn(__fmul_rn(__fmul_rn(pva[c], ra), gain_a[i + c]), __fmul_rn(__fmul_rn(pvb[c], rb), gain_b[i + c])), scale);
+                pva[c] = __fmul_rn(__fadd_rn(__fmul_rn(__fmul_rn(pva[c], ra), ga[c]), __fmul_rn(__fmul_rn(pvb[c], rb), gb[c])), scale);
         }
     }
     float sv = 0.f;
@@ -1045,8 +1078,10 @@ norm_chain_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef
         if (i4 >= n4) break;
         const float* pva = reinterpret_cast<const float*>(&va[j]);
         float* pvx = reinterpret_cast<float*>(&vx[j]);
+        const float4 gp4 = gain_post.four(4 * i4);
+        const float gp[4] = {gp4.x, gp4.y, gp4.z, gp4.w};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) pvx[c] = __fadd_rn(pvx[c], __fmul_rn(__fmul_rn(pva[c], rv), gain_post[4 * i4 + c]));
+        for (int c = 0; c < 4; ++c) pvx[c] = __fadd_rn(pvx[c], __fmul_rn(__fmul_rn(pva[c], rv), gp[c]));
         px[i4] = vx[j];
         sx = squares(vx[j], sx);
     }
@@ -1059,9 +1094,11 @@ norm_chain_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef
         const int i4 = threadIdx.x + 256 * j;
         if (i4 >= n4) break;
         const float* pvx = reinterpret_cast<const float*>(&vx[j]);
+        const float4 gn4 = gain_next.four(4 * i4);
+        const float gn[4] = {gn4.x, gn4.y, gn4.z, gn4.w};
         float o[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) o[c] = __fmul_rn(__fmul_rn(pvx[c], rx), gain_next[4 * i4 + c]);
+        for (int c = 0; c < 4; ++c) o[c] = __fmul_rn(__fmul_rn(pvx[c], rx), gn[c]);
         if constexpr (sizeof(Tnext) == 4) {
             reinterpret_cast<float4*>(pn)[i4] = make_float4(o[0], o[1], o[2], o[3]);
         } else {
