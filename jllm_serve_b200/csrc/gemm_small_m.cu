@@ -15,14 +15,23 @@
 // (t * k_blocks + kb) * 16 KB; padded with zeros). A warp's load of 8 rows x 64 bytes then comes from one 1 KB
 // stretch of memory instead of 8 rows that lie a whole row apart.
 //
+// A matrix of few rows and a long k (a down projection of a narrow model) has a block for fewer SMs than there are, each with a
+// long way through k: there a cluster of two blocks takes the same rows, half of the k blocks each, and their sums meet through
+// distributed shared memory (first half + second half).
+//
 // Requirements (else the caller uses the CUDA-core kernel): bfloat16 inputs, K a multiple of 8,
 // 16-byte aligned rows (lda a multiple of 8; aligned base pointers), 1 <= M <= 64.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace {
 
 constexpr int WARPS = 8;
 constexpr int KCHUNK = 32;
+// From so many k blocks on two blocks share the way (8 rows, a block for each 16 rows and two: 2,048 x 12,288 13.4 and 11.1 us, x 8,192 9.7 and
+// 8.4, x 4,096 6.0 and 5.9, x 2,048 3.9 and 4.3).
+constexpr int HALVES_MIN_K_BLOCKS = 96;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                uint32_t b0, uint32_t b1) {
@@ -45,7 +54,7 @@ __device__ __forceinline__ uint4 load_16_stream(const __nv_bfloat16* p) {
     return v;
 }
 
-template <int NT, int RT, int UNROLL, typename Tout>
+template <int NT, int RT, int UNROLL, bool HALVES, typename Tout>
 __global__ void __launch_bounds__(WARPS * 32, 2)
 gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w, int k_blocks,
                     VecRef bias, int has_bias, Tout* __restrict__ out, int ldo, int accumulate, int M, int N, int K,
@@ -53,7 +62,8 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
     extern __shared__ float red[];  // [WARPS][RT * 16][NT * 8]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int n0 = blockIdx.x * (16 * RT);
+    const int half = HALVES ? (int)(blockIdx.x & 1) : 0;           // (clusters lie along x)
+    const int n0 = (HALVES ? (int)(blockIdx.x >> 1) : (int)blockIdx.x) * (16 * RT);
     float acc[RT][NT][4];
 #pragma unroll
     for (int r = 0; r < RT; ++r)
@@ -85,7 +95,9 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
         arow[j] = a + (size_t)(aok[j] ? m : 0) * lda;
     }
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    const int chunks = (K + KCHUNK - 1) / KCHUNK;
+    // this block's k blocks [k_lo, k_hi), 32-wide chunks below `chunks`
+    const int all_blocks = (K + 63) >> 6, k_lo = HALVES && half ? all_blocks >> 1 : 0, k_hi = HALVES && !half ? all_blocks >> 1 : all_blocks;
+    const int chunks = HALVES ? min((K + KCHUNK - 1) / KCHUNK, 2 * k_hi) : (K + KCHUNK - 1) / KCHUNK;
     uint4 wv[UNROLL][RT][2];
     static_assert(UNROLL % 2 == 0, "a warp takes the two halves of a k block together");
     // the u-th 32-wide chunk of the batch that starts at k block c0: k blocks c0, c0 + WARPS, ..., two chunks each
@@ -109,11 +121,10 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
     // The weights do not depend on the kernel before this one: the first batch is requested while that kernel
     // is still running. The kernels between two products (norms, RoPE, the attention combine) are tiny: the weight
     // stream would otherwise pause for them.
-    load_weights(warp);
+    load_weights(k_lo + warp);
     pdl_wait();
     pdl_trigger();
-    const int k_blocks_here = (chunks + 1) >> 1;
-    for (int c0 = warp; c0 < k_blocks_here; c0 += WARPS * (UNROLL / 2)) {
+    for (int c0 = k_lo + warp; c0 < k_hi; c0 += WARPS * (UNROLL / 2)) {
         // the activations of these chunks: issued before any of the weights is waited for, so that their
         // (L2) latency overlaps the weights' (HBM) latency instead of following it
         uint4 xv[UNROLL][NT];
@@ -138,7 +149,7 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
                 }
             }
         }
-        if (c0 + WARPS * (UNROLL / 2) < k_blocks_here) load_weights(c0 + WARPS * (UNROLL / 2));
+        if (c0 + WARPS * (UNROLL / 2) < k_hi) load_weights(c0 + WARPS * (UNROLL / 2));
     }
     // partial sums of the 8 warps -> shared memory, laid out [warp][token][row] so the final pass writes
     // consecutive output features from consecutive threads
@@ -155,19 +166,44 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
             mine[(tok + 1) * ROWS + row + 8] = acc[r][j][3];
         }
     __syncthreads();
+    const float *first = red, *second = red;
+    auto sum = [&](int e) {
+        float v = 0.f;
+        if constexpr (HALVES) {
+            v = first[e] + second[e];
+        } else {
+#pragma unroll
+            for (int wi = 0; wi < WARPS; ++wi) v += red[(size_t)wi * ROWS * TOK + e];
+        }
+        return v;
+    };
+    if constexpr (HALVES) {
+        // the block's own sum goes over warp 0's part, then both blocks read both
+        float own[(ROWS * TOK + WARPS * 32 - 1) / (WARPS * 32)];
+        int u = 0;
+#pragma unroll
+        for (int e = threadIdx.x; e < ROWS * TOK; e += WARPS * 32, ++u) {
+            own[u] = 0.f;
+#pragma unroll
+            for (int wi = 0; wi < WARPS; ++wi) own[u] += red[(size_t)wi * ROWS * TOK + e];
+        }
+        u = 0;
+#pragma unroll
+        for (int e = threadIdx.x; e < ROWS * TOK; e += WARPS * 32, ++u) red[e] = own[u];
+        const auto cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        first = cluster.map_shared_rank(red, 0);
+        second = cluster.map_shared_rank(red, 1);
+    }
     for (int e = threadIdx.x; e < ROWS * TOK; e += WARPS * 32) {
         const int tok = e / ROWS, row = e % ROWS;
         const int n = n0 + row;
-        if (tok >= M || n >= N) continue;
-        float v = 0.f;
-#pragma unroll
-        for (int wi = 0; wi < WARPS; ++wi) v += red[(size_t)wi * ROWS * TOK + e];
+        if (tok >= M || n >= N || (HALVES && (tok & 1) != half)) continue;       // (of a cluster's tokens each block finishes every other one)
+        float v = sum(e);
         if (swiglu) {
             // rows come in blocks of 16: 8 gate rows, then the 8 up rows of the same hidden units
             if ((row & 15) >= 8) continue;
-            float u = 0.f;
-#pragma unroll
-            for (int wi = 0; wi < WARPS; ++wi) u += red[(size_t)wi * ROWS * TOK + e + 8];
+            const float u = sum(e + 8);
             out[(size_t)tok * ldo + (n >> 4) * 8 + (row & 7)] = from_float<Tout>(swiglu.apply<false>(v, u, tok, (n >> 4) * 8 + (row & 7)));
             continue;
         }
@@ -177,6 +213,7 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
         if (accumulate == EPI_ADD) v += to_float(*dst);
         *dst = from_float<Tout>(v);
     }
+    if constexpr (HALVES) cooperative_groups::this_cluster().sync();        // nobody leaves while its sums are being read
 }
 
 template <int NT, int RT, int UNROLL>
@@ -185,16 +222,39 @@ int launch(const void* a, int lda, const void* w, int k_blocks, VecRef bias, int
     const int grid = (N + 16 * RT - 1) / (16 * RT);
     const size_t smem = (size_t)WARPS * RT * 16 * NT * 8 * sizeof(float);
     if (out_dtype == JLLM_F32) {
-        auto kern = gemm_small_m_kernel<NT, RT, UNROLL, float>;
+        auto kern = gemm_small_m_kernel<NT, RT, UNROLL, false, float>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         jllm_launch(kern, dim3(grid), dim3(WARPS * 32), smem, stream, LAUNCH_DEPENDENT_WANTS_L1, (const __nv_bfloat16*)a, lda,
                     (const __nv_bfloat16*)w, k_blocks, bias, has_bias, (float*)out, ldo, accumulate, M, N, K, swiglu);
     } else {
-        auto kern = gemm_small_m_kernel<NT, RT, UNROLL, __nv_bfloat16>;
+        auto kern = gemm_small_m_kernel<NT, RT, UNROLL, false, __nv_bfloat16>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         jllm_launch(kern, dim3(grid), dim3(WARPS * 32), smem, stream, LAUNCH_DEPENDENT_WANTS_L1, (const __nv_bfloat16*)a, lda,
                     (const __nv_bfloat16*)w, k_blocks, bias, has_bias, (__nv_bfloat16*)out, ldo, accumulate, M, N, K, swiglu);
     }
+    return jllm_check_launch("gemm_small_m");
+}
+
+// Two blocks to 16 rows, half of k each
+template <int NT, typename Tout>
+int launch_halves(const void* a, int lda, const void* w, int k_blocks, VecRef bias, int has_bias, void* out, int ldo, int accumulate,
+                  int M, int N, int K, GluArgs swiglu, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * ((N + 15) / 16));
+    cfg.blockDim = dim3(WARPS * 32);
+    cfg.dynamicSmemBytes = (size_t)WARPS * 16 * NT * 8 * sizeof(float);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = jllm_launch_overlaps(cfg.dynamicSmemBytes, LAUNCH_DEPENDENT_WANTS_L1) ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, gemm_small_m_kernel<NT, 1, 4, true, Tout>, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, k_blocks, bias,
+                       has_bias, (Tout*)out, ldo, accumulate, M, N, K, swiglu);
     return jllm_check_launch("gemm_small_m");
 }
 
@@ -233,6 +293,16 @@ JLLM_EXPORT int jllm_gemm_small_m(const void* a, int lda, const void* w, int k_b
     if (M <= 8) wide = blocks32 > sms && blocks32 <= 2 * sms;
     // (with the packed weight a warp's batch of four k blocks is four contiguous 2 KB pieces: twice as deep an unroll,
     // which paid on row-major weights, is slower here: gate_up at 8 rows 37.7 us against 34.8)
+    if (M <= 16 && (N + 15) / 16 <= sms && k_blocks >= HALVES_MIN_K_BLOCKS) {
+#define JLLM_HALVES(NT, T) return launch_halves<NT, T>(a, lda, w, k_blocks, b, hb, out, ldo, accumulate, M, N, K, swiglu, stream)
+        if (out_dtype == JLLM_F32) {
+            if (M <= 8) JLLM_HALVES(1, float);
+            JLLM_HALVES(2, float);
+        }
+        if (M <= 8) JLLM_HALVES(1, __nv_bfloat16);
+        JLLM_HALVES(2, __nv_bfloat16);
+#undef JLLM_HALVES
+    }
 #define JLLM_GO(NT, RT, UN) return launch<NT, RT, UN>(a, lda, w, k_blocks, b, hb, out, out_dtype, ldo, accumulate, M, N, K, swiglu, stream)
     if (M <= 8) { if (wide) { if (deep) JLLM_GO(1, 2, 8); JLLM_GO(1, 2, 4); } if (deep) JLLM_GO(1, 1, 8); JLLM_GO(1, 1, 4); }
     if (M <= 16) { if (wide) JLLM_GO(2, 2, 4); if (deep) JLLM_GO(2, 1, 8); JLLM_GO(2, 1, 4); }

@@ -937,3 +937,22 @@ def test_gemm_pair_swap(ops, M, N, K, tokens):
                 units = torch.full((M, N // 2), float("nan"), dtype=dtype, device=DEV)
                 ops.gemm_pair_swap(a, packed, units, tokens, swiglu=True, max_pairs=pairs)
                 assert torch.allclose(units.float().cpu(), want, rtol=t, atol=1e-3)
+
+
+@pytest.mark.parametrize("M", [1, 7, 16])
+@pytest.mark.parametrize("N,K", [(16, 6144), (40, 6200), (2048, 12288), (2368, 6152)])
+def test_gemm_small_m_halves_of_k(ops, M, N, K):
+    """Few weight rows and a long k: two blocks of a cluster take half of the k blocks each (an odd number of them, k no multiple of 64,
+    a last block of rows that is not full). Three runs give the same bits; float64 within 1e-4 sqrt(K) of a product's size (0.05)."""
+    a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
+    packed, base, bias = ops.pack_weight(w), rnd(M, N, seed=3), rnd(N, dtype=torch.bfloat16, seed=2)
+    want, outs = gemm_want(a, w, bias, base), [base.clone() for _ in range(3)]
+    for out in outs:
+        ops.gemm_small_m(a, packed, out, bias, accumulate=True)
+    assert torch.allclose(outs[0].cpu(), want, rtol=1e-4, atol=1e-4 * math.sqrt(K) * 0.05)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    if N % 16 == 0:
+        units = torch.empty(M, N // 2, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_small_m(a, packed, units, swiglu=True)
+        z = gemm_want(a, w).view(M, N // 16, 2, 8)
+        assert torch.allclose(units.float().cpu(), (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2), rtol=2 ** -7, atol=2e-3)
