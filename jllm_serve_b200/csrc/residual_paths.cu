@@ -610,6 +610,72 @@ norm_conv_kernel(const float* __restrict__ x, VecRef gain, VecRef conv, float* _
     }
 }
 
+// A step of single rows (8 rows of 2,048, four taps: the kernel above took 5 us of a step, most of it trips to L2 one after the other):
+// gains and taps are in registers before the kernel in front has ended, the row and the state are asked for together behind the wait,
+// and nothing is read twice. P pieces of four channels a thread; value by value the arithmetic is that of the kernel above.
+template <typename Tout, int TAPS, int P>
+__global__ void __launch_bounds__(256)
+norm_conv_step_kernel(const float* __restrict__ x, VecRef gain, VecRef conv, float* __restrict__ state, int num_slots,
+                      const int* __restrict__ row_seg, const int* __restrict__ state_slots, Tout* __restrict__ out, int dim, float eps) {
+    __shared__ float scratch[33];
+    const int r = blockIdx.x, n4 = dim >> 2;
+    int slot = state_slots[row_seg[r]];                      // (the step's tables are older than the kernel in front)
+    if (!jllm_in_bounds(slot, num_slots, BOUNDS_SLOT)) slot = -1;
+    float4 g[P], w[P][TAPS];                                 // w: the 4 x TAPS weights of a piece as they lie in memory
+#pragma unroll
+    for (int u = 0; u < P; ++u) {
+        const int i = threadIdx.x + 256 * u;
+        if (i >= n4) continue;
+        g[u] = gain.four(4 * i);
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) w[u][j] = conv.four(4 * (i * TAPS + j));
+    }
+    pdl_wait();
+    pdl_trigger();
+    float* st = state + (size_t)max(slot, 0) * (TAPS - 1) * dim;
+    Pack<4> h[P], win[P][TAPS - 1];
+    float ss = 0.f;
+#pragma unroll
+    for (int u = 0; u < P; ++u) {
+        const int i = threadIdx.x + 256 * u;
+        h[u] = Pack<4>{};
+        if (i >= n4) continue;
+        h[u] = load_pack<4>(x + (size_t)r * dim + 4 * i);
+#pragma unroll
+        for (int j = 0; j + 1 < TAPS; ++j) win[u][j] = slot >= 0 ? load_pack<4>(st + (size_t)j * dim + 4 * i) : Pack<4>{};
+    }
+#pragma unroll
+    for (int u = 0; u < P; ++u) {
+        if (threadIdx.x + 256 * u >= n4) continue;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ss = fmaf(h[u].v[k], h[u].v[k], ss);
+    }
+    const float f = 1.f / sqrtf(block_sum(ss, scratch) / (float)dim + eps);
+#pragma unroll
+    for (int u = 0; u < P; ++u) {
+        const int i = threadIdx.x + 256 * u;
+        if (i >= n4) continue;
+        const float gv[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+        float taps[4 * TAPS];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            taps[4 * j] = w[u][j].x; taps[4 * j + 1] = w[u][j].y; taps[4 * j + 2] = w[u][j].z; taps[4 * j + 3] = w[u][j].w;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) h[u].v[k] = __fmul_rn(__fmul_rn(h[u].v[k], f), gv[k]);
+        Pack<4> acc = h[u];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc.v[k] = fmaf(taps[k * TAPS + j], j + 1 < TAPS ? win[u][j < TAPS - 1 ? j : 0].v[k] : h[u].v[k], acc.v[k]);
+        store_pack<4>(out + (size_t)r * dim + 4 * i, acc);
+        if (slot >= 0) {
+#pragma unroll
+            for (int j = 0; j + 1 < TAPS; ++j) store_pack<4>(st + (size_t)j * dim + 4 * i, j + 2 < TAPS ? win[u][j + 2 < TAPS ? j + 1 : 0] : h[u]);
+        }
+    }
+}
+
 // behind it, for steps with portions: the state's new entry j is the normed row of local index n - (taps - 1) + j
 __global__ void __launch_bounds__(256)
 norm_conv_save_kernel(const float* __restrict__ x, VecRef gain, float* __restrict__ state, int num_slots,
@@ -778,6 +844,30 @@ JLLM_EXPORT int jllm_norm_conv(const float* x, const void* gain, int gain_dtype,
     if (rows == 0) return JLLM_OK;
     const VecRef g{gain, gain_dtype}, c{conv, conv_dtype};
     const bool vec = dim % 4 == 0 && (((uintptr_t)x | (uintptr_t)state | (uintptr_t)out) % 16) == 0;
+#define JLLM_CONV_STEP(T, TAPS, P)                                                                                             \
+    do {                                                                                                                       \
+        jllm_launch(norm_conv_step_kernel<T, TAPS, P>, dim3(rows), dim3(256), 0, stream, LAUNCH_DEPENDENT, x, g, c, state,     \
+                    num_slots, row_seg, state_slots, (T*)out, dim, eps);                                                       \
+        return jllm_check_launch("norm_conv");                                                                                 \
+    } while (0)
+#define JLLM_CONV_STEP_TAPS(T, P)                                                                                              \
+    do {                                                                                                                       \
+        if (taps == 2) JLLM_CONV_STEP(T, 2, P);                                                                                \
+        if (taps == 3) JLLM_CONV_STEP(T, 3, P);                                                                                \
+        JLLM_CONV_STEP(T, 4, P);                                                                                               \
+    } while (0)
+    if (single && vec && taps >= 2 && taps <= 4 && dim <= 4096) {
+        if (out_dtype == JLLM_F32) {
+            if (dim <= 1024) JLLM_CONV_STEP_TAPS(float, 1);
+            if (dim <= 2048) JLLM_CONV_STEP_TAPS(float, 2);
+            JLLM_CONV_STEP_TAPS(float, 4);
+        }
+        if (dim <= 1024) JLLM_CONV_STEP_TAPS(__nv_bfloat16, 1);
+        if (dim <= 2048) JLLM_CONV_STEP_TAPS(__nv_bfloat16, 2);
+        JLLM_CONV_STEP_TAPS(__nv_bfloat16, 4);
+    }
+#undef JLLM_CONV_STEP_TAPS
+#undef JLLM_CONV_STEP
 #define JLLM_NORM_CONV(T, RUN, V, TAPS)                                                                                        \
     jllm_launch(norm_conv_kernel<T, RUN, V, TAPS>, dim3((rows + RUN - 1) / RUN), dim3(256), 0, stream, LAUNCH_DEPENDENT, x, g, c,   \
                 state, num_slots, row_seg, seg_start, state_slots, (T*)out, rows, dim, taps, eps, single)
