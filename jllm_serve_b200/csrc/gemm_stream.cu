@@ -374,8 +374,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __nv_bfloat1
 // tokens, the others write their parts of it straight into its shared memory (st.shared::cluster), and after the cluster's
 // barrier it adds them up in k order. Launched back to back, equal runs and clusters: 64 rows against O (4,096 x 4,096) 14.0 and
 // 11.5 us, against down (4,096 x 12,288) 24.5 and 21.7, 24 rows against them 13.8 and 10.5, 23.4 and 20.3; 64 rows against 2,048 x
-// 8,192 16.5 and 12.7. What bounds it is what an SM takes in, 60 GB/s of weights and activations (0.33 us per k block with 32 tokens,
-// 0.40 with 64) on the SMs that have a block, and about 5 us from launch to first bytes and for the meeting.
+// 8,192 16.5 and 12.7. (These with one lane in the issuing loops, 0.33 us a k block with 32 tokens; with whole warps, see tcgen05_common.cuh,
+// clusters take 9.3 us for 64 rows of O, 23.0 of down, 13.4 of QKV.) What bounds it is what an SM takes in on the SMs that have a block,
+// and about 5 us from launch to first bytes and for the meeting.
 // `overlay`: the parts lie over the ring (many tokens leave no room beside it); the cluster then meets once more, when every block
 // is done with its ring, before anything is written.
 constexpr int CLUSTER_MAX = 8;
