@@ -1030,12 +1030,17 @@ def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str
     42.5 and 38.1; O of 512 17.7 and 15.9; gate_up of 144 47.7 and 38.6, of 400 73.0 and 63.3, of 613 101 and 88; down of 300
     47.3 and 35.5, of 613 59.6 and 50.7. From there on 256 x 256 tiles with the tokens as the M side are as good (gate_up of 1,536 rows
     195 and 213): it takes a twelfth less by this count to change. Below 129 rows there are too few tiles; of few k blocks a pair's start and
-    end are most of it (3,072 x 768, 613 rows 6.6 and 7.4); matrices much longer than high stay with `gemm_stream` up to 208 rows
-    (down of 200 rows 38.4 and 40, of 256 48.5 and 45.4). A matrix of few rows, which the streamed pairs took between 257 and 512
-    rows, was worst off there (768 x 2,048, 300 rows: 49.6 and 7.1)."""
+    end are most of it (3,072 x 768, 613 rows 6.6 and 7.4). A matrix of few rows, which the streamed pairs took between 257 and 512
+    rows, was worst off there (768 x 2,048, 300 rows: 49.6 and 7.1).
+
+    `gemm_stream` ("swap") cuts k up over all SMs where a pair walks all of it, so there the whole product is counted: a pair's
+    rounds of (T + 256) clocks a k block against a meeting of 75 clocks a token and, on every SM, its share of all tiles' k blocks at
+    3 (128 + tokens) clocks each (16 KB of weights and 128 bytes a token); where the two are within 3 % the pairs have it. Behind a norm, us, swap and pairs: 512 x 16,384 of
+    240 rows 21.0 and 39.7, 1,024 x 8,192 16.9 and 21.8, 2,048 x 12,288 of 212 22.3 and 31.7, 1,536 x 8,960 of 256 18.3 and 23.7; about
+    even at 4,096 x 8,192 of 212 (24.2 both), 2,048 x 8,192 of 256 (22.2 and 22.7), 4,096 x 12,288 of 212 (33.2 and 33.8); 4,096 x 12,288 of 256
+    37.8 and 34.0, 2,048 x 5,120 of 256 19.3 and 15.5, 768 x 3,072 13.7 and 10.4, 4,096 x 4,096 of 144 15.3 and 14.2, 6,144 x 4,096
+    20.1 and 15.5, 4,096 x 512 10.1 and 5.2 (few k blocks do not count against the pairs here: swap is the worse for them)."""
     if pairs <= 0 or rows <= TILE_ROWS or kernel not in ("swap", "tiles", "pair", "pair-streamed"):
-        return 0
-    if kernel == "swap" and rows <= 208 and in_features >= 2 * out_features:
         return 0
     if kernel in ("tiles", "pair") and in_features < 1024:
         return 0
@@ -1050,12 +1055,16 @@ def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str
         c = cost(-(-rows // t) * high, pairs, 256 + t, 2 * t)
         if t >= 48 and (not tokens or c < best):
             best, tokens = c, t
+    if kernel == "pair-streamed":
+        return tokens
+    if kernel == "swap":
+        k_blocks, n = -(-in_features // 64), -(-rows // 16) * 16
+        stream = 75 * n + 3.0 * (128 + n) * k_blocks * -(-out_features // 128) / sms
+        return tokens if 0.97 * -(-(-(-rows // tokens) * high) // pairs) * (256 + tokens) * k_blocks <= stream else 0
     if kernel == "pair":
         other = cost(-(-rows // 256) * high, pairs, 512, 512)
-    elif kernel == "tiles":
-        other = min(cost(-(-rows // 128) * -(-out_features // w), sms, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
     else:
-        return tokens
+        other = min(cost(-(-rows // 128) * -(-out_features // w), sms, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
     return tokens if best < 0.92 * other else 0
 
 

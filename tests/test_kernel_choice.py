@@ -1,4 +1,6 @@
 """Which kernel a step's work goes to: decisions taken on the host from sizes alone (no GPU, nothing launched)."""
+import math
+
 import torch
 
 from jllm_serve_b200.csrc import ops
@@ -133,13 +135,51 @@ def test_a_wait_that_ran_out_is_reported_with_its_kernel(monkeypatch):
 
 
 def test_tokens_of_a_tile_with_the_weight_rows_as_m_side():
-    """Where the product of a pair with the weight rows as its M side takes another kernel's place, and the tiles it then has cover the rows."""
+    """Where the product of a pair with the weight rows as its M side takes another kernel's place: its tiles cover the rows and none of
+    them is empty, no other multiple of 16 makes cheaper tiles, and what it replaces costs more by the count that the rule states."""
     def tokens(rows, n, k, **more):
         return ops.pair_swap_tokens(rows, n, k, ops.gemm_kernel_for(rows, n, k), **more)
     assert tokens(613, 24576, 4096) == 208 and tokens(613, 4096, 12288) == 160 and tokens(300, 4096, 12288) == 80
     assert tokens(128, 6144, 4096) == 0 and tokens(2048, 24576, 4096) == 0 and tokens(200, 4096, 12288) == 0
     assert tokens(613, 24576, 4096, pairs=0) == 0 and ops.pair_swap_tokens(613, 24576, 4096, "rows") == 0
+
+    def clocks(tiles, places, round_, multiply):       # a k block of all tiles: rounds, and the power that all multiply-adds share
+        return math.ceil(tiles / places) * round_ + 2 * tiles * multiply / places
+    taken = left = 0
     for rows in list(range(129, 700, 13)) + [1000, 1536, 2048, 5000]:
-        for n, k in ((6144, 4096), (4096, 4096), (24576, 4096), (4096, 12288), (2048, 2048), (768, 2048), (64, 2048)):
-            t = tokens(rows, n, k)
-            assert t % 16 == 0 and 0 <= t <= 256 and (t == 0 or t >= 48)
+        for n, k in ((6144, 4096), (4096, 4096), (24576, 4096), (4096, 12288), (2048, 2048), (768, 2048), (64, 2048), (3072, 768)):
+            kernel, t, high = ops.gemm_kernel_for(rows, n, k), tokens(rows, n, k), math.ceil(n / 256)
+            # (sizes that cut the rows into at most eight tiles more than need be)
+            every = {u: clocks(math.ceil(rows / u) * high, 74, 256 + u, 2 * u) for u in range(48, 257, 16)
+                     if math.ceil(rows / u) <= math.ceil(rows / 256) + 8}
+            if t:
+                taken, cut = taken + 1, math.ceil(rows / t)
+                assert (cut - 1) * t < rows <= cut * t and every[t] == min(every.values())
+            else:
+                left += 1
+            if 256 < rows <= 512 and k >= 2 * n:
+                assert t > 0
+            elif kernel in ("tiles", "pair") and k < 1024:
+                assert t == 0
+            elif kernel == "tiles":
+                other = min(clocks(math.ceil(rows / 128) * math.ceil(n / w), 148, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
+                assert (t > 0) == (min(every.values()) < 0.92 * other)
+            elif kernel == "pair":
+                assert (t > 0) == (min(every.values()) < 0.92 * clocks(math.ceil(rows / 256) * high, 74, 512, 512))
+    assert taken > 100 and left > 20
+
+
+def test_long_products_of_few_weight_rows_stay_where_k_is_cut_up():
+    """129 to 256 rows: `gemm_stream` cuts k up over all SMs, a pair of the swapped product walks all of it. Few weight rows against a
+    long k have a handful of tiles, each as long as k (240 rows of 512 x 16,384: 21 us against 40)."""
+    def tokens(rows, n, k):
+        assert ops.gemm_kernel_for(rows, n, k) == "swap"
+        return ops.pair_swap_tokens(rows, n, k, "swap")
+    for rows, n, k in ((240, 512, 16384), (256, 512, 16384), (240, 1024, 8192), (212, 2048, 12288), (256, 2048, 12288), (256, 1536, 8960),
+                       (160, 4096, 8192), (208, 4096, 12288), (130, 256, 4096)):
+        assert tokens(rows, n, k) == 0, (rows, n, k)
+    for rows, n, k in ((256, 4096, 12288), (256, 5120, 17408), (256, 2048, 5120), (256, 768, 3072), (144, 4096, 4096), (160, 6144, 4096),
+                       (144, 8192, 8192), (150, 4096, 512)):
+        assert tokens(rows, n, k) >= 48, (rows, n, k)
+    # more SMs shorten the streamed product
+    assert ops.pair_swap_tokens(256, 4096, 12288, "swap", sms=300) == 0
