@@ -927,13 +927,6 @@ def _packed(w) -> "PackedWeight":
     return w if isinstance(w, PackedWeight) else pack_weight(w)
 
 
-def _rows_fit(a, w) -> bool:
-    """Whether the weight-row kernel (`gemm_small_m`) takes this product."""
-    M, K = a.shape
-    return (1 <= M <= 64 and K >= 8 and K % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) == 1
-            and a.data_ptr() % 16 == 0)
-
-
 def _tcgen05_fits(a, w) -> bool:
     M, K = a.shape
     return M >= 1 and K >= 8 and K % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) == 1 and a.data_ptr() % 16 == 0
@@ -1018,7 +1011,6 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
     return "tiles"
 
 
-@functools.lru_cache(maxsize=4096)
 def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str, sms: int = 148, pairs: int = 74) -> int:
     """The tokens of a tile with which `gemm_pair_swap` takes a product of `rows` rows that would else go to `kernel`
     (`gemm_kernel_for`), or 0 where it is not the faster one.
@@ -1068,18 +1060,24 @@ def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str
     return tokens if best < 0.92 * other else 0
 
 
+@functools.lru_cache(maxsize=16384)
+def product_choice(rows: int, out_features: int, in_features: int, fits: bool = True, sms: int = 148, pairs: int = 74) -> tuple:
+    """(kernel, tokens) of a bfloat16 product: what `gemm_kernel_for` names and 0, or "pair-swap" and the tokens of its tile. `fits`:
+    whether the tensor-core kernels take its strides and alignment. Worked out once per size: a step asks it for every product."""
+    kernel = gemm_kernel_for(rows, out_features, in_features, fits and rows <= 64, fits, sms, pairs)
+    tokens = pair_swap_tokens(rows, out_features, in_features, kernel, sms, pairs) if fits else 0
+    return ("pair-swap", tokens) if tokens else (kernel, 0)
+
+
 def gemm_bf16(a, w, out, bias=None, accumulate=False, swiglu=False) -> None:
     """out (+)= a @ w.T (+ bias) on the tensor cores: bfloat16 operands, float32 accumulation; `w` a PackedWeight (a
     plain [out, in] matrix is packed on the spot). With `swiglu` the rows of w are blocks of 8 gate rows followed by
     their 8 up rows and out[m, j] = silu(gate_j) * up_j."""
     w = _packed(w)
     rows = a.shape[0]
-    kernel = gemm_kernel_for(rows, w.rows, w.cols, _rows_fit(a, w), _tcgen05_fits(a, w), sm_count(),
-                             resident_pairs() if rows > 128 else 0)
-    if rows > TILE_ROWS and kernel and _tcgen05_fits(a, w):
-        tokens = pair_swap_tokens(rows, w.rows, w.cols, kernel, sm_count(), resident_pairs())
-        if tokens:
-            return gemm_pair_swap(a, w, out, tokens, bias, accumulate, swiglu=swiglu)
+    kernel, tokens = product_choice(rows, w.rows, w.cols, _tcgen05_fits(a, w), sm_count(), resident_pairs() if rows > TILE_ROWS else 0)
+    if kernel == "pair-swap":
+        return gemm_pair_swap(a, w, out, tokens, bias, accumulate, swiglu=swiglu)
     if kernel == "rows":
         return gemm_small_m(a, w, out, bias, accumulate, swiglu=swiglu)
     if kernel == "swap":

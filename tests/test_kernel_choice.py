@@ -183,3 +183,30 @@ def test_long_products_of_few_weight_rows_stay_where_k_is_cut_up():
         assert tokens(rows, n, k) >= 48, (rows, n, k)
     # more SMs shorten the streamed product
     assert ops.pair_swap_tokens(256, 4096, 12288, "swap", sms=300) == 0
+
+
+def test_a_product_asks_once_which_kernel_takes_it(monkeypatch):
+    """Alignment, SMs and pairs are asked once a product, the choice is worked out once per size: prompts of some hundreds of rows wait
+    for the host, and a product's choice is a part of its launch."""
+    asked = []
+
+    def counted(name, answer):
+        monkeypatch.setattr(ops, name, lambda *a, **k: (asked.append(name), answer(*a, **k))[1])
+    counted("_tcgen05_fits", ops._tcgen05_fits)
+    counted("sm_count", lambda: 148)
+    counted("resident_pairs", lambda: 74)
+    counted("gemm_kernel_for", ops.gemm_kernel_for)
+    for name in ("gemm_small_m", "gemm_stream", "gemm_tcgen05", "gemm_pair", "gemm_pair_swap"):
+        monkeypatch.setattr(ops, name, lambda *a, name=name, **k: asked.append(name))
+    ops.product_choice.cache_clear()
+    for rows, n, k, kernel in ((8, 4096, 4096, "gemm_small_m"), (64, 6144, 4096, "gemm_stream"), (613, 24576, 4096, "gemm_pair_swap"),
+                               (2048, 24576, 4096, "gemm_pair"), (300, 3072, 512, "gemm_tcgen05")):
+        w = ops.PackedWeight(torch.zeros(1, dtype=torch.bfloat16).expand(-(-n // 128), -(-k // 64), 1), n, k)
+        a, out = torch.zeros(rows, k, dtype=torch.bfloat16), torch.zeros(1)
+        asked.clear()
+        ops.gemm_bf16(a, w, out)
+        ops.gemm_bf16(a, w, out)
+        assert asked.count(kernel) == 2 and asked.count("gemm_kernel_for") == 1, asked
+        assert asked.count("_tcgen05_fits") == 2 and asked.count("sm_count") == 2 and asked.count("resident_pairs") == (2 if rows > 128 else 0), asked
+    assert ops.product_choice(64, 4096, 4096, fits=False) == ("", 0)
+    ops.product_choice.cache_clear()
