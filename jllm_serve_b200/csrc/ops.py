@@ -1011,6 +1011,23 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
     return "tiles"
 
 
+def _round_clocks(tiles: int, places: int, per_round: int, multiply: int) -> float:
+    """Clocks a k block of 64 of all tiles: rounds of them, and twice their multiply-adds, which share one power limit."""
+    return -(-tiles // places) * per_round + 2.0 * tiles * multiply / places
+
+
+def pair_swap_tile(rows: int, out_features: int, pairs: int) -> tuple:
+    """(clocks a k block, tokens) of the tile that `gemm_pair_swap` is fastest with by the count of `pair_swap_tokens`."""
+    best = tokens = 0
+    high = -(-out_features // 256)
+    for cut in range(-(-rows // 256), -(-rows // 256) + 9):
+        t = -(-rows // (16 * cut)) * 16
+        c = _round_clocks(-(-rows // t) * high, pairs, 256 + t, 2 * t)
+        if t >= 48 and (not tokens or c < best):
+            best, tokens = c, t
+    return best, tokens
+
+
 def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str, sms: int = 148, pairs: int = 74) -> int:
     """The tokens of a tile with which `gemm_pair_swap` takes a product of `rows` rows that would else go to `kernel`
     (`gemm_kernel_for`), or 0 where it is not the faster one.
@@ -1036,17 +1053,8 @@ def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str
         return 0
     if kernel in ("tiles", "pair") and in_features < 1024:
         return 0
+    best, tokens = pair_swap_tile(rows, out_features, pairs)
     high = -(-out_features // 256)
-
-    def cost(tiles, places, per_round, multiply):
-        return -(-tiles // places) * per_round + 2.0 * tiles * multiply / places
-
-    best = tokens = 0
-    for cut in range(-(-rows // 256), -(-rows // 256) + 9):
-        t = -(-rows // (16 * cut)) * 16
-        c = cost(-(-rows // t) * high, pairs, 256 + t, 2 * t)
-        if t >= 48 and (not tokens or c < best):
-            best, tokens = c, t
     if kernel == "pair-streamed":
         return tokens
     if kernel == "swap":
@@ -1054,9 +1062,9 @@ def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str
         stream = 75 * n + 3.0 * (128 + n) * k_blocks * -(-out_features // 128) / sms
         return tokens if 0.97 * -(-(-(-rows // tokens) * high) // pairs) * (256 + tokens) * k_blocks <= stream else 0
     if kernel == "pair":
-        other = cost(-(-rows // 256) * high, pairs, 512, 512)
+        other = _round_clocks(-(-rows // 256) * high, pairs, 512, 512)
     else:
-        other = min(cost(-(-rows // 128) * -(-out_features // w), sms, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
+        other = min(_round_clocks(-(-rows // 128) * -(-out_features // w), sms, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
     return tokens if best < 0.92 * other else 0
 
 

@@ -18,6 +18,20 @@ import sys
 import torch
 
 
+def product_kernels(ops, rows: int, out_features: int, in_features: int, pairs: int):
+    """The name of the kernel that `ops.gemm_bf16` runs for such a product, and all that take it: name -> (function, arguments)."""
+    kernels = {"tiles": (ops.gemm_tcgen05, {})}
+    if pairs > 0:
+        kernels["pair"] = (ops.gemm_pair, {})
+        kernels["pair-streamed"] = (ops.gemm_pair, {"stream_mode": 1})
+        kernels["pair-swap"] = (ops.gemm_pair_swap, {"tokens": ops.pair_swap_tile(rows, out_features, pairs)[1]})
+    if rows <= ops.SWAP_MAX_ROWS:
+        kernels["swap"] = (ops.gemm_stream, {})
+    if rows <= 64:
+        kernels["rows"] = (ops.gemm_small_m, {})
+    return ops.product_choice(rows, out_features, in_features, True, ops.sm_count(), pairs)[0], kernels
+
+
 def main() -> int:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawTextHelpFormatter)
     ap.add_argument("--rows", type=int, default=8, help="rows of a decode step")
@@ -115,24 +129,18 @@ def main() -> int:
                 ("down (+= residual)", h_p, w_down, x_p, True, False, 2 * T * D * F)]
     pairs = ops.resident_pairs() if T > 128 else 0
     for what, a_, ws_, out_, acc_, glu_, flops_ in products:
-        chosen = ops.gemm_kernel_for(T, ws_[0].rows, ws_[0].cols, T <= 64, True, ops.sm_count(), pairs)
+        chosen, kernels = product_kernels(ops, T, ws_[0].rows, ws_[0].cols, pairs)
         case(f"prefill gemm {what} [{chosen}]",
              lambda i, a_=a_, ws_=ws_, out_=out_, acc_=acc_, glu_=glu_: ops.gemm_bf16(a_, ws_[i], out_, None, acc_, glu_),
              len(ws_), flops=flops_)
         if not args.all_kernels:
             continue
         # every product kernel that takes this shape, side by side on the same packed weights
-        kernels = {"tiles": lambda i, a_=a_, ws_=ws_, out_=out_, acc_=acc_, glu_=glu_: ops.gemm_tcgen05(a_, ws_[i], out_, None, acc_, swiglu=glu_)}
-        if pairs > 0:
-            kernels["pair"] = lambda i, a_=a_, ws_=ws_, out_=out_, acc_=acc_, glu_=glu_: ops.gemm_pair(a_, ws_[i], out_, None, acc_, swiglu=glu_)
-            kernels["pair-streamed"] = lambda i, a_=a_, ws_=ws_, out_=out_, acc_=acc_, glu_=glu_: ops.gemm_pair(a_, ws_[i], out_, None, acc_, swiglu=glu_, stream_mode=1)
-        if T <= ops.SWAP_MAX_ROWS:
-            kernels["swap"] = lambda i, a_=a_, ws_=ws_, out_=out_, acc_=acc_, glu_=glu_: ops.gemm_stream(a_, ws_[i], out_, None, acc_, swiglu=glu_)
-        if T <= 64:
-            kernels["rows"] = lambda i, a_=a_, ws_=ws_, out_=out_, acc_=acc_, glu_=glu_: ops.gemm_small_m(a_, ws_[i], out_, None, acc_, swiglu=glu_)
-        for kernel, fn in kernels.items():
+        for kernel, (fn, more) in kernels.items():
             if kernel != chosen:
-                case(f"prefill gemm {what} on {kernel}", fn, len(ws_), flops=flops_)
+                case(f"prefill gemm {what} on {kernel}",
+                     lambda i, a_=a_, ws_=ws_, out_=out_, acc_=acc_, glu_=glu_, fn_=fn, more_=more:
+                     fn_(a_, ws_[i], out_, bias=None, accumulate=acc_, swiglu=glu_, **more_), len(ws_), flops=flops_)
     pp = T // page + 1
     kc, vc = torch.randn(pp, Hkv, page, hd, device=dev).to(bf), torch.randn(pp, Hkv, page, hd, device=dev).to(bf)
     tp = torch.arange(pp, dtype=torch.int32, device=dev).reshape(1, -1).contiguous()

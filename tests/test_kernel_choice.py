@@ -210,3 +210,29 @@ def test_a_product_asks_once_which_kernel_takes_it(monkeypatch):
         assert asked.count("_tcgen05_fits") == 2 and asked.count("sm_count") == 2 and asked.count("resident_pairs") == (2 if rows > 128 else 0), asked
     assert ops.product_choice(64, 4096, 4096, fits=False) == ("", 0)
     ops.product_choice.cache_clear()
+
+
+def test_the_kernel_bench_names_the_kernel_that_runs(monkeypatch):
+    """`kernel_bench`'s label of a product is the kernel that `gemm_bf16` calls, with the same tile, and that kernel is one of those it
+    times side by side."""
+    from jllm_serve_b200.kernel_bench import product_kernels
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    monkeypatch.setattr(ops, "resident_pairs", lambda: 74)
+    ran = []
+    for name in ("gemm_small_m", "gemm_stream", "gemm_tcgen05", "gemm_pair", "gemm_pair_swap"):
+        monkeypatch.setattr(ops, name, lambda a, w, out, *args, name=name, **more: ran.append((name, args, more)))
+    seen = set()
+    for rows in (8, 47, 64, 150, 200, 300, 613, 1024, 2048):
+        for n, k in ((6144, 4096), (4096, 4096), (24576, 4096), (4096, 12288)):
+            chosen, kernels = product_kernels(ops, rows, n, k, 74 if rows > 128 else 0)
+            w = ops.PackedWeight(torch.zeros(1, dtype=torch.bfloat16).expand(-(-n // 128), -(-k // 64), 1), n, k)
+            ran.clear()
+            ops.gemm_bf16(torch.zeros(1, dtype=torch.bfloat16).expand(rows, k).contiguous(), w, torch.zeros(1))
+            fn, more = kernels[chosen]
+            by_bench = ran.pop()
+            fn(None, None, None, **more)
+            assert ran[-1][0] == by_bench[0], (rows, n, k, chosen)
+            if chosen == "pair-swap":
+                assert by_bench[1][0] == more["tokens"]
+            seen.add(chosen)
+    assert seen >= {"rows", "swap", "tiles", "pair", "pair-swap"}
