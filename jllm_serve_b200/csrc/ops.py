@@ -943,12 +943,16 @@ def gemm_bf16_fits(a, w, out) -> bool:
 #            and for small matrices up to 64 rows;
 #   "swap"   gemm_stream: tcgen05 with the weight rows as the M side, one 16 KB bulk copy per tile, the k blocks dealt
 #            out evenly over the SMs; from 17 to 128 rows for matrices of 40 MB or more (QKV, down), from 41 rows for
-#            smaller ones (O), where the row kernel's time grows with the rows; up to 160 rows for all of these and up to
-#            256 for matrices much longer than high (down); not for very wide matrices (gate_up), which whole tiles of
-#            the tiles kernel fill the SMs with;
-#   "tiles"  gemm_tcgen05: tokens as the M side, 128 x BN tiles; above that, and from 16 rows for very wide matrices.
-# From 129 rows on `pair_swap_tokens` then says whether pairs of SMs with the weight rows as their M side (gemm_pair_swap) are faster
-# than the kernel named here.
+#            smaller ones (O), where the row kernel's time grows with the rows; not for very wide matrices (gate_up), which
+#            whole tiles of the tiles kernel fill the SMs with. Of 129 to 256 rows what the swapped pairs are not ahead of:
+#            matrices much longer than high (down to 208 rows; the fewer weight rows, the further up);
+#   "tiles"  gemm_tcgen05: tokens as the M side, 128 x BN tiles; from 16 rows for very wide matrices, and above 128 rows what
+#            pairs do not take (few k blocks, sizes whose tiles come out better);
+#   "pair"   gemm_pair: two SMs to a 256 x 256 tile; from some 1,000 rows on;
+#   "pair-swap"  gemm_pair_swap: two SMs to a tile of 256 weight rows by as many tokens as the rows are cut into; nearly everything from
+#            129 to some hundreds of rows, in between up to 1,500.
+# `gemm_kernel_for` chooses among the first three and "pair", `pair_swap_tokens` says where the swapped pairs are faster than that one;
+# `product_choice` is both.
 SWAP_MAX_ROWS = 256      # gemm_stream: the tokens are the N side of one tcgen05.mma
 TILE_ROWS = 128          # rows of a tcgen05 product tile (BM in gemm_tcgen05.cu): a step of 129 rows pays for 256
 SMALL_M_ROWS = int(os.environ.get("JLLM_B200_SMALL_M_ROWS", "64"))
@@ -974,8 +978,9 @@ def gemm_workspace(key, floats: int = 8 << 20) -> torch.Tensor:
 
 def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_fit: bool = True,
                     tiles_fit: bool = True, sms: int = 148, pairs: int = 74) -> str:
-    """"rows", "swap", "tiles", "pair", "pair-streamed" or "" for a bfloat16 product of `rows` rows against a [out_features, in_features]
-    weight, given which kernels take its strides and alignment, the SMs and the pairs of them the device runs at a time."""
+    """"rows", "swap", "tiles", "pair" or "" for a bfloat16 product of `rows` rows against a [out_features, in_features] weight, given
+    which kernels take its strides and alignment, the SMs and the pairs of them the device runs at a time. From 129 rows on this is
+    what `pair_swap_tokens` weighs the swapped pairs against."""
     # 16 or more rows against a wide matrix (gate_up): 128 or more 192-wide tcgen05 tiles stream it faster than the
     # weight-row kernel, whose blocks have half their loads in flight once they hold more than two token tiles
     wide = rows >= 16 and out_features >= WIDE_ROWS and tiles_fit
@@ -992,11 +997,6 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
         return "rows"
     if not tiles_fit:
         return ""
-    # 257 to 512 rows against a matrix much longer than high (down): its few 256 x 256 tiles cut up over ALL pairs, the
-    # parts of a tile meeting in a workspace (8B shape, 384 rows: 49 us against 59 on one-SM tiles; 512 rows: 52 against
-    # 67; the shorter matrices lose that way, and above 512 rows the whole tiles are enough)
-    if pairs > 0 and tiles_fit and 256 < rows <= 512 and in_features >= 2 * out_features:
-        return "pair-streamed"
     # Many rows: two SMs to a 256 x 256 tile take in a third less per multiply-add than one SM with a 128 x 256 tile,
     # which is what bounds these products. It pays where its tiles keep three quarters of the pairs busy or more and its
     # rounds of tiles, each about a tenth shorter than a round of one-SM tiles of the same width, take less than the
@@ -1039,8 +1039,10 @@ def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str
     42.5 and 38.1; O of 512 17.7 and 15.9; gate_up of 144 47.7 and 38.6, of 400 73.0 and 63.3, of 613 101 and 88; down of 300
     47.3 and 35.5, of 613 59.6 and 50.7. From there on 256 x 256 tiles with the tokens as the M side are as good (gate_up of 1,536 rows
     195 and 213): it takes a twelfth less by this count to change. Below 129 rows there are too few tiles; of few k blocks a pair's start and
-    end are most of it (3,072 x 768, 613 rows 6.6 and 7.4). A matrix of few rows, which the streamed pairs took between 257 and 512
-    rows, was worst off there (768 x 2,048, 300 rows: 49.6 and 7.1).
+    end are most of it (3,072 x 768, 613 rows 6.6 and 7.4). 257 to 512 rows against matrices much longer than high are the swapped pairs'
+    without a count: behind a norm, us, one-SM tiles and they, 512 x 16,384 of 300 and 500 rows 41.3 and 39.7, 41.3 and 39.6, 1,024 x
+    8,192 22.4 and 21.7, 22.6 and 22.0, 2,048 x 8,192 23.7 and 22.9, 24.2 and 23.3, 256 x 4,096 12.6 and 12.2, 12.6 both (256 x 256 tiles
+    cut up over all pairs, `gemm_pair`'s stream_mode, take 70, 45, 32 and 113 there).
 
     `gemm_stream` ("swap") cuts k up over all SMs where a pair walks all of it, so there the whole product is counted: a pair's
     rounds of (T + 256) clocks a k block against a meeting of 75 clocks a token and, on every SM, its share of all tiles' k blocks at
@@ -1049,13 +1051,14 @@ def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str
     even at 4,096 x 8,192 of 212 (24.2 both), 2,048 x 8,192 of 256 (22.2 and 22.7), 4,096 x 12,288 of 212 (33.2 and 33.8); 4,096 x 12,288 of 256
     37.8 and 34.0, 2,048 x 5,120 of 256 19.3 and 15.5, 768 x 3,072 13.7 and 10.4, 4,096 x 4,096 of 144 15.3 and 14.2, 6,144 x 4,096
     20.1 and 15.5, 4,096 x 512 10.1 and 5.2 (few k blocks do not count against the pairs here: swap is the worse for them)."""
-    if pairs <= 0 or rows <= TILE_ROWS or kernel not in ("swap", "tiles", "pair", "pair-streamed"):
+    if pairs <= 0 or rows <= TILE_ROWS or kernel not in ("swap", "tiles", "pair"):
         return 0
-    if kernel in ("tiles", "pair") and in_features < 1024:
+    long = 256 < rows <= 512 and in_features >= 2 * out_features
+    if kernel != "swap" and in_features < 1024 and not long:
         return 0
     best, tokens = pair_swap_tile(rows, out_features, pairs)
     high = -(-out_features // 256)
-    if kernel == "pair-streamed":
+    if long:
         return tokens
     if kernel == "swap":
         k_blocks, n = -(-in_features // 64), -(-rows // 16) * 16
@@ -1092,8 +1095,6 @@ def gemm_bf16(a, w, out, bias=None, accumulate=False, swiglu=False) -> None:
         return gemm_stream(a, w, out, bias, accumulate, swiglu=swiglu)
     if kernel == "pair":
         return gemm_pair(a, w, out, bias, accumulate, swiglu=swiglu)
-    if kernel == "pair-streamed":
-        return gemm_pair(a, w, out, bias, accumulate, swiglu=swiglu, stream_mode=1)
     if kernel == "tiles":
         return gemm_tcgen05(a, w, out, bias, accumulate, swiglu=swiglu)
     raise KernelError("the tensor-core matrix product is not built for this shape")
