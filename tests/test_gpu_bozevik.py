@@ -141,6 +141,70 @@ def test_depth_mix_alone_and_behind_the_last_norm(planes, rows, dim):
         assert torch.equal(state[0], kept[0]) and torch.equal(state[rows + 1], kept[rows + 1])
 
 
+def off_by_one(t, odd):
+    """The tensor on the device; with `odd` in a buffer of its own one element further, where four values are no aligned access."""
+    if not odd:
+        return t.to(DEV)
+    room = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+    room[1:] = t.reshape(-1).to(DEV)
+    return room[1:].view(t.shape)
+
+
+# widths: eight and sixteen values of a row in a thread's registers, their last pieces full and not, and the first width that is read twice
+# again; where the vectors (gain, mu, weights) or the rows themselves begin at an odd element, values go one by one
+@pytest.mark.parametrize("dim", [1028, 2048, 2052, 4096, 4100])
+@pytest.mark.parametrize("odd", ["", "vectors", "rows"])
+def test_norms_added_to_the_stream_at_widths_held_in_registers(dim, odd):
+    o_, rows = ops(), 3
+    g = torch.Generator().manual_seed(dim + len(odd))
+    x, a = torch.randn(rows, dim, generator=g), torch.randn(rows, dim, generator=g) * 7 - 2
+    for gain in (torch.randn(dim, generator=g), torch.randn(dim, generator=g).bfloat16()):
+        for center in (True, False):
+            for next_dtype in (None, torch.float32, torch.bfloat16):
+                xd = off_by_one(x, odd == "rows")
+                nxt = torch.empty(rows, dim, dtype=next_dtype, device=DEV) if next_dtype is not None else None
+                o_.norm_add(xd, off_by_one(a, odd == "rows"), off_by_one(gain, odd == "vectors"), 1e-6, next_out=nxt, center=center)
+                normed = P.layer_norm(a.double(), gain.double(), 1e-6) if center else P.rms(a.double(), 1e-6) * gain.double()
+                close(xd, x.double() + normed, torch.float32, f"stream, center={center}")
+                if nxt is not None:
+                    assert torch.equal(nxt, xd.to(next_dtype))
+
+
+@pytest.mark.parametrize("planes", [1, 2, 4, 9])
+@pytest.mark.parametrize("dim", [2048, 2052, 4096, 4100])
+@pytest.mark.parametrize("odd", ["", "vectors", "rows"])
+def test_the_mix_behind_a_norm_at_widths_held_in_registers(dim, planes, odd):
+    """Planes come four at a time up to 2,048 values a row, two at a time above."""
+    o_, rows = ops(), 3
+    g = torch.Generator().manual_seed(dim + planes)
+    first = torch.randn(planes + 1, rows + 2, dim, generator=g)
+    a, gain = torch.randn(rows, dim, generator=g) * 3, torch.randn(dim, generator=g).bfloat16()
+    weights, mu = torch.randn(planes, generator=g).bfloat16(), torch.rand(dim, generator=g).bfloat16()
+    kept = torch.randn(rows + 2, dim, generator=g)
+    for center in (True, False):
+        normed = P.layer_norm(a.double(), gain.double(), 1e-5) if center else P.rms(a.double(), 1e-5) * gain.double()
+        x_new = first[planes - 1, :rows].double() + normed
+        want = sum(weights[j].double() * (x_new if j == planes - 1 else first[j, :rows].double()) for j in range(planes))
+        for h_dtype in (None, torch.float32, torch.bfloat16):
+            view = off_by_one(first, odd == "rows")[:, :rows]
+            batch, _ = step_tables([1] * rows, list(range(rows, 0, -1)))
+            state = off_by_one(kept, odd == "rows")
+            h = torch.empty(rows, dim, dtype=h_dtype, device=DEV) if h_dtype is not None else None
+            o_.norm_add_mix(view[planes - 1], off_by_one(a, odd == "rows"), off_by_one(gain, odd == "vectors"), 1e-5, view,
+                            off_by_one(weights, odd == "vectors"), planes, view[planes], center,
+                            shift=(off_by_one(mu, odd == "vectors"), state) if h is not None else None, batch=batch, h_out=h)
+            close(view[planes - 1], x_new, torch.float32, "the layer's result")
+            close(view[planes], want, torch.float32, "what the layer hands on")
+            assert torch.equal(view[:planes - 1].cpu(), first[:planes - 1, :rows])
+            if h is None:
+                assert torch.equal(state.cpu(), kept)
+                continue
+            prev = kept[batch.state_slots.long().cpu()].double()
+            close(h, want + (prev - want) * mu.double(), h_dtype, "the next layer's shifted rows")
+            assert torch.equal(state[batch.state_slots.long()], view[planes])
+            assert torch.equal(state[0].cpu(), kept[0]) and torch.equal(state[rows + 1].cpu(), kept[rows + 1])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("q_rank, rank, rope_dim, rotary", [(24, 32, 8, 8), (20, 40, 12, 12), (80, 96, 32, 32), (0, 24, 6, 4)])
 def test_query_latent_norm_and_the_cached_row(dtype, q_rank, rank, rope_dim, rotary):

@@ -89,6 +89,36 @@ def test_norm_and_convolution_over_portions_and_slots(dtype, dim, taps):
     assert bool((state[1] == 7.0).all())
 
 
+@pytest.mark.parametrize("dim", [1024, 2052, 4096, 4100])
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("odd", [False, True])
+def test_norm_and_convolution_of_single_rows_at_widths_held_in_registers(dim, taps, odd):
+    """Steps of single rows: up to 4,096 channels a thread has gains, taps, the row and the state in registers, above that the step is
+    the portions' kernel; with `odd` the gain and the taps begin at an odd element."""
+    o = ops()
+    g = torch.Generator().manual_seed(taps * 100 + dim)
+
+    def vector(t):
+        room = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        room[1:] = t.reshape(-1).to(DEV)
+        return room[1:].view(t.shape) if odd else t.to(DEV)
+    xs = torch.randn(6, 3, dim, generator=g)
+    for dtype in (torch.float32, torch.bfloat16):
+        gain, conv = torch.randn(dim, generator=g).to(dtype), (torch.randn(dim, taps, generator=g) * 0.5).to(dtype)
+        hs = P.norm(xs.double(), gain.double(), 1e-5)
+        state = torch.zeros(4, taps - 1, dim, device=DEV)
+        state[1] = 7.0
+        got = []
+        for x in xs:
+            out = torch.empty(3, dim, dtype=dtype, device=DEV)
+            o.norm_conv(x.to(DEV), vector(gain), 1e-5, vector(conv), state, FakeBatch([1, 1, 1], [2, 0, 3]), out)
+            got.append(out.float().cpu())
+        for i, slot in enumerate((2, 0, 3)):
+            close(torch.stack(got)[:, i], P.input_convolution(hs[:, i], conv.double()), dtype, f"request {i}")
+            close(state[slot], hs[-(taps - 1):, i], torch.float32, f"state of request {i}")
+        assert bool((state[1] == 7.0).all())
+
+
 # ---- the delta rule ----------------------------------------------------------------------------------------------------
 
 def delta_case(H, dk, dv, lens, seed, strong=False):

@@ -956,3 +956,49 @@ def test_gemm_small_m_halves_of_k(ops, M, N, K):
         ops.gemm_small_m(a, packed, units, swiglu=True)
         z = gemm_want(a, w).view(M, N // 16, 2, 8)
         assert torch.allclose(units.float().cpu(), (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2), rtol=2 ** -7, atol=2e-3)
+
+
+@pytest.mark.parametrize("dim", [512, 1028, 2048, 3000, 4096, 8192, 8196])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norms_whose_gain_begins_at_an_odd_element(ops, dim, dtype):
+    """Gains are read four at a time where their start allows it and one by one where not: the same bits, for every number of values that a
+    thread holds (rmsnorm, the sandwich norms and the sum of two branches) and for the rotated heads."""
+    def odd(t):
+        room = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        room[1:] = t
+        return room[1:]
+    x, a, b = (rnd(5, dim, seed=i, scale=3.0) for i in range(3))
+    gains = [(1 + 0.1 * rnd(dim, seed=4 + i)).to(dtype) for i in range(4)]
+    results = []
+    for place in (lambda t: t, odd):
+        g = [place(t) for t in gains]
+        out, xs, chain, nxt = torch.empty(5, dim, device=DEV), x.clone(), x.clone(), torch.empty(5, dim, dtype=torch.bfloat16, device=DEV)
+        ops.rmsnorm(x, g[0], 1e-5, out)
+        ops.norm_sum(xs, a, g[0], 1e-5, b, g[1], scale=0.5)
+        ops.norm_chain(chain, a, g[2], 1e-5, b, g[0], g[1], 0.5, next_out=nxt, gain_next=g[3])
+        results.append((out, xs, chain, nxt))
+    assert all(torch.equal(u, v) for u, v in zip(*results))
+    want = P.rmsnorm(x.cpu(), gains[0].float().cpu(), 1e-5)
+    assert torch.allclose(results[0][0].cpu(), want, rtol=2e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("M,N,K,tokens", [(150, 4096, 1024, 80), (257, 528, 4096, 96), (613, 2048, 2048, 208)])
+def test_gemm_pair_swap_gives_the_bits_of_whole_tiles(ops, M, N, K, tokens):
+    """An element's sum runs over k in the same order with one accumulator, whichever operand is the M side: the results are those of
+    one-SM tiles, stored, behind bias and relu squared, added to a residual, gated."""
+    a, w = rnd(M, K, dtype=torch.bfloat16), ops.pack_weight(rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05))
+    bias, base = rnd(N, dtype=torch.float32, seed=2), rnd(M, N, seed=3)
+    for dtype in (torch.float32, torch.bfloat16):
+        for how in (False, True, ops.EPILOGUE_RELU2, "glu"):
+            got, want = (base[:, :N // 2].to(dtype).contiguous() if how == "glu" else base.to(dtype) for _ in range(2))
+            more = dict(swiglu=True) if how == "glu" else dict(bias=bias, accumulate=how)
+            ops.gemm_pair_swap(a, w, got, tokens, **more)
+            ops.gemm_tcgen05(a, w, want, **more)
+            assert torch.equal(got, want), (dtype, how)
+    wide = torch.full((M, N + 6), float("nan"), dtype=torch.bfloat16, device=DEV)       # added into a bfloat16 row that is wider
+    wide[:, :N] = base
+    ops.gemm_pair_swap(a, w, wide[:, :N], tokens, bias, accumulate=True)
+    want = a.double().cpu() @ w.unpack().double().cpu().t() + bias.double().cpu() + base.bfloat16().double().cpu()
+    # a sum of float32 and a rounding to 8 bits of the result
+    assert torch.allclose(wide[:, :N].double().cpu(), want, rtol=2 ** -8, atol=1e-4 * math.sqrt(K) * 0.05) and wide[:, N:].isnan().all()
+    assert ops.gemm_tcgen05_error() == 0
