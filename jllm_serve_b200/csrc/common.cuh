@@ -111,8 +111,10 @@ __device__ __forceinline__ long long jllm_page_of(const int* __restrict__ table,
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Weights are nobody's output: a kernel may ask for its own before it waits for its predecessor. `bytes` from `p` on, whole lines,
-// asked of memory by the block's threads together.
+// Weights are nobody's output: a kernel may ask for its own, or read them, before it waits for its predecessor (packed weights, a
+// norm's gain, a convolution's taps, the weights of a sum over planes; also a step's tables, which are copied in front of the step).
+// Whoever would have one of THIS library's kernels write such a vector puts a copy, an event or a launch without the attribute between.
+// `bytes` from `p` on, whole lines, asked of memory by the block's threads together.
 __device__ __forceinline__ void prefetch_lines(const void* p, size_t bytes) {
     const char* c = static_cast<const char*>(p);
     for (size_t i = (size_t)threadIdx.x * 128; i < bytes; i += (size_t)blockDim.x * 128)

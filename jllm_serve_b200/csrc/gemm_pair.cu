@@ -4,18 +4,18 @@
 // What bounds the one-SM product (gemm_tcgen05.cu) on big shapes is what an SM can take in: 48 KB per k block (128
 // rows of A, 256 rows of W) for 128 x 256 x 64 multiply-adds. Here two blocks, a cluster of two on neighbouring SMs,
 // share a 256 x 256 tile: each brings 128 rows of A and 128 of the tile's 256 rows of W (32 KB per k block for the
-// same multiply-adds), one thread of the pair's first block issues MMAs of M 256 that read both blocks' shared memory,
+// same multiply-adds), one lane of the pair's first block issues MMAs of M 256 that read both blocks' shared memory,
 // and each block ends up with its 128 rows of the tile in its own tensor memory.
 //
-//   * warp 0 (one lane) of BOTH blocks is a producer: it waits for its free stage and brings its A tile (tiled TMA
+//   * warp 0 of BOTH blocks is a producer (the warp walks, one elected lane issues: tcgen05_common.cuh): it waits for its free stage and brings its A tile (tiled TMA
 //     copy, 128-byte swizzle) and its W tile (the PACKED weight is that shared-memory image already: a tiled copy
 //     without swizzle of its 16 KB). Every copy completes on the FIRST block's "full" barrier of the stage, which
 //     expects the bytes of both blocks;
-//   * warp 1 (one lane) of the first block issues 4 x tcgen05.mma.cta_group::2 (M 256, N 256, K 16) per k block;
+//   * warp 1 of the first block, again by one elected lane, issues 4 x tcgen05.mma.cta_group::2 (M 256, N 256, K 16) per k block;
 //     tcgen05.commit, multicast to both blocks, frees the stage in both and, after a tile's last k block, tells both
 //     blocks' epilogues that the accumulator is full;
 //   * warps 2-5 of both blocks are the epilogue of their block's 128 rows (gemm_epilogue.cuh); when a block's four
-//     warps have read an accumulator they tell the first block, whose MMA thread may then use it again.
+//     warps have read an accumulator they tell the first block, whose MMA warp may then use it again.
 // Tensor memory holds two accumulators, so a tile's epilogue overlaps the next tile's main loop. The pairs walk the
 // tiles with m fastest. Edges: TMA fills rows beyond M and k beyond K with zeros; a block whose half of the W rows lies
 // beyond the (padded) matrix brings none, and its columns are never stored.

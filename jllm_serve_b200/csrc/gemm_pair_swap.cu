@@ -8,10 +8,10 @@
 // side, in steps of 256: 613 tokens are 768 there (640 in 128-row tiles). Here a tile's tokens are cut to what is there (613 = 3 x 208),
 // or to what fills the pairs: T is chosen so that the rounds of tiles, times T + 256 clocks a k block, come out least.
 //
-//   * warp 0 (one lane) of BOTH blocks is a producer: its 128 rows of W (one packed tile: a tiled copy without swizzle of its 16 KB) and
+//   * warp 0 of BOTH blocks is a producer (the warp walks, one elected lane issues: tcgen05_common.cuh): its 128 rows of W (one packed tile: a tiled copy without swizzle of its 16 KB) and
 //     half of the tile's tokens (tiled copy, 128-byte swizzle), all completing on the FIRST block's barrier of the stage. The first
 //     stages' weights are asked for before the wait for the kernel in front;
-//   * warp 1 (one lane) of the first block issues 4 x tcgen05.mma.cta_group::2 (M 256, N T, K 16) per k block and commits to both blocks;
+//   * warp 1 of the first block, again by one elected lane, issues 4 x tcgen05.mma.cta_group::2 (M 256, N T, K 16) per k block and commits to both blocks;
 //   * warps 2-9 of both blocks are the epilogue of their block's 128 weight rows: a thread has one weight row and 16 tokens at a time, so
 //     that a warp's store of one token is 32 neighbouring outputs. Gate and up rows lie 8 lanes apart and meet by shuffles.
 // Tensor memory holds two accumulators of at most 256 columns, so a tile's epilogue lies under the next tile's main loop. Tiles are walked

@@ -17,7 +17,7 @@
 //   * the activations' tile of a k block (tokens x 64) comes by TMA from the [rows, K] matrix (L2 resident);
 //   * the producer requests its first weights BEFORE it waits for the kernel in front of it (programmatic dependent
 //     launch): weights do not depend on it.
-// Roles: warp 0 (one lane) producer, warp 1 (one lane) MMA issuer, warps 2-5 epilogue (bias / float32 residual add /
+// Roles: warp 0 producer, warp 1 MMA issuer (both walk as a warp, one elected lane issues: tcgen05_common.cuh), warps 2-5 epilogue (bias / float32 residual add /
 // SwiGLU over interleaved gate and up rows / store). Every wait is bounded and raises the error word of
 // gemm_tcgen05 (codes 11-13; the clusters' kernel 14-16).
 #include <mutex>

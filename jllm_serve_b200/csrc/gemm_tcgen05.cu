@@ -2,12 +2,12 @@
 //
 // The prefill product. A persistent kernel, one block per SM, walks 128 x BN output tiles (BN = 256 for big
 // products, narrower when the rows are few):
-//   * warp 0 (one lane) is the producer: for every 64-wide k block it waits for a free stage and brings a
+//   * warp 0 is the producer (the warp walks, one elected lane issues: tcgen05_common.cuh): for every 64-wide k block it waits for a free stage and brings a
 //     128 x 64 tile of A (a tiled TMA copy into 128-byte-swizzled shared memory) and a BN x 64 tile of W, which
 //     is kept PACKED in exactly that shared-memory image (ops.pack_weight), so its tile is one or two plain
 //     contiguous bulk copies of up to 16 KB; all complete on the stage's "full" mbarrier (no multicast: every
 //     block loads its own copy);
-//   * warp 1 (one lane) issues the MMAs: 4 x tcgen05.mma (M 128, N 256, K 16) per k block, operands
+//   * warp 1, again by one elected lane, issues the MMAs: 4 x tcgen05.mma (M 128, N 256, K 16) per k block, operands
 //     described by shared-memory descriptors, the float32 accumulator in tensor memory (TMEM);
 //     tcgen05.commit frees the stage, and after the last k block signals "accumulator full";
 //   * warps 2-5 are the epilogue: each reads its 32 TMEM lanes (= 32 rows of the tile) with

@@ -986,11 +986,12 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
     wide = rows >= 16 and out_features >= WIDE_ROWS and tiles_fit
     if tiles_fit and not wide and 16 < rows <= 128 and (out_features * in_features * 2 >= SWAP_MIN_BYTES or rows > 40):
         return "swap"
+    # (The line at 40 rows was drawn before a cluster took a tile of such a matrix; since then swap is ahead of the row kernel from 17
+    # rows on: 24 rows of O 10.3 us against 12.3, 40 rows 11.5 against 18.2.)
     # 129 to 256 rows (the tokens are still one tcgen05 N side): what the tiles kernel is worst at, matrices much longer than
     # high (down: 12,288 k for 4,096 rows; 160, 200, 256 rows 28.6, 32.9, 37.7 us against 59), and everything up to 160 rows
-    # (QKV 22.7 us against 24.6, O 16.3 against 22.8; at 200 rows QKV 26.2 against 24.8). The lines of O were drawn before a
-    # cluster took a tile of it: since then swap is ahead of the row kernel from 17 rows on (24 rows 10.3 us against 12.3, 40 rows
-    # 11.5 against 18.2) and of the tiles up to 256 (200 rows 19.1 against 22.7, 256 rows 21.3 against 22.8).
+    # (QKV 22.7 us against 24.6, O 16.3 against 22.8; at 200 rows QKV 26.2 against 24.8). Most of these are then the swapped pairs';
+    # all of them are swap's where the device runs no pairs.
     if tiles_fit and not wide and 128 < rows <= SWAP_MAX_ROWS and (rows <= 160 or in_features >= 2 * out_features):
         return "swap"
     if rows <= min(SMALL_M_ROWS, 64) and rows_fit and not wide:

@@ -1027,10 +1027,10 @@ __global__ void __launch_bounds__(256)
 norm_chain_vec_kernel(float* __restrict__ x, const float* __restrict__ a, VecRef gain_a, const float* __restrict__ b,
                       VecRef gain_b, float scale, VecRef gain_post, VecRef gain_next, Tnext* __restrict__ next, int dim, float eps) {
     __shared__ float scratch[33];
-    const size_t row = (size_t)blockIdx.x * dim;
-    const int n4 = dim >> 2;
     pdl_wait();
     pdl_trigger();
+    const size_t row = (size_t)blockIdx.x * dim;
+    const int n4 = dim >> 2;
     const float4* pa = reinterpret_cast<const float4*>(a + row);
     const float4* pb = b ? reinterpret_cast<const float4*>(b + row) : nullptr;
     float4* px = reinterpret_cast<float4*>(x + row);

@@ -48,7 +48,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // tcgen05.mma, tcgen05.commit and the bulk copies take their operands from the warp's uniform registers. Issued under `if (lane == 0)`
 // every operand is moved there one by one behind a branch that the compiler has to think divergent, and a loop of one wait, four MMAs and
 // a commit takes 330 ns whatever the tile (205 ns with nothing but the barriers): longer than the MMAs of every tile but the largest.
-// So the WHOLE warp walks the loop, its control flow follows from votes (which are uniform), and one elected lane issues: 115 ns for the
+// So the WHOLE warp walks the loop, its control flow follows from votes (which are uniform), and one elected lane issues (the same lane
+// every time: a commit stands for the MMAs that its own thread issued, and those complete in order): 115 ns for the
 // barriers alone, and from there on the MMAs are what is waited for (128 weight rows a block x 160 tokens: 318 -> 176 ns a k block of 64).
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ bool elect_one() {
