@@ -139,7 +139,6 @@ class _Signatures:
     jllm_gemm_small_m = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, P, P]
     jllm_gemm_tcgen05 = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, I, P]
     jllm_gemm_pair = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, P]
-    jllm_gemm_pair_swap = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, I, I, P, P]
     jllm_gemm_pair_resident = []
     jllm_gemm_plain_stores = [I]
     jllm_gemm_stream = [P, I, P, I, P, I, P, I, I, I, I, I, I, I, P, P, ctypes.c_longlong, I, I, P]
@@ -944,15 +943,10 @@ def gemm_bf16_fits(a, w, out) -> bool:
 #   "swap"   gemm_stream: tcgen05 with the weight rows as the M side, one 16 KB bulk copy per tile, the k blocks dealt
 #            out evenly over the SMs; from 17 to 128 rows for matrices of 40 MB or more (QKV, down), from 41 rows for
 #            smaller ones (O), where the row kernel's time grows with the rows; not for very wide matrices (gate_up), which
-#            whole tiles of the tiles kernel fill the SMs with. Of 129 to 256 rows what the swapped pairs are not ahead of:
-#            matrices much longer than high (down to 208 rows; the fewer weight rows, the further up);
-#   "tiles"  gemm_tcgen05: tokens as the M side, 128 x BN tiles; from 16 rows for very wide matrices, and above 128 rows what
-#            pairs do not take (few k blocks, sizes whose tiles come out better);
-#   "pair"   gemm_pair: two SMs to a 256 x 256 tile; from some 1,000 rows on;
-#   "pair-swap"  gemm_pair_swap: two SMs to a tile of 256 weight rows by as many tokens as the rows are cut into; nearly everything from
-#            129 to some hundreds of rows, in between up to 1,500.
-# `gemm_kernel_for` chooses among the first three and "pair", `pair_swap_tokens` says where the swapped pairs are faster than that one;
-# `product_choice` is both.
+#            whole tiles of the tiles kernel fill the SMs with; to 256 rows where k is long for the rows of the matrix (down);
+#   "tiles"  gemm_tcgen05: tokens as the M side, 128 x BN tiles; from 16 rows for very wide matrices, and above 128 rows
+#            what swap and the pairs do not take;
+#   "pair"   gemm_pair: two SMs to a 256 x 256 tile, where such tiles fill three quarters of the pairs and more.
 SWAP_MAX_ROWS = 256      # gemm_stream: the tokens are the N side of one tcgen05.mma
 TILE_ROWS = 128          # rows of a tcgen05 product tile (BM in gemm_tcgen05.cu): a step of 129 rows pays for 256
 SMALL_M_ROWS = int(os.environ.get("JLLM_B200_SMALL_M_ROWS", "64"))
@@ -979,8 +973,7 @@ def gemm_workspace(key, floats: int = 8 << 20) -> torch.Tensor:
 def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_fit: bool = True,
                     tiles_fit: bool = True, sms: int = 148, pairs: int = 74) -> str:
     """"rows", "swap", "tiles", "pair" or "" for a bfloat16 product of `rows` rows against a [out_features, in_features] weight, given
-    which kernels take its strides and alignment, the SMs and the pairs of them the device runs at a time. From 129 rows on this is
-    what `pair_swap_tokens` weighs the swapped pairs against."""
+    which kernels take its strides and alignment, the SMs and the pairs of them the device runs at a time."""
     # 16 or more rows against a wide matrix (gate_up): 128 or more 192-wide tcgen05 tiles stream it faster than the
     # weight-row kernel, whose blocks have half their loads in flight once they hold more than two token tiles
     wide = rows >= 16 and out_features >= WIDE_ROWS and tiles_fit
@@ -988,16 +981,25 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
         return "swap"
     # (The line at 40 rows was drawn before a cluster took a tile of such a matrix; since then swap is ahead of the row kernel from 17
     # rows on: 24 rows of O 10.3 us against 12.3, 40 rows 11.5 against 18.2.)
-    # 129 to 256 rows (the tokens are still one tcgen05 N side): what the tiles kernel is worst at, matrices much longer than
-    # high (down: 12,288 k for 4,096 rows; 160, 200, 256 rows 28.6, 32.9, 37.7 us against 59), and everything up to 160 rows
-    # (QKV 22.7 us against 24.6, O 16.3 against 22.8; at 200 rows QKV 26.2 against 24.8). Most of these are then the swapped pairs';
-    # all of them are swap's where the device runs no pairs.
-    if tiles_fit and not wide and 128 < rows <= SWAP_MAX_ROWS and (rows <= 160 or in_features >= 2 * out_features):
-        return "swap"
+    # 129 to 256 rows (the tokens are still one tcgen05 N side). Swap cuts k up over all SMs and pays for a meeting, counted as 75 clocks
+    # a token and, on every SM, its share of all tiles' k blocks at 3 (128 + tokens) clocks each (16 KB of weights, 128 bytes a token);
+    # tiles of 128 x w walk all of k, rounds of 256 + 2 w clocks a k block, and take some tenth less than that. Behind a norm, us, swap and
+    # tiles: down (4,096 x 12,288) of 160, 212, 256 rows 26.8 and 34.9, 33.2 and 35.7, 35.1 and 35.4, 5,120 x 17,408 of 256 54.1 and
+    # 61.8, 512 x 16,384 21.3 and 41.2, 2,048 x 8,192 of 200 19.0 and 22.9, 5,120 x 5,120 of 144 18.1 and 21.0; QKV (6,144 x 4,096) of 152
+    # 21.4 and 18.5, O (4,096 x 4,096) 15.6 and 14.2, 2,048 x 2,048 of 144 10.0 and 8.3, 4,096 x 512 10.1 and 5.2, 768 x 3,072 of 256 13.7
+    # and 10.6.
+    if tiles_fit and not wide and 128 < rows <= SWAP_MAX_ROWS:
+        tokens, k_blocks = -(-rows // 16) * 16, -(-in_features // 64)
+        swap = 75 * tokens + 3.0 * (128 + tokens) * k_blocks * -(-out_features // 128) / sms
+        if 1.2 * swap <= k_blocks * min(-(-2 * -(-out_features // w) // sms) * (256 + 2 * w) for w in (256, 192, 128, 64, 32)):
+            return "swap"
     if rows <= min(SMALL_M_ROWS, 64) and rows_fit and not wide:
         return "rows"
     if not tiles_fit:
         return ""
+    # (257 to 512 rows against matrices much longer than high went to 256 x 256 tiles cut up over all pairs, `gemm_pair`'s stream_mode, while
+    # one lane's issue held the tiles kernel back: down of 300 rows 49.3 us there and 60.5 on tiles, now 48.7 and 43.4; of 512 50.6 and 44.9;
+    # 5,120 x 17,408 of 300 70 and 62, of 512 77 and 80.)
     # Many rows: two SMs to a 256 x 256 tile take in a third less per multiply-add than one SM with a 128 x 256 tile,
     # which is what bounds these products. It pays where its tiles keep three quarters of the pairs busy or more and its
     # rounds of tiles, each about a tenth shorter than a round of one-SM tiles of the same width, take less than the
@@ -1012,73 +1014,11 @@ def gemm_kernel_for(rows: int, out_features: int, in_features: int = 4096, rows_
     return "tiles"
 
 
-def _round_clocks(tiles: int, places: int, per_round: int, multiply: int) -> float:
-    """Clocks a k block of 64 of all tiles: rounds of them, and twice their multiply-adds, which share one power limit."""
-    return -(-tiles // places) * per_round + 2.0 * tiles * multiply / places
-
-
-def pair_swap_tile(rows: int, out_features: int, pairs: int) -> tuple:
-    """(clocks a k block, tokens) of the tile that `gemm_pair_swap` is fastest with by the count of `pair_swap_tokens`."""
-    best = tokens = 0
-    high = -(-out_features // 256)
-    for cut in range(-(-rows // 256), -(-rows // 256) + 9):
-        t = -(-rows // (16 * cut)) * 16
-        c = _round_clocks(-(-rows // t) * high, pairs, 256 + t, 2 * t)
-        if t >= 48 and (not tokens or c < best):
-            best, tokens = c, t
-    return best, tokens
-
-
-def pair_swap_tokens(rows: int, out_features: int, in_features: int, kernel: str, sms: int = 148, pairs: int = 74) -> int:
-    """The tokens of a tile with which `gemm_pair_swap` takes a product of `rows` rows that would else go to `kernel`
-    (`gemm_kernel_for`), or 0 where it is not the faster one.
-
-    What a product takes is counted in clocks a k block of 64: a round of tiles takes T + 256 (shared memory: 128 weight rows
-    and half of the T tokens of every block are written and read once at 128 bytes a clock), one-SM tiles of 128 x w 2 w + 256,
-    pairs of 256 x 256 512; and because the SMs share one power limit, twice the multiply-adds of all tiles, spread over all
-    pairs, come on top. 8B layer shapes, us, before and with it: QKV of 300 rows 18.5 and 16.5, of 613 28.9 and 24.7, of 1,024
-    42.5 and 38.1; O of 512 17.7 and 15.9; gate_up of 144 47.7 and 38.6, of 400 73.0 and 63.3, of 613 101 and 88; down of 300
-    47.3 and 35.5, of 613 59.6 and 50.7. From there on 256 x 256 tiles with the tokens as the M side are as good (gate_up of 1,536 rows
-    195 and 213): it takes a twelfth less by this count to change. Below 129 rows there are too few tiles; of few k blocks a pair's start and
-    end are most of it (3,072 x 768, 613 rows 6.6 and 7.4). 257 to 512 rows against matrices much longer than high are the swapped pairs'
-    without a count: behind a norm, us, one-SM tiles and they, 512 x 16,384 of 300 and 500 rows 41.3 and 39.7, 41.3 and 39.6, 1,024 x
-    8,192 22.4 and 21.7, 22.6 and 22.0, 2,048 x 8,192 23.7 and 22.9, 24.2 and 23.3, 256 x 4,096 12.6 and 12.2, 12.6 both (256 x 256 tiles
-    cut up over all pairs, `gemm_pair`'s stream_mode, take 70, 45, 32 and 113 there).
-
-    `gemm_stream` ("swap") cuts k up over all SMs where a pair walks all of it, so there the whole product is counted: a pair's
-    rounds of (T + 256) clocks a k block against a meeting of 75 clocks a token and, on every SM, its share of all tiles' k blocks at
-    3 (128 + tokens) clocks each (16 KB of weights and 128 bytes a token); where the two are within 3 % the pairs have it. Behind a norm, us, swap and pairs: 512 x 16,384 of
-    240 rows 21.0 and 39.7, 1,024 x 8,192 16.9 and 21.8, 2,048 x 12,288 of 212 22.3 and 31.7, 1,536 x 8,960 of 256 18.3 and 23.7; about
-    even at 4,096 x 8,192 of 212 (24.2 both), 2,048 x 8,192 of 256 (22.2 and 22.7), 4,096 x 12,288 of 212 (33.2 and 33.8); 4,096 x 12,288 of 256
-    37.8 and 34.0, 2,048 x 5,120 of 256 19.3 and 15.5, 768 x 3,072 13.7 and 10.4, 4,096 x 4,096 of 144 15.3 and 14.2, 6,144 x 4,096
-    20.1 and 15.5, 4,096 x 512 10.1 and 5.2 (few k blocks do not count against the pairs here: swap is the worse for them)."""
-    if pairs <= 0 or rows <= TILE_ROWS or kernel not in ("swap", "tiles", "pair"):
-        return 0
-    long = 256 < rows <= 512 and in_features >= 2 * out_features
-    if kernel != "swap" and in_features < 1024 and not long:
-        return 0
-    best, tokens = pair_swap_tile(rows, out_features, pairs)
-    high = -(-out_features // 256)
-    if long:
-        return tokens
-    if kernel == "swap":
-        k_blocks, n = -(-in_features // 64), -(-rows // 16) * 16
-        stream = 75 * n + 3.0 * (128 + n) * k_blocks * -(-out_features // 128) / sms
-        return tokens if 0.97 * -(-(-(-rows // tokens) * high) // pairs) * (256 + tokens) * k_blocks <= stream else 0
-    if kernel == "pair":
-        other = _round_clocks(-(-rows // 256) * high, pairs, 512, 512)
-    else:
-        other = min(_round_clocks(-(-rows // 128) * -(-out_features // w), sms, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
-    return tokens if best < 0.92 * other else 0
-
-
 @functools.lru_cache(maxsize=16384)
-def product_choice(rows: int, out_features: int, in_features: int, fits: bool = True, sms: int = 148, pairs: int = 74) -> tuple:
-    """(kernel, tokens) of a bfloat16 product: what `gemm_kernel_for` names and 0, or "pair-swap" and the tokens of its tile. `fits`:
-    whether the tensor-core kernels take its strides and alignment. Worked out once per size: a step asks it for every product."""
-    kernel = gemm_kernel_for(rows, out_features, in_features, fits and rows <= 64, fits, sms, pairs)
-    tokens = pair_swap_tokens(rows, out_features, in_features, kernel, sms, pairs) if fits else 0
-    return ("pair-swap", tokens) if tokens else (kernel, 0)
+def product_choice(rows: int, out_features: int, in_features: int, fits: bool = True, sms: int = 148, pairs: int = 74) -> str:
+    """`gemm_kernel_for`, worked out once per size: a step asks it for every product. `fits`: whether the tensor-core kernels take the
+    product's strides and alignment."""
+    return gemm_kernel_for(rows, out_features, in_features, fits and rows <= 64, fits, sms, pairs)
 
 
 def gemm_bf16(a, w, out, bias=None, accumulate=False, swiglu=False) -> None:
@@ -1087,9 +1027,7 @@ def gemm_bf16(a, w, out, bias=None, accumulate=False, swiglu=False) -> None:
     their 8 up rows and out[m, j] = silu(gate_j) * up_j."""
     w = _packed(w)
     rows = a.shape[0]
-    kernel, tokens = product_choice(rows, w.rows, w.cols, _tcgen05_fits(a, w), sm_count(), resident_pairs() if rows > TILE_ROWS else 0)
-    if kernel == "pair-swap":
-        return gemm_pair_swap(a, w, out, tokens, bias, accumulate, swiglu=swiglu)
+    kernel = product_choice(rows, w.rows, w.cols, _tcgen05_fits(a, w), sm_count(), resident_pairs() if rows > TILE_ROWS else 0)
     if kernel == "rows":
         return gemm_small_m(a, w, out, bias, accumulate, swiglu=swiglu)
     if kernel == "swap":
@@ -1130,16 +1068,6 @@ def gemm_pair(a, w, out, bias=None, accumulate=False, swiglu=False, max_pairs: i
           _DT[bias.dtype] if bias is not None else F32, out.data_ptr(), _DT[out.dtype], out.stride(0),
           int(accumulate), a.shape[0], w.rows, w.cols, int(max_pairs), glu_kind(swiglu), glu_more(swiglu), _p(ws),
           ws.numel() if ws is not None else 0, int(stream_mode), _stream())
-
-
-def gemm_pair_swap(a, w, out, tokens: int, bias=None, accumulate=False, swiglu=False, max_pairs: int = 0) -> None:
-    """As `gemm_pair`, with the weight rows as the M side: tiles of 256 weight rows by `tokens` tokens (a multiple of 16 up to 256)."""
-    w = _packed(w)
-    assert a.dtype == torch.bfloat16 and out.stride(-1) == 1 and a.shape[1] == w.cols
-    _call("jllm_gemm_pair_swap", a.data_ptr(), a.stride(0), w.data.data_ptr(), w.k_blocks, _p(bias),
-          _DT[bias.dtype] if bias is not None else F32, out.data_ptr(), _DT[out.dtype], out.stride(0),
-          int(accumulate), a.shape[0], w.rows, w.cols, int(tokens), int(max_pairs) or resident_pairs(), glu_kind(swiglu), glu_more(swiglu),
-          _stream())
 
 
 _resident_pairs = None
@@ -1262,7 +1190,7 @@ def bounds_errors() -> dict:
 
 
 # Which kernel a code in an error word is from: the products share one word, the attention kernels another.
-WAIT_KERNELS = {"products": ((1, 3, "gemm_tcgen05"), (11, 13, "gemm_stream"), (14, 16, "gemm_stream (clusters)"), (21, 23, "gemm_pair"), (34, 36, "gemm_pair_swap")),
+WAIT_KERNELS = {"products": ((1, 3, "gemm_tcgen05"), (11, 13, "gemm_stream"), (14, 16, "gemm_stream (clusters)"), (21, 23, "gemm_pair")),
                 "attention": ((21, 23, "attention_prefill_tc"), (31, 33, "attention_prefill_pair"), (41, 43, "attention_prefill_latent"),
                               (51, 52, "attention_decode_ring"))}
 

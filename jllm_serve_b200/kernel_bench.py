@@ -24,12 +24,11 @@ def product_kernels(ops, rows: int, out_features: int, in_features: int, pairs: 
     if pairs > 0:
         kernels["pair"] = (ops.gemm_pair, {})
         kernels["pair-streamed"] = (ops.gemm_pair, {"stream_mode": 1})
-        kernels["pair-swap"] = (ops.gemm_pair_swap, {"tokens": ops.pair_swap_tile(rows, out_features, pairs)[1]})
     if rows <= ops.SWAP_MAX_ROWS:
         kernels["swap"] = (ops.gemm_stream, {})
     if rows <= 64:
         kernels["rows"] = (ops.gemm_small_m, {})
-    return ops.product_choice(rows, out_features, in_features, True, ops.sm_count(), pairs)[0], kernels
+    return ops.product_choice(rows, out_features, in_features, True, ops.sm_count(), pairs), kernels
 
 
 def main() -> int:

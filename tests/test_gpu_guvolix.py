@@ -842,6 +842,37 @@ def test_a_captured_decode_step_equals_a_launched_one():
     assert torch.equal(rows[False], rows[True])
 
 
+def test_requests_one_behind_the_other_without_a_wait():
+    """Four prompts of 609 tokens in one step at the benchmark's layer sizes, thirteen tokens each, and again, with nobody waiting for the
+    device: launches of the passes overlap as they may, every pass ends, and the last one's logits are the first one's."""
+    from bench import guvolix_shape
+    from jllm_serve_b200.engine import Engine, Segment
+    config = guvolix_shape(2048, 16, 8, 8192, 8)
+    for layer in config["layers"]:
+        layer["mlp"] = {"kind": "dense", "ff": 8192}
+    engine = Engine(config=config, seed=3, dtype="bfloat16", ctx=256, page_size=16, num_pages=64, max_batch_tokens=640, max_running=4)
+    lengths = [122, 142, 162, 183]
+    tokens = [random_tokens(n + 13, 32768, 50 + i) for i, n in enumerate(lengths)]
+    steps = [[Segment(i, t[:n], 0, [n - 1]) for i, (t, n) in enumerate(zip(tokens, lengths))]]
+    steps += [[Segment(i, [t[n + k]], n + k, [0]) for i, (t, n) in enumerate(zip(tokens, lengths))] for k in range(13)]
+    results = []
+    for turn in range(60):
+        first = engine.step(steps[0])
+        first = first.clone() if turn in (0, 59) else first
+        for segments in steps[1:]:
+            last = engine.step(segments)
+        for i in range(4):
+            engine.finish(i)
+        if turn in (0, 59):
+            results.append((first, last.clone()))
+    torch.cuda.synchronize()
+    ops().check_kernel_errors()
+    assert all(torch.isfinite(t).all() for pair in results for t in pair)
+    # (pass 0's decode steps were launched, the others' replayed: the same bits)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    engine.close()
+
+
 @pytest.mark.parametrize("seed", [9001, 9002, 9003, 9004, 9005, 9006, 9007, 9008, 9009, 9010])
 def test_a_random_configuration_mixed_and_decoded(seed):
     """Configurations drawn at random: sizes, layer orders, windows and constants in combinations that the fixed test models

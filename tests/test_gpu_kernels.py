@@ -911,34 +911,6 @@ def test_attention_prefill_over_rows_that_are_key_and_value(ops, H, Hkv, page, w
         rows_close(got, want.float().cpu().view(-1, H, hd)[:, :, :cols].reshape(q.shape[0], -1), f"latent {far}")
 
 
-@pytest.mark.parametrize("M,N,K,tokens", [(1, 8, 8, 16), (130, 40, 72, 48), (257, 517, 200, 256), (300, 256, 4096, 112), (613, 1040, 1032, 208),
-                                          (500, 2500, 136, 80)])
-def test_gemm_pair_swap(ops, M, N, K, tokens):
-    """Weight rows as the M side of a pair's tile: edges of tokens, rows and k, tiles whose second block has no weight rows, many tiles on
-    few pairs (both accumulators in turn), bias, residual add, relu squared, bfloat16 results into a wider row, gate and up rows."""
-    a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
-    packed, bias, base = ops.pack_weight(w), rnd(N, dtype=torch.float32, seed=2), rnd(M, N, seed=3)
-    tol, plain = 1e-4 * math.sqrt(K) * 0.05, gemm_want(a, w, bias)
-    for pairs in (0, 2):
-        acc, again, sq = base.clone(), base.clone(), torch.full((M, N), float("nan"), device=DEV)
-        ops.gemm_pair_swap(a, packed, acc, tokens, bias, accumulate=True, max_pairs=pairs)
-        ops.gemm_pair_swap(a, packed, again, tokens, bias, accumulate=True, max_pairs=pairs)
-        ops.gemm_pair_swap(a, packed, sq, tokens, bias, accumulate=ops.EPILOGUE_RELU2, max_pairs=pairs)
-        out16 = torch.zeros(M, N + 6, dtype=torch.bfloat16, device=DEV)
-        ops.gemm_pair_swap(a, packed, out16[:, :N], tokens, max_pairs=pairs)
-        assert ops.gemm_tcgen05_error() == 0
-        assert torch.allclose(acc.cpu(), plain + base.cpu(), rtol=1e-4, atol=tol) and torch.equal(acc, again)
-        assert torch.allclose(sq.cpu(), torch.relu(plain) ** 2, rtol=1e-3, atol=4 * tol)
-        assert torch.allclose(out16[:, :N].float().cpu(), gemm_want(a, w), rtol=2 ** -7, atol=2e-3) and float(out16[:, N:].abs().max()) == 0
-        if N % 16 == 0:
-            z = gemm_want(a, w).view(M, N // 16, 2, 8)
-            want = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(M, N // 2)
-            for dtype, t in ((torch.float32, 1e-3), (torch.bfloat16, 2 ** -7)):
-                units = torch.full((M, N // 2), float("nan"), dtype=dtype, device=DEV)
-                ops.gemm_pair_swap(a, packed, units, tokens, swiglu=True, max_pairs=pairs)
-                assert torch.allclose(units.float().cpu(), want, rtol=t, atol=1e-3)
-
-
 @pytest.mark.parametrize("M", [1, 7, 16])
 @pytest.mark.parametrize("N,K", [(16, 6144), (40, 6200), (2048, 12288), (2368, 6152)])
 def test_gemm_small_m_halves_of_k(ops, M, N, K):
@@ -980,25 +952,3 @@ def test_norms_whose_gain_begins_at_an_odd_element(ops, dim, dtype):
     assert all(torch.equal(u, v) for u, v in zip(*results))
     want = P.rmsnorm(x.cpu(), gains[0].float().cpu(), 1e-5)
     assert torch.allclose(results[0][0].cpu(), want, rtol=2e-6, atol=1e-6)
-
-
-@pytest.mark.parametrize("M,N,K,tokens", [(150, 4096, 1024, 80), (257, 528, 4096, 96), (613, 2048, 2048, 208)])
-def test_gemm_pair_swap_gives_the_bits_of_whole_tiles(ops, M, N, K, tokens):
-    """An element's sum runs over k in the same order with one accumulator, whichever operand is the M side: the results are those of
-    one-SM tiles, stored, behind bias and relu squared, added to a residual, gated."""
-    a, w = rnd(M, K, dtype=torch.bfloat16), ops.pack_weight(rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05))
-    bias, base = rnd(N, dtype=torch.float32, seed=2), rnd(M, N, seed=3)
-    for dtype in (torch.float32, torch.bfloat16):
-        for how in (False, True, ops.EPILOGUE_RELU2, "glu"):
-            got, want = (base[:, :N // 2].to(dtype).contiguous() if how == "glu" else base.to(dtype) for _ in range(2))
-            more = dict(swiglu=True) if how == "glu" else dict(bias=bias, accumulate=how)
-            ops.gemm_pair_swap(a, w, got, tokens, **more)
-            ops.gemm_tcgen05(a, w, want, **more)
-            assert torch.equal(got, want), (dtype, how)
-    wide = torch.full((M, N + 6), float("nan"), dtype=torch.bfloat16, device=DEV)       # added into a bfloat16 row that is wider
-    wide[:, :N] = base
-    ops.gemm_pair_swap(a, w, wide[:, :N], tokens, bias, accumulate=True)
-    want = a.double().cpu() @ w.unpack().double().cpu().t() + bias.double().cpu() + base.bfloat16().double().cpu()
-    # a sum of float32 and a rounding to 8 bits of the result
-    assert torch.allclose(wide[:, :N].double().cpu(), want, rtol=2 ** -8, atol=1e-4 * math.sqrt(K) * 0.05) and wide[:, N:].isnan().all()
-    assert ops.gemm_tcgen05_error() == 0

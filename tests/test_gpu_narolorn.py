@@ -382,30 +382,6 @@ def test_limits_and_weights_in_every_products_epilogue(rows, K, E, ff, shared):
     o.check_kernel_errors()
 
 
-@pytest.mark.parametrize("rows, K, E, ff, shared, tokens, dtype", [(40, 64, 3, 16, 8, 48, torch.bfloat16), (150, 512, 4, 64, 32, 80, torch.float32),
-                                                                   (300, 256, 2, 40, 16, 112, torch.bfloat16), (513, 512, 4, 96, 96, 176, torch.float32),
-                                                                   (200, 128, 3, 24, 0, 208, torch.bfloat16)])
-def test_limits_and_weights_in_the_swapped_pairs_epilogue(rows, K, E, ff, shared, tokens, dtype):
-    """The same with the weight rows as a pair's M side, where a unit's gate and up rows meet by shuffles: 16-bit results two units to a
-    store, at an address that does not allow that one by one, and 32-bit results."""
-    o = ops()
-    x, gate, up, weights, want = clamped_case(rows, K, E, ff, shared, rows + ff, torch.bfloat16)
-    hidden = E * ff + shared
-    stacked = torch.stack([gate.view(hidden // 8, 8, K), up.view(hidden // 8, 8, K)], dim=1).reshape(2 * hidden, K).contiguous().to(DEV)
-    words = [o.glu_descriptor("swish_clamped", l) for l in (0.9, 1.6)]
-    table = weights.to(DEV) if shared else weights[:, :E].contiguous().to(DEV)
-    packed, a = o.pack_weight(stacked), x.to(DEV)
-    for start in (0, 1):
-        room = torch.full((rows, hidden + 4 + 4 * start), float("nan"), dtype=dtype, device=DEV)
-        out = room[:, start:start + hidden]
-        o.gemm_pair_swap(a, packed, out, tokens, swiglu=o.GluUnits(words[0], ff, E * ff if shared else 0, words[1], table))
-        close(out, want, torch.bfloat16, "weighted")
-        o.gemm_pair_swap(a, packed, out, tokens, swiglu=o.GluUnits(words[0], ff, E * ff if shared else 0, words[1], None))
-        close(out, clamped_case_unweighted(x, gate, up, E * ff, (0.9, 1.6)), torch.bfloat16, "not weighted")
-        assert room[:, :start].isnan().all() and room[:, start + hidden:].isnan().all()
-    o.check_kernel_errors()
-
-
 def clamped_case_unweighted(x, gate, up, routed, limits):
     limit = torch.full((gate.shape[0],), limits[1], dtype=torch.float64)
     limit[:routed] = limits[0]

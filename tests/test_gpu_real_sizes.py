@@ -97,14 +97,15 @@ def test_bfloat16_follows_float32_far_into_a_long_prompt():
 
 
 def test_bfloat16_follows_float32_with_portions_of_some_hundred_rows():
-    """Steps of 129 to 512 rows (portions of 150, 220 and 440 rows beside two decoding requests). The swapped pairs have nearly all
-    products there; the down product stays with the weight-stream product up to 208 rows, whose N side 256 tokens still are."""
+    """Steps of 129 to 512 rows (portions of 150, 220 and 440 rows beside two decoding requests). Up to 256 rows the
+    tokens are still one N side of the weight-stream product, which takes the down product there; the others, and the down
+    product of more rows, are one-SM tiles, gate_up of 442 rows pairs."""
     from jllm_serve_b200.csrc import ops
     from jllm_serve_b200.precision_check import compare_precisions
+    assert ops.gemm_kernel_for(222, 4096, 12288) == "swap" and ops.gemm_kernel_for(152, 6144, 4096) == "tiles"
     if ops.resident_pairs() > 0:
-        chosen = {(rows, n): ops.product_choice(rows, n, k, True, ops.sm_count(), ops.resident_pairs())[0]
-                  for rows in (152, 222, 442) for n, k in ((6144, 4096), (4096, 12288))}
-        assert chosen.pop((152, 4096)) == "swap" and set(chosen.values()) == {"pair-swap"}
+        assert ops.gemm_kernel_for(442, 4096, 12288, pairs=ops.resident_pairs()) == "tiles"
+        assert ops.gemm_kernel_for(442, 24576, 4096, pairs=ops.resident_pairs()) == "pair"
     for portion in (150, 220, 440):
         got = compare_precisions(CONFIG, seed=9, prompt=2 * portion, tail=4, portion=portion)
         print(f"portions of {portion}, layers {CONFIG['num_hidden_layers']} of {QWEN3_8B_LAYERS}: {got}")

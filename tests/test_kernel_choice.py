@@ -1,6 +1,4 @@
 """Which kernel a step's work goes to: decisions taken on the host from sizes alone (no GPU, nothing launched)."""
-import math
-
 import torch
 
 from jllm_serve_b200.csrc import ops
@@ -13,14 +11,12 @@ def test_product_kernel_by_rows_and_shape():
     assert k(16, 24576, 4096) == "tiles"                   # 16 rows against gate_up: tcgen05 tiles
     assert k(16, 6144, 4096) == "rows"
     assert k(17, 6144, 4096) == "swap"                     # QKV (50 MB) from 17 rows: weight rows as the MMA's M side
-    assert k(64, 6144, 4096) == "swap" and k(128, 6144, 4096) == "swap" and k(160, 6144, 4096) == "swap"
-    assert k(161, 6144, 4096) == "tiles" and k(161, 4096, 4096) == "tiles"      # above 160 rows its parked parts cost too much
+    assert k(64, 6144, 4096) == "swap" and k(128, 6144, 4096) == "swap" and k(129, 6144, 4096) == "tiles"
+    assert k(161, 6144, 4096) == "tiles" and k(161, 4096, 4096) == "tiles"      # above 128 rows its parked parts cost too much
     # ... except against matrices much longer than high (down), up to the 256 tokens of one tcgen05 N side
-    assert k(64, 4096, 12288) == "swap" and k(128, 4096, 12288) == "swap" and k(256, 4096, 12288) == "swap"
+    assert k(64, 4096, 12288) == "swap" and k(128, 4096, 12288) == "swap" and k(212, 4096, 12288) == "swap" and k(257, 4096, 12288) == "tiles"
     assert k(256, 5120, 17408) == "swap" and k(200, 24576, 4096) == "tiles"
-    # 257 to 512 rows against such a matrix: the swapped pairs, whatever the other rule names
-    assert ops.product_choice(257, 4096, 12288)[0] == "pair-swap" and ops.product_choice(512, 5120, 17408)[0] == "pair-swap"
-    assert k(257, 4096, 12288) == "tiles" and k(513, 4096, 12288) == "tiles" and k(400, 6144, 4096) == "tiles" and k(400, 4096, 12288, pairs=0) == "tiles"
+    assert k(513, 4096, 12288) == "tiles" and k(400, 6144, 4096) == "tiles" and k(400, 4096, 12288, pairs=0) == "tiles"
     assert k(40, 4096, 4096) == "rows" and k(41, 4096, 4096) == "swap"         # O (34 MB): from 41 rows
     assert k(64, 24576, 4096) == "tiles"                                       # gate_up: whole tiles fill the SMs
     # many rows: two SMs to a 256 x 256 tile where such tiles keep the pairs busy in no more rounds than one-SM tiles
@@ -134,55 +130,17 @@ def test_a_wait_that_ran_out_is_reported_with_its_kernel(monkeypatch):
     ops.check_kernel_errors()
 
 
-def test_tokens_of_a_tile_with_the_weight_rows_as_m_side():
-    """Where the product of a pair with the weight rows as its M side takes another kernel's place: its tiles cover the rows and none of
-    them is empty, no other multiple of 16 makes cheaper tiles, and what it replaces costs more by the count that the rule states."""
-    def tokens(rows, n, k, **more):
-        return ops.pair_swap_tokens(rows, n, k, ops.gemm_kernel_for(rows, n, k), **more)
-    assert tokens(613, 24576, 4096) == 208 and tokens(613, 4096, 12288) == 160 and tokens(300, 4096, 12288) == 80
-    assert tokens(128, 6144, 4096) == 0 and tokens(2048, 24576, 4096) == 0 and tokens(200, 4096, 12288) == 0
-    assert tokens(613, 24576, 4096, pairs=0) == 0 and ops.pair_swap_tokens(613, 24576, 4096, "rows") == 0
-
-    def clocks(tiles, places, round_, multiply):       # a k block of all tiles: rounds, and the power that all multiply-adds share
-        return math.ceil(tiles / places) * round_ + 2 * tiles * multiply / places
-    taken = left = 0
-    for rows in list(range(129, 700, 13)) + [1000, 1536, 2048, 5000]:
-        for n, k in ((6144, 4096), (4096, 4096), (24576, 4096), (4096, 12288), (2048, 2048), (768, 2048), (64, 2048), (3072, 768)):
-            kernel, t, high = ops.gemm_kernel_for(rows, n, k), tokens(rows, n, k), math.ceil(n / 256)
-            # (sizes that cut the rows into at most eight tiles more than need be)
-            every = {u: clocks(math.ceil(rows / u) * high, 74, 256 + u, 2 * u) for u in range(48, 257, 16)
-                     if math.ceil(rows / u) <= math.ceil(rows / 256) + 8}
-            if t:
-                taken, cut = taken + 1, math.ceil(rows / t)
-                assert (cut - 1) * t < rows <= cut * t and every[t] == min(every.values())
-            else:
-                left += 1
-            if 256 < rows <= 512 and k >= 2 * n:
-                assert t > 0
-            elif kernel in ("tiles", "pair") and k < 1024:
-                assert t == 0
-            elif kernel == "tiles":
-                other = min(clocks(math.ceil(rows / 128) * math.ceil(n / w), 148, 256 + 2 * w, 2 * w) for w in (256, 192, 128, 64, 32))
-                assert (t > 0) == (min(every.values()) < 0.92 * other)
-            elif kernel == "pair":
-                assert (t > 0) == (min(every.values()) < 0.92 * clocks(math.ceil(rows / 256) * high, 74, 512, 512))
-    assert taken > 100 and left > 20
-
-
-def test_long_products_of_few_weight_rows_stay_where_k_is_cut_up():
-    """129 to 256 rows: `gemm_stream` cuts k up over all SMs, a pair of the swapped product walks all of it. Few weight rows against a
-    long k have a handful of tiles, each as long as k (240 rows of 512 x 16,384: 21 us against 40)."""
-    def tokens(rows, n, k):
-        assert ops.gemm_kernel_for(rows, n, k) == "swap"
-        return ops.pair_swap_tokens(rows, n, k, "swap")
-    for rows, n, k in ((240, 512, 16384), (256, 512, 16384), (240, 1024, 8192), (212, 2048, 12288), (256, 2048, 12288), (256, 1536, 8960),
-                       (160, 4096, 8192), (208, 4096, 12288), (130, 256, 4096)):
-        assert tokens(rows, n, k) == 0, (rows, n, k)
-    for rows, n, k in ((256, 4096, 12288), (256, 5120, 17408), (256, 2048, 5120), (256, 768, 3072), (144, 4096, 4096), (160, 6144, 4096),
-                       (144, 8192, 8192), (150, 4096, 512)):
-        assert tokens(rows, n, k) >= 48, (rows, n, k)
-    # more SMs shorten the streamed product
-    assert ops.pair_swap_tokens(256, 4096, 12288, "swap", sms=300) == 0
+def test_products_of_129_to_256_rows_are_counted_on_both_kernels():
+    """`gemm_stream` cuts k up over all SMs, the tiles walk all of it: what is long for its rows goes there, what is short or has enough
+    tiles does not (each shape was measured on both)."""
+    k = ops.gemm_kernel_for
+    for rows, n, kk in ((144, 512, 16384), (256, 512, 16384), (240, 1024, 8192), (256, 2048, 12288), (256, 1536, 8960), (200, 2048, 8192),
+                        (160, 4096, 8192), (212, 4096, 12288), (144, 256, 4096), (144, 5120, 5120), (212, 5120, 17408), (150, 2048, 5120)):
+        assert k(rows, n, kk) == "swap", (rows, n, kk)
+    for rows, n, kk in ((130, 4096, 4096), (160, 6144, 4096), (144, 7168, 5120), (144, 2048, 2048), (150, 4096, 512), (150, 512, 128),
+                        (256, 768, 3072), (256, 2048, 5120), (256, 4096, 8192), (150, 1024, 2816), (240, 256, 4096)):
+        assert k(rows, n, kk) == "tiles", (rows, n, kk)
+    assert k(200, 4096, 12288, tiles_fit=False) == "" and k(256, 2048, 5120, sms=1000) == "swap"
 
 
 def test_a_product_asks_once_which_kernel_takes_it(monkeypatch):
@@ -196,10 +154,10 @@ def test_a_product_asks_once_which_kernel_takes_it(monkeypatch):
     counted("sm_count", lambda: 148)
     counted("resident_pairs", lambda: 74)
     counted("gemm_kernel_for", ops.gemm_kernel_for)
-    for name in ("gemm_small_m", "gemm_stream", "gemm_tcgen05", "gemm_pair", "gemm_pair_swap"):
+    for name in ("gemm_small_m", "gemm_stream", "gemm_tcgen05", "gemm_pair"):
         monkeypatch.setattr(ops, name, lambda *a, name=name, **k: asked.append(name))
     ops.product_choice.cache_clear()
-    for rows, n, k, kernel in ((8, 4096, 4096, "gemm_small_m"), (64, 6144, 4096, "gemm_stream"), (613, 24576, 4096, "gemm_pair_swap"),
+    for rows, n, k, kernel in ((8, 4096, 4096, "gemm_small_m"), (64, 6144, 4096, "gemm_stream"), (613, 4096, 4096, "gemm_tcgen05"),
                                (2048, 24576, 4096, "gemm_pair"), (300, 3072, 512, "gemm_tcgen05")):
         w = ops.PackedWeight(torch.zeros(1, dtype=torch.bfloat16).expand(-(-n // 128), -(-k // 64), 1), n, k)
         a, out = torch.zeros(rows, k, dtype=torch.bfloat16), torch.zeros(1)
@@ -208,18 +166,17 @@ def test_a_product_asks_once_which_kernel_takes_it(monkeypatch):
         ops.gemm_bf16(a, w, out)
         assert asked.count(kernel) == 2 and asked.count("gemm_kernel_for") == 1, asked
         assert asked.count("_tcgen05_fits") == 2 and asked.count("sm_count") == 2 and asked.count("resident_pairs") == (2 if rows > 128 else 0), asked
-    assert ops.product_choice(64, 4096, 4096, fits=False) == ("", 0)
+    assert ops.product_choice(64, 4096, 4096, fits=False) == ""
     ops.product_choice.cache_clear()
 
 
 def test_the_kernel_bench_names_the_kernel_that_runs(monkeypatch):
-    """`kernel_bench`'s label of a product is the kernel that `gemm_bf16` calls, with the same tile, and that kernel is one of those it
-    times side by side."""
+    """`kernel_bench`'s label of a product is the kernel that `gemm_bf16` calls, and that kernel is one of those it times side by side."""
     from jllm_serve_b200.kernel_bench import product_kernels
     monkeypatch.setattr(ops, "sm_count", lambda: 148)
     monkeypatch.setattr(ops, "resident_pairs", lambda: 74)
     ran = []
-    for name in ("gemm_small_m", "gemm_stream", "gemm_tcgen05", "gemm_pair", "gemm_pair_swap"):
+    for name in ("gemm_small_m", "gemm_stream", "gemm_tcgen05", "gemm_pair"):
         monkeypatch.setattr(ops, name, lambda a, w, out, *args, name=name, **more: ran.append((name, args, more)))
     seen = set()
     for rows in (8, 47, 64, 150, 200, 300, 613, 1024, 2048):
@@ -232,7 +189,5 @@ def test_the_kernel_bench_names_the_kernel_that_runs(monkeypatch):
             by_bench = ran.pop()
             fn(None, None, None, **more)
             assert ran[-1][0] == by_bench[0], (rows, n, k, chosen)
-            if chosen == "pair-swap":
-                assert by_bench[1][0] == more["tokens"]
             seen.add(chosen)
-    assert seen >= {"rows", "swap", "tiles", "pair", "pair-swap"}
+    assert seen == {"rows", "swap", "tiles", "pair"}
