@@ -16,21 +16,21 @@
 // stretch of memory instead of 8 rows that lie a whole row apart.
 //
 // A matrix of few rows and a long k (a down projection of a narrow model) has a block for fewer SMs than there are, each with a
-// long way through k: there a cluster of two blocks takes the same rows, half of the k blocks each, and their sums meet through
-// distributed shared memory (first half + second half).
+// long way through k: there a block has 16 warps, the first eight with the first half of the k blocks, the others with the second (sum of
+// the first half + sum of the second), so that an SM has as many bytes on their way as two blocks would.
 //
 // Requirements (else the caller uses the CUDA-core kernel): bfloat16 inputs, K a multiple of 8,
 // 16-byte aligned rows (lda a multiple of 8; aligned base pointers), 1 <= M <= 64.
-#include <cooperative_groups.h>
-
 #include "common.cuh"
 
 namespace {
 
 constexpr int WARPS = 8;
 constexpr int KCHUNK = 32;
-// From so many k blocks on two blocks share the way (8 rows, a block for each 16 rows and two: 2,048 x 12,288 13.4 and 11.1 us, x 8,192 9.7 and
-// 8.4, x 4,096 6.0 and 5.9, x 2,048 3.9 and 4.3).
+// From so many k blocks on a block takes the two halves (8 rows, a block of 8 warps and of 16: 2,048 x 12,288 13.4 and 11.5 us, x 8,192 9.7
+// and 8.7). Two blocks of a cluster, which add up through distributed shared memory, were 0.4 us faster still, also spread over the SMs
+// that are left without a block here, but clusters in a captured decode step made the first pass of a new model dearer (eight such
+// products a step: 17.9 to 26.6 ms, without clusters 16.0 to 16.7) and its steady pass no shorter (11.88 ms and 11.89). The same bits.
 constexpr int HALVES_MIN_K_BLOCKS = 96;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -55,15 +55,16 @@ __device__ __forceinline__ uint4 load_16_stream(const __nv_bfloat16* p) {
 }
 
 template <int NT, int RT, int UNROLL, bool HALVES, typename Tout>
-__global__ void __launch_bounds__(WARPS * 32, 2)
+__global__ void __launch_bounds__((HALVES ? 2 : 1) * WARPS * 32, HALVES ? 1 : 2)
 gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w, int k_blocks,
                     VecRef bias, int has_bias, Tout* __restrict__ out, int ldo, int accumulate, int M, int N, int K,
                     GluArgs swiglu) {
-    extern __shared__ float red[];  // [WARPS][RT * 16][NT * 8]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int THREADS = (HALVES ? 2 : 1) * WARPS * 32;
+    extern __shared__ float red[];  // [THREADS / 32][NT * 8][RT * 16]
+    const int half = HALVES ? (int)threadIdx.x / (WARPS * 32) : 0;
+    const int warp = (threadIdx.x >> 5) % WARPS, lane = threadIdx.x & 31;          // (warp: of this half)
     const int g = lane >> 2, t = lane & 3;
-    const int half = HALVES ? (int)(blockIdx.x & 1) : 0;           // (clusters lie along x)
-    const int n0 = (HALVES ? (int)(blockIdx.x >> 1) : (int)blockIdx.x) * (16 * RT);
+    const int n0 = blockIdx.x * (16 * RT);
     float acc[RT][NT][4];
 #pragma unroll
     for (int r = 0; r < RT; ++r)
@@ -95,7 +96,7 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
         arow[j] = a + (size_t)(aok[j] ? m : 0) * lda;
     }
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    // this block's k blocks [k_lo, k_hi), 32-wide chunks below `chunks`
+    // this warp's half has k blocks [k_lo, k_hi), 32-wide chunks below `chunks`
     const int all_blocks = (K + 63) >> 6, k_lo = HALVES && half ? all_blocks >> 1 : 0, k_hi = HALVES && !half ? all_blocks >> 1 : all_blocks;
     const int chunks = HALVES ? min((K + KCHUNK - 1) / KCHUNK, 2 * k_hi) : (K + KCHUNK - 1) / KCHUNK;
     uint4 wv[UNROLL][RT][2];
@@ -151,10 +152,10 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
         }
         if (c0 + WARPS * (UNROLL / 2) < k_hi) load_weights(c0 + WARPS * (UNROLL / 2));
     }
-    // partial sums of the 8 warps -> shared memory, laid out [warp][token][row] so the final pass writes
+    // partial sums of the warps -> shared memory, laid out [warp][token][row] so the final pass writes
     // consecutive output features from consecutive threads
     constexpr int ROWS = RT * 16, TOK = NT * 8;
-    float* mine = red + (size_t)warp * ROWS * TOK;
+    float* mine = red + (size_t)(half * WARPS + warp) * ROWS * TOK;
 #pragma unroll
     for (int r = 0; r < RT; ++r)
 #pragma unroll
@@ -166,39 +167,21 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
             mine[(tok + 1) * ROWS + row + 8] = acc[r][j][3];
         }
     __syncthreads();
-    const float *first = red, *second = red;
-    auto sum = [&](int e) {
+    auto sum_of = [&](const float* part, int e) {
         float v = 0.f;
-        if constexpr (HALVES) {
-            v = first[e] + second[e];
-        } else {
 #pragma unroll
-            for (int wi = 0; wi < WARPS; ++wi) v += red[(size_t)wi * ROWS * TOK + e];
-        }
+        for (int wi = 0; wi < WARPS; ++wi) v += part[(size_t)wi * ROWS * TOK + e];
         return v;
     };
-    if constexpr (HALVES) {
-        // the block's own sum goes over warp 0's part, then both blocks read both
-        float own[(ROWS * TOK + WARPS * 32 - 1) / (WARPS * 32)];
-        int u = 0;
-#pragma unroll
-        for (int e = threadIdx.x; e < ROWS * TOK; e += WARPS * 32, ++u) {
-            own[u] = 0.f;
-#pragma unroll
-            for (int wi = 0; wi < WARPS; ++wi) own[u] += red[(size_t)wi * ROWS * TOK + e];
-        }
-        u = 0;
-#pragma unroll
-        for (int e = threadIdx.x; e < ROWS * TOK; e += WARPS * 32, ++u) red[e] = own[u];
-        const auto cluster = cooperative_groups::this_cluster();
-        cluster.sync();
-        first = cluster.map_shared_rank(red, 0);
-        second = cluster.map_shared_rank(red, 1);
-    }
-    for (int e = threadIdx.x; e < ROWS * TOK; e += WARPS * 32) {
+    auto sum = [&](int e) {
+        const float first = sum_of(red, e);
+        if constexpr (HALVES) return first + sum_of(red + (size_t)WARPS * ROWS * TOK, e);
+        return first;
+    };
+    for (int e = threadIdx.x; e < ROWS * TOK; e += THREADS) {
         const int tok = e / ROWS, row = e % ROWS;
         const int n = n0 + row;
-        if (tok >= M || n >= N || (HALVES && (tok & 1) != half)) continue;       // (of a cluster's tokens each block finishes every other one)
+        if (tok >= M || n >= N) continue;
         float v = sum(e);
         if (swiglu) {
             // rows come in blocks of 16: 8 gate rows, then the 8 up rows of the same hidden units
@@ -213,7 +196,6 @@ gemm_small_m_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfl
         if (accumulate == EPI_ADD) v += to_float(*dst);
         *dst = from_float<Tout>(v);
     }
-    if constexpr (HALVES) cooperative_groups::this_cluster().sync();        // nobody leaves while its sums are being read
 }
 
 template <int NT, int RT, int UNROLL>
@@ -235,26 +217,13 @@ int launch(const void* a, int lda, const void* w, int k_blocks, VecRef bias, int
     return jllm_check_launch("gemm_small_m");
 }
 
-// Two blocks to 16 rows, half of k each
+// 16 warps to 16 rows, half of k to eight of them
 template <int NT, typename Tout>
 int launch_halves(const void* a, int lda, const void* w, int k_blocks, VecRef bias, int has_bias, void* out, int ldo, int accumulate,
                   int M, int N, int K, GluArgs swiglu, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * ((N + 15) / 16));
-    cfg.blockDim = dim3(WARPS * 32);
-    cfg.dynamicSmemBytes = (size_t)WARPS * 16 * NT * 8 * sizeof(float);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = jllm_launch_overlaps(cfg.dynamicSmemBytes, LAUNCH_DEPENDENT_WANTS_L1) ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_small_m_kernel<NT, 1, 4, true, Tout>, (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, k_blocks, bias,
-                       has_bias, (Tout*)out, ldo, accumulate, M, N, K, swiglu);
+    const size_t smem = (size_t)2 * WARPS * 16 * NT * 8 * sizeof(float);           // (16 KB at most)
+    jllm_launch(gemm_small_m_kernel<NT, 1, 4, true, Tout>, dim3((N + 15) / 16), dim3(2 * WARPS * 32), smem, stream, LAUNCH_DEPENDENT_WANTS_L1,
+                (const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, k_blocks, bias, has_bias, (Tout*)out, ldo, accumulate, M, N, K, swiglu);
     return jllm_check_launch("gemm_small_m");
 }
 

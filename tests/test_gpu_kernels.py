@@ -914,7 +914,7 @@ def test_attention_prefill_over_rows_that_are_key_and_value(ops, H, Hkv, page, w
 @pytest.mark.parametrize("M", [1, 7, 16])
 @pytest.mark.parametrize("N,K", [(16, 6144), (40, 6200), (2048, 12288), (2368, 6152)])
 def test_gemm_small_m_halves_of_k(ops, M, N, K):
-    """Few weight rows and a long k: two blocks of a cluster take half of the k blocks each (an odd number of them, k no multiple of 64,
+    """Few weight rows and a long k: the two halves of a block's warps take half of the k blocks each (an odd number of them, k no multiple of 64,
     a last block of rows that is not full). Three runs give the same bits; float64 within 1e-4 sqrt(K) of a product's size (0.05)."""
     a, w = rnd(M, K, dtype=torch.bfloat16), rnd(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
     packed, base, bias = ops.pack_weight(w), rnd(M, N, seed=3), rnd(N, dtype=torch.bfloat16, seed=2)
