@@ -28,9 +28,9 @@ namespace {
 constexpr int WARPS = 8;
 constexpr int KCHUNK = 32;
 // From so many k blocks on a block takes the two halves (8 rows, a block of 8 warps and of 16: 2,048 x 12,288 13.4 and 11.5 us, x 8,192 9.7
-// and 8.7). Two blocks of a cluster, which add up through distributed shared memory, were 0.4 us faster still, also spread over the SMs
-// that are left without a block here, but clusters in a captured decode step made the first pass of a new model dearer (eight such
-// products a step: 17.9 to 26.6 ms, without clusters 16.0 to 16.7) and its steady pass no shorter (11.88 ms and 11.89). The same bits.
+// and 8.7). Two blocks of a cluster, which add up through distributed shared memory and reach the SMs that have no block here, take 0.4 us
+// less by themselves (11.0 and 8.3); in a model's pass with eight such products a step that does not show (11.87 and 11.88 ms, 11.88 and
+// 11.90), and here no block waits for another. The same bits.
 constexpr int HALVES_MIN_K_BLOCKS = 96;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
